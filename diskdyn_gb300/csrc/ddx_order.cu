@@ -23,8 +23,8 @@
 //    fine for the tracers: each tracer's result depends on its own data and the sources;
 //  - sorted by (code, index) (the sources: 5 bits per axis).  The sources' order is the
 //    order of the FP32 sums over them, so it must not depend on timing: equal codes keep
-//    their index order.  Up to 8,192 bodies one block does it all (box, keys, a bitonic sort
-//    of code << 13 | index in shared memory, the slots), in one launch; beyond that a stable
+//    their index order.  Up to 8,192 bodies one block finds the box and the keys
+//    code << 13 | index and a second launch counts the smaller keys of each; beyond that a stable
 //    LSD radix sort of (code, index) with 8-bit digits: per digit pass every block counts the
 //    digits of its tile, digit-major; an exclusive scan gives every (digit, block) its first
 //    output slot; the scatter ranks equal digits inside a warp with __match_any_sync and
@@ -153,24 +153,34 @@ __device__ __forceinline__ uint32_t cell_code(const float* v, const float* lo, c
     return hilbert ? hilbert_index(c[0], c[1], c[2], bits) : spread3(c[0]) << 2 | spread3(c[1]) << 1 | spread3(c[2]);
 }
 
-// The whole stable order of up to kSmallOrder bodies in one block.
+// The stable order of up to kSmallOrder bodies in two launches: one block finds the box and
+// the keys code << 13 | index, all distinct, and a body's position is the number of smaller
+// keys, counted by brute force over the whole GPU (4,096 bodies: 36 us for a bitonic sort in
+// one block, 10 us so).
 constexpr int kSmallOrder = 8192;        // index < 2^13 below the 15-bit code + removed bit
 constexpr int kSmallThreads = 1024;
 __global__ void __launch_bounds__(kSmallThreads)
-order_small_kernel(ddx_state s, int first, int n, bool dead_last, bool hilbert, int* __restrict__ perm,
-                   int* __restrict__ inv) {
-    __shared__ uint32_t keys[kSmallOrder];
+order_small_keys_kernel(ddx_state s, int first, int n, bool dead_last, bool hilbert, uint32_t* __restrict__ key,
+                        int* __restrict__ pos) {
     __shared__ float red[kSmallThreads / 32][6];
     __shared__ float box[6];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    constexpr int kBits = kOrderBits - 1;
+    constexpr int kBits = kOrderBits - 1, kPer = kSmallOrder / kSmallThreads;
+    float x[kPer][3];
+    bool in[kPer];
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int k = t; k < n; k += kSmallThreads) {
-        if (dead_last && removed(s, first + k)) continue;
-        const float v[3] = {d2f_toward0(s.x[first + k]), d2f_toward0(s.y[first + k]), d2f_toward0(s.z[first + k])};
 #pragma unroll
-        for (int a = 0; a < 3; ++a) { lo[a] = fminf(lo[a], v[a]); hi[a] = fmaxf(hi[a], v[a]); }
+    for (int j = 0; j < kPer; ++j) {
+        const int k = t + j * kSmallThreads;
+        in[j] = k < n && !(dead_last && removed(s, first + k));
+        if (!in[j]) continue;
+        x[j][0] = d2f_toward0(s.x[first + k]); x[j][1] = d2f_toward0(s.y[first + k]); x[j][2] = d2f_toward0(s.z[first + k]);
     }
+#pragma unroll
+    for (int j = 0; j < kPer; ++j)
+        if (in[j])
+#pragma unroll
+            for (int a = 0; a < 3; ++a) { lo[a] = fminf(lo[a], x[j][a]); hi[a] = fmaxf(hi[a], x[j][a]); }
 #pragma unroll
     for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -187,37 +197,37 @@ order_small_kernel(ddx_state s, int first, int n, bool dead_last, bool hilbert, 
         box[t] = v;
     }
     __syncthreads();
-    int m = 1;
-    while (m < n) m <<= 1;
-    for (int k = t; k < m; k += kSmallThreads) {
-        uint32_t key = 0xFFFFFFFFu;   // padding sorts last
-        if (k < n) {
-            uint32_t code = 1u << (3 * kBits);
-            if (!(dead_last && removed(s, first + k))) {
-                const float v[3] = {d2f_toward0(s.x[first + k]), d2f_toward0(s.y[first + k]),
-                                    d2f_toward0(s.z[first + k])};
-                code = cell_code(v, box, box + 3, kBits, hilbert);
-            }
-            key = code << 13 | (uint32_t)k;
-        }
-        keys[k] = key;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        const int k = t + j * kSmallThreads;
+        if (k >= n) break;
+        const uint32_t code = in[j] ? cell_code(x[j], box, box + 3, kBits, hilbert) : 1u << (3 * kBits);
+        key[k] = code << 13 | (uint32_t)k;
+        pos[k] = 0;
     }
+}
+
+// pos[k] += the keys of this block's part of the list that are smaller than key k.
+constexpr int kRankKeys = 1024;
+__global__ void __launch_bounds__(kThreads)
+order_small_rank_kernel(int n, const uint32_t* __restrict__ key, int* __restrict__ pos) {
+    __shared__ __align__(16) uint32_t other[kRankKeys];
+    const int k = blockIdx.x * kThreads + threadIdx.x, j0 = blockIdx.y * kRankKeys;
+    for (int j = threadIdx.x; j < kRankKeys; j += kThreads) other[j] = j0 + j < n ? key[j0 + j] : 0xFFFFFFFFu;
+    const uint32_t mine = k < n ? key[k] : 0u;
     __syncthreads();
-    // bitonic sort, ascending, of the m keys (all distinct)
-    for (int size = 2; size <= m; size <<= 1)
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int i = t; i < m / 2; i += kSmallThreads) {
-                const int a = 2 * i - (i & (stride - 1)), b = a + stride;
-                const uint32_t ka = keys[a], kb = keys[b];
-                if ((ka > kb) == ((a & size) == 0)) { keys[a] = kb; keys[b] = ka; }
-            }
-            __syncthreads();
-        }
-    for (int p = t; p < n; p += kSmallThreads) {
-        const int k = (int)(keys[p] & 0x1FFFu);
-        if (perm) perm[p] = k;
-        if (inv) inv[k] = p;
+    int less = 0;
+#pragma unroll 8
+    for (int j = 0; j < kRankKeys / 4; ++j) {
+        const uint4 q = reinterpret_cast<const uint4*>(other)[j];
+        less += (q.x < mine) + (q.y < mine) + (q.z < mine) + (q.w < mine);
     }
+    if (k < n) atomicAdd(&pos[k], less);
+}
+
+__global__ void order_from_pos_kernel(int n, const int* __restrict__ pos, int* __restrict__ perm) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) perm[pos[k]] = k;
 }
 
 // Code of each body's cell (bits per axis; removed bodies get 1 << 3 bits when
@@ -377,7 +387,11 @@ cudaError_t order_bodies(const ddx_state& s, int first, int n, bool dead_last, c
     if (n <= 0) return cudaSuccess;
     if (n > o.cap) return cudaErrorInvalidValue;
     if (o.stable && n <= kSmallOrder) {
-        order_small_kernel<<<1, kSmallThreads, 0, st>>>(s, first, n, dead_last, hilbert, perm, inv);
+        int* const pos = inv ? inv : reinterpret_cast<int*>(o.rank);
+        order_small_keys_kernel<<<1, kSmallThreads, 0, st>>>(s, first, n, dead_last, hilbert, o.key, pos);
+        order_small_rank_kernel<<<dim3((n + kThreads - 1) / kThreads, (n + kRankKeys - 1) / kRankKeys), kThreads, 0, st>>>(
+            n, o.key, pos);
+        if (perm) order_from_pos_kernel<<<(n + kThreads - 1) / kThreads, kThreads, 0, st>>>(n, pos, perm);
         return cudaGetLastError();
     }
     const int blk = (n + kThreads - 1) / kThreads;

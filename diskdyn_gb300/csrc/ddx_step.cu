@@ -261,8 +261,8 @@ __global__ void massive_pass2_kernel(ddx_state s, StepArgs a, MassiveScratch ms)
 // ---------------------------------------------------------------------------------------
 // A few thousand targets leave most of the GPU idle when one warp serves one target, so
 // the FP32 pulls of the planetesimals are split over source slices: block (target group of
-// kSliceThreads, slice k) stages the slice's pair records of the pass's two stages in
-// shared memory, every thread (one target) reads each record at once (broadcast) and
+// kSliceThreads, slice k, one of the pass's two stages) stages the slice's pair records in
+// shared memory, every thread (two targets) reads each record at once (broadcast) and
 // works on both sources of a record with one f32x2 instruction, in plain sums over spans
 // of kPairSpan records with a Kahan sum across spans (the dust kernel's scheme).  A
 // target's own slot gives RR = 0 and is masked.  The star (target 0) takes the
@@ -348,11 +348,17 @@ __device__ __forceinline__ void near_span_massive(const BodyPair* R, int q0, f2 
     }
 }
 
+// Threads of a slice block.  A thread takes two targets at one stage, which share every
+// record read: broadcasting a record's 56 bytes to 32 lanes costs the shared-memory pipe 14
+// cycles, a target's FP32 operations on it 9 (4,099 bodies: 38 us a pass with one target at
+// both stages per thread, 26 us with two at one).
+constexpr int kSliceWorkers = kSliceThreads / 2;
+
 // Deterministic block sum of v (fixed tree order); the result in thread 0.
 __device__ __forceinline__ double block_sum(double v, double* red) {
     red[threadIdx.x] = v;
     __syncthreads();
-    for (int o = kSliceThreads / 2; o > 0; o >>= 1) {
+    for (int o = kSliceWorkers / 2; o > 0; o >>= 1) {
         if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
         __syncthreads();
     }
@@ -361,91 +367,95 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
     return r;
 }
 
-__global__ void __launch_bounds__(kSliceThreads)
+// One target of a slice block.
+struct SliceTarget {
+    f2 XH, XL, YH, YL, ZH, ZL;
+    f2 S[3], C[3];             // Kahan sums of the spans
+    double N[3];               // FP64 pulls of near sources, added to the slice's total
+    float inv_near;
+};
+
+__global__ void __launch_bounds__(kSliceWorkers)
 massive_slice_kernel(StepArgs a, MassiveScratch ms, int sa, int per, int np, double* __restrict__ part) {
-    __shared__ __align__(16) BodyPair tile[2][kSliceTile];
-    const int k = blockIdx.y;
-    const int sb = sa + 1;
+    __shared__ __align__(16) BodyPair tile[kSliceTile];
+    const int k = blockIdx.y, st = sa + blockIdx.z;
     const int n_src = a.n_grav - a.n_exact;
     const int npairs = pair_count(n_src);
     const int r0 = k * per, r1 = min(r0 + per, npairs);
     const int c = ms.cap;
+    double* const o = part + ((size_t)k * 6 + 3 * blockIdx.z) * np;
     if (blockIdx.x == gridDim.x - 1) {
         // the star's row: the whole block takes the slice's planetesimals in FP64
-        const Body pa = ms.P[sa * c], pb = ms.P[sb * c];
-        double d[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        const Body ps = ms.P[st * c];
+        double d[3] = {0.0, 0.0, 0.0};
         const int q1 = min(2 * r1, n_src);
-        for (int q = 2 * r0 + threadIdx.x; q < q1; q += kSliceThreads) {
-            pair64(pa, ms.P[sa * c + a.n_exact + q], d[0], d[1], d[2]);
-            pair64(pb, ms.P[sb * c + a.n_exact + q], d[3], d[4], d[5]);
-        }
-        double* red = reinterpret_cast<double*>(&tile[0][0]);     // 2 KiB of the tile space
-        double* o = part + (size_t)k * 6 * np;
-        for (int q = 0; q < 6; ++q) {
+        for (int q = 2 * r0 + threadIdx.x; q < q1; q += kSliceWorkers)
+            pair64(ps, ms.P[st * c + a.n_exact + q], d[0], d[1], d[2]);
+        double* red = reinterpret_cast<double*>(&tile[0]);        // 1 KiB of the tile space
+        for (int q = 0; q < 3; ++q) {
             const double t = block_sum(d[q], red);
             if (threadIdx.x == 0) o[(size_t)q * np] = t;
         }
         return;
     }
-    const int i = blockIdx.x * kSliceThreads + threadIdx.x;
-    const bool active = i > 0 && i < a.n_grav;                   // the star has its own row
-    float4 ha = make_float4(0.f, 0.f, 0.f, 0.f), la = ha, hb = ha, lb = ha;
-    if (active) {
-        ha = ms.Phi[sa * c + i]; la = ms.Plo[sa * c + i];
-        hb = ms.Phi[sb * c + i]; lb = ms.Plo[sb * c + i];
+    const int i0 = blockIdx.x * kSliceThreads + threadIdx.x;      // targets i0 and i0 + kSliceWorkers
+    SliceTarget t[2];
+    bool any = false;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int i = i0 + q * kSliceWorkers;
+        const bool active = i > 0 && i < a.n_grav;                // the star has its own row
+        any = any || active;
+        float4 h = make_float4(0.f, 0.f, 0.f, 0.f), l = h;
+        if (active) { h = ms.Phi[st * c + i]; l = ms.Plo[st * c + i]; }
+        t[q].XH = f2_dup(h.x); t[q].XL = f2_dup(l.x); t[q].YH = f2_dup(h.y); t[q].YL = f2_dup(l.y);
+        t[q].ZH = f2_dup(h.z); t[q].ZL = f2_dup(l.z);
+        // a thread without a target finds nothing near
+        t[q].inv_near = active ? near_inv(a.near_eta, fmaxf(fabsf(h.x), fmaxf(fabsf(h.y), fabsf(h.z)))) : INFINITY;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) t[q].S[d] = t[q].C[d] = 0, t[q].N[d] = 0.0;
     }
-    const f2 XHa = f2_dup(ha.x), XLa = f2_dup(la.x), YHa = f2_dup(ha.y), YLa = f2_dup(la.y);
-    const f2 ZHa = f2_dup(ha.z), ZLa = f2_dup(la.z);
-    const f2 XHb = f2_dup(hb.x), XLb = f2_dup(lb.x), YHb = f2_dup(hb.y), YLb = f2_dup(lb.y);
-    const f2 ZHb = f2_dup(hb.z), ZLb = f2_dup(lb.z);
-    f2 SA[3] = {0, 0, 0}, CA[3] = {0, 0, 0}, SB[3] = {0, 0, 0}, CB[3] = {0, 0, 0};
-    // near sources: FP64 pulls, summed apart and added to the slice's total
-    const float inv_a = near_inv(a.near_eta, fmaxf(fabsf(ha.x), fmaxf(fabsf(ha.y), fabsf(ha.z))));
-    const float inv_b = near_inv(a.near_eta, fmaxf(fabsf(hb.x), fmaxf(fabsf(hb.y), fabsf(hb.z))));
-    double NA[3] = {0.0, 0.0, 0.0}, NB[3] = {0.0, 0.0, 0.0};
     for (int t0 = r0; t0 < r1; t0 += kSliceTile) {
         const int cnt = min(kSliceTile, r1 - t0);          // a multiple of kPairSpan
         __syncthreads();                                   // the previous tile is consumed
-        const uint4* ga = reinterpret_cast<const uint4*>(ms.PP + (size_t)sa * ms.pcap + t0);
-        const uint4* gb = reinterpret_cast<const uint4*>(ms.PP + (size_t)sb * ms.pcap + t0);
-        uint4* ta = reinterpret_cast<uint4*>(tile[0]);
-        uint4* tb = reinterpret_cast<uint4*>(tile[1]);
-        for (int w = threadIdx.x; w < cnt * 4; w += kSliceThreads) {
-            ta[w] = ga[w];
-            tb[w] = gb[w];
-        }
+        const uint4* g = reinterpret_cast<const uint4*>(ms.PP + (size_t)st * ms.pcap + t0);
+        for (int w = threadIdx.x; w < cnt * 4; w += kSliceWorkers) reinterpret_cast<uint4*>(tile)[w] = g[w];
         __syncthreads();
-        if (!active) continue;
+        if (!any) continue;
         for (int u0 = 0; u0 < cnt; u0 += kPairSpan) {
-            f2 ax = 0, ay = 0, az = 0, bx = 0, by = 0, bz = 0;
-            float mxa = 0.f, mxb = 0.f;
+            f2 x[2] = {0, 0}, y[2] = {0, 0}, z[2] = {0, 0};
+            float mx[2] = {0.f, 0.f};
 #pragma unroll 4
-            for (int u = 0; u < kPairSpan; ++u) {
-                pair_f2_max(tile[0][u0 + u], XHa, XLa, YHa, YLa, ZHa, ZLa, ax, ay, az, mxa);
-                pair_f2_max(tile[1][u0 + u], XHb, XLb, YHb, YLb, ZHb, ZLb, bx, by, bz, mxb);
+            for (int u = 0; u < kPairSpan; ++u)
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+                    pair_f2_max(tile[u0 + u], t[q].XH, t[q].XL, t[q].YH, t[q].YL, t[q].ZH, t[q].ZL, x[q], y[q], z[q],
+                                mx[q]);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                if (mx[q] > t[q].inv_near)   // rare: a source of this span within the near radius
+                    near_span_massive(&tile[u0], 2 * (t0 + u0), t[q].XH, t[q].XL, t[q].YH, t[q].YL, t[q].ZH, t[q].ZL,
+                                      t[q].inv_near, ms.P[st * c + i0 + q * kSliceWorkers],
+                                      ms.P + (size_t)st * c + a.n_exact, ms.slot ? ms.src : nullptr, x[q], y[q], z[q],
+                                      t[q].N);
+                kahan2(t[q].S[0], t[q].C[0], x[q]); kahan2(t[q].S[1], t[q].C[1], y[q]); kahan2(t[q].S[2], t[q].C[2], z[q]);
             }
-            if (mxa > inv_a)   // rare: a source of this span within the near radius at stage sa
-                near_span_massive(&tile[0][u0], 2 * (t0 + u0), XHa, XLa, YHa, YLa, ZHa, ZLa, inv_a, ms.P[sa * c + i],
-                                  ms.P + (size_t)sa * c + a.n_exact, ms.slot ? ms.src : nullptr, ax, ay, az, NA);
-            if (mxb > inv_b)
-                near_span_massive(&tile[1][u0], 2 * (t0 + u0), XHb, XLb, YHb, YLb, ZHb, ZLb, inv_b, ms.P[sb * c + i],
-                                  ms.P + (size_t)sb * c + a.n_exact, ms.slot ? ms.src : nullptr, bx, by, bz, NB);
-            kahan2(SA[0], CA[0], ax); kahan2(SA[1], CA[1], ay); kahan2(SA[2], CA[2], az);
-            kahan2(SB[0], CB[0], bx); kahan2(SB[1], CB[1], by); kahan2(SB[2], CB[2], bz);
         }
     }
-    if (!active) return;
-    double* o = part + (size_t)k * 6 * np + i;
-    o[0] = f2_total(SA[0], CA[0]) + NA[0]; o[np] = f2_total(SA[1], CA[1]) + NA[1];
-    o[2 * np] = f2_total(SA[2], CA[2]) + NA[2];
-    o[3 * np] = f2_total(SB[0], CB[0]) + NB[0]; o[4 * np] = f2_total(SB[1], CB[1]) + NB[1];
-    o[5 * np] = f2_total(SB[2], CB[2]) + NB[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int i = i0 + q * kSliceWorkers;
+        if (!(i > 0 && i < a.n_grav)) continue;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) o[(size_t)d * np + i] = f2_total(t[q].S[d], t[q].C[d]) + t[q].N[d];
+    }
 }
 
-// 32 targets per block of 8 warps.  Each warp adds the slices of 4 targets (the lanes take
-// slices lane, lane + 32, ..., a fixed butterfly adds the lanes: the same order on every
-// run); then warp 0 finishes the 32 targets, one per lane, so the FP64 update runs on full
-// warps.
+// 32 targets per block of 8 warps, a target per lane (coalesced reads of the slice sums).  Warp
+// w adds slices w, w + 8, ... , the warps' sums are added in warp order (the same on every
+// run), two warps add the FP64 pulls of bodies 0..n_exact-1 at the pass's two stages, and
+// warp 0 applies the pass's update (4,099 bodies: 25 us with a warp per target's slices and
+// every FP64 pull in warp 0, 9 us so).
 constexpr int kGatherTargets = 32;
 constexpr int kGatherThreads = 256;
 
@@ -453,38 +463,41 @@ template <int PASS>
 __global__ void __launch_bounds__(kGatherThreads)
 massive_gather_kernel(ddx_state s, StepArgs a, MassiveScratch ms, int slices, int np,
                       const double* __restrict__ part) {
-    __shared__ double sums[kGatherTargets][6];
+    constexpr int kWarps = kGatherThreads / 32;
+    __shared__ double sums[kWarps][6][kGatherTargets];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i0 = blockIdx.x * kGatherTargets;
-    constexpr int per_warp = kGatherTargets / (kGatherThreads / 32);
-    for (int t = warp * per_warp; t < (warp + 1) * per_warp; ++t) {
-        const int it = i0 + t;
-        double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-        if (it < a.n_grav)
-            for (int k = lane; k < slices; k += 32)
+    const int i = blockIdx.x * kGatherTargets + lane;
+    double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (i < a.n_grav)
+        for (int k = warp; k < slices; k += kWarps)
 #pragma unroll
-                for (int q = 0; q < 6; ++q) acc[q] += part[((size_t)k * 6 + q) * np + it];
+            for (int q = 0; q < 6; ++q) acc[q] += part[((size_t)k * 6 + q) * np + i];
 #pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            const double v = warp_sum(acc[q]);
-            if (lane == 0) sums[t][q] = v;
-        }
+    for (int q = 0; q < 6; ++q) sums[warp][q][lane] = acc[q];
+    __syncthreads();
+    if (warp < 6) {
+        double v = sums[0][warp][lane];
+        for (int k = 1; k < kWarps; ++k) v += sums[k][warp][lane];
+        sums[0][warp][lane] = v;
     }
     __syncthreads();
-    if (warp != 0) return;
-    const int i = i0 + lane;
-    if (i >= a.n_grav) return;
+    if (warp >= 2) return;
     const int c = ms.cap;
-    const int sa = PASS == 1 ? 0 : 2, sb = sa + 1;
-    double acc[6];
+    const int st = (PASS == 1 ? 0 : 2) + warp;
+    if (i < a.n_grav) {
+        double d[3];
 #pragma unroll
-    for (int q = 0; q < 6; ++q) acc[q] = sums[lane][q];
-    const Body pa = ms.P[sa * c + i], pb = ms.P[sb * c + i];
-    for (int j = 0; j < a.n_exact && j < a.n_grav; ++j) {
-        if (j == i) continue;
-        pair64(pa, ms.P[sa * c + j], acc[0], acc[1], acc[2]);
-        pair64(pb, ms.P[sb * c + j], acc[3], acc[4], acc[5]);
+        for (int q = 0; q < 3; ++q) d[q] = sums[0][3 * warp + q][lane];
+        const Body p = ms.P[st * c + i];
+        for (int j = 0; j < a.n_exact && j < a.n_grav; ++j)
+            if (j != i) pair64(p, ms.P[st * c + j], d[0], d[1], d[2]);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) sums[0][3 * warp + q][lane] = d[q];
     }
+    asm volatile("bar.sync 1, 64;" ::: "memory");          // the two warps
+    if (warp != 0 || i >= a.n_grav) return;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) acc[q] = sums[0][q][lane];
     if (PASS == 1) pass1_update(s, a, ms, i, acc, DDX_PREC_MIXED);
     else pass2_update(s, a, ms, i, acc);
 }
@@ -681,8 +694,8 @@ cudaError_t launch_sliced(const ddx_state& s, const StepArgs& a, MassiveScratch&
     const int np = slice_stride(a.n_grav);
     if (S > 0) {
         const int per = (spans + S - 1) / S * kPairSpan;
-        const dim3 grid((a.n_grav + kSliceThreads - 1) / kSliceThreads + 1, S);   // + the star's row
-        massive_slice_kernel<<<grid, kSliceThreads, 0, st>>>(a, slotted(ms, a), PASS == 1 ? 0 : 2, per, np, ms.part);
+        const dim3 grid((a.n_grav + kSliceThreads - 1) / kSliceThreads + 1, S, 2);   // + the star's row; two stages
+        massive_slice_kernel<<<grid, kSliceWorkers, 0, st>>>(a, slotted(ms, a), PASS == 1 ? 0 : 2, per, np, ms.part);
     }
     massive_gather_kernel<PASS><<<(a.n_grav + kGatherTargets - 1) / kGatherTargets, kGatherThreads, 0, st>>>(
         s, a, slotted(ms, a), S, np, ms.part);
