@@ -72,6 +72,7 @@ void free_massive(MassiveScratch& ms) {
     cudaFree(ms.part); cudaFree(ms.slot); cudaFree(ms.src);
     order_free(ms.src_order);
     order_free(ms.dust_order);
+    cells_free(ms.cells);
     ms = MassiveScratch{};   // the status word belongs to the context, not to the scratch
 }
 
@@ -90,6 +91,9 @@ int ensure_massive(ddx_ctx* c, int n_grav, int n_dust, int precision) {
             return DDX_ERR_NOMEM;
         }
     }
+    // without room for the cells' scratch the mixed step takes every planetesimal one by one
+    if (precision == DDX_PREC_MIXED && n_grav > kCellMinSources && cells_ensure(c->ms.cells, n_grav) != cudaSuccess)
+        cudaGetLastError();
     return DDX_OK;
 }
 
@@ -142,6 +146,7 @@ int make_step_args(const ddx_ctx* c, const ddx_phys* p, int n_grav, int n_dust, 
     a.Bstar = p->Bstar;
     a.Rstar = p->Rstar;
     a.vswAU = p->vsw_AUyr;
+    a.inv_vsw = 1.0 / p->vsw_AUyr;
     a.Rmin = p->Rmin;
     a.mode = mode;
     a.lose_tile = -1;

@@ -63,6 +63,8 @@
 // only on its own state and the massive set.
 #include "ddx_internal.cuh"
 #include "ddx_f32x2.cuh"
+#include "ddx_cells.cuh"
+#include "ddx_pull.cuh"
 
 namespace ddx {
 namespace {
@@ -311,50 +313,6 @@ __device__ __forceinline__ float rest3(double v, float hi, float lo) {
     return __double2float_rn((v - (double)hi) - (double)lo);
 }
 
-// One span of kPairSpan pair records (slots q0 .. q0 + 2 kPairSpan - 1) summed again for a
-// tracer with a near source among them: the FP32 partial sum of the sources at or beyond the
-// near radius (the same operations as the main loop, so each of their pulls is the same),
-// and the FP64 pull of each near source from its FP64 stage position (P: the stage's
-// records of bodies n_exact.., src: source of each slot, null when slot q holds source q),
-// added to k.  A zero FP64 separation gives an infinite pull, which removes the tracer as in
-// the FP64 step.
-__device__ __forceinline__ void near_span(const BodyPair* R, int q0, f2 XH, f2 XL, f2 YH, f2 YL, f2 ZH, f2 ZL,
-                                          float xr, float yr, float zr, float inv_near, const Body* __restrict__ P,
-                                          const int* __restrict__ src, f2& px, f2& py, f2& pz, double& kx,
-                                          double& ky, double& kz) {
-    const double xt = join3(XH, XL, xr), yt = join3(YH, YL, yr), zt = join3(ZH, ZL, zr);
-    px = 0; py = 0; pz = 0;
-    for (int u = 0; u < kPairSpan; ++u) {
-        const BodyPair* r = R + u;
-        const ulonglong2 q0v = *reinterpret_cast<const ulonglong2*>(r->hx);
-        const ulonglong2 q1v = *reinterpret_cast<const ulonglong2*>(r->hz);
-        const ulonglong2 q2v = *reinterpret_cast<const ulonglong2*>(r->lx);
-        const f2 lz = *reinterpret_cast<const f2*>(r->lz);
-        const f2 dX = add2(sub2(q0v.x, XH), sub2(q2v.x, XL));
-        const f2 dY = add2(sub2(q0v.y, YH), sub2(q2v.y, YL));
-        const f2 dZ = add2(sub2(q1v.x, ZH), sub2(lz, ZL));
-        const f2 RR = fma2(dX, dX, fma2(dY, dY, mul2(dZ, dZ)));
-        float r0, r1;
-        f2_split(RR, r0, r1);
-        const float i0 = rsqrt_approx(r0), i1 = rsqrt_approx(r1);
-        const bool n0 = i0 > inv_near, n1 = i1 > inv_near;
-        const f2 ri = f2_join(n0 ? 0.f : i0, n1 ? 0.f : i1);
-        const f2 f = mul2(mul2(q1v.y, ri), mul2(ri, ri));
-        px = fma2(f, dX, px); py = fma2(f, dY, py); pz = fma2(f, dZ, pz);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (!(h ? n1 : n0)) continue;
-            const int q = q0 + 2 * u + h;
-            const Body p = P[src ? src[q] : q];
-            const double ex = p.x - xt, ey = p.y - yt, ez = p.z - zt;
-            const double rr = ex * ex + ey * ey + ez * ez;
-            const double ri64 = rsqrt(rr);
-            const double f64 = p.m * (ri64 * ri64 * ri64);
-            kx = fma(f64, ex, kx); ky = fma(f64, ey, ky); kz = fma(f64, ez, kz);
-        }
-    }
-}
-
 // One float-float span summed again for a tracer with a near source among its pair records:
 // the float-float sums of the other sources into (SH, SL), and the FP64 pull of each near
 // source (reciprocal FP32 distance above inv_near) from its FP64 stage record, added to k
@@ -381,30 +339,6 @@ __device__ __forceinline__ void near_span_ff(const BodyPair* R, const f2* ML, in
         }
     }
 }
-
-// Kahan sums across the FP32 spans.  The compensated variant keeps both lanes (its
-// float-float spans go to the FP64 acceleration instead, ff_total).  The FP32 forms add
-// the span's two lanes (one rounding, against the 16 of each lane's plain sum) and carry one
-// FP32 sum per axis: six registers fewer in the loop, which the dusty-ring dust kernel took
-// from 8.18 to 8.00 ms.
-template <bool F2> struct SpanAcc;
-template <> struct SpanAcc<true> {
-    f2 S = 0, C = 0;
-    __device__ __forceinline__ void add(f2 v) { kahan2(S, C, v); }
-    __device__ __forceinline__ double total() const { return f2_total(S, C); }
-};
-template <> struct SpanAcc<false> {
-    float S = 0.f, C = 0.f;
-    __device__ __forceinline__ void add(f2 v) {
-        float a, b;
-        f2_split(v, a, b);
-        const float y = __fsub_rn(__fadd_rn(a, b), C);
-        const float t = __fadd_rn(S, y);
-        C = __fsub_rn(__fsub_rn(t, S), y);
-        S = t;
-    }
-    __device__ __forceinline__ double total() const { return (double)S - (double)C; }
-};
 
 // A float-float span sum (both lanes' high parts H and low parts L) in FP64: the lanes' high
 // parts added exactly (TwoSum), the error and the low parts in FP32, then two FP64 adds.  The
@@ -714,9 +648,12 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
                         const f2 f = mul2(mul2(q1.y, ri), mul2(ri, ri));
                         px = fma2(f, dX, px); py = fma2(f, dY, py); pz = fma2(f, dZ, pz);
                     }
-                    if (mx > inv_near)   // rare: a source of this span lies within the near radius
-                        near_span(T + k, 2 * (tt * kTilePairs + k), XH, XL, YH, YL, ZH, ZL, xr, yr, zr, inv_near,
-                                  Pn, src, px, py, pz, kx, ky, kz);
+                    if (mx > inv_near) {   // rare: a source of this span lies within the near radius
+                        px = py = pz = 0;
+                        near_span<kPairSpan>(T + k, 2 * (tt * kTilePairs + k), XH, XL, YH, YL, ZH, ZL, join3(XH, XL, xr),
+                                             join3(YH, YL, yr), join3(ZH, ZL, zr), inv_near, Pn, src, px, py, pz, kx, ky,
+                                             kz);
+                    }
                 }
                 ax.add(px); ay.add(py); az.add(pz);
             }
@@ -765,6 +702,9 @@ cudaError_t launch_dust_mixed(const ddx_state& s, const StepArgs& a, const Massi
                               const SizeBin* bins, int precision, cudaStream_t st) {
     if (a.n_dust <= 0) return cudaSuccess;
     const bool comp = precision == DDX_PREC_COMPENSATED;
+    // cell expansions from kCellMinSources planetesimals on (the lost-copy test hook needs tiles)
+    if (!comp && ms.cells && ms.dust_order.cap >= a.n_dust && a.n_grav - a.n_exact >= kCellMinSources && a.lose_tile < 0)
+        return launch_dust_cells(s, a, ms, bins, st);
     const size_t smem = 2 * (size_t)kTilePairs * sizeof(BodyPair);
     static bool attr_set[128] = {};   // the attributes are set once per device
     int dev = 0;

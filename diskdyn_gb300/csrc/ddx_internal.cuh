@@ -33,7 +33,7 @@ struct StepArgs {
     int    n_exact;         // bodies 0..n_exact-1 (star, planets) act in FP64 in the mixed path
     double dt, dt2, dt6;    // dt, dt/2, dt/6 formed exactly as the reference forms them
     int    SWQ, FLQ;
-    double Wz, Bstar, Rstar, vswAU, Rmin;
+    double Wz, Bstar, Rstar, vswAU, inv_vsw, Rmin;
     int    mode;            // DDX_MODE_*
     int    lose_tile;       // test hook: tile whose copy is never issued (-1: none)
     unsigned long long wait_ns;   // bound on any one device-side wait
@@ -135,6 +135,17 @@ __host__ __device__ inline bool spatial_order_on(const StepArgs& a) {
     return a.n_grav - a.n_exact >= kOrderMinSources;
 }
 
+// Buffers of the mixed step's cell expansions (ddx_cells.cu), for up to n_src planetesimals.
+struct CellScratch;
+cudaError_t cells_ensure(CellScratch*& c, int n_src);
+void cells_free(CellScratch*& c);
+
+// The mixed step takes far planetesimals through cell expansions (ddx_cells.cu) from this many
+// on; with fewer, building them costs small numbers of tracers more than it saves (us a step
+// with every pair / with cells: 1,100 planetesimals and 50,000 tracers 395 / 517, 2,100 and 10,000
+// 519 / 491, 2,100 and 500,000 2312 / 1513).
+constexpr int kCellMinSources = 2048;
+
 // Stage scratch for the massive set.  Positions of the four RK4 stages are kept as
 // {x, y, z, m} records for the FP64 dust kernels.  The mixed path also keeps an FP32
 // hi/lo split of each stage position, per body (Phi/Plo, for the massive passes) and in
@@ -158,6 +169,7 @@ struct MassiveScratch {
     int      *src;       // [cap] its inverse: FP32 source of pair slot q (written with slot)
     OrderScratch src_order;    // ordering of the FP32 sources (cap bodies)
     OrderScratch dust_order;   // ordering of the tracers of one dust launch
+    CellScratch *cells;        // trees of the mixed dust kernel with many planetesimals (ddx_cells.cu)
 };
 
 // Makes `device` current for the scope of an entry point and makes the caller's current
@@ -214,6 +226,59 @@ __device__ __forceinline__ float d2f_toward0(double v) {
 __device__ __forceinline__ void split_hilo(double v, float& hi, float& lo) {
     hi = __double2float_rn(v);
     lo = __double2float_rn(v - (double)hi);
+}
+
+// f as FP64, exactly, by moving its bits (f finite; subnormal f give 0): the FP64 pipe is left
+// alone, as in d2f_toward0.
+__device__ __forceinline__ double f2d_bits(float f) {
+    const uint32_t b = __float_as_uint(f), m = b & 0x7FFFFFFFu;
+    const uint32_t hi = m < 0x00800000u ? 0u : (m >> 3) + 0x38000000u;
+    return __hiloint2double((int)(hi | (b & 0x80000000u)), m < 0x00800000u ? 0 : (int)(m << 29));
+}
+
+// v = hi + lo within 2^-48 |v|: each rounded to 24 bits (halves away from zero) by moving bits;
+// one exact FP64 subtraction a call.
+__device__ __forceinline__ double round24(double v) {
+    return __longlong_as_double((__double_as_longlong(v) + 0x10000000ll) & ~0x1FFFFFFFll);
+}
+__device__ __forceinline__ void split2(double v, float& hi, float& lo) {
+    const double h = round24(v);
+    hi = d2f_toward0(h);
+    lo = d2f_toward0(round24(v - h));
+}
+
+// Star term of the mixed dust kernel with cells: the same force as star_term below with its
+// factors that do not change over a step formed once per tracer, one rsqrt in place of four
+// divisions and a square root (28 FP64 operations against about 100, which took half of the
+// kernel: FP64 issues at 1/64 of the FP32 rate).  Results agree to a few FP64 roundings;
+// the sublimation test is the same expression.
+struct StarCoef {
+    double g, c, l;      // (1 - beta - beta_sw) m0; drag factor times m0; q Bstar Rstar^3 / m
+};
+__device__ __forceinline__ StarCoef star_coef(double m0, float bet, float betsw, float qe, double m, const StepArgs& a) {
+    StarCoef k;
+    k.g = (1.0 - bet - betsw) * m0;
+    const double pr = bet * (1.0 / kLightAU);
+    k.c = (a.SWQ == 1 ? fma((double)betsw, a.inv_vsw, pr) : pr) * m0;
+    k.l = a.FLQ == 1 ? qe * (a.Bstar * a.Rstar * a.Rstar * a.Rstar) / m : 0.0;
+    return k;
+}
+__device__ __forceinline__ bool star_term(double dx, double dy, double dz, double rx, double ry, double rz,
+                                          const StarCoef& k, const StepArgs& a, double& kx, double& ky, double& kz) {
+    const double RR = fma(dz, dz, fma(dy, dy, dx * dx));
+    if (RR <= a.Rmin * a.Rmin) return false;
+    const double ri = rsqrt(RR), iRR = ri * ri, iR3 = ri * iRR;
+    const double f1 = k.c * iRR;
+    const double f = fma(f1, fma(dz, rz, fma(dy, ry, dx * rx)) * iRR, k.g * iR3);
+    kx = -fma(f, dx, f1 * rx);
+    ky = -fma(f, dy, f1 * ry);
+    kz = -fma(f, dz, f1 * rz);
+    if (a.FLQ == 1) {
+        const double b = k.l * iR3;
+        kx = fma(b, fma(-a.Wz, dx, ry), kx);
+        ky = fma(-b, fma(a.Wz, dy, rx), ky);
+    }
+    return true;
 }
 
 // Star term of one stage (src/gpu_functions.cu:680-718): gravity reduced by beta+beta_sw,

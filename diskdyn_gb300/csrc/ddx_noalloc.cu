@@ -141,6 +141,7 @@ extern "C" int ddx_step_noalloc(int device, const ddx_state* s, int n_grav, int 
     a.Bstar = p->Bstar;
     a.Rstar = p->Rstar;
     a.vswAU = p->vsw_AUyr;
+    a.inv_vsw = 1.0 / p->vsw_AUyr;
     a.Rmin = p->Rmin;
     a.mode = mode;
     a.lose_tile = -1;

@@ -1,0 +1,78 @@
+// Pieces of the planetesimals' FP32 pull shared by the mixed dust kernels: the FP64 pull of
+// near sources and the sums across spans of pair records.
+#pragma once
+#include "ddx_internal.cuh"
+#include "ddx_f32x2.cuh"
+
+namespace ddx {
+namespace {
+
+// N pair records (slots q0 .. q0 + 2 N - 1) summed again for a tracer with a near source
+// among them: the FP32 partial sum, added to (px, py, pz), of the sources at or beyond the
+// near radius (the same operations as the main loop, so each of their pulls is the same), and
+// the FP64 pull of each near source from its FP64 stage position (P: the stage's records of
+// bodies n_exact.., src: source of each slot, null when slot q holds source q) and the
+// tracer's (xt, yt, zt), added to k.  A zero FP64 separation gives an infinite pull, which
+// removes the tracer as in the FP64 step.
+template <int N>
+__device__ __forceinline__ void near_span(const BodyPair* R, int q0, f2 XH, f2 XL, f2 YH, f2 YL, f2 ZH, f2 ZL,
+                                          double xt, double yt, double zt, float inv_near, const Body* __restrict__ P,
+                                          const int* __restrict__ src, f2& px, f2& py, f2& pz, double& kx,
+                                          double& ky, double& kz) {
+    for (int u = 0; u < N; ++u) {
+        const BodyPair* r = R + u;
+        const ulonglong2 q0v = *reinterpret_cast<const ulonglong2*>(r->hx);
+        const ulonglong2 q1v = *reinterpret_cast<const ulonglong2*>(r->hz);
+        const ulonglong2 q2v = *reinterpret_cast<const ulonglong2*>(r->lx);
+        const f2 lz = *reinterpret_cast<const f2*>(r->lz);
+        const f2 dX = add2(sub2(q0v.x, XH), sub2(q2v.x, XL));
+        const f2 dY = add2(sub2(q0v.y, YH), sub2(q2v.y, YL));
+        const f2 dZ = add2(sub2(q1v.x, ZH), sub2(lz, ZL));
+        const f2 RR = fma2(dX, dX, fma2(dY, dY, mul2(dZ, dZ)));
+        float r0, r1;
+        f2_split(RR, r0, r1);
+        const float i0 = rsqrt_approx(r0), i1 = rsqrt_approx(r1);
+        const bool n0 = i0 > inv_near, n1 = i1 > inv_near;
+        const f2 ri = f2_join(n0 ? 0.f : i0, n1 ? 0.f : i1);
+        const f2 f = mul2(mul2(q1v.y, ri), mul2(ri, ri));
+        px = fma2(f, dX, px); py = fma2(f, dY, py); pz = fma2(f, dZ, pz);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (!(h ? n1 : n0)) continue;
+            const int q = q0 + 2 * u + h;
+            const Body p = P[src ? src[q] : q];
+            const double ex = p.x - xt, ey = p.y - yt, ez = p.z - zt;
+            const double rr = fma(ez, ez, fma(ey, ey, ex * ex));
+            const double ri64 = rsqrt(rr);
+            const double f64 = p.m * (ri64 * ri64 * ri64);
+            kx = fma(f64, ex, kx); ky = fma(f64, ey, ky); kz = fma(f64, ez, kz);
+        }
+    }
+}
+
+// Kahan sums across the FP32 spans.  The compensated variant keeps both lanes (its
+// float-float spans go to the FP64 acceleration instead, ff_total).  The FP32 forms add
+// the span's two lanes (one rounding, against the 16 of each lane's plain sum) and carry one
+// FP32 sum per axis: six registers fewer in the loop, which the dusty-ring dust kernel took
+// from 8.18 to 8.00 ms.
+template <bool F2> struct SpanAcc;
+template <> struct SpanAcc<true> {
+    f2 S = 0, C = 0;
+    __device__ __forceinline__ void add(f2 v) { kahan2(S, C, v); }
+    __device__ __forceinline__ double total() const { return f2_total(S, C); }
+};
+template <> struct SpanAcc<false> {
+    float S = 0.f, C = 0.f;
+    __device__ __forceinline__ void add(f2 v) {
+        float a, b;
+        f2_split(v, a, b);
+        const float y = __fsub_rn(__fadd_rn(a, b), C);
+        const float t = __fadd_rn(S, y);
+        C = __fsub_rn(__fsub_rn(t, S), y);
+        S = t;
+    }
+    __device__ __forceinline__ double total() const { return (double)S - (double)C; }
+};
+
+}  // namespace
+}  // namespace ddx

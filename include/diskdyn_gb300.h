@@ -132,7 +132,10 @@ int ddx_set_optics(ddx_ctx *ctx, int n_grid, int n_wav, int n_theta, const doubl
  * DDX_PREC_MIXED with 1,024 planetesimals or more visits the tracers and reads the FP32
  * planetesimals in a spatial order (Hilbert cells) and takes spans of 32 planetesimals that
  * lie at least a quarter of the largest |coordinate| of the two away from a tracer with the
- * FP32 high parts alone.
+ * FP32 high parts alone.  From 2,048 planetesimals on, those far from a tracer's cell of
+ * space act through the cell's expansion (harmonics to degree 10; at most 2.6e-6 of one
+ * such pull is left out, the size of the FP32 pulls' own rounding over all of them) and only
+ * the others one by one.
  * Each tracer's result depends on its own data and the massive set only (not on the
  * other tracers or their order), and the result is the same from run to run. */
 int ddx_step(ddx_ctx *ctx, const ddx_state *s, int n_grav, int n_dust, double dt,
@@ -374,7 +377,8 @@ int ddx_set_compensated_radius(ddx_ctx *ctx, double eta);
  * dust launch of this context leaves the TMA copy of source tile `tile` (counted over the
  * four stages) unissued and bounds its waits by wait_ns instead of 2 s, so the blocks
  * give up, report DDX_ERR_TIMEOUT through ddx_sync_status and leave their tracers
- * unchanged.  Nothing faults or hangs; the context stays usable. */
+ * unchanged.  Nothing faults or hangs; the context stays usable.  That launch takes every
+ * planetesimal one by one (cell expansions have no tiles). */
 int ddx_debug_lose_tile_copy(ddx_ctx *ctx, int tile, unsigned long long wait_ns);
 
 /* Error string for a status code. */

@@ -63,3 +63,80 @@ def test_massive_set_pulls(engine, n_plsml):
     rows = np.arange(3, s.n_grav)
     rows = rows if len(rows) <= 1024 else np.concatenate([rows[:300], rows[300:-300:13], rows[-300:]])
     check_velocities(s, f, m, rows)
+
+
+# Cell expansions of far planetesimals.  Their series stops at degree 10; for one source at the
+# least far distance of 4.5 cell edges and a tracer at the corner of the reach of 0.55 edges
+# (ratio 0.21) the rest is at most sum over n > 10 of n 0.21^(n - 1) = 2.6e-6 of the pull;
+# with the FP32 roundings above 4e-6.
+CELLS = 4e-6
+
+
+def scattered(n_plsml, n_dust, seed=78):
+    """The heavy ring with grains everywhere: half in the ring, the rest at 15 to 5,000 AU in
+    all directions, and every 100th planetesimal moved to 300 to 30,000 AU."""
+    s = heavy_ring(n_plsml, n_dust, seed)
+    g = np.random.default_rng(seed)
+    ng = s.n_grav
+
+    def move(rows, lo, hi):
+        u = g.normal(size=(3, len(rows)))
+        u *= 10 ** g.uniform(np.log10(lo), np.log10(hi), len(rows)) / np.linalg.norm(u, axis=0)
+        for k, c in enumerate("xyz"):
+            s.state[c][rows] = u[k]
+            s.state["v" + c][rows] *= 0.1
+    move(np.arange(ng + 1, ng + n_dust, 2), 15.0, 5000.0)
+    move(np.arange(3, ng, 100), 300.0, 30000.0)
+    return s
+
+
+# 2,048 planetesimals is where the cells begin, 8,192 where the grid becomes finer
+@pytest.mark.parametrize("n_plsml", [2047, 2048, 2049, 4096, 8192, 8193, 16385])
+@pytest.mark.parametrize("make", [heavy_ring, scattered])
+def test_tracer_pulls(engine, n_plsml, make):
+    s = make(n_plsml, 3000)
+    f = one_step(engine, s, s.state, abi.DDX_PREC_FP64)
+    m = one_step(engine, s, s.state, abi.DDX_PREC_MIXED)
+    np.testing.assert_array_equal(m["N"] == 0, f["N"] == 0)
+    rows = np.arange(s.n_grav, s.n_grav + 3000)
+    check_velocities(s, f, m, rows[f["N"][rows] != 0], CELLS)
+
+
+def test_lanes_per_tracer_give_the_same_bits(engine):
+    """Few tracers are shared by 8 or 4 lanes each; the first 100 grains come out the same
+    among 100, 7,999, 8,000, 47,999 and 48,000."""
+    s = scattered(3000, 48000)
+    ng = s.n_grav
+    first = None
+    for n in (100, 7999, 8000, 47999, 48000):
+        state = {k: np.asarray(v)[:ng + n].copy() for k, v in s.state.items()}
+        m = one_step(engine, s, state, abi.DDX_PREC_MIXED)
+        got = np.stack([m[c][:ng + 100] for c in ("x", "y", "z", "vx", "vy", "vz", "N")])
+        if first is None:
+            first = got
+        np.testing.assert_array_equal(got, first)
+
+
+@pytest.mark.parametrize("far", [0.0, 1e12, 1e30])
+def test_star_and_planetesimals_far_from_the_origin(engine, far):
+    """The whole system displaced by 2^20 AU and more, or a planetesimal at a huge distance or
+    with no finite position: tracers take every planetesimal when no cell serves them, and stay as
+    close to FP64 as its own rounding allows."""
+    s = heavy_ring(2500, 2000)
+    st = {k: v.copy() for k, v in s.state.items()}
+    if far == 0.0:
+        for c, d in (("x", 2.0 ** 21), ("y", -2.0 ** 21), ("z", 2.0 ** 20)):
+            st[c] += d
+    else:
+        st["x"][s.n_grav - 1] = far
+    f = one_step(engine, s, st, abi.DDX_PREC_FP64)
+    m = one_step(engine, s, st, abi.DDX_PREC_MIXED)
+    np.testing.assert_array_equal(m["N"] == 0, f["N"] == 0)
+    rows = np.arange(s.n_grav, s.n_grav + 2000)
+    rows = rows[f["N"][rows] != 0]
+    # hi + lo hold a coordinate to 2^-48 of itself: 7.5e-9 AU at 2^21 AU against separations beyond
+    # the near radius (which is there larger than the ring): every pull is FP64's
+    a = pull_sums(st, s.n_grav, rows)
+    e = np.linalg.norm(np.stack([m["v" + c][rows] - f["v" + c][rows] for c in "xyz"]), axis=0)
+    v = np.linalg.norm(np.stack([f["v" + c][rows] for c in "xyz"]), axis=0)
+    assert (e <= CELLS * s.dt * a + 1e-14 * v + (1e-12 * v if far == 0.0 else 0.0)).all()
