@@ -141,22 +141,29 @@ __device__ __forceinline__ double dust_temperature(double R, int id, const Optic
     return exp(lTd[Rid - 1] + (lTd[Rid] - lTd[Rid - 1]) * frac);
 }
 
-// Flux of one tracer at table wavelength wj, in Jy, before the multiplicity N
-// (src/gpu_functions.cu:1064-1078): Planck*pi thermal emission + scattered starlight
-// with a log-linear phase-function interpolation in the scattering-angle cosine.
-__device__ __forceinline__ double tracer_flux(double n, int id, int wj, double R, double T,
-                                              int cosinm, double wt, const OpticsDev& o,
-                                              double dist, double w5, double wvl) {
-    const double I = (2 * kHplank * kCspeed * kCspeed) /
-                     (w5 * (exp(kHplank * kCspeed / (wvl * kKboltz * T)) - 1.0)) * kPI;
+// Flux of one tracer at table wavelength j, in Jy (src/gpu_functions.cu:1064-1078): Planck*pi
+// thermal emission + scattered starlight with a log-linear phase-function interpolation in
+// the scattering-angle cosine.  Factors of the wavelength alone and of the tracer alone are
+// formed once, which leaves one of nine FP64 divisions per tracer and wavelength.
+struct WaveFactor {
+    double c2, ct, cs;       // h c / (lambda k); factors of the thermal and of the scattered part
+};
+__device__ __forceinline__ WaveFactor wave_factor(int j, const OpticsDev& o) {
+    const double wvl = o.w[j], jy = 1e26 * wvl * wvl / kCspeed;
+    WaveFactor f;
+    f.c2 = kHplank * kCspeed / (wvl * kKboltz);
+    f.ct = (2 * kHplank * kCspeed * kCspeed) * kPI / o.w5[j] * jy;
+    f.cs = o.in[j] * kPI / (kAU * kAU) * jy;
+    return f;
+}
+// (gt, gs) = N s^2 (1 / dist^2, 1 / R^2); row: the phase table's row of the bracket's lower angle.
+__device__ __forceinline__ double tracer_flux(double gt, double gs, double inv_T, double wt, size_t row, int id, int j,
+                                              const WaveFactor& f, const OpticsDev& o) {
     const int nw = o.n_wav;
-    const double lm = o.lQp[(size_t)nw * (o.n_theta * id + cosinm) + wj];
-    const double lp = o.lQp[(size_t)nw * (o.n_theta * id + cosinm + 1) + wj];
-    const double P = exp(lm + (lp - lm) * wt);
-    const double s = o.size[id];
-    const double Fscat = o.in[wj] * kPI * s * s * o.Qsca[(size_t)nw * id + wj] * P / R / R / kAU / kAU;
-    const double Fther = I * s * s * o.Qabs[(size_t)nw * id + wj] / dist / dist;
-    return n * (Fther + Fscat) * 1e26 * wvl * wvl / kCspeed;
+    const double lm = o.lQp[row + j], lp = o.lQp[row + nw + j];
+    const double ther = gt * f.ct * o.Qabs[(size_t)nw * id + j] / (exp(f.c2 * inv_T) - 1.0);
+    const double scat = gs * f.cs * o.Qsca[(size_t)nw * id + j];
+    return fma(scat, exp(fma(lp - lm, wt, lm)), ther);
 }
 
 // Phase-function bracket of a scattering-angle cosine (src/gpu_functions.cu:1066-1072).
@@ -173,13 +180,9 @@ __global__ void __launch_bounds__(256)
 image_kernel(ddx_state s, int n_grav, int n_dust, const ViewConst* __restrict__ vcp,
              OpticsDev o, ImageList il, double* __restrict__ Fd, unsigned long long* __restrict__ nexact) {
     __shared__ ViewConst v;
-    __shared__ double w5s[kMaxImages], wvls[kMaxImages];
+    __shared__ WaveFactor wf[kMaxImages];
     if (threadIdx.x == 0) v = *vcp;
-    if (threadIdx.x < il.n) {
-        const double wvl = o.w[il.wj[threadIdx.x]];
-        wvls[threadIdx.x] = wvl;
-        w5s[threadIdx.x] = pow(wvl, 5);
-    }
+    if (threadIdx.x < il.n) wf[threadIdx.x] = wave_factor(il.wj[threadIdx.x], o);
     __syncthreads();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_dust) return;
@@ -214,13 +217,13 @@ image_kernel(ddx_state s, int n_grav, int n_dust, const ViewConst* __restrict__ 
     }
     int cosinm; double wt;
     phase_bracket(cossc, v.ntheta, cosinm, wt);
-    const double T = dust_temperature(R, id, o);
+    const double inv_T = 1.0 / dust_temperature(R, id, o), area = n * o.size[id] * o.size[id];
+    const double gt = area / v.dist / v.dist, gs = area / R / R;
     const size_t npix = (size_t)v.xsize * v.ysize;
     const size_t pix = (size_t)v.ysize * xim + yim;
-    for (int k = 0; k < il.n; ++k) {
-        const double F = tracer_flux(n, id, il.wj[k], R, T, cosinm, wt, o, v.dist, w5s[k], wvls[k]);
-        atomicAdd(&Fd[k * npix + pix], F);
-    }
+    const size_t row = (size_t)o.n_wav * (o.n_theta * id + cosinm);
+    for (int k = 0; k < il.n; ++k)
+        atomicAdd(&Fd[k * npix + pix], tracer_flux(gt, gs, inv_T, wt, row, id, il.wj[k], wf[k], o));
 }
 
 // Pixel index of every tracer (ysize*xim + yim, or -1 when it has no optics or falls
@@ -255,75 +258,119 @@ __global__ void pixel_kernel(ddx_state s, int n_grav, int n_dust, const ViewCons
     pix[i] = v.ysize * xim + yim;
 }
 
-// SED: each block accumulates, per wavelength, the flux of the tracers of its chunks in a
-// fixed order; a second kernel sums the block partials in block order.  Deterministic.
+// SED in FP64.  A block takes kSedBatch tracers at a time: a thread each works out what does not
+// depend on the wavelength, then thread t adds up, over every S-th tracer of the batch, the
+// flux at wavelength t % n_wav (S = sed_slices(n_wav)), so the tables are read side by side and
+// nothing is summed across lanes inside the loop.  FP64 issue bounds it: two exponentials and a division
+// per tracer and wavelength are about 50 operations of the 60.  Factors of the wavelength or the
+// tracer alone are formed once (with eight more divisions per value, and a block-wide sum
+// per wavelength, 262,144 tracers at 200 wavelengths took 12.8 ms, so 5.2 ms).  Fixed order:
+// deterministic.
 constexpr int kSedThreads = 256;
+constexpr int kSedBatch = 32, kSedMaxThreads = 512;
 
-__global__ void __launch_bounds__(kSedThreads)
-sed_partial_kernel(ddx_state s, int n_grav, int n_dust, const ViewConst* __restrict__ vcp,
-                   OpticsDev o, int mode, double* __restrict__ partial) {
-    extern __shared__ double sed_smem[];
-    double* acc = sed_smem;                      // [n_wav] block accumulator
-    double* red = sed_smem + o.n_wav;            // [kSedThreads/32] warp partials
-    __shared__ ViewConst v;
-    if (threadIdx.x == 0) v = *vcp;
-    for (int j = threadIdx.x; j < o.n_wav; j += blockDim.x) acc[j] = 0.0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int base = blockIdx.x * blockDim.x; base < n_dust; base += gridDim.x * blockDim.x) {
-        const int i = base + threadIdx.x;
-        bool on = false;
-        int id = 0, cosinm = 0;
-        double R = 1.0, T = 1.0, wt = 0.0, n = 0.0;
-        if (i < n_dust) {
-            const int t = n_grav + i;
-            id = s.id[t];
-            if (id >= 0 && id < o.n_grid) {
-                const double x = s.x[t], y = s.y[t], z = s.z[t];
-                n = s.N[t];
-                R = sqrt(x * x + y * y + z * z);
-                // The reference rotates by the spherical radius here (src/gpu_functions.cu:1106-1107);
-                // the image kernel uses the cylindrical one.
-                double x1 = x * v.cr - y * v.sr;
-                double y1 = x * v.sr + y * v.cr;
-                if (mode == DDX_MODE_REFERENCE) {
-                    const double Rd = sqrt(x * x + y * y);
-                    if (Rd > 0.0) { x1 *= R / Rd; y1 *= R / Rd; }
-                    else { x1 = R * v.cr; y1 = R * v.sr; }
-                }
-                const double cossc = scatter_cos(x1, y1, z, R, v);
-                phase_bracket(cossc, v.ntheta, cosinm, wt);
-                T = dust_temperature(R, id, o);
-                on = R > o.Rmin;
-            }
-        }
-        for (int j = 0; j < o.n_wav; ++j) {
-            double F = 0.0;
-            if (on) {
-                const double wvl = o.w[j];
-                F = tracer_flux(n, id, j, R, T, cosinm, wt, o, v.dist, o.w5[j], wvl);
-            }
-            F = warp_sum_d(F);
-            if (lane == 0) red[warp] = F;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                double b = 0.0;
-                for (int k = 0; k < kSedThreads / 32; ++k) b += red[k];
-                acc[j] += b;
-            }
-            __syncthreads();
-        }
+// Slices of a batch: as many threads of whole warps as possible have a wavelength.
+int sed_slices(int n_wav) {
+    int best = 1;
+    double used = 0.0;
+    for (int S = 1; S <= 8 && S * n_wav <= kSedMaxThreads; ++S) {
+        const double u = (double)(S * n_wav) / ((S * n_wav + 31) / 32 * 32);
+        if (u > used + 0.01) { best = S; used = u; }
     }
-    for (int j = threadIdx.x; j < o.n_wav; j += blockDim.x)
-        partial[(size_t)blockIdx.x * o.n_wav + j] = acc[j];
+    return best;
 }
 
-__global__ void sed_final_kernel(const double* __restrict__ partial, int nblocks, int n_wav,
-                                 double* __restrict__ Fsed) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n_wav) return;
+__global__ void __launch_bounds__(kSedMaxThreads)
+sed_partial_kernel(ddx_state s, int n_grav, int n_dust, const ViewConst* __restrict__ vcp,
+                   OpticsDev o, int mode, int S, double* __restrict__ partial) {
+    __shared__ ViewConst v;
+    __shared__ double inv_T[kSedBatch], wts[kSedBatch], gt[kSedBatch], gs[kSedBatch], part[kSedMaxThreads];
+    __shared__ size_t row[kSedBatch];
+    __shared__ int ids[kSedBatch];
+    if (threadIdx.x == 0) v = *vcp;
+    __syncthreads();
+    const int nw = o.n_wav, items = S * nw;
+    double* const mine = partial + (size_t)blockIdx.x * nw;
+    const bool single = items <= (int)blockDim.x;    // an item per thread, else S = 1 and sums in the block's row
+    WaveFactor f{};
+    if (single) f = wave_factor(threadIdx.x % nw, o);
+    else
+        for (int j = threadIdx.x; j < nw; j += blockDim.x) mine[j] = 0.0;
+    double acc = 0.0;
+    for (int base = blockIdx.x * kSedBatch; base < n_dust; base += gridDim.x * kSedBatch) {
+        __syncthreads();                         // the last batch has been read
+        if (threadIdx.x < kSedBatch) {
+            const int i = base + threadIdx.x;
+            int id = -1;
+            if (i < n_dust) {
+                const int t = n_grav + i;
+                id = s.id[t];
+                if (id >= 0 && id < o.n_grid) {
+                    const double x = s.x[t], y = s.y[t], z = s.z[t];
+                    const double R = sqrt(x * x + y * y + z * z);
+                    // The reference rotates by the spherical radius here (src/gpu_functions.cu:1106-1107);
+                    // the image kernel uses the cylindrical one.
+                    double x1 = x * v.cr - y * v.sr;
+                    double y1 = x * v.sr + y * v.cr;
+                    if (mode == DDX_MODE_REFERENCE) {
+                        const double Rd = sqrt(x * x + y * y);
+                        if (Rd > 0.0) { x1 *= R / Rd; y1 *= R / Rd; }
+                        else { x1 = R * v.cr; y1 = R * v.sr; }
+                    }
+                    if (R > o.Rmin) {
+                        int cosinm;
+                        double wt;
+                        phase_bracket(scatter_cos(x1, y1, z, R, v), v.ntheta, cosinm, wt);
+                        const double g = s.N[t] * o.size[id] * o.size[id];
+                        wts[threadIdx.x] = wt;
+                        row[threadIdx.x] = (size_t)nw * (o.n_theta * id + cosinm);
+                        inv_T[threadIdx.x] = 1.0 / dust_temperature(R, id, o);
+                        gt[threadIdx.x] = g / v.dist / v.dist;
+                        gs[threadIdx.x] = g / R / R;
+                    } else {
+                        id = -1;
+                    }
+                } else {
+                    id = -1;
+                }
+            }
+            ids[threadIdx.x] = id;
+        }
+        __syncthreads();
+        for (int item = threadIdx.x; item < items; item += blockDim.x) {
+            const int slice = item / nw, j = item - slice * nw;
+            if (!single) f = wave_factor(j, o);
+            double F = 0.0;
+            for (int q = slice; q < kSedBatch; q += S)
+                if (ids[q] >= 0) F += tracer_flux(gt[q], gs[q], inv_T[q], wts[q], row[q], ids[q], j, f, o);
+            if (single) acc += F;
+            else mine[j] += F;
+        }
+    }
+    if (!single) return;
+    if (threadIdx.x < items) part[threadIdx.x] = acc;
+    __syncthreads();
+    for (int j = threadIdx.x; j < nw; j += blockDim.x) {
+        double b = 0.0;
+        for (int k = 0; k < S; ++k) b += part[k * nw + j];
+        mine[j] = b;
+    }
+}
+
+// Sums of the blocks' rows: a warp takes 32 wavelengths and every kFinalWarps-th row, the warps'
+// sums are added in order (1,024 rows of 200: 72 us with a thread per wavelength).
+constexpr int kFinalWarps = 32;
+__global__ void __launch_bounds__(32 * kFinalWarps)
+sed_final_kernel(const double* __restrict__ partial, int nblocks, int n_wav, double* __restrict__ Fsed) {
+    __shared__ double part[kFinalWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = blockIdx.x * 32 + lane;
     double s = 0.0;
-    for (int b = 0; b < nblocks; ++b) s += partial[(size_t)b * n_wav + j];
+    if (j < n_wav)
+        for (int b = warp; b < nblocks; b += kFinalWarps) s += partial[(size_t)b * n_wav + j];
+    part[warp][lane] = s;
+    __syncthreads();
+    if (warp != 0 || j >= n_wav) return;
+    for (int w = 1; w < kFinalWarps; ++w) s += part[w][lane];
     Fsed[j] = s;
 }
 
@@ -394,9 +441,10 @@ cudaError_t launch_pixels(const ddx_state& s, int n_grav, int n_dust, const ddx_
     return cudaGetLastError();
 }
 
+// Blocks of the FP64 SED (eight per SM at most), never fewer than the mixed one's.
 int sed_blocks(int n_dust) {
-    int b = (n_dust + kSedThreads - 1) / kSedThreads;
-    return b < 1 ? 1 : (b > 1216 ? 1216 : b);
+    const int b = n_dust / kSedBatch + 1;
+    return b > 1216 ? 1216 : b;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -867,7 +915,10 @@ sed_mixed_kernel(ddx_state s, int n_grav, int n_dust, View32 v32, OpticsDev o,
     }
 }
 
-int sed_mixed_blocks(int n_dust) { return sed_blocks(n_dust); }
+int sed_mixed_blocks(int n_dust) {
+    const int b = n_dust / kSedThreads + (n_dust % kSedThreads != 0);
+    return b < 1 ? 1 : (b > 1216 ? 1216 : b);
+}
 
 cudaError_t launch_photo_prepare(const OpticsDev& o, const ViewConst* vc, const ImageList* il,
                                  PhotoConst pc, cudaStream_t st) {
@@ -908,7 +959,7 @@ cudaError_t launch_sed_mixed(const ddx_state& s, int n_grav, int n_dust, const d
         sed_mixed_kernel<<<nb, kSedThreads, 0, st>>>(s, n_grav, n_dust, v32, o, pc, mode, lam0, partial);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    sed_final_kernel<<<(o.n_wav + 127) / 128, 128, 0, st>>>(partial, nb, o.n_wav, Fsed);
+    sed_final_kernel<<<(o.n_wav + 31) / 32, 32 * kFinalWarps, 0, st>>>(partial, nb, o.n_wav, Fsed);
     return cudaGetLastError();
 }
 
@@ -919,11 +970,12 @@ cudaError_t launch_sed(const ddx_state& s, int n_grav, int n_dust, const ddx_vie
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const int nb = sed_blocks(n_dust);
-    const size_t smem = sizeof(double) * (o.n_wav + kSedThreads / 32);
-    sed_partial_kernel<<<nb, kSedThreads, smem, st>>>(s, n_grav, n_dust, vc, o, mode, partial);
+    const int S = sed_slices(o.n_wav), items = S * o.n_wav;
+    const int threads = items > kSedMaxThreads ? kSedMaxThreads : (items + 31) / 32 * 32;
+    sed_partial_kernel<<<nb, threads, 0, st>>>(s, n_grav, n_dust, vc, o, mode, S, partial);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    sed_final_kernel<<<(o.n_wav + 127) / 128, 128, 0, st>>>(partial, nb, o.n_wav, Fsed);
+    sed_final_kernel<<<(o.n_wav + 31) / 32, 32 * kFinalWarps, 0, st>>>(partial, nb, o.n_wav, Fsed);
     return cudaGetLastError();
 }
 

@@ -55,12 +55,6 @@ cudaError_t launch_sed_mixed(const ddx_state& s, int n_grav, int n_dust, const d
                              double* Fsed, cudaStream_t st);
 int sed_mixed_blocks(int n_dust);
 
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 cudaError_t launch_optics_prepare(OpticsDev& o, OpticsDev* o_dev, cudaStream_t st);
 cudaError_t launch_image(const ddx_state& s, int n_grav, int n_dust, const ddx_view& view,
                          const OpticsDev& o, const ImageList& il, ViewConst* vc, double* Fd,
