@@ -81,7 +81,7 @@ __device__ __forceinline__ StarConst star_const(const AdjArgs& A, double m0, flo
 }
 
 // Acceleration of a tracer at (x, r) for the stage whose body records are P[0..ng), with one
-// square root and one division for the star and one rsqrt per body.  Returns false on
+// rsqrt64 for the star and one per body.  Returns false on
 // sublimation (R <= Rmin) or an exact coincidence with a body.  rc (optional, stride rs):
 // receives 1/R^2 and 1/R of the star and 1/|e| of bodies 1..nir, which the reverse sweep
 // reuses instead of dividing and taking roots again (FP64 division and square root are
@@ -92,8 +92,8 @@ __device__ __forceinline__ bool tracer_accel(const AdjArgs& A, const StarConst& 
     const double dx = x - P[0].x, dy = y - P[0].y, dz = z - P[0].z;
     const double RR = dx * dx + dy * dy + dz * dz;
     if (RR <= A.sa.Rmin * A.sa.Rmin) return false;
-    const double iRR = 1.0 / RR;
-    const double iR = sqrt(iRR);
+    const double iR = rsqrt64(RR);
+    const double iRR = iR * iR;
     const double iR3 = iR * iRR;
     if (rc) { rc[0] = iRR; rc[rs] = iR; }
     const double Fg = K.g0 * iR3, Fb1 = K.c1 * iRR, Fb2 = (dx * rx + dy * ry + dz * rz) * iRR;
@@ -108,7 +108,7 @@ __device__ __forceinline__ bool tracer_accel(const AdjArgs& A, const StarConst& 
         const double ex = P[j].x - x, ey = P[j].y - y, ez = P[j].z - z;
         const double R2 = ex * ex + ey * ey + ez * ez;
         if (R2 == 0.0) return false;
-        const double ir = rsqrt(R2);
+        const double ir = rsqrt64(R2);
         if (rc && j <= A.nir) rc[(1 + j) * rs] = ir;
         const double f = P[j].m * (ir * ir * ir);
         ax += f * ex; ay += f * ey; az += f * ez;
@@ -127,8 +127,8 @@ __device__ __forceinline__ void massive_acc(const double (*sp)[4], int ng, int j
         if (k == j) continue;
         const double dx = sp[k][0] - sp[j][0], dy = sp[k][1] - sp[j][1], dz = sp[k][2] - sp[j][2];
         const double RR = dx * dx + dy * dy + dz * dz;
-        if (RR > 0.0) {
-            const double f = sp[k][3] / (RR * sqrt(RR));
+        if (positive64(RR)) {
+            const double f = pull64(sp[k][3], RR);
             ax += f * dx; ay += f * dy; az += f * dz;
         }
     }
@@ -191,8 +191,8 @@ __device__ __forceinline__ void massive_vjp(const double (*sp)[4], const double 
         if (k == j) continue;
         const double dx = sp[j][0] - sp[k][0], dy = sp[j][1] - sp[k][1], dz = sp[j][2] - sp[k][2];
         const double RR = dx * dx + dy * dy + dz * dz;
-        if (!(RR > 0.0)) continue;
-        const double ri3 = 1.0 / (RR * sqrt(RR)), ri5 = ri3 / RR;
+        if (!positive64(RR)) continue;
+        const double ri = rsqrt64(RR), ri2 = ri * ri, ri3 = ri * ri2, ri5 = ri3 * ri2;
         const double vx = mj * sg[k][0] - sp[k][3] * sg[j][0];
         const double vy = mj * sg[k][1] - sp[k][3] * sg[j][1];
         const double vz = mj * sg[k][2] - sp[k][3] * sg[j][2];
@@ -415,7 +415,7 @@ __device__ __forceinline__ void tracer_vjp(const AdjArgs& A, const StarConst& K,
         double v4[4] = {0, 0, 0, 0};
         if (on) {
             const double dx = P[j].x - pos[0], dy = P[j].y - pos[1], dz = P[j].z - pos[2];
-            const double ir = (j <= A.nir) ? rc[(1 + j) * rs] : rsqrt(dx * dx + dy * dy + dz * dz);
+            const double ir = (j <= A.nir) ? rc[(1 + j) * rs] : rsqrt64(dx * dx + dy * dy + dz * dz);
             const double ir2 = ir * ir;
             const double ri3 = ir2 * ir, ri5 = ri3 * ir2;
             const double gd = g[0] * dx + g[1] * dy + g[2] * dz;
@@ -546,7 +546,7 @@ __device__ __forceinline__ double warp_sum_d(double v) {
 }
 
 // Acceleration of body j from every other body at one stage (records P[0..ng)), the
-// m / (RR sqrt(RR)) form of massive_acc, lanes strided over the sources with a fixed
+// pull64 form of massive_acc, lanes strided over the sources with a fixed
 // butterfly sum.  All 32 lanes call it.
 __device__ __forceinline__ void massive_acc_warp(const Body* __restrict__ P, int ng, int j, double& ax, double& ay,
                                                  double& az) {
@@ -558,8 +558,8 @@ __device__ __forceinline__ void massive_acc_warp(const Body* __restrict__ P, int
         const Body pk = P[k];
         const double dx = pk.x - pj.x, dy = pk.y - pj.y, dz = pk.z - pj.z;
         const double RR = dx * dx + dy * dy + dz * dz;
-        if (RR > 0.0) {
-            const double f = pk.m / (RR * sqrt(RR));
+        if (positive64(RR)) {
+            const double f = pull64(pk.m, RR);
             ax += f * dx; ay += f * dy; az += f * dz;
         }
     }
@@ -659,8 +659,8 @@ __global__ void massive_rev_stage_kernel(int ng, double dt, const Body* __restri
         const Body pk = P[k];
         const double dx = pj.x - pk.x, dy = pj.y - pk.y, dz = pj.z - pk.z;
         const double RR = dx * dx + dy * dy + dz * dz;
-        if (!(RR > 0.0)) continue;
-        const double ri3 = 1.0 / (RR * sqrt(RR)), ri5 = ri3 / RR;
+        if (!positive64(RR)) continue;
+        const double ri = rsqrt64(RR), ri2 = ri * ri, ri3 = ri * ri2, ri5 = ri3 * ri2;
         const double gk[3] = {G[k], G[ng + k], G[2 * ng + k]};
         const double vx = pj.m * gk[0] - pk.m * gj[0];
         const double vy = pj.m * gk[1] - pk.m * gj[1];

@@ -170,8 +170,7 @@ __device__ __forceinline__ void finish_tracer(const Column& col, const StepArgs&
 // The FP64 pull of one body added to the column's acceleration of stage st.
 __device__ __noinline__ void add_point(const Body p, const Column col, int st, const StepArgs& a) {
     const double ex = p.x - stage_pos(col, 0, st, a), ey = p.y - stage_pos(col, 1, st, a), ez = p.z - stage_pos(col, 2, st, a);
-    const double ri = rsqrt(fma(ez, ez, fma(ey, ey, ex * ex)));
-    const double f = p.m * (ri * ri * ri);
+    const double f = pull64(p.m, fma(ez, ez, fma(ey, ey, ex * ex)));
     const int kc = qK1 + 3 * st;
     col.put(kc, fma(f, ex, col.get(kc)));
     col.put(kc + 1, fma(f, ey, col.get(kc + 1)));
@@ -396,8 +395,7 @@ dust_cells_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __r
                     removed = 2;
                     break;
                 }
-                const double ri = rsqrt(RR);
-                const double f = p.m * (ri * ri * ri);
+                const double f = pull64(p.m, RR);
                 kx = fma(f, ex, kx); ky = fma(f, ey, ky); kz = fma(f, ez, kz);
             }
             const int kc = qK1 + 3 * st;
@@ -429,15 +427,17 @@ dust_cells_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __r
                         ms.P + (size_t)st * ms.cap + a.n_exact, src};
         pull_groups<T>(v, node, alive, S, p, col, st, a);
         if (alive) {
+            const int kc = qK1 + 3 * st;
+            const double kx = col.get(kc), ky = col.get(kc + 1), kz = col.get(kc + 2);
             // An exact coincidence makes RR = 0, the rsqrt infinite and the sum NaN.
-            if (!(isfinite(p.ax.S + fx) && isfinite(p.ay.S + fy) && isfinite(p.az.S + fz))) {
+            if (!(isfinite(p.ax.S + fx) && isfinite(p.ay.S + fy) && isfinite(p.az.S + fz) && finite64(kx) &&
+                  finite64(ky) && finite64(kz))) {
                 alive = false;
                 removed = 2;
             }
-            const int kc = qK1 + 3 * st;
-            col.put(kc, (col.get(kc) + f2d_bits(p.ax.S)) + f2d_bits(fx - p.ax.C));
-            col.put(kc + 1, (col.get(kc + 1) + f2d_bits(p.ay.S)) + f2d_bits(fy - p.ay.C));
-            col.put(kc + 2, (col.get(kc + 2) + f2d_bits(p.az.S)) + f2d_bits(fz - p.az.C));
+            col.put(kc, (kx + f2d_bits(p.ax.S)) + f2d_bits(fx - p.ax.C));
+            col.put(kc + 1, (ky + f2d_bits(p.ay.S)) + f2d_bits(fy - p.ay.C));
+            col.put(kc + 2, (kz + f2d_bits(p.az.S)) + f2d_bits(fz - p.az.C));
         }
     }
     if (i >= a.n_dust || (T > 1 && (threadIdx.x & (T - 1)))) return;

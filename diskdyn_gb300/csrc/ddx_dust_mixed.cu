@@ -333,8 +333,7 @@ __device__ __forceinline__ void near_span_ff(const BodyPair* R, const f2* ML, in
             const Body p = P[src ? src[q] : q];
             const double ex = p.x - xt, ey = p.y - yt, ez = p.z - zt;
             const double rr = ex * ex + ey * ey + ez * ez;
-            const double ri64 = rsqrt(rr);
-            const double f64 = p.m * (ri64 * ri64 * ri64);
+            const double f64 = pull64(p.m, rr);
             kx = fma(f64, ex, kx); ky = fma(f64, ey, ky); kz = fma(f64, ez, kz);
         }
     }
@@ -438,6 +437,7 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
     };
     if (tid == 0 && G > 0) issue(0);
 
+    const StarCoef star = star_coef(ms.P[0].m, bet, betsw, qe, m, a);
     const double dt = a.dt, dt2 = a.dt / 2.0, dt6 = a.dt / 6.0;
     // RK4 of src/gpu_functions.cu:627-943 with running sums, so that little FP64 state is
     // live across the FP32 loop: stage s evaluates the acceleration at
@@ -465,8 +465,7 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
         double kx = 0, ky = 0, kz = 0;
         if (alive) {
             const Body ps = ms.P[st * ms.cap + 0];
-            if (!star_term(xt - ps.x, yt - ps.y, zt - ps.z, rx, ry, rz, ps.m, bet, betsw, qe, m, a,
-                           kx, ky, kz)) {
+            if (!star_term(xt - ps.x, yt - ps.y, zt - ps.z, rx, ry, rz, star, a, kx, ky, kz)) {
                 alive = false; removed = 1; removed_stage = st;
             }
         }
@@ -476,8 +475,7 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
             const double ex = p.x - xt, ey = p.y - yt, ez = p.z - zt;
             const double RR = ex * ex + ey * ey + ez * ez;
             if (RR == 0.0) { alive = false; removed = 2; removed_stage = st; break; }
-            const double ri = rsqrt(RR);
-            const double f = p.m * (ri * ri * ri);
+            const double f = pull64(p.m, RR);
             kx = fma(f, ex, kx); ky = fma(f, ey, ky); kz = fma(f, ez, kz);
         }
         float xh, xl, yh, yl, zh, zl;

@@ -247,11 +247,42 @@ __device__ __forceinline__ void split2(double v, float& hi, float& lo) {
     lo = d2f_toward0(round24(v - h));
 }
 
-// Star term of the mixed dust kernel with cells: the same force as star_term below with its
-// factors that do not change over a step formed once per tracer, one rsqrt in place of four
-// divisions and a square root (28 FP64 operations against about 100, which took half of the
-// kernel: FP64 issues at 1/64 of the FP32 rate).  Results agree to a few FP64 roundings;
-// the sublimation test is the same expression.
+// x^(-1/2) and m x^(-3/2) in FP64 for the pulls, from rsqrt.approx.ftz.f64 (20 bits: e below is at most
+// 2^-19.0) and the binomial series in e = 1 - x y^2, which stops where the next term is below
+// 2^-55: x^(-1/2) = y (1 - e)^(-1/2), x^(-3/2) = y^3 (1 - e)^(-3/2).  Five and seven FP64 operations (the
+// FP64 pipe, at 1/64 of the FP32 rate, bounds every kernel with FP64 pulls), no branch, and
+// m x^(-3/2) within 2.3e-16 where the cube of rsqrt(double) is within 5.5e-16 (no faster in the
+// pair loops: one operation fewer of 17).
+// Zero and subnormal x give NaN, as the sum of a coincident source always did; infinite x
+// gives 0.
+__device__ __forceinline__ double rsqrt_seed(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    return y;
+}
+__device__ __forceinline__ double zero_at_infinity(double x, double f) {
+    return (__double2hiint(x) & 0x7FFFFFFF) >= 0x7FF00000 ? 0.0 : f;
+}
+__device__ __forceinline__ double rsqrt64(double x) {
+    const double y = rsqrt_seed(x), e = fma(-x, y * y, 1.0);
+    return zero_at_infinity(x, fma(y * e, fma(e, 0.375, 0.5), y));
+}
+__device__ __forceinline__ double pull64(double m, double x) {
+    const double y = rsqrt_seed(x), y2 = y * y, e = fma(-x, y2, 1.0), f = (m * y) * y2;
+    return zero_at_infinity(x, fma(f * e, fma(e, 1.875, 1.5), f));
+}
+__device__ __forceinline__ bool finite64(double x) { return (__double2hiint(x) & 0x7FFFFFFF) < 0x7FF00000; }
+// x > 0, normal and finite, without the FP64 pipe.
+__device__ __forceinline__ bool positive64(double x) {
+    return (unsigned)__double2hiint(x) - 0x00100000u < 0x7FE00000u;
+}
+
+// Star term of the dust kernels but DDX_MODE_REFERENCE's FP64 one: the same force as star_term
+// below with its factors that do not change over a step formed once per tracer, and one rsqrt
+// in place of nine divisions and a square root: 28 FP64 operations against about 100, at 1/64 of the
+// FP32 rate (262,144 charged grains with 256 planetesimals: 462 -> 350 us a step; 16,384 grains with a star and
+// eight planets in FP64: 63.5 -> 53.1 us).
+// Results agree to a few FP64 roundings; the sublimation test is the same expression.
 struct StarCoef {
     double g, c, l;      // (1 - beta - beta_sw) m0; drag factor times m0; q Bstar Rstar^3 / m
 };
@@ -267,7 +298,7 @@ __device__ __forceinline__ bool star_term(double dx, double dy, double dz, doubl
                                           const StarCoef& k, const StepArgs& a, double& kx, double& ky, double& kz) {
     const double RR = fma(dz, dz, fma(dy, dy, dx * dx));
     if (RR <= a.Rmin * a.Rmin) return false;
-    const double ri = rsqrt(RR), iRR = ri * ri, iR3 = ri * iRR;
+    const double ri = rsqrt64(RR), iRR = ri * ri, iR3 = ri * iRR;
     const double f1 = k.c * iRR;
     const double f = fma(f1, fma(dz, rz, fma(dy, ry, dx * rx)) * iRR, k.g * iR3);
     kx = -fma(f, dx, f1 * rx);

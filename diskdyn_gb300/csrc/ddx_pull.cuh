@@ -12,8 +12,8 @@ namespace {
 // near radius (the same operations as the main loop, so each of their pulls is the same), and
 // the FP64 pull of each near source from its FP64 stage position (P: the stage's records of
 // bodies n_exact.., src: source of each slot, null when slot q holds source q) and the
-// tracer's (xt, yt, zt), added to k.  A zero FP64 separation gives an infinite pull, which
-// removes the tracer as in the FP64 step.
+// tracer's (xt, yt, zt), added to k.  A zero FP64 separation makes the sum NaN, which removes
+// the tracer as in the FP64 step.
 template <int N>
 __device__ __forceinline__ void near_span(const BodyPair* R, int q0, f2 XH, f2 XL, f2 YH, f2 YL, f2 ZH, f2 ZL,
                                           double xt, double yt, double zt, float inv_near, const Body* __restrict__ P,
@@ -43,8 +43,7 @@ __device__ __forceinline__ void near_span(const BodyPair* R, int q0, f2 XH, f2 X
             const Body p = P[src ? src[q] : q];
             const double ex = p.x - xt, ey = p.y - yt, ez = p.z - zt;
             const double rr = fma(ez, ez, fma(ey, ey, ex * ex));
-            const double ri64 = rsqrt(rr);
-            const double f64 = p.m * (ri64 * ri64 * ri64);
+            const double f64 = pull64(p.m, rr);
             kx = fma(f64, ex, kx); ky = fma(f64, ey, ky); kz = fma(f64, ez, kz);
         }
     }

@@ -104,9 +104,8 @@ __device__ __forceinline__ void pair64(const Body pi, const Body pj, double& ax,
                                        double& ay, double& az) {
     const double dX = pj.x - pi.x, dY = pj.y - pi.y, dZ = pj.z - pi.z;
     const double RR = dX * dX + dY * dY + dZ * dZ;
-    if (RR > 0.0) {
-        const double ri = rsqrt(RR);
-        const double f = pj.m * (ri * ri * ri);
+    if (positive64(RR)) {
+        const double f = pull64(pj.m, RR);
         ax = fma(f, dX, ax); ay = fma(f, dY, ay); az = fma(f, dZ, az);
     }
 }
@@ -550,8 +549,7 @@ __device__ __forceinline__ bool dust_perturb(const MassiveScratch& ms, int ng, i
                         const Body p = sP[k];
                         const double dx = xt - p.x, dy = yt - p.y, dz = zt - p.z;
                         const double RR = dx * dx + dy * dy + dz * dz;
-                        const double ri = rsqrt(RR);
-                        const double f = p.m * (ri * ri * ri);
+                        const double f = pull64(p.m, RR);
                         kx = fma(-f, dx, kx); ky = fma(-f, dy, ky); kz = fma(-f, dz, kz);
                     }
                 }
@@ -586,6 +584,7 @@ dust_rk4_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __res
             }
         }
     }
+    const StarCoef star = star_coef(ms.P[0].m, bet, betsw, qe, m, a);
     const double dt = a.dt, dt2 = a.dt / 2.0, dt6 = a.dt / 6.0;
     double k1vx = 0, k1vy = 0, k1vz = 0, k2vx = 0, k2vy = 0, k2vz = 0;
     double k3vx = 0, k3vy = 0, k3vz = 0, k4vx = 0, k4vy = 0, k4vz = 0;
@@ -614,10 +613,11 @@ dust_rk4_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __res
         double kx = 0, ky = 0, kz = 0;
         if (alive) {
             const Body ps = ms.P[st * ms.cap + 0];
-            if (!star_term(xt - ps.x, yt - ps.y, zt - ps.z, rx, ry, rz, ps.m, bet, betsw, qe, m,
-                           a, kx, ky, kz)) {
-                alive = false; removed = 1; removed_stage = st;
-            }
+            const double dx = xt - ps.x, dy = yt - ps.y, dz = zt - ps.z;
+            const bool outside = VAR == kDustFP64Exact
+                                     ? star_term(dx, dy, dz, rx, ry, rz, ps.m, bet, betsw, qe, m, a, kx, ky, kz)
+                                     : star_term(dx, dy, dz, rx, ry, rz, star, a, kx, ky, kz);
+            if (!outside) { alive = false; removed = 1; removed_stage = st; }
         }
         if (!dust_perturb<VAR>(ms, ng, st, alive, xt, yt, zt, kx, ky, kz, smem)) {
             alive = false; removed = 2; removed_stage = st;
