@@ -511,61 +511,96 @@ enum DustVariant {
     kDustFP64 = 1,       // FP64 with rsqrt
 };
 
-constexpr int kDustThreads = 256;
-constexpr int kDustTile = 1024;    // sources per shared-memory tile (32 KiB)
+// Small blocks spread the tracers evenly: FP64 issue bounds the kernel, so the SM with the most
+// warps sets its time, and 65,536 tracers in blocks of 256 put 512 of them on two thirds of the
+// SMs and 256 on the rest (4,096 planetesimals: 41.1 ms in blocks of 256, 37.5 ms so).
+constexpr int kDustThreads = 64;
+constexpr int kDustTile = 256;     // sources per shared-memory tile (8 KiB)
+// Four lanes share a tracer of the FP64 kernel while that pays for repeating its star term: one
+// thread's chain of sources leaves the FP64 pipe waiting (us a step with one / four lanes: star and
+// 8 planets, 1,000 tracers 56 / 41, 16,384 tracers 57 / 75; 200 planetesimals, 2,000 tracers
+// 518 / 172, 65,536 tracers 1819 / 1750; 4,096 planetesimals, 65,536 tracers 37500 / 34000; 300
+// planetesimals, 262,144 tracers 9540 / 10010).
+constexpr int kLanesMinSources = 128, kLanesFew = 4864, kLanesMany = 131072;
 
 // FP64 gravity of massive bodies 1..n_grav-1 at stage `st` on every tracer of the block.
 // Sources are staged through shared memory tile by tile; every thread of the block takes
 // part in the loads and barriers whether or not its tracer is still alive.
+// kDustFP64 sums source j into partial sum j mod 4, and adds the four in pairs: with T = 4 lanes
+// per tracer each lane has one of them (the butterfly gives every lane the same bits as T = 1).
 // Returns false (for the calling thread) on an exact coincidence with a body.
-template <int VAR>
+template <int VAR, int T>
 __device__ __forceinline__ bool dust_perturb(const MassiveScratch& ms, int ng, int st, bool alive,
                                              double xt, double yt, double zt, double& kx,
                                              double& ky, double& kz, unsigned char* smem) {
     const int nsrc = ng - 1;
     bool ok = true;
-    {
-        Body* sP = reinterpret_cast<Body*>(smem);
-        for (int base = 0; base < nsrc; base += kDustTile) {
-            const int cnt = min(kDustTile, nsrc - base);
-            __syncthreads();
-            for (int k = threadIdx.x; k < cnt; k += blockDim.x)
-                sP[k] = ms.P[st * ms.cap + 1 + base + k];
-            __syncthreads();
-            if (alive && ok) {
-                if (VAR == kDustFP64Exact) {
-                    // src/gpu_functions.cu:722-735, in order, with its early exit.
-                    for (int k = 0; k < cnt; ++k) {
-                        const Body p = sP[k];
-                        const double dx = xt - p.x, dy = yt - p.y, dz = zt - p.z;
-                        const double RR = dx * dx + dy * dy + dz * dz;
-                        if (RR == 0) { ok = false; break; }
-                        const double f = p.m / RR / sqrt(RR);
-                        kx += -f * dx; ky += -f * dy; kz += -f * dz;
-                    }
-                } else {
+    constexpr int kSums = VAR == kDustFP64 && T == 1 ? 4 : 1;
+    double s[kSums][3];
+#pragma unroll
+    for (int q = 0; q < kSums; ++q) s[q][0] = s[q][1] = s[q][2] = 0.0;
+    Body* sP = reinterpret_cast<Body*>(smem);
+    for (int base = 0; base < nsrc; base += kDustTile) {
+        const int cnt = min(kDustTile, nsrc - base);
+        __syncthreads();
+        for (int k = threadIdx.x; k < cnt; k += blockDim.x)
+            sP[k] = ms.P[st * ms.cap + 1 + base + k];
+        __syncthreads();
+        if (!alive || !ok) continue;
+        if (VAR == kDustFP64Exact) {
+            // src/gpu_functions.cu:722-735, in order, with its early exit.
+            for (int k = 0; k < cnt; ++k) {
+                const Body p = sP[k];
+                const double dx = xt - p.x, dy = yt - p.y, dz = zt - p.z;
+                const double RR = dx * dx + dy * dy + dz * dz;
+                if (RR == 0) { ok = false; break; }
+                const double f = p.m / RR / sqrt(RR);
+                kx += -f * dx; ky += -f * dy; kz += -f * dz;
+            }
+        } else {
+            auto add = [&](int k, double (&a)[3]) {
+                const Body p = sP[k];
+                const double dx = p.x - xt, dy = p.y - yt, dz = p.z - zt;
+                const double f = pull64(p.m, fma(dz, dz, fma(dy, dy, dx * dx)));
+                a[0] = fma(f, dx, a[0]); a[1] = fma(f, dy, a[1]); a[2] = fma(f, dz, a[2]);
+            };
+            if (T == 1) {
+                int k = 0;
+                for (; k + 4 <= cnt; k += 4)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) add(k + q, s[q % kSums]);
+#pragma unroll
+                for (int q = 0; q < 3; ++q)
+                    if (k + q < cnt) add(k + q, s[q % kSums]);
+            } else {
 #pragma unroll 4
-                    for (int k = 0; k < cnt; ++k) {
-                        const Body p = sP[k];
-                        const double dx = xt - p.x, dy = yt - p.y, dz = zt - p.z;
-                        const double RR = dx * dx + dy * dy + dz * dz;
-                        const double f = pull64(p.m, RR);
-                        kx = fma(-f, dx, kx); ky = fma(-f, dy, ky); kz = fma(-f, dz, kz);
-                    }
-                }
+                for (int k = threadIdx.x & (T - 1); k < cnt; k += T) add(k, s[0]);
             }
         }
-        if (VAR == kDustFP64 && alive && !(isfinite(kx) && isfinite(ky) && isfinite(kz))) ok = false;
+    }
+    if (VAR == kDustFP64) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            double t = s[0][c];
+            if (T == 1) {
+                t = (s[0][c] + s[1 % kSums][c]) + (s[2 % kSums][c] + s[3 % kSums][c]);
+            } else {
+                t += __shfl_xor_sync(0xffffffffu, t, 1);
+                t += __shfl_xor_sync(0xffffffffu, t, 2);
+            }
+            (c == 0 ? kx : c == 1 ? ky : kz) += t;
+        }
+        if (alive && !(finite64(kx) && finite64(ky) && finite64(kz))) ok = false;
     }
     return ok;
 }
 
-// Full RK4 of one dust tracer per thread (src/gpu_functions.cu:627-943).
-template <int VAR>
-__global__ void __launch_bounds__(kDustThreads)
+// Full RK4 of one dust tracer per thread, or per T = 4 lanes (src/gpu_functions.cu:627-943).
+template <int VAR, int T>
+__global__ void __launch_bounds__(kDustThreads, VAR == kDustFP64 ? 8 : 1)
 dust_rk4_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __restrict__ bins) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) / T;
     const int ng = a.n_grav;
     const int t = ng + i;
     bool alive = false;
@@ -619,7 +654,7 @@ dust_rk4_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __res
                                      : star_term(dx, dy, dz, rx, ry, rz, star, a, kx, ky, kz);
             if (!outside) { alive = false; removed = 1; removed_stage = st; }
         }
-        if (!dust_perturb<VAR>(ms, ng, st, alive, xt, yt, zt, kx, ky, kz, smem)) {
+        if (!dust_perturb<VAR, T>(ms, ng, st, alive, xt, yt, zt, kx, ky, kz, smem)) {
             alive = false; removed = 2; removed_stage = st;
         }
         if (st == 0)      { k1vx = kx; k1vy = ky; k1vz = kz; }
@@ -627,7 +662,7 @@ dust_rk4_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __res
         else if (st == 2) { k3vx = kx; k3vy = ky; k3vz = kz; }
         else              { k4vx = kx; k4vy = ky; k4vz = kz; }
     }
-    if (i >= a.n_dust) return;
+    if (i >= a.n_dust || (T > 1 && (threadIdx.x & (T - 1)))) return;
     if (removed) {
         // src/gpu_functions.cu:878 zeroes N[i] (i is the dust-relative index) on a stage-4
         // sublimation and leaves the grain alive; DDX_MODE_REFERENCE reproduces it.
@@ -745,13 +780,13 @@ int dust_block_threads(int n_dust) {
     static int sm_count[128] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 128) return kDustThreads;
+    if (dev < 0 || dev >= 128) return 256;
     if (sm_count[dev] == 0) {
         int n = 0;
         if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 1;
         sm_count[dev] = n;
     }
-    int threads = kDustThreads;
+    int threads = 256;
     while (threads > 64 && (n_dust + threads - 1) / threads < 2 * sm_count[dev]) threads /= 2;
     return threads;
 }
@@ -759,15 +794,17 @@ int dust_block_threads(int n_dust) {
 cudaError_t launch_dust(const ddx_state& s, const StepArgs& a, const MassiveScratch& ms,
                         const SizeBin* bins, int precision, cudaStream_t st) {
     if (a.n_dust <= 0) return cudaSuccess;
-    const int threads = dust_block_threads(a.n_dust);
-    const int blocks = (a.n_dust + threads - 1) / threads;
+    const int threads = kDustThreads;
     const size_t smem = (size_t)kDustTile * 32;
     if (precision == DDX_PREC_MIXED || precision == DDX_PREC_COMPENSATED) {
         return launch_dust_mixed(s, a, ms, bins, precision, st);
     } else if (a.mode == DDX_MODE_REFERENCE) {
-        dust_rk4_kernel<kDustFP64Exact><<<blocks, threads, smem, st>>>(s, a, ms, bins);
+        dust_rk4_kernel<kDustFP64Exact, 1><<<(a.n_dust + threads - 1) / threads, threads, smem, st>>>(s, a, ms, bins);
+    } else if (a.n_dust <= (a.n_grav > kLanesMinSources ? kLanesMany : kLanesFew)) {
+        const int blocks = (int)((4LL * a.n_dust + threads - 1) / threads);
+        dust_rk4_kernel<kDustFP64, 4><<<blocks, threads, smem, st>>>(s, a, ms, bins);
     } else {
-        dust_rk4_kernel<kDustFP64><<<blocks, threads, smem, st>>>(s, a, ms, bins);
+        dust_rk4_kernel<kDustFP64, 1><<<(a.n_dust + threads - 1) / threads, threads, smem, st>>>(s, a, ms, bins);
     }
     return cudaGetLastError();
 }

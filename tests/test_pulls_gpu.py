@@ -140,3 +140,32 @@ def test_star_and_planetesimals_far_from_the_origin(engine, far):
     e = np.linalg.norm(np.stack([m["v" + c][rows] - f["v" + c][rows] for c in "xyz"]), axis=0)
     v = np.linalg.norm(np.stack([f["v" + c][rows] for c in "xyz"]), axis=0)
     assert (e <= CELLS * s.dt * a + 1e-14 * v + (1e-12 * v if far == 0.0 else 0.0)).all()
+
+
+def test_fp64_lanes_per_tracer_give_the_same_bits(engine):
+    """Four lanes share a tracer of the FP64 step up to 4,864 tracers, or 131,072 with 128 massive
+    bodies and more; the first 50 grains come out the same on either side."""
+    for n_plsml, counts in ((3, (50, 4864, 4865)), (123, (50, 4864, 4865)), (127, (50, 131072, 131073))):
+        s = synth.dusty_ring(n_dust=counts[-1], n_plsml=n_plsml, seed=12, n_steps=1)
+        first = None
+        for n in counts:
+            state = {k: np.asarray(v)[:s.n_grav + n].copy() for k, v in s.state.items()}
+            m = one_step(engine, s, state, abi.DDX_PREC_FP64)
+            got = np.stack([m[c][:s.n_grav + 50] for c in ("x", "y", "z", "vx", "vy", "vz", "N")])
+            first = got if first is None else first
+            np.testing.assert_array_equal(got, first)
+
+
+# massive bodies at the ends of a group of four sources and of a tile of 256
+@pytest.mark.parametrize("n_plsml", [1, 2, 3, 4, 5, 253, 254, 255, 256, 257])
+def test_fp64_tracer_pulls(engine, n_plsml):
+    """Against the same sums in FP64 on the CPU: velocities after one step to 1e-13 (some 50
+    roundings of a sum whose terms are at most the star's pull)."""
+    import oracle.cpu as oc
+    s = heavy_ring(n_plsml, 300)
+    f = one_step(engine, s, s.state, abi.DDX_PREC_FP64)
+    o = oc.step(s.state, s.n_grav, s.dt, s.size_table, s.phys, 1, ref_mode=False)
+    np.testing.assert_array_equal(f["N"] == 0, o["N"] == 0)
+    vf, vo = (np.stack([q["v" + c][s.n_grav:] for c in "xyz"]) for q in (f, o))
+    live = o["N"][s.n_grav:] != 0
+    assert (np.linalg.norm(vf - vo, axis=0) / np.linalg.norm(vo, axis=0))[live].max() < 1e-13
