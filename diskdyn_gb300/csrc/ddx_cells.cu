@@ -545,8 +545,7 @@ __device__ __forceinline__ void kahan_sum(float& S, float& C, float v) {
 __device__ __forceinline__ void p2l(float dx, float dy, float dz, float mass, f2 (&acc)[kAcc], float (&S)[3],
                                     float (&C)[3]) {
     const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    float ri = rsqrt_approx(r2);
-    ri = ri * fmaf(-0.5f * r2, ri * ri, 1.5f);            // one Newton step
+    const float ri = rsqrt_newton(r2);
     const float v = ri * ri, zv = dz * v, ux = dx * v, uy = dy * v, t0 = mass * ri;
     kahan_sum(S[0], C[0], t0 * zv);
     kahan_sum(S[1], C[1], t0 * ux);

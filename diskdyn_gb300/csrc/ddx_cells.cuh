@@ -116,6 +116,16 @@ cudaError_t cells_build(CellScratch* c, const ddx_state& s, const StepArgs& a, c
 cudaError_t launch_dust_cells(const ddx_state& s, const StepArgs& a, const MassiveScratch& ms, const SizeBin* bins,
                               cudaStream_t st);
 
+// x^(-1/2) within an FP32 rounding: rsqrt.approx and one Newton step whose residual 1 - x y^2 is
+// formed with the square's rounding error.  (With a factor near one instead, y (1.5 - x y^2 / 2),
+// the unequal spacing of FP32 on both sides of one made the far pulls of a belt weaker by 3e-9 in
+// the mean, the same for every tracer.)
+__device__ __forceinline__ float rsqrt_newton(float x) {
+    const float y = rsqrt_approx(x), u = y * y;
+    const float e = fmaf(-x, fmaf(y, y, -u), fmaf(-x, u, 1.f));
+    return fmaf(0.5f * y, e, y);
+}
+
 // 1 - beta - beta_sw of a tracer's bin (1 without one), as cell_predict takes it.
 __device__ __forceinline__ float star_reduction(const SizeBin* __restrict__ bins, int id, int n_grid) {
     if (id < 0 || id >= n_grid) return 1.f;

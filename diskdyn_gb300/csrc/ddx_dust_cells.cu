@@ -85,8 +85,7 @@ __device__ __forceinline__ void l2p(const float4* __restrict__ F, float x, float
 __device__ __forceinline__ void m2p(const float4* __restrict__ F, float x, float y, float z, float& ax, float& ay,
                                     float& az) {
     const float r2 = fmaf(x, x, fmaf(y, y, z * z));
-    float ri = rsqrt_approx(r2);
-    ri = ri * fmaf(-0.5f * r2, ri * ri, 1.5f);            // one Newton step
+    const float ri = rsqrt_newton(r2);
     const float v = ri * ri, zv = z * v, ux = x * v, uy = y * v;
     f2 SX = 0, SY = 0, SZ = 0;
     float ex = 1.f, ey = 0.f;
