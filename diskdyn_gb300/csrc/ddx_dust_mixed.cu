@@ -71,6 +71,12 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kTilePairs = 256;                 // pair records per tile (16 KiB)
+// Four lanes share a tracer up to these numbers of tracers, from kLanesMinSources planetesimals on: one
+// thread's chain of pulls then takes longer than four threads' shares with the star term and the
+// sums repeated in each (us a step with one / four lanes; mixed, 900 planetesimals: 2,003 tracers 220 / 174,
+// 6,003 222 / 196, 12,003 231 / 288; compensated, 1,500: 2,003 1202 / 850, 12,003 1163 / 909,
+// 20,003 1169 / 1117, 30,003 1194 / 1367; star and planets alone: 2,003 69 / 71).
+constexpr int kLanesMinSources = 128, kLanesFew = 6144, kLanesFewComp = 16384;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
@@ -377,7 +383,9 @@ __device__ __forceinline__ uint32_t span_bits(const uint32_t* w, int j0, int n) 
 // 8.55 ms at 12 KiB, 8.47 ms at 16 KiB, 8.53 ms at 20 KiB.
 // COMP: the compensated variant, three blocks per SM (80 registers; its float-float pair
 // needs more than 64): 22.75 ms on the dusty ring against 23.0 ms with two blocks of 128.
-template <bool COMP>
+// T = 4: four lanes share a tracer.  Each takes every fourth span of a tile; the spans' sums are then
+// added by all four in span order, so the bits are those of T = 1.
+template <bool COMP, int T>
 __global__ void __launch_bounds__(kThreads, COMP ? 3 : 4)
 dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __restrict__ bins,
                       const int* __restrict__ perm, bool boxes, const int* __restrict__ src) {
@@ -390,7 +398,9 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
     __shared__ uint32_t allcomp[COMP ? kFlagSpans / 32 : 1], nocomp[COMP ? kFlagSpans / 32 : 1];
     BodyPair* const tiles = reinterpret_cast<BodyPair*>(smem);
     const int tid = threadIdx.x;
-    const int slot = blockIdx.x * blockDim.x + tid;   // position in the visiting order
+    const int slot = (blockIdx.x * blockDim.x + tid) / T;   // position in the visiting order
+    const int sub = T > 1 ? tid & (T - 1) : 0, team0 = tid & 31 & ~(T - 1);
+    const unsigned team = T > 1 ? ((1u << T) - 1u) << team0 : 0u;
     const int i = perm && slot < a.n_dust ? perm[slot] : slot;
     const int ng = a.n_grav;
     const int t = ng + i;
@@ -549,7 +559,7 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
             if (!mbar_wait(mb[g & 1], (g >> 1) & 1, a.wait_ns)) { lost = 1; continue; }
             if (tid == 0) in_flight[g & 1] = -1;
             if (!alive) continue;
-            const BodyPair* T = tiles + (g & 1) * kTilePairs;
+            const BodyPair* const T_ = tiles + (g & 1) * kTilePairs;
             const int cnt = min(kTilePairs, npairs - tt * kTilePairs);   // a multiple of kPairSpan
             static_assert(kTilePairs / kPairSpan <= 32, "one mask bit per span of a tile");
             uint32_t fm = 0u, cm = 0u;   // far spans, compensated spans (compensated wins)
@@ -570,7 +580,7 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
                         open &= open - 1;
                         float2 bx, by, bz;
                         float xm;
-                        span_box(T + j * kPairSpan, bx, by, bz, xm);
+                        span_box(T_ + j * kPairSpan, bx, by, bz, xm);
                         if (lane_dist2(bx, by, bz, xh, yh, zh) < __fmul_rn(Dc, Dc)) cm |= 1u << j;
                     }
                 }
@@ -588,33 +598,36 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
                     open &= open - 1;
                     float2 bx, by, bz;
                     float xm;
-                    span_box(T + j * kPairSpan, bx, by, bz, xm);
+                    span_box(T_ + j * kPairSpan, bx, by, bz, xm);
                     if (lane_far(bx, by, bz, xm, xh, yh, zh, own)) fm |= 1u << j;
                 }
             }
-            for (int k = 0; k < cnt; k += kPairSpan) {
+            for (int k0 = 0; k0 < cnt; k0 += T * kPairSpan) {
+                const int k = k0 + sub * kPairSpan;               // this lane's span
+                const f2* ML = COMP ? reinterpret_cast<const f2*>(ms.PM + (size_t)st * ms.pcap + tt * kTilePairs) : nullptr;
+                // span k's pulls again with the near ones, in FP64, added to the acceleration
+                auto with_near = [&](int k, f2& px, f2& py, f2& pz) {
+                    px = py = pz = 0;
+                    near_span<kPairSpan>(T_ + k, 2 * (tt * kTilePairs + k), XH, XL, YH, YL, ZH, ZL, join3(XH, XL, xr),
+                                         join3(YH, YL, yr), join3(ZH, ZL, zr), inv_near, Pn, src, px, py, pz, kx, ky, kz);
+                };
                 f2 px = 0, py = 0, pz = 0;
-                if (COMP && ((cm >> (k / kPairSpan)) & 1u)) {
+                f2 SH[3] = {0, 0, 0}, SL[3] = {0, 0, 0};
+                float mx = 0.f;                                   // largest reciprocal distance of the span
+                const bool mine = T == 1 || k < cnt;
+                const bool ff = COMP && mine && ((cm >> (k / kPairSpan)) & 1u);
+                if (ff) {
                     // float-float span sums, added to the stage's FP64 acceleration
-                    f2 SH[3] = {0, 0, 0}, SL[3] = {0, 0, 0};
-                    const f2* ML = reinterpret_cast<const f2*>(ms.PM + (size_t)st * ms.pcap + tt * kTilePairs + k);
-                    float mx = 0.f;
 #pragma unroll 2
                     for (int u = 0; u < kPairSpan; ++u) {
                         float y0, y1;
-                        pair_ff<false>(T + k + u, __ldg(ML + u), XH, XL, YH, YL, ZH, ZL, SH, SL, inv_near, y0, y1);
+                        pair_ff<false>(T_ + k + u, __ldg(ML + k + u), XH, XL, YH, YL, ZH, ZL, SH, SL, inv_near, y0, y1);
                         mx = fmax3(mx, y0, y1);
                     }
-                    if (mx > inv_near)   // a source within the near radius: its pull in FP64
-                        near_span_ff(T + k, ML, 2 * (tt * kTilePairs + k), XH, XL, YH, YL, ZH, ZL, xr, yr, zr,
-                                     inv_near, Pn, src, SH, SL, kx, ky, kz);
-                    kx += ff_total(SH[0], SL[0]); ky += ff_total(SH[1], SL[1]); kz += ff_total(SH[2], SL[2]);
-                    continue;
-                }
-                if ((fm >> (k / kPairSpan)) & 1u) {
+                } else if (mine && ((fm >> (k / kPairSpan)) & 1u)) {
 #pragma unroll
                     for (int u = 0; u < kPairSpan; ++u) {
-                        const BodyPair* r = T + k + u;
+                        const BodyPair* r = T_ + k + u;
                         const ulonglong2 q0 = *reinterpret_cast<const ulonglong2*>(r->hx);  // hx, hy
                         const ulonglong2 q1 = *reinterpret_cast<const ulonglong2*>(r->hz);  // hz, m
                         const f2 dX = sub2(q0.x, XH), dY = sub2(q0.y, YH), dZ = sub2(q1.x, ZH);
@@ -625,11 +638,10 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
                         const f2 f = mul2(mul2(q1.y, ri), mul2(ri, ri));
                         px = fma2(f, dX, px); py = fma2(f, dY, py); pz = fma2(f, dZ, pz);
                     }
-                } else {
-                    float mx = 0.f;   // largest reciprocal distance of the span
+                } else if (mine) {
 #pragma unroll
                     for (int u = 0; u < kPairSpan; ++u) {
-                        const BodyPair* r = T + k + u;
+                        const BodyPair* r = T_ + k + u;
                         const ulonglong2 q0 = *reinterpret_cast<const ulonglong2*>(r->hx);  // hx, hy
                         const ulonglong2 q1 = *reinterpret_cast<const ulonglong2*>(r->hz);  // hz, m
                         const ulonglong2 q2 = *reinterpret_cast<const ulonglong2*>(r->lx);  // lx, ly
@@ -646,14 +658,47 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
                         const f2 f = mul2(mul2(q1.y, ri), mul2(ri, ri));
                         px = fma2(f, dX, px); py = fma2(f, dY, py); pz = fma2(f, dZ, pz);
                     }
-                    if (mx > inv_near) {   // rare: a source of this span lies within the near radius
-                        px = py = pz = 0;
-                        near_span<kPairSpan>(T + k, 2 * (tt * kTilePairs + k), XH, XL, YH, YL, ZH, ZL, join3(XH, XL, xr),
-                                             join3(YH, YL, yr), join3(ZH, ZL, zr), inv_near, Pn, src, px, py, pz, kx, ky,
-                                             kz);
+                }
+                if (T == 1) {
+                    if (ff) {
+                        if (mx > inv_near)   // a source within the near radius: its pull in FP64
+                            near_span_ff(T_ + k, ML + k, 2 * (tt * kTilePairs + k), XH, XL, YH, YL, ZH, ZL, xr, yr, zr,
+                                         inv_near, Pn, src, SH, SL, kx, ky, kz);
+                        kx += ff_total(SH[0], SL[0]); ky += ff_total(SH[1], SL[1]); kz += ff_total(SH[2], SL[2]);
+                        continue;
+                    }
+                    if (mx > inv_near) with_near(k, px, py, pz);   // rare
+                    ax.add(px); ay.add(py); az.add(pz);
+                    continue;
+                }
+                // the team's spans in order: each one's sum (FP64 or two FP32 lanes) from its lane
+                if (ff) {
+                    px = (f2)__double_as_longlong(ff_total(SH[0], SL[0]));
+                    py = (f2)__double_as_longlong(ff_total(SH[1], SL[1]));
+                    pz = (f2)__double_as_longlong(ff_total(SH[2], SL[2]));
+                }
+                const unsigned nears = __ballot_sync(team, mx > inv_near) >> team0;
+#pragma unroll
+                for (int q = 0; q < T; ++q) {
+                    const int kq = k0 + q * kPairSpan;
+                    if (kq >= cnt) break;
+                    f2 vx_ = __shfl_sync(team, px, team0 + q), vy_ = __shfl_sync(team, py, team0 + q);
+                    f2 vz_ = __shfl_sync(team, pz, team0 + q);
+                    if (COMP && ((cm >> (kq / kPairSpan)) & 1u)) {
+                        double t[3] = {__longlong_as_double((long long)vx_), __longlong_as_double((long long)vy_),
+                                       __longlong_as_double((long long)vz_)};
+                        if ((nears >> q) & 1u) {
+                            f2 H[3], L[3];
+                            near_span_ff(T_ + kq, ML + kq, 2 * (tt * kTilePairs + kq), XH, XL, YH, YL, ZH, ZL, xr, yr, zr,
+                                         inv_near, Pn, src, H, L, kx, ky, kz);
+                            for (int c = 0; c < 3; ++c) t[c] = ff_total(H[c], L[c]);
+                        }
+                        kx += t[0]; ky += t[1]; kz += t[2];
+                    } else {
+                        if ((nears >> q) & 1u) with_near(kq, vx_, vy_, vz_);
+                        ax.add(vx_); ay.add(vy_); az.add(vz_);
                     }
                 }
-                ax.add(px); ay.add(py); az.add(pz);
             }
         }
         if (ntiles > 0) lost = __syncthreads_or(lost);   // block-uniform before branching on it
@@ -681,7 +726,7 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
         }
         return;
     }
-    if (i >= a.n_dust) return;
+    if (i >= a.n_dust || sub != 0) return;
     if (removed) {
         if (removed == 1 && removed_stage == 3 && a.mode == DDX_MODE_REFERENCE) s.N[i] = 0;
         else s.N[t] = 0;
@@ -704,21 +749,23 @@ cudaError_t launch_dust_mixed(const ddx_state& s, const StepArgs& a, const Massi
     if (!comp && ms.cells && ms.dust_order.cap >= a.n_dust && a.n_grav - a.n_exact >= kCellMinSources && a.lose_tile < 0)
         return launch_dust_cells(s, a, ms, bins, st);
     const size_t smem = 2 * (size_t)kTilePairs * sizeof(BodyPair);
+    const bool lanes = a.n_grav - a.n_exact >= kLanesMinSources && a.n_dust <= (comp ? kLanesFewComp : kLanesFew);
+    auto* const kernel = comp ? (lanes ? dust_rk4_mixed_kernel<true, 4> : dust_rk4_mixed_kernel<true, 1>)
+                              : (lanes ? dust_rk4_mixed_kernel<false, 4> : dust_rk4_mixed_kernel<false, 1>);
     static bool attr_set[128] = {};   // the attributes are set once per device
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 128) return cudaErrorInvalidDevice;
     if (!attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(dust_rk4_mixed_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(dust_rk4_mixed_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem);
-        if (e != cudaSuccess) return e;
+        for (const void* f : {(const void*)dust_rk4_mixed_kernel<true, 4>, (const void*)dust_rk4_mixed_kernel<true, 1>,
+                              (const void*)dust_rk4_mixed_kernel<false, 4>, (const void*)dust_rk4_mixed_kernel<false, 1>}) {
+            const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return e;
+        }
         attr_set[dev] = true;
     }
-    const int threads = dust_block_threads(a.n_dust);   // 256 unless the grains are few
-    const int blocks = (a.n_dust + threads - 1) / threads;
+    const int threads = dust_block_threads(lanes ? 4 * a.n_dust : a.n_dust);   // 256 unless the grains are few
+    const int blocks = (int)((a.n_dust * (lanes ? 4LL : 1LL) + threads - 1) / threads);
     // the tracers' visiting order and the spans' boxes, when the context keeps their scratch
     const int* perm = nullptr;
     bool boxes = false;
@@ -735,8 +782,7 @@ cudaError_t launch_dust_mixed(const ddx_state& s, const StepArgs& a, const Massi
     // the source of each pair slot, for the FP64 pulls of near sources: the sources sit in
     // cell order when the step ordered them (massive_prepare), else slot q holds source q
     const int* src = ms.slot && spatial_order_on(a) ? ms.src : nullptr;
-    if (comp) dust_rk4_mixed_kernel<true><<<blocks, threads, smem, st>>>(s, a, ms, bins, perm, boxes, src);
-    else dust_rk4_mixed_kernel<false><<<blocks, threads, smem, st>>>(s, a, ms, bins, perm, boxes, src);
+    kernel<<<blocks, threads, smem, st>>>(s, a, ms, bins, perm, boxes, src);
     return cudaGetLastError();
 }
 

@@ -169,3 +169,30 @@ def test_fp64_tracer_pulls(engine, n_plsml):
     vf, vo = (np.stack([q["v" + c][s.n_grav:] for c in "xyz"]) for q in (f, o))
     live = o["N"][s.n_grav:] != 0
     assert (np.linalg.norm(vf - vo, axis=0) / np.linalg.norm(vo, axis=0))[live].max() < 1e-13
+
+
+# index order and spatial order, few and many spans; four lanes up to 6,144 and 16,384 tracers
+@pytest.mark.parametrize("n_plsml", [127, 128, 300, 1500])
+@pytest.mark.parametrize("prec,counts", [(abi.DDX_PREC_MIXED, (70, 6144, 6145)),
+                                         (abi.DDX_PREC_COMPENSATED, (70, 16384, 16385))])
+def test_span_lanes_per_tracer_give_the_same_bits(engine, prec, counts, n_plsml):
+    s = scattered(n_plsml, counts[-1])
+    ng = s.n_grav
+    first = None
+    for n in counts:
+        state = {k: np.asarray(v)[:ng + n].copy() for k, v in s.state.items()}
+        m = one_step(engine, s, state, prec)
+        got = np.stack([m[c][:ng + 70] for c in ("x", "y", "z", "vx", "vy", "vz", "N")])
+        first = got if first is None else first
+        np.testing.assert_array_equal(got, first)
+
+
+@pytest.mark.parametrize("n_plsml", [127, 128, 129, 511, 512, 513, 1500])
+def test_few_tracers_pulls(engine, n_plsml):
+    s = heavy_ring(n_plsml, 500)
+    f = one_step(engine, s, s.state, abi.DDX_PREC_FP64)
+    rows = np.arange(s.n_grav, s.n_grav + 500)
+    for prec, rel in ((abi.DDX_PREC_MIXED, 2e-6), (abi.DDX_PREC_COMPENSATED, 6e-7)):
+        m = one_step(engine, s, s.state, prec)
+        np.testing.assert_array_equal(m["N"] == 0, f["N"] == 0)
+        check_velocities(s, f, m, rows[f["N"][rows] != 0], rel)
