@@ -422,6 +422,7 @@ int ddx_step_host(ddx_ctx* c, const ddx_host_state* in, ddx_host_state* out, con
             return DDX_ERR_CUDA;
         StepArgs ac = a;
         ac.n_dust = len;
+        ac.after_event = true;
         if (o > 0) ac.lose_tile = -1;
         if (launch_dust(shifted(*s, o), ac, c->ms, c->bins, precision, st) != cudaSuccess) return DDX_ERR_CUDA;
         if (cudaEventRecord(c->ev_comp, st) != cudaSuccess || cudaStreamWaitEvent(c->s_out, c->ev_comp, 0) != cudaSuccess ||

@@ -39,6 +39,7 @@
 #include <complex>
 #include <cstring>
 #include <vector>
+#include "ddx_launch.cuh"
 #include "ddx_cells.cuh"
 #include "ddx_scan.cuh"
 
@@ -197,6 +198,7 @@ constexpr int kSetupThreads = 256;
 __global__ void __launch_bounds__(kSetupThreads)
 cells_setup_kernel(const Body* __restrict__ P, int n_exact, int n_src, int G, unsigned long long* __restrict__ sums,
                    CellGrid* __restrict__ grid) {
+    after_previous();
     __shared__ bool last;
     const Body s = P[0];
     const int k = blockIdx.x * kSetupThreads + threadIdx.x;
@@ -336,6 +338,7 @@ __device__ __forceinline__ void mark_cell(const CellView& v, int set, const Cell
 __global__ void cells_keys_kernel(ddx_state s, StepArgs a, const SizeBin* __restrict__ bins, CellView v,
                                   uint32_t* __restrict__ key, uint32_t* __restrict__ rank,
                                   uint32_t* __restrict__ count) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.n_dust) return;
     const int t = a.n_grav + i;
@@ -372,6 +375,7 @@ __global__ void cells_keys_kernel(ddx_state s, StepArgs a, const SizeBin* __rest
 
 __global__ void cells_scatter_kernel(int n, const uint32_t* __restrict__ key, const uint32_t* __restrict__ rank,
                                      const uint32_t* __restrict__ start, int* __restrict__ perm) {
+    after_previous();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < n) perm[start[key[k]] + rank[k]] = k;
 }
@@ -381,6 +385,7 @@ __global__ void cells_scatter_kernel(int n, const uint32_t* __restrict__ key, co
 // them level by level in shared memory, and follows the last cell up to the top.
 __global__ void __launch_bounds__(1024)
 cells_ancestors_kernel(CellView v) {
+    after_previous();
     __shared__ uint32_t row[2][1024];
     // which level and which chunk of it
     int b = blockIdx.x, level = 0;
@@ -435,6 +440,7 @@ cells_ancestors_kernel(CellView v) {
 // Per stage: the sources in slot order as (high parts, mass) and (low parts), and the boxes of
 // the source groups (a lane per source, high parts).
 __global__ void cells_boxes_kernel(const BodyPair* __restrict__ PP, int pcap, CellView v) {
+    after_previous();
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) / kGroupSrc;             // stage * n_groups + group
     const int u = threadIdx.x % kGroupSrc;
     const unsigned part = ((1u << kGroupSrc) - 1u) << (threadIdx.x & 31 & ~(kGroupSrc - 1));
@@ -510,6 +516,7 @@ __device__ __forceinline__ void set_node(const CellView& v, const CellGrid& g, i
 constexpr int kRootThreads = 256;
 __global__ void __launch_bounds__(kRootThreads)
 cells_roots_kernel(CellView v) {
+    after_previous();
     const int top = v.levels - 1, c = blockIdx.x * kRootThreads + threadIdx.x;   // cell of the top grid
     const CellGrid& g = *v.grid;
     int first = -1;
@@ -610,6 +617,7 @@ __device__ __forceinline__ int level_nodes(const CellView& v, int level, int& fi
 // it is split, and its children.
 __global__ void __launch_bounds__(kNodeThreads)
 cells_split_kernel(CellView v, int level, float near_eta) {
+    after_previous();
     CellGrid& g = *v.grid;
     const int lane = threadIdx.x & 31;
     const bool top = level == v.levels - 1;       // the levels' nodes lie one after the other
@@ -968,6 +976,7 @@ __device__ __forceinline__ void distant_sums(const CellView& v, int stage, int b
 
 __global__ void __launch_bounds__(kNodeThreads, 3)
 cells_far_kernel(CellView v, int distant_blocks) {
+    after_previous();
     union Shared {
         FarShared far;
         DistantShared distant;
@@ -1018,6 +1027,7 @@ constexpr int kForceSplit = kShiftThreads / kCellForce;     // nodes whose force
 
 __global__ void __launch_bounds__(kShiftThreads)
 cells_shift_kernel(CellView v, int level) {
+    after_previous();
     __shared__ __align__(16) float par[kReal][kShiftNodes];    // parents' coefficients, reflected to (+, +, +)
     __shared__ __align__(8) float lam[kShiftNodes][kReal];
     __shared__ int neg[kShiftNodes], parent[kShiftNodes];
@@ -1244,26 +1254,27 @@ cudaError_t cells_build(CellScratch* c, const ddx_state& s, const StepArgs& a, c
     if (e == cudaSuccess) e = cudaMemsetAsync(c->count, 0, 4 * ((size_t)kCellBins + 1), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->sums, 0, 5 * sizeof(unsigned long long) + 4 * (1 + (size_t)v.words) * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
-    cells_setup_kernel<<<(v.n_src + kSetupThreads - 1) / kSetupThreads, kSetupThreads, 0, st>>>(
-        ms.P, a.n_exact, v.n_src, v.G, c->sums, v.grid);
-    cells_boxes_kernel<<<(4 * v.n_groups * kGroupSrc + 127) / 128, 128, 0, st>>>(ms.PP, ms.pcap, v);
+    launch_first(cells_setup_kernel, (v.n_src + kSetupThreads - 1) / kSetupThreads, kSetupThreads, 0, st, ms.P,
+                 a.n_exact,
+                 v.n_src, v.G, c->sums, v.grid);
+    launch_after(cells_boxes_kernel, (4 * v.n_groups * kGroupSrc + 127) / 128, 128, 0, st, ms.PP, ms.pcap, v);
     const int blk = (a.n_dust + 255) / 256;
-    cells_keys_kernel<<<blk, 256, 0, st>>>(s, a, bins, v, o.key, o.rank, c->count);
+    launch_after(cells_keys_kernel, blk, 256, 0, st, s, a, bins, v, o.key, o.rank, c->count);
     e = exclusive_scan(c->count, c->start, (int)kCellBins + 1, c->temp, nullptr, st);
     if (e != cudaSuccess) return e;
-    cells_scatter_kernel<<<blk, 256, 0, st>>>(a.n_dust, o.key, o.rank, c->start, o.perm);
+    launch_after(cells_scatter_kernel, blk, 256, 0, st, a.n_dust, o.key, o.rank, c->start, o.perm);
     int chunks = 0;
     for (int l = 0; l < v.levels; ++l) {
         const int n = cell_dim(v.G, l) / 32;
         chunks += n * n * n;
     }
-    cells_ancestors_kernel<<<dim3(chunks, 3), 1024, 0, st>>>(v);
-    cells_roots_kernel<<<kCellTop * kCellTop * kCellTop / kRootThreads, kRootThreads, 0, st>>>(v);
+    launch_after(cells_ancestors_kernel, dim3(chunks, 3), 1024, 0, st, v);
+    launch_after(cells_roots_kernel, kCellTop * kCellTop * kCellTop / kRootThreads, kRootThreads, 0, st, v);
     for (int l = v.levels - 1; l >= 0; --l)
-        cells_split_kernel<<<608, kNodeThreads, 0, st>>>(v, l, a.near_eta);
+        launch_after(cells_split_kernel, 608, kNodeThreads, 0, st, v, l, a.near_eta);
     const int db = (v.n_src + 4 * kNodeThreads - 1) / (4 * kNodeThreads);
-    cells_far_kernel<<<456, kNodeThreads, 0, st>>>(v, db < kMultiBlocks ? db : kMultiBlocks);
-    for (int l = v.levels - 1; l >= 0; --l) cells_shift_kernel<<<1520, kShiftThreads, 0, st>>>(v, l);
+    launch_after(cells_far_kernel, 456, kNodeThreads, 0, st, v, db < kMultiBlocks ? db : kMultiBlocks);
+    for (int l = v.levels - 1; l >= 0; --l) launch_after(cells_shift_kernel, 1520, kShiftThreads, 0, st, v, l);
     return cudaGetLastError();
 }
 

@@ -38,6 +38,7 @@
 // The order of the tracers inside a bucket depends on the atomics, but nothing written does:
 // every tracer's partners are sorted by j, and a segment cut by the buffer's end keeps the
 // smallest j, so the output is the first cap pairs of the ordered list.
+#include "ddx_launch.cuh"
 #include "ddx_internal.cuh"
 #include "ddx_scan.cuh"
 
@@ -143,6 +144,7 @@ __device__ __forceinline__ long long half_cell(double x, double inv2, float inv2
 __global__ void keys_kernel(ddx_state s, int i0, int n, double inv2, float inv2f, uint32_t mask, uint32_t sentinel,
                             uint32_t* __restrict__ bsize, uint32_t* __restrict__ bucket, uint32_t* __restrict__ rank,
                             unsigned long long* __restrict__ cellid, uint32_t* __restrict__ count) {
+    after_previous();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     const int idx = i0 + p;
@@ -165,6 +167,7 @@ __global__ void keys_kernel(ddx_state s, int i0, int n, double inv2, float inv2f
 __global__ void scatter_kernel(ddx_state s, int i0, int n, uint32_t sentinel, const uint32_t* __restrict__ bucket,
                                const uint32_t* __restrict__ rank, const unsigned long long* __restrict__ cellid,
                                uint4* table, CellRec* __restrict__ rec, uint32_t* __restrict__ vals) {
+    after_previous();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     const uint32_t b = bucket[p];
@@ -216,6 +219,7 @@ __global__ void write_kernel(const CellRec* __restrict__ rec, const uint32_t* __
                              double h2, float hf, uint32_t mask, const uint32_t* __restrict__ count,
                              const int* __restrict__ slots, const uint32_t* __restrict__ offs,
                              int2* __restrict__ pairs, long long cap) {
+    after_previous();
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;   // bucket order
     if (q >= *n_live) return;
     const uint32_t p = vals[q];
@@ -327,6 +331,7 @@ __global__ void __launch_bounds__(kCountThreads, 4) count_kernel(const CellRec* 
                                                               const uint32_t* __restrict__ n_live, int i0, double h2,
                                                               float hf, uint32_t mask, uint32_t* __restrict__ count,
                                                               int* __restrict__ slots) {
+    after_previous();
     __shared__ uint8_t queue[kCountThreads / 32][256];
     __shared__ uint32_t found[kCountThreads];
     const uint32_t FULL = 0xffffffffu;
@@ -517,17 +522,19 @@ int collide_run(CollideScratch*& cs, const ddx_state& s, int i0, int i1, double 
     uint32_t* n_live = cs->total;
     uint32_t* n_found = cs->total + 1;
     cudaMemsetAsync(cs->bsize, 0, 4ull * T, st);
-    keys_kernel<<<blk, thr, 0, st>>>(s, i0, n, inv2, (float)inv2, mask, sentinel, cs->bsize, cs->bucket, cs->rank, cs->cellid,
+    launch_first(keys_kernel, blk, thr, 0, st, s, i0, n, inv2, (float)inv2, mask, sentinel, cs->bsize, cs->bucket,
+                 cs->rank, cs->cellid,
                                      cs->count);
     // entries {start, size, lin of the first two cells (written by the scatter)}
     if (exclusive_scan_table(cs->bsize, cs->table, (int)T, cs->temp, n_live, st) != cudaSuccess) return DDX_ERR_CUDA;
-    scatter_kernel<<<blk, thr, 0, st>>>(s, i0, n, sentinel, cs->bucket, cs->rank, cs->cellid, cs->table, cs->rec,
+    launch_after(scatter_kernel, blk, thr, 0, st, s, i0, n, sentinel, cs->bucket, cs->rank, cs->cellid, cs->table,
+                 cs->rec,
                                         cs->vals);
-    count_kernel<<<(n + kCountThreads - 1) / kCountThreads, kCountThreads, 0, st>>>(
-        cs->rec, cs->vals, cs->table, n_live, i0, h2, hf, mask, cs->count, cs->slots);
+    launch_after(count_kernel, (n + kCountThreads - 1) / kCountThreads, kCountThreads, 0, st, cs->rec, cs->vals,
+                 cs->table, n_live, i0, h2, hf, mask, cs->count, cs->slots);
     if (exclusive_scan(cs->count, cs->offs, n, cs->temp, n_found, st) != cudaSuccess) return DDX_ERR_CUDA;
     if (pairs && cap > 0)
-        write_kernel<<<blk, thr, 0, st>>>(cs->rec, cs->vals, cs->table, n_live, i0, h2, hf, mask, cs->count,
+        launch_after(write_kernel, blk, thr, 0, st, cs->rec, cs->vals, cs->table, n_live, i0, h2, hf, mask, cs->count,
                                                 cs->slots, cs->offs, pairs, cap);
     if (cudaGetLastError() != cudaSuccess) return DDX_ERR_CUDA;
     uint32_t tot = 0;

@@ -14,6 +14,7 @@
 // a million tracers 1575 -> 1515 us, 3,001 planetesimals with 30,000 tracers 234 -> 171 us).
 // A tracer outside every grid, with a non-finite position, or further from its cell's centre
 // than kReach edges (it moved more in the step than expected) takes every planetesimal.
+#include "ddx_launch.cuh"
 #include "ddx_cells.cuh"
 #include "ddx_pull.cuh"
 
@@ -341,6 +342,7 @@ template <int T>
 __global__ void __launch_bounds__(kThreads, 8)
 dust_cells_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __restrict__ bins,
                   const int* __restrict__ perm, CellView v, const int* __restrict__ src) {
+    after_previous();
     __shared__ double held[qKept][kThreads];
     const Column col{(uint32_t)__cvta_generic_to_shared(&held[0][threadIdx.x])};
     const int slot = (blockIdx.x * blockDim.x + threadIdx.x) / T;
@@ -459,9 +461,9 @@ cudaError_t launch_dust_cells(const ddx_state& s, const StepArgs& a, const Massi
     const int* const src = ms.slot ? ms.src : nullptr;
     const int lanes = a.n_dust < kLanes8 ? 8 : a.n_dust < kLanes4 ? 4 : 1;
     const int blocks = (int)(((long long)a.n_dust * lanes + kThreads - 1) / kThreads);
-    if (lanes == 8) dust_cells_kernel<8><<<blocks, kThreads, 0, st>>>(s, a, ms, bins, perm, v, src);
-    else if (lanes == 4) dust_cells_kernel<4><<<blocks, kThreads, 0, st>>>(s, a, ms, bins, perm, v, src);
-    else dust_cells_kernel<1><<<blocks, kThreads, 0, st>>>(s, a, ms, bins, perm, v, src);
+    if (lanes == 8) launch_first(dust_cells_kernel<8>, blocks, kThreads, 0, st, s, a, ms, bins, perm, v, src);
+    else if (lanes == 4) launch_first(dust_cells_kernel<4>, blocks, kThreads, 0, st, s, a, ms, bins, perm, v, src);
+    else launch_first(dust_cells_kernel<1>, blocks, kThreads, 0, st, s, a, ms, bins, perm, v, src);
     return cudaGetLastError();
 }
 

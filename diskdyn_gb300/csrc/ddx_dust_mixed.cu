@@ -61,6 +61,7 @@
 // still take the exact FP64 pull inside those spans.  The per-span choice is made like the
 // far-span choice (block box first, then per tracer), so a tracer's result again depends
 // only on its own state and the massive set.
+#include "ddx_launch.cuh"
 #include "ddx_internal.cuh"
 #include "ddx_f32x2.cuh"
 #include "ddx_cells.cuh"
@@ -215,6 +216,7 @@ __device__ __forceinline__ void pair_ff(const BodyPair* r, f2 ml, f2 XH, f2 XL, 
 // never counts as far).
 // One warp per (stage, span): lane u reads source slot u of the span's 32.
 __global__ void span_box_kernel(BodyPair* __restrict__ PP, int pcap, int n_src, int nspans) {
+    after_previous();
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;   // stage * nspans + span
     const int u = threadIdx.x & 31;
     if (k >= 4 * nspans) return;                                   // whole warps leave together
@@ -389,6 +391,7 @@ template <bool COMP, int T>
 __global__ void __launch_bounds__(kThreads, COMP ? 3 : 4)
 dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __restrict__ bins,
                       const int* __restrict__ perm, bool boxes, const int* __restrict__ src) {
+    after_previous();
     constexpr int NB = COMP ? 8 : 7;              // box values: 3 x (min, max), largest own[, smallest own]
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) unsigned long long mbar[2];
@@ -775,14 +778,15 @@ cudaError_t launch_dust_mixed(const ddx_state& s, const StepArgs& a, const Massi
             order_bodies(s, a.n_grav, a.n_dust, true, ms.dust_order, ms.dust_order.perm, nullptr, !comp, st);
         if (e != cudaSuccess) return e;
         const int nspans = pair_count(n_src) / kPairSpan;
-        span_box_kernel<<<(4 * nspans * 32 + 127) / 128, 128, 0, st>>>(ms.PP, ms.pcap, n_src, nspans);
+        launch_after(span_box_kernel, (4 * nspans * 32 + 127) / 128, 128, 0, st, ms.PP, ms.pcap, n_src, nspans);
         perm = ms.dust_order.perm;
         boxes = true;
     }
     // the source of each pair slot, for the FP64 pulls of near sources: the sources sit in
     // cell order when the step ordered them (massive_prepare), else slot q holds source q
     const int* src = ms.slot && spatial_order_on(a) ? ms.src : nullptr;
-    kernel<<<blocks, threads, smem, st>>>(s, a, ms, bins, perm, boxes, src);
+    launch_with(a.n_grav <= kOverlapDust && !a.after_event, kernel, blocks, threads, smem, st, s, a, ms, bins, perm,
+                boxes, src);
     return cudaGetLastError();
 }
 

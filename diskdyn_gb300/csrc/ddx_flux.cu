@@ -13,6 +13,7 @@
 // farther than the guard width from a pixel edge the floor is the same.  Tracers inside
 // the guard band take the reference's exact expression sequence, so every pixel index is
 // identical to the reference kernel's on the same GPU.
+#include "ddx_launch.cuh"
 #include "ddx_internal.cuh"
 #include "ddx_flux.cuh"
 
@@ -21,6 +22,7 @@ namespace ddx {
 // Constants of one view, computed on the device with the device math library so that
 // every quantity the reference recomputes per thread has the same bits here.
 __global__ void view_setup_kernel(ViewConst* vc, ddx_view v, int n_theta) {
+    after_previous();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     ViewConst c;
     c.dist = v.dist;
@@ -179,6 +181,7 @@ __device__ __forceinline__ void phase_bracket(double cossc, int ntheta, int& cos
 __global__ void __launch_bounds__(256)
 image_kernel(ddx_state s, int n_grav, int n_dust, const ViewConst* __restrict__ vcp,
              OpticsDev o, ImageList il, double* __restrict__ Fd, unsigned long long* __restrict__ nexact) {
+    after_previous();
     __shared__ ViewConst v;
     __shared__ WaveFactor wf[kMaxImages];
     if (threadIdx.x == 0) v = *vcp;
@@ -230,6 +233,7 @@ image_kernel(ddx_state s, int n_grav, int n_dust, const ViewConst* __restrict__ 
 // outside the image) and whether the exact reference sequence decided it.
 __global__ void pixel_kernel(ddx_state s, int n_grav, int n_dust, const ViewConst* __restrict__ vcp,
                              int* __restrict__ pix, int* __restrict__ exact) {
+    after_previous();
     __shared__ ViewConst v;
     if (threadIdx.x == 0) v = *vcp;
     __syncthreads();
@@ -283,6 +287,7 @@ int sed_slices(int n_wav) {
 __global__ void __launch_bounds__(kSedMaxThreads)
 sed_partial_kernel(ddx_state s, int n_grav, int n_dust, const ViewConst* __restrict__ vcp,
                    OpticsDev o, int mode, int S, double* __restrict__ partial) {
+    after_previous();
     __shared__ ViewConst v;
     __shared__ double inv_T[kSedBatch], wts[kSedBatch], gt[kSedBatch], gs[kSedBatch], part[kSedMaxThreads];
     __shared__ size_t row[kSedBatch];
@@ -362,6 +367,7 @@ sed_partial_kernel(ddx_state s, int n_grav, int n_dust, const ViewConst* __restr
 constexpr int kFinalWarps = 32;
 __global__ void __launch_bounds__(32 * kFinalWarps)
 sed_final_kernel(const double* __restrict__ partial, int nblocks, int n_wav, double* __restrict__ Fsed) {
+    after_previous();
     __shared__ double part[kFinalWarps][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = blockIdx.x * 32 + lane;
     double s = 0.0;
@@ -414,7 +420,7 @@ cudaError_t launch_optics_prepare(OpticsDev& o, OpticsDev* o_dev, cudaStream_t s
 cudaError_t launch_image(const ddx_state& s, int n_grav, int n_dust, const ddx_view& view,
                          const OpticsDev& o, const ImageList& il, ViewConst* vc, double* Fd,
                          unsigned long long* nexact, cudaStream_t st) {
-    view_setup_kernel<<<1, 32, 0, st>>>(vc, view, o.n_theta);
+    launch_first(view_setup_kernel, 1, 32, 0, st, vc, view, o.n_theta);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const size_t npix = (size_t)view.xsize * view.ysize;
@@ -423,21 +429,21 @@ cudaError_t launch_image(const ddx_state& s, int n_grav, int n_dust, const ddx_v
     if (n_dust <= 0) return cudaSuccess;
     const int threads = 256;
     const int blocks = (n_dust + threads - 1) / threads;
-    image_kernel<<<blocks, threads, 0, st>>>(s, n_grav, n_dust, vc, o, il, Fd, nexact);
+    launch_after(image_kernel, blocks, threads, 0, st, s, n_grav, n_dust, vc, o, il, Fd, nexact);
     return cudaGetLastError();
 }
 
 cudaError_t launch_view_setup(ViewConst* vc, const ddx_view& view, int n_theta, cudaStream_t st) {
-    view_setup_kernel<<<1, 32, 0, st>>>(vc, view, n_theta);
+    launch_first(view_setup_kernel, 1, 32, 0, st, vc, view, n_theta);
     return cudaGetLastError();
 }
 
 cudaError_t launch_pixels(const ddx_state& s, int n_grav, int n_dust, const ddx_view& view,
                           int n_theta, ViewConst* vc, int* pix, int* exact, cudaStream_t st) {
-    view_setup_kernel<<<1, 32, 0, st>>>(vc, view, n_theta);
+    launch_first(view_setup_kernel, 1, 32, 0, st, vc, view, n_theta);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || n_dust <= 0) return e;
-    pixel_kernel<<<(n_dust + 255) / 256, 256, 0, st>>>(s, n_grav, n_dust, vc, pix, exact);
+    launch_after(pixel_kernel, (n_dust + 255) / 256, 256, 0, st, s, n_grav, n_dust, vc, pix, exact);
     return cudaGetLastError();
 }
 
@@ -652,6 +658,7 @@ __device__ __forceinline__ float flux32(const Tracer32& t, const float2* lq2, co
 // At, As, C2, esh for the wavelength slots of one call: one block per slot.
 __global__ void photo_prepare_kernel(OpticsDev o, const ViewConst* __restrict__ vcp, ImageList il, int use_list,
                                      PhotoConst pc) {
+    after_previous();
     __shared__ double smax[256];
     const int j = blockIdx.x;
     const int J = use_list ? il.wj[j] : j;
@@ -702,6 +709,7 @@ __global__ void __launch_bounds__(256)
 image_mixed_kernel(ddx_state s, int n_grav, int n_dust, const ViewConst* __restrict__ vcp, View32 v32, OpticsDev o,
                    ImageList il, PhotoConst pc, float* __restrict__ Fi, int K4,
                    unsigned long long* __restrict__ counters) {
+    after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     bool valid = false;
@@ -810,6 +818,7 @@ image_mixed_kernel(ddx_state s, int n_grav, int n_dust, const ViewConst* __restr
 // Fd[k][pixel] = Fi[pixel][k] 2^-esh[k] (an exact power-of-two scaling).
 __global__ void image_convert_kernel(const float* __restrict__ Fi, int K4, int n_img, size_t npix,
                                      const int* __restrict__ esh, double* __restrict__ Fd) {
+    after_previous();
     const size_t pix = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (pix >= npix) return;
     const float4* row = reinterpret_cast<const float4*>(Fi + pix * K4);
@@ -833,6 +842,7 @@ constexpr int kSedChunks = 8;   // wavelengths per pass: 32 * kSedChunks
 __global__ void __launch_bounds__(kSedThreads, 3)
 sed_mixed_kernel(ddx_state s, int n_grav, int n_dust, View32 v32, OpticsDev o,
                  PhotoConst pc, int mode, int lam0, double* __restrict__ partial) {
+    after_previous();
     __shared__ double red[kSedThreads / 32][32 * kSedChunks];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int gw = blockIdx.x * (kSedThreads / 32) + warp, nw = gridDim.x * (kSedThreads / 32);
@@ -923,14 +933,14 @@ int sed_mixed_blocks(int n_dust) {
 cudaError_t launch_photo_prepare(const OpticsDev& o, const ViewConst* vc, const ImageList* il,
                                  PhotoConst pc, cudaStream_t st) {
     ImageList none{};
-    photo_prepare_kernel<<<pc.n_lam, 256, 0, st>>>(o, vc, il ? *il : none, il ? 1 : 0, pc);
+    launch_after(photo_prepare_kernel, pc.n_lam, 256, 0, st, o, vc, il ? *il : none, il ? 1 : 0, pc);
     return cudaGetLastError();
 }
 
 cudaError_t launch_image_mixed(const ddx_state& s, int n_grav, int n_dust, const ddx_view& view,
                                const OpticsDev& o, const ImageList& il, ViewConst* vc, PhotoConst pc,
                                double* Fd, float* Fi, unsigned long long* counters, cudaStream_t st) {
-    view_setup_kernel<<<1, 32, 0, st>>>(vc, view, o.n_theta);
+    launch_first(view_setup_kernel, 1, 32, 0, st, vc, view, o.n_theta);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     pc.n_lam = il.n;
@@ -939,16 +949,17 @@ cudaError_t launch_image_mixed(const ddx_state& s, int n_grav, int n_dust, const
     const int K4 = image_k4(il.n);
     if ((e = cudaMemsetAsync(Fi, 0, sizeof(float) * npix * K4, st)) != cudaSuccess) return e;
     if (n_dust > 0)
-        image_mixed_kernel<<<(n_dust + 255) / 256, 256, 0, st>>>(s, n_grav, n_dust, vc, make_view32(view, o), o, il,
+        launch_after(image_mixed_kernel, (n_dust + 255) / 256, 256, 0, st, s, n_grav, n_dust, vc, make_view32(view,
+                     o), o, il,
                                                                  pc, Fi, K4, counters);
-    image_convert_kernel<<<(unsigned)((npix + 255) / 256), 256, 0, st>>>(Fi, K4, il.n, npix, pc.esh, Fd);
+    launch_after(image_convert_kernel, (unsigned)((npix + 255) / 256), 256, 0, st, Fi, K4, il.n, npix, pc.esh, Fd);
     return cudaGetLastError();
 }
 
 cudaError_t launch_sed_mixed(const ddx_state& s, int n_grav, int n_dust, const ddx_view& view,
                              const OpticsDev& o, ViewConst* vc, PhotoConst pc, double* partial, int mode,
                              double* Fsed, cudaStream_t st) {
-    view_setup_kernel<<<1, 32, 0, st>>>(vc, view, o.n_theta);
+    launch_first(view_setup_kernel, 1, 32, 0, st, vc, view, o.n_theta);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     pc.n_lam = o.n_wav;
@@ -956,26 +967,26 @@ cudaError_t launch_sed_mixed(const ddx_state& s, int n_grav, int n_dust, const d
     const int nb = sed_mixed_blocks(n_dust);
     const View32 v32 = make_view32(view, o);
     for (int lam0 = 0; lam0 < o.n_wav; lam0 += 32 * kSedChunks) {
-        sed_mixed_kernel<<<nb, kSedThreads, 0, st>>>(s, n_grav, n_dust, v32, o, pc, mode, lam0, partial);
+        launch_after(sed_mixed_kernel, nb, kSedThreads, 0, st, s, n_grav, n_dust, v32, o, pc, mode, lam0, partial);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    sed_final_kernel<<<(o.n_wav + 31) / 32, 32 * kFinalWarps, 0, st>>>(partial, nb, o.n_wav, Fsed);
+    launch_after(sed_final_kernel, (o.n_wav + 31) / 32, 32 * kFinalWarps, 0, st, partial, nb, o.n_wav, Fsed);
     return cudaGetLastError();
 }
 
 cudaError_t launch_sed(const ddx_state& s, int n_grav, int n_dust, const ddx_view& view,
                        const OpticsDev& o, ViewConst* vc, double* partial, int mode,
                        double* Fsed, cudaStream_t st) {
-    view_setup_kernel<<<1, 32, 0, st>>>(vc, view, o.n_theta);
+    launch_first(view_setup_kernel, 1, 32, 0, st, vc, view, o.n_theta);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const int nb = sed_blocks(n_dust);
     const int S = sed_slices(o.n_wav), items = S * o.n_wav;
     const int threads = items > kSedMaxThreads ? kSedMaxThreads : (items + 31) / 32 * 32;
-    sed_partial_kernel<<<nb, threads, 0, st>>>(s, n_grav, n_dust, vc, o, mode, S, partial);
+    launch_after(sed_partial_kernel, nb, threads, 0, st, s, n_grav, n_dust, vc, o, mode, S, partial);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    sed_final_kernel<<<(o.n_wav + 31) / 32, 32 * kFinalWarps, 0, st>>>(partial, nb, o.n_wav, Fsed);
+    launch_after(sed_final_kernel, (o.n_wav + 31) / 32, 32 * kFinalWarps, 0, st, partial, nb, o.n_wav, Fsed);
     return cudaGetLastError();
 }
 

@@ -37,6 +37,7 @@ struct StepArgs {
     int    mode;            // DDX_MODE_*
     int    lose_tile;       // test hook: tile whose copy is never issued (-1: none)
     unsigned long long wait_ns;   // bound on any one device-side wait
+    bool   after_event = false;   // the dust launch follows an event wait: keep the stream's full order
     float  near_eta;        // mixed path: an FP32 source nearer to a body than near_eta times the
                             // body's largest |coordinate| takes the FP64 pair force instead (0: none)
     float  comp_eta;        // compensated path: spans nearer to a tracer than comp_eta times its

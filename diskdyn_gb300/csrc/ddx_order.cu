@@ -29,6 +29,7 @@
 //    digits of its tile, digit-major; an exclusive scan gives every (digit, block) its first
 //    output slot; the scatter ranks equal digits inside a warp with __match_any_sync and
 //    orders warps and rounds by counts in shared memory.  Both give the same order.
+#include "ddx_launch.cuh"
 #include "ddx_internal.cuh"
 #include "ddx_scan.cuh"
 
@@ -51,6 +52,7 @@ __device__ __forceinline__ bool removed(const ddx_state& s, int i) {
 }
 
 __global__ void order_init_kernel(uint32_t* __restrict__ count, int* __restrict__ box) {
+    after_previous();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k <= kOrderBins) count[k] = 0;
     if (k < 3) {
@@ -62,6 +64,7 @@ __global__ void order_init_kernel(uint32_t* __restrict__ count, int* __restrict_
 // Bounding box of the bodies' FP32 positions (NaN left out): a block reduction, then one
 // atomic per block and bound.
 __global__ void order_box_kernel(ddx_state s, int first, int n, bool dead_last, int* __restrict__ box) {
+    after_previous();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     if (k < n && !(dead_last && removed(s, first + k))) {
@@ -162,6 +165,7 @@ constexpr int kSmallThreads = 1024;
 __global__ void __launch_bounds__(kSmallThreads)
 order_small_keys_kernel(ddx_state s, int first, int n, bool dead_last, bool hilbert, uint32_t* __restrict__ key,
                         int* __restrict__ pos) {
+    after_previous();
     __shared__ float red[kSmallThreads / 32][6];
     __shared__ float box[6];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -211,6 +215,7 @@ order_small_keys_kernel(ddx_state s, int first, int n, bool dead_last, bool hilb
 constexpr int kRankKeys = 1024;
 __global__ void __launch_bounds__(kThreads)
 order_small_rank_kernel(int n, const uint32_t* __restrict__ key, int* __restrict__ pos) {
+    after_previous();
     __shared__ __align__(16) uint32_t other[kRankKeys];
     const int k = blockIdx.x * kThreads + threadIdx.x, j0 = blockIdx.y * kRankKeys;
     for (int j = threadIdx.x; j < kRankKeys; j += kThreads) other[j] = j0 + j < n ? key[j0 + j] : 0xFFFFFFFFu;
@@ -226,6 +231,7 @@ order_small_rank_kernel(int n, const uint32_t* __restrict__ key, int* __restrict
 }
 
 __global__ void order_from_pos_kernel(int n, const int* __restrict__ pos, int* __restrict__ perm) {
+    after_previous();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < n) perm[pos[k]] = k;
 }
@@ -237,6 +243,7 @@ __global__ void order_keys_kernel(ddx_state s, int first, int n, bool dead_last,
                                   const int* __restrict__ box,
                                   uint32_t* __restrict__ key, uint32_t* __restrict__ rank,
                                   uint32_t* __restrict__ count) {
+    after_previous();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     uint32_t bin = 1u << (3 * bits);
@@ -252,6 +259,7 @@ __global__ void order_keys_kernel(ddx_state s, int first, int n, bool dead_last,
 
 __global__ void hist_kernel(const uint32_t* __restrict__ keys, int n, int shift, uint32_t* __restrict__ hist,
                             int nblocks) {
+    after_previous();
     __shared__ uint32_t cnt[256];
     cnt[threadIdx.x] = 0;
     __syncthreads();
@@ -267,6 +275,7 @@ __global__ void hist_kernel(const uint32_t* __restrict__ keys, int n, int shift,
 __global__ void radix_scatter_kernel(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
                                      uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, int n, int shift,
                                      const uint32_t* __restrict__ offs, int nblocks) {
+    after_previous();
     __shared__ uint32_t wcnt[kThreads / 32][257];
     __shared__ uint32_t run[256];
     __shared__ uint32_t gofs[256];
@@ -326,10 +335,10 @@ cudaError_t radix_sort_stable(uint32_t* keys, uint32_t* vals, int n, int key_bit
     uint32_t* v2 = k2 + n;
     uint32_t *ka = keys, *va = vals, *kb = k2, *vb = v2;
     for (int shift = 0; shift < key_bits; shift += 8) {
-        hist_kernel<<<nb, kThreads, 0, st>>>(ka, n, shift, hist, nb);
+        launch_after(hist_kernel, nb, kThreads, 0, st, ka, n, shift, hist, nb);
         const cudaError_t e = exclusive_scan(hist, offs, nh, stmp, nullptr, st);
         if (e != cudaSuccess) return e;
-        radix_scatter_kernel<<<nb, kThreads, 0, st>>>(ka, va, kb, vb, n, shift, offs, nb);
+        launch_after(radix_scatter_kernel, nb, kThreads, 0, st, ka, va, kb, vb, n, shift, offs, nb);
         uint32_t* tk = ka; ka = kb; kb = tk;
         uint32_t* tv = va; va = vb; vb = tv;
     }
@@ -340,6 +349,7 @@ cudaError_t radix_sort_stable(uint32_t* keys, uint32_t* vals, int n, int key_bit
 
 __global__ void order_from_sorted_kernel(int n, const uint32_t* __restrict__ sorted, int* __restrict__ perm,
                                          int* __restrict__ inv) {
+    after_previous();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     const uint32_t k = sorted[p];
@@ -350,6 +360,7 @@ __global__ void order_from_sorted_kernel(int n, const uint32_t* __restrict__ sor
 __global__ void order_scatter_kernel(int n, const uint32_t* __restrict__ key, const uint32_t* __restrict__ rank,
                                      const uint32_t* __restrict__ start, int* __restrict__ perm,
                                      int* __restrict__ inv) {
+    after_previous();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const uint32_t pos = start[key[k]] + rank[k];
@@ -388,30 +399,32 @@ cudaError_t order_bodies(const ddx_state& s, int first, int n, bool dead_last, c
     if (n > o.cap) return cudaErrorInvalidValue;
     if (o.stable && n <= kSmallOrder) {
         int* const pos = inv ? inv : reinterpret_cast<int*>(o.rank);
-        order_small_keys_kernel<<<1, kSmallThreads, 0, st>>>(s, first, n, dead_last, hilbert, o.key, pos);
-        order_small_rank_kernel<<<dim3((n + kThreads - 1) / kThreads, (n + kRankKeys - 1) / kRankKeys), kThreads, 0, st>>>(
-            n, o.key, pos);
-        if (perm) order_from_pos_kernel<<<(n + kThreads - 1) / kThreads, kThreads, 0, st>>>(n, pos, perm);
+        launch_first(order_small_keys_kernel, 1, kSmallThreads, 0, st, s, first, n, dead_last, hilbert, o.key, pos);
+        launch_after(order_small_rank_kernel, dim3((n + kThreads - 1) / kThreads, (n + kRankKeys - 1) / kRankKeys),
+                     kThreads, 0, st, n, o.key, pos);
+        if (perm) launch_after(order_from_pos_kernel, (n + kThreads - 1) / kThreads, kThreads, 0, st, n, pos, perm);
         return cudaGetLastError();
     }
     const int blk = (n + kThreads - 1) / kThreads;
-    order_init_kernel<<<(kOrderBins + 1 + kThreads - 1) / kThreads, kThreads, 0, st>>>(o.count, o.box);
-    order_box_kernel<<<blk, kThreads, 0, st>>>(s, first, n, dead_last, o.box);
+    launch_first(order_init_kernel, (kOrderBins + 1 + kThreads - 1) / kThreads, kThreads, 0, st, o.count, o.box);
+    launch_after(order_box_kernel, blk, kThreads, 0, st, s, first, n, dead_last, o.box);
     if (o.stable) {
         constexpr int kBits = kOrderBits - 1;   // 32^3 cells: two 8-bit digit passes
-        order_keys_kernel<<<blk, kThreads, 0, st>>>(s, first, n, dead_last, kBits, hilbert, o.box, o.key, o.rank,
+        launch_after(order_keys_kernel, blk, kThreads, 0, st, s, first, n, dead_last, kBits, hilbert, o.box, o.key,
+                     o.rank,
                                                     nullptr);
         uint32_t *ko = nullptr, *vo = nullptr;
         cudaError_t e = radix_sort_stable(o.key, o.rank, n, 3 * kBits + 1, o.temp, &ko, &vo, st);
         if (e != cudaSuccess) return e;
-        order_from_sorted_kernel<<<blk, kThreads, 0, st>>>(n, vo, perm, inv);
+        launch_after(order_from_sorted_kernel, blk, kThreads, 0, st, n, vo, perm, inv);
         return cudaGetLastError();
     }
-    order_keys_kernel<<<blk, kThreads, 0, st>>>(s, first, n, dead_last, kOrderBits, hilbert, o.box, o.key, o.rank,
+    launch_after(order_keys_kernel, blk, kThreads, 0, st, s, first, n, dead_last, kOrderBits, hilbert, o.box, o.key,
+                 o.rank,
                                                 o.count);
     cudaError_t e = exclusive_scan(o.count, o.start, (int)kOrderBins + 1, o.temp, nullptr, st);
     if (e != cudaSuccess) return e;
-    order_scatter_kernel<<<blk, kThreads, 0, st>>>(n, o.key, o.rank, o.start, perm, inv);
+    launch_after(order_scatter_kernel, blk, kThreads, 0, st, n, o.key, o.rank, o.start, perm, inv);
     return cudaGetLastError();
 }
 

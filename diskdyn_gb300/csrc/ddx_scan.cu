@@ -9,6 +9,7 @@
 // and store instruction of a warp then covers 512 contiguous bytes of the counts (one 16-byte
 // vector per lane) or 2,048 contiguous bytes of the bucket table, every sector written in
 // full.
+#include "ddx_launch.cuh"
 #include "ddx_scan.cuh"
 
 namespace ddx {
@@ -53,6 +54,7 @@ __device__ __forceinline__ void load_items(const uint32_t* __restrict__ in, long
 }
 
 __global__ void scan_sums_kernel(const uint32_t* __restrict__ in, long long n, bool vec, uint32_t* __restrict__ sums) {
+    after_previous();
     uint32_t v[16];
     load_items(in, n, (long long)blockIdx.x * kTile, vec, v);
     uint32_t s = 0;
@@ -72,6 +74,7 @@ __global__ void scan_sums_kernel(const uint32_t* __restrict__ in, long long n, b
 
 // One block scans the tile sums (a sequential chunk per thread).
 __global__ void scan_top_kernel(uint32_t* __restrict__ sums, int nb, uint32_t* __restrict__ total) {
+    after_previous();
     const int per = (nb + kThreads - 1) / kThreads;
     const int b0 = threadIdx.x * per;
     uint32_t s = 0;
@@ -97,6 +100,7 @@ __global__ void scan_top_kernel(uint32_t* __restrict__ sums, int nb, uint32_t* _
 template <bool TABLE>
 __global__ void scan_apply_kernel(const uint32_t* __restrict__ in, long long n, bool vec,
                                   const uint32_t* __restrict__ sums, void* __restrict__ out) {
+    after_previous();
     const long long t0 = (long long)blockIdx.x * kTile;
     uint32_t v[16];
     load_items(in, n, t0, vec, v);
@@ -147,12 +151,12 @@ cudaError_t scan(const uint32_t* in, void* out, bool table, int n, uint32_t* tem
     if (n <= 0) return total ? cudaMemsetAsync(total, 0, sizeof(uint32_t), st) : cudaSuccess;
     const int nb = (n + kTile - 1) / kTile;
     const bool vin = aligned16(in);
-    scan_sums_kernel<<<nb, kThreads, 0, st>>>(in, n, vin, temp);
-    scan_top_kernel<<<1, kThreads, 0, st>>>(temp, nb, total);
+    launch_after(scan_sums_kernel, nb, kThreads, 0, st, in, n, vin, temp);
+    launch_after(scan_top_kernel, 1, kThreads, 0, st, temp, nb, total);
     if (table)
-        scan_apply_kernel<true><<<nb, kThreads, 0, st>>>(in, n, vin, temp, out);
+        launch_after(scan_apply_kernel<true>, nb, kThreads, 0, st, in, n, vin, temp, out);
     else
-        scan_apply_kernel<false><<<nb, kThreads, 0, st>>>(in, n, vin && aligned16(out), temp, out);
+        launch_after(scan_apply_kernel<false>, nb, kThreads, 0, st, in, n, vin && aligned16(out), temp, out);
     return cudaGetLastError();
 }
 

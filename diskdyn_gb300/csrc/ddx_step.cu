@@ -14,6 +14,7 @@
 // pass 2 evaluates A3 (at P3) and A4 (at P4).  The reference issues 4*(num+1)+4 launches
 // per step with CAS atomics; here it is prepare + pass1 + pass2 + dust, deterministic, with
 // no atomics.
+#include "ddx_launch.cuh"
 #include "ddx_internal.cuh"
 #include "ddx_f32x2.cuh"
 
@@ -65,6 +66,7 @@ static MassiveScratch slotted(const MassiveScratch& ms, const StepArgs& a) {
 
 // P1 = x, P2 = x + v dt/2 (src/gpu_functions.cu:90-99, 219-230).
 __global__ void massive_prepare_kernel(ddx_state s, StepArgs a, MassiveScratch ms, int prec) {
+    after_previous();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.n_grav) return;
     const double x = s.x[i], y = s.y[i], z = s.z[i], m = s.m[i];
@@ -217,6 +219,7 @@ __device__ __forceinline__ void pass1_update(const ddx_state& s, const StepArgs&
 // FP32 records its dust kernel reads).
 template <int PREC, int STORE = PREC>
 __global__ void massive_pass1_kernel(ddx_state s, StepArgs a, MassiveScratch ms) {
+    after_previous();
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (i >= a.n_grav) return;  // warp-uniform
     double acc[6];
@@ -247,6 +250,7 @@ __device__ __forceinline__ void pass2_update(const ddx_state& s, const StepArgs&
 
 template <int PREC>
 __global__ void massive_pass2_kernel(ddx_state s, StepArgs a, MassiveScratch ms) {
+    after_previous();
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (i >= a.n_grav) return;
     double acc[6];
@@ -376,6 +380,7 @@ struct SliceTarget {
 
 __global__ void __launch_bounds__(kSliceWorkers)
 massive_slice_kernel(StepArgs a, MassiveScratch ms, int sa, int per, int np, double* __restrict__ part) {
+    after_previous();
     __shared__ __align__(16) BodyPair tile[kSliceTile];
     const int k = blockIdx.y, st = sa + blockIdx.z;
     const int n_src = a.n_grav - a.n_exact;
@@ -462,6 +467,7 @@ template <int PASS>
 __global__ void __launch_bounds__(kGatherThreads)
 massive_gather_kernel(ddx_state s, StepArgs a, MassiveScratch ms, int slices, int np,
                       const double* __restrict__ part) {
+    after_previous();
     constexpr int kWarps = kGatherThreads / 32;
     __shared__ double sums[kWarps][6][kGatherTargets];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -599,6 +605,7 @@ __device__ __forceinline__ bool dust_perturb(const MassiveScratch& ms, int ng, i
 template <int VAR, int T>
 __global__ void __launch_bounds__(kDustThreads, VAR == kDustFP64 ? 8 : 1)
 dust_rk4_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __restrict__ bins) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem[];
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) / T;
     const int ng = a.n_grav;
@@ -688,7 +695,8 @@ dust_rk4_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __res
 cudaError_t launch_massive_prepare(const ddx_state& s, const StepArgs& a, MassiveScratch& ms,
                                    int precision, cudaStream_t st) {
     // the FP32 sources' pair slots in cell order, from their positions at the start of the step
-    if (precision != DDX_PREC_FP64 && ms.slot && spatial_order_on(a)) {
+    const bool ordered = precision != DDX_PREC_FP64 && ms.slot && spatial_order_on(a);
+    if (ordered) {
         const cudaError_t e =
             order_bodies(s, a.n_exact, a.n_grav - a.n_exact, false, ms.src_order, nullptr, ms.slot,
                          precision == DDX_PREC_MIXED, st);
@@ -696,7 +704,7 @@ cudaError_t launch_massive_prepare(const ddx_state& s, const StepArgs& a, Massiv
     }
     const int threads = 128;
     const int blocks = (a.n_grav + threads - 1) / threads;
-    massive_prepare_kernel<<<blocks, threads, 0, st>>>(s, a, slotted(ms, a), precision);
+    launch_with(ordered, massive_prepare_kernel, blocks, threads, 0, st, s, a, slotted(ms, a), precision);
     return cudaGetLastError();
 }
 
@@ -730,10 +738,11 @@ cudaError_t launch_sliced(const ddx_state& s, const StepArgs& a, MassiveScratch&
     if (S > 0) {
         const int per = (spans + S - 1) / S * kPairSpan;
         const dim3 grid((a.n_grav + kSliceThreads - 1) / kSliceThreads + 1, S, 2);   // + the star's row; two stages
-        massive_slice_kernel<<<grid, kSliceWorkers, 0, st>>>(a, slotted(ms, a), PASS == 1 ? 0 : 2, per, np, ms.part);
+        launch_with(a.n_grav <= kOverlapPasses, massive_slice_kernel, grid, kSliceWorkers, 0, st, a, slotted(ms, a),
+                    PASS == 1 ? 0 : 2, per, np, ms.part);
     }
-    massive_gather_kernel<PASS><<<(a.n_grav + kGatherTargets - 1) / kGatherTargets, kGatherThreads, 0, st>>>(
-        s, a, slotted(ms, a), S, np, ms.part);
+    launch_after(massive_gather_kernel<PASS>, (a.n_grav + kGatherTargets - 1) / kGatherTargets, kGatherThreads, 0, st,
+                 s, a, slotted(ms, a), S, np, ms.part);
     return cudaGetLastError();
 }
 }  // namespace
@@ -756,10 +765,12 @@ cudaError_t launch_massive_pass1(const ddx_state& s, const StepArgs& a, MassiveS
     const int threads = 128;  // 4 targets per block
     const int blocks = (a.n_grav * 32 + threads - 1) / threads;
     if (precision == DDX_PREC_COMPENSATED)   // the massive set in FP64
-        massive_pass1_kernel<DDX_PREC_FP64, DDX_PREC_MIXED><<<blocks, threads, 0, st>>>(s, a, slotted(ms, a));
+        launch_with(a.n_grav <= kOverlapPasses, (massive_pass1_kernel<DDX_PREC_FP64, DDX_PREC_MIXED>), blocks,
+                    threads, 0, st, s, a, slotted(ms, a));
     else if (precision == DDX_PREC_MIXED)
-        massive_pass1_kernel<DDX_PREC_MIXED><<<blocks, threads, 0, st>>>(s, a, slotted(ms, a));
-    else massive_pass1_kernel<DDX_PREC_FP64><<<blocks, threads, 0, st>>>(s, a, ms);
+        launch_with(a.n_grav <= kOverlapPasses, massive_pass1_kernel<DDX_PREC_MIXED>, blocks, threads, 0, st, s, a,
+                    slotted(ms, a));
+    else launch_with(a.n_grav <= kOverlapPasses, massive_pass1_kernel<DDX_PREC_FP64>, blocks, threads, 0, st, s, a, ms);
     return cudaGetLastError();
 }
 
@@ -769,10 +780,11 @@ cudaError_t launch_massive_pass2(const ddx_state& s, const StepArgs& a, MassiveS
     const int threads = 128;
     const int blocks = (a.n_grav * 32 + threads - 1) / threads;
     if (precision == DDX_PREC_COMPENSATED)
-        massive_pass2_kernel<DDX_PREC_FP64><<<blocks, threads, 0, st>>>(s, a, ms);
+        launch_with(a.n_grav <= kOverlapPasses, massive_pass2_kernel<DDX_PREC_FP64>, blocks, threads, 0, st, s, a, ms);
     else if (precision == DDX_PREC_MIXED)
-        massive_pass2_kernel<DDX_PREC_MIXED><<<blocks, threads, 0, st>>>(s, a, slotted(ms, a));
-    else massive_pass2_kernel<DDX_PREC_FP64><<<blocks, threads, 0, st>>>(s, a, ms);
+        launch_with(a.n_grav <= kOverlapPasses, massive_pass2_kernel<DDX_PREC_MIXED>, blocks, threads, 0, st, s, a,
+                    slotted(ms, a));
+    else launch_with(a.n_grav <= kOverlapPasses, massive_pass2_kernel<DDX_PREC_FP64>, blocks, threads, 0, st, s, a, ms);
     return cudaGetLastError();
 }
 
@@ -795,16 +807,19 @@ cudaError_t launch_dust(const ddx_state& s, const StepArgs& a, const MassiveScra
                         const SizeBin* bins, int precision, cudaStream_t st) {
     if (a.n_dust <= 0) return cudaSuccess;
     const int threads = kDustThreads;
+    const bool overlap = a.n_grav <= kOverlapDust && !a.after_event;
     const size_t smem = (size_t)kDustTile * 32;
     if (precision == DDX_PREC_MIXED || precision == DDX_PREC_COMPENSATED) {
         return launch_dust_mixed(s, a, ms, bins, precision, st);
     } else if (a.mode == DDX_MODE_REFERENCE) {
-        dust_rk4_kernel<kDustFP64Exact, 1><<<(a.n_dust + threads - 1) / threads, threads, smem, st>>>(s, a, ms, bins);
+        launch_with(overlap, (dust_rk4_kernel<kDustFP64Exact, 1>), (a.n_dust + threads - 1) / threads, threads, smem,
+                    st, s, a, ms, bins);
     } else if (a.n_dust <= (a.n_grav > kLanesMinSources ? kLanesMany : kLanesFew)) {
         const int blocks = (int)((4LL * a.n_dust + threads - 1) / threads);
-        dust_rk4_kernel<kDustFP64, 4><<<blocks, threads, smem, st>>>(s, a, ms, bins);
+        launch_with(overlap, (dust_rk4_kernel<kDustFP64, 4>), blocks, threads, smem, st, s, a, ms, bins);
     } else {
-        dust_rk4_kernel<kDustFP64, 1><<<(a.n_dust + threads - 1) / threads, threads, smem, st>>>(s, a, ms, bins);
+        launch_with(overlap, (dust_rk4_kernel<kDustFP64, 1>), (a.n_dust + threads - 1) / threads, threads, smem, st,
+                    s, a, ms, bins);
     }
     return cudaGetLastError();
 }
