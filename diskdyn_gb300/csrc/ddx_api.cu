@@ -647,18 +647,25 @@ int ddx_image(ddx_ctx* c, const ddx_state* s, int n_grav, int n_dust, const ddx_
     }
     DeviceGuard dg(c->device);
     if (precision == DDX_PREC_MIXED) {
-        const size_t need = (size_t)view->xsize * view->ysize * image_k4(n_img);
-        if (need > c->img32_words) {
+        // the sums, then the wavelengths' table rows where there is room for them
+        const size_t sums = (size_t)view->xsize * view->ysize * image_k4(n_img), rows = image_row_words(c->od, n_img);
+        if (sums + rows > c->img32_words) {
             cudaFree(c->img32);
             c->img32 = nullptr;
             c->img32_words = 0;
+            size_t need = sums + rows;
             if (dalloc(&c->img32, need) != cudaSuccess) {
                 cudaGetLastError();
-                return DDX_ERR_NOMEM;
+                need = sums;
+                if (dalloc(&c->img32, need) != cudaSuccess) {
+                    cudaGetLastError();
+                    return DDX_ERR_NOMEM;
+                }
             }
             c->img32_words = need;
         }
-        return cuda_status(launch_image_mixed(*s, n_grav, n_dust, *view, c->od, il, c->vc, c->photo, Fd, c->img32,
+        float2* const at = rows && c->img32_words >= sums + rows ? reinterpret_cast<float2*>(c->img32 + sums) : nullptr;
+        return cuda_status(launch_image_mixed(*s, n_grav, n_dust, *view, c->od, il, c->vc, c->photo, Fd, c->img32, at,
                                               c->counters, (cudaStream_t)stream));
     }
     return cuda_status(launch_image(*s, n_grav, n_dust, *view, c->od, il, c->vc, Fd, c->counters,

@@ -694,6 +694,26 @@ __global__ void photo_prepare_kernel(OpticsDev o, const ViewConst* __restrict__ 
     }
 }
 
+// The image wavelengths' columns of the phase table side by side, rows[bin, angle][K4]: a tracer
+// then reads its wavelengths from neighbouring sectors instead of one sector each, which
+// bounded image_mixed_kernel (2,097,152 tracers, ten images of 512 x 400: 182 -> 139 us).  A thread per
+// entry.
+__global__ void image_rows_kernel(OpticsDev o, ImageList il, int K4, float2* __restrict__ rows) {
+    after_previous();
+    const int n = o.n_grid * (o.n_theta - 1) * K4;
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+        const int row = e / K4, k = e - row * K4;
+        rows[e] = k < il.n ? o.lQp32p[(size_t)row * o.n_wav + il.wj[k]] : make_float2(0.f, 0.f);
+    }
+}
+// From this many tracers on: below, the tables' launch costs what the rows save (ten images, us with / without:
+// 60,000 tracers 38 / 42 at best and 38 / 36 at worst, 200,000 43 / 53, 500,000 55 / 71).
+constexpr int kRowTracers = 100000;
+size_t image_row_words(const OpticsDev& o, int n_img) {
+    const size_t n = (size_t)o.n_grid * (o.n_theta - 1) * image_k4(n_img);
+    return n < (1u << 27) ? 2 * n : 0;
+}
+
 // Images, mixed precision: one thread per tracer, every image wavelength in one pass.  The
 // sums go to an FP32 buffer interleaved by wavelength, Fi[pixel][K4] (K4 = n_img rounded up
 // to 4), in the wavelengths' scaled domain (2^esh), as 16-byte vector atomics: one request
@@ -705,9 +725,10 @@ __global__ void photo_prepare_kernel(OpticsDev o, const ViewConst* __restrict__ 
 // The gain grows with the tracers per pixel that sit next to each other in the state (all
 // of them when the tracers are stored in pixel order).
 // image_convert_kernel then writes the FP64 x-major images.
+template <bool ROWS>
 __global__ void __launch_bounds__(256)
 image_mixed_kernel(ddx_state s, int n_grav, int n_dust, const ViewConst* __restrict__ vcp, View32 v32, OpticsDev o,
-                   ImageList il, PhotoConst pc, float* __restrict__ Fi, int K4,
+                   ImageList il, PhotoConst pc, const float2* __restrict__ rows, float* __restrict__ Fi, int K4,
                    unsigned long long* __restrict__ counters) {
     after_previous();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -770,7 +791,8 @@ image_mixed_kernel(ddx_state s, int n_grav, int n_dust, const ViewConst* __restr
             if (lane + (1 << k) < 32 && so == seg) take |= 1u << k;
         }
     }
-    const float2* lq2 = valid ? o.lQp32p + ((size_t)tr.id * (o.n_theta - 1) + tr.cm) * o.n_wav : nullptr;
+    const size_t at = valid ? (size_t)tr.id * (o.n_theta - 1) + tr.cm : 0;
+    const float2* lq2 = ROWS ? rows + at * K4 : o.lQp32p + at * o.n_wav;
     const float2* A = valid ? pc.A + (size_t)tr.id * pc.n_lam : nullptr;
     float* row = Fi + pix * K4;
     // eight wavelengths at a time, their table loads issued together before the arithmetic
@@ -781,7 +803,13 @@ image_mixed_kernel(ddx_state s, int n_grav, int n_dust, const ViewConst* __restr
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
                 const int k = g + u;
-                lv[u] = k < il.n ? lq2[il.wj[k]] : make_float2(0.f, 0.f);
+                if (!ROWS) {
+                    lv[u] = k < il.n ? lq2[il.wj[k]] : make_float2(0.f, 0.f);
+                } else if (u % 2 == 0) {
+                    const float4 q = k < K4 ? *reinterpret_cast<const float4*>(lq2 + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    lv[u] = make_float2(q.x, q.y);
+                    lv[u + 1] = make_float2(q.z, q.w);
+                }
                 av[u] = k < il.n ? A[k] : make_float2(0.f, 0.f);
             }
 #pragma unroll
@@ -939,7 +967,7 @@ cudaError_t launch_photo_prepare(const OpticsDev& o, const ViewConst* vc, const 
 
 cudaError_t launch_image_mixed(const ddx_state& s, int n_grav, int n_dust, const ddx_view& view,
                                const OpticsDev& o, const ImageList& il, ViewConst* vc, PhotoConst pc,
-                               double* Fd, float* Fi, unsigned long long* counters, cudaStream_t st) {
+                               double* Fd, float* Fi, float2* rows, unsigned long long* counters, cudaStream_t st) {
     launch_first(view_setup_kernel, 1, 32, 0, st, vc, view, o.n_theta);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -948,10 +976,11 @@ cudaError_t launch_image_mixed(const ddx_state& s, int n_grav, int n_dust, const
     const size_t npix = (size_t)view.xsize * view.ysize;
     const int K4 = image_k4(il.n);
     if ((e = cudaMemsetAsync(Fi, 0, sizeof(float) * npix * K4, st)) != cudaSuccess) return e;
+    if (n_dust < kRowTracers) rows = nullptr;
+    if (rows) launch_after(image_rows_kernel, 608, 256, 0, st, o, il, K4, rows);
     if (n_dust > 0)
-        launch_after(image_mixed_kernel, (n_dust + 255) / 256, 256, 0, st, s, n_grav, n_dust, vc, make_view32(view,
-                     o), o, il,
-                                                                 pc, Fi, K4, counters);
+        launch_after(rows ? image_mixed_kernel<true> : image_mixed_kernel<false>, (n_dust + 255) / 256, 256, 0, st, s,
+                     n_grav, n_dust, vc, make_view32(view, o), o, il, pc, rows, Fi, K4, counters);
     launch_after(image_convert_kernel, (unsigned)((npix + 255) / 256), 256, 0, st, Fi, K4, il.n, npix, pc.esh, Fd);
     return cudaGetLastError();
 }

@@ -47,9 +47,11 @@ cudaError_t launch_photo_prepare(const OpticsDev& o, const ViewConst* vc, const 
                                  PhotoConst pc, cudaStream_t st);
 // Mixed images: Fi is an FP32 scratch of npix * image_k4(n_img) floats (256-byte aligned).
 inline int image_k4(int n_img) { return (n_img + 3) / 4 * 4; }
+// 32-bit words of the rows scratch of launch_image_mixed, which takes null as well (0: none).
+size_t image_row_words(const OpticsDev& o, int n_img);
 cudaError_t launch_image_mixed(const ddx_state& s, int n_grav, int n_dust, const ddx_view& view,
                                const OpticsDev& o, const ImageList& il, ViewConst* vc, PhotoConst pc,
-                               double* Fd, float* Fi, unsigned long long* counters, cudaStream_t st);
+                               double* Fd, float* Fi, float2* rows, unsigned long long* counters, cudaStream_t st);
 cudaError_t launch_sed_mixed(const ddx_state& s, int n_grav, int n_dust, const ddx_view& view,
                              const OpticsDev& o, ViewConst* vc, PhotoConst pc, double* partial, int mode,
                              double* Fsed, cudaStream_t st);
