@@ -35,6 +35,7 @@
 // one rsqrt per body per stage, and the reverse reuses them from the record.
 // Tracers removed during the forward (N = 0) or without optical data emit nothing, so
 // their adjoint is zero and they are skipped.
+#include <type_traits>
 #include "ddx_internal.cuh"
 #include "ddx_flux.cuh"
 
@@ -44,7 +45,10 @@ namespace {
 // Massive sets up to this size run the one-warp kernels (every step in one launch); larger
 // ones the launch-per-pass kernels of the "large massive sets" section.
 constexpr int kMaxGrav = 32;
-constexpr int kThreads = 128;
+// FP64 issue bounds the dust kernels, so the SM with the most warps sets their time: 65,536 tracers
+// over 50 steps take 9.35 ms in blocks of 128 threads, 8.90 ms in 64 and 8.79 ms in 32, which doubles
+// the blocks' sums once more.
+constexpr int kThreads = 64;
 constexpr int kWarps = kThreads / 32;
 constexpr int kSegComp = 15;   // per tracer per step: x, y, z, vx, vy, vz, a1, a2, a3
 constexpr int kMaxStoredIr = 3; // bodies whose 1/|e| the recompute keeps (n_grav <= 4)
@@ -107,7 +111,7 @@ __device__ __forceinline__ bool tracer_accel(const AdjArgs& A, const StarConst& 
     for (int j = 1; j < A.ng; ++j) {
         const double ex = P[j].x - x, ey = P[j].y - y, ez = P[j].z - z;
         const double R2 = ex * ex + ey * ey + ez * ez;
-        if (R2 == 0.0) return false;
+        if (((unsigned long long)__double_as_longlong(R2) << 1) == 0) return false;
         const double ir = rsqrt64(R2);
         if (rc && j <= A.nir) rc[(1 + j) * rs] = ir;
         const double f = P[j].m * (ir * ir * ir);
@@ -132,6 +136,32 @@ __device__ __forceinline__ void massive_acc(const double (*sp)[4], int ng, int j
             ax += f * dx; ay += f * dy; az += f * dz;
         }
     }
+}
+
+// Up to kPairBodies bodies every ordered pair (j, k) has a lane of the warp, lane j ng + k, and lane j
+// adds its ng results: half the FP64 instructions of a lane per body, whose sequence
+// is the time of these one-warp kernels (three bodies, 50 steps: trajectory 447 -> 341 us, reverse
+// 536 -> 303 us a 25 steps).
+constexpr int kPairBodies = 5;
+
+__device__ __forceinline__ double pair_sum(double v, int ng) {
+    double t = 0.0;
+    for (int k = 0; k < ng; ++k) t += __shfl_sync(0xffffffffu, v, (threadIdx.x * ng + k) & 31);
+    return t;
+}
+// Every lane of the warp calls it; lanes j < ng get body j's acceleration.
+__device__ __forceinline__ void massive_acc_pairs(const double (*sp)[4], int ng, double& ax, double& ay, double& az) {
+    const int j = threadIdx.x / ng, k = threadIdx.x - j * ng;
+    double vx = 0.0, vy = 0.0, vz = 0.0;
+    if (j < ng && j != k) {
+        const double dx = sp[k][0] - sp[j][0], dy = sp[k][1] - sp[j][1], dz = sp[k][2] - sp[j][2];
+        const double RR = dx * dx + dy * dy + dz * dz;
+        if (positive64(RR)) {
+            const double f = pull64(sp[k][3], RR);
+            vx = f * dx; vy = f * dy; vz = f * dz;
+        }
+    }
+    ax = pair_sum(vx, ng); ay = pair_sum(vy, ng); az = pair_sum(vz, ng);
 }
 
 __global__ void massive_traj_kernel(int ng, int n_steps, double dt, double* xv, Body* Ps) {
@@ -162,8 +192,9 @@ __global__ void massive_traj_kernel(int ng, int n_steps, double dt, double* xv, 
             __syncwarp();
             if (on) { sp[j][0] = px[s]; sp[j][1] = py[s]; sp[j][2] = pz[s]; sp[j][3] = m; }
             __syncwarp();
+            if (ng <= kPairBodies) massive_acc_pairs(sp, ng, ax[s], ay[s], az[s]);
+            else if (on) massive_acc(sp, ng, j, ax[s], ay[s], az[s]);
             if (on) {
-                massive_acc(sp, ng, j, ax[s], ay[s], az[s]);
                 Ps[((size_t)n * 4 + s) * ng + j] = make_body(px[s], py[s], pz[s], m);
             }
         }
@@ -182,26 +213,30 @@ __global__ void massive_traj_kernel(int ng, int n_steps, double dt, double* xv, 
 
 // Vector-Jacobian product of the all-pairs accelerations at one stage for body j:
 // out_j = sum_k J_jk (m_j g_k - m_k g_j), J(d) v = v/r^3 - 3 (d.v) d/r^5, and the mass
-// adjoint sum_k g_k.(P_j - P_k)/r^3.
-__device__ __forceinline__ void massive_vjp(const double (*sp)[4], const double (*sg)[3], int ng, int j,
-                                            double& ox, double& oy, double& oz, double& om) {
-    ox = oy = oz = om = 0.0;
+// adjoint sum_k g_k.(P_j - P_k)/r^3.  This adds the term of k.
+__device__ __forceinline__ void massive_vjp_pair(const double (*sp)[4], const double (*sg)[3], int j, int k,
+                                                 double& ox, double& oy, double& oz, double& om) {
     const double mj = sp[j][3];
-    for (int k = 0; k < ng; ++k) {
-        if (k == j) continue;
-        const double dx = sp[j][0] - sp[k][0], dy = sp[j][1] - sp[k][1], dz = sp[j][2] - sp[k][2];
-        const double RR = dx * dx + dy * dy + dz * dz;
-        if (!positive64(RR)) continue;
-        const double ri = rsqrt64(RR), ri2 = ri * ri, ri3 = ri * ri2, ri5 = ri3 * ri2;
-        const double vx = mj * sg[k][0] - sp[k][3] * sg[j][0];
-        const double vy = mj * sg[k][1] - sp[k][3] * sg[j][1];
-        const double vz = mj * sg[k][2] - sp[k][3] * sg[j][2];
-        const double dv = dx * vx + dy * vy + dz * vz;
-        ox += vx * ri3 - 3.0 * dv * dx * ri5;
-        oy += vy * ri3 - 3.0 * dv * dy * ri5;
-        oz += vz * ri3 - 3.0 * dv * dz * ri5;
-        om += (sg[k][0] * dx + sg[k][1] * dy + sg[k][2] * dz) * ri3;
-    }
+    const double dx = sp[j][0] - sp[k][0], dy = sp[j][1] - sp[k][1], dz = sp[j][2] - sp[k][2];
+    const double RR = dx * dx + dy * dy + dz * dz;
+    if (!positive64(RR)) return;
+    const double ri = rsqrt64(RR), ri2 = ri * ri, ri3 = ri * ri2, ri5 = ri3 * ri2;
+    const double vx = mj * sg[k][0] - sp[k][3] * sg[j][0];
+    const double vy = mj * sg[k][1] - sp[k][3] * sg[j][1];
+    const double vz = mj * sg[k][2] - sp[k][3] * sg[j][2];
+    const double dv = 3.0 * (dx * vx + dy * vy + dz * vz) * ri5;
+    ox += vx * ri3 - dv * dx;
+    oy += vy * ri3 - dv * dy;
+    oz += vz * ri3 - dv * dz;
+    om += (sg[k][0] * dx + sg[k][1] * dy + sg[k][2] * dz) * ri3;
+}
+// For every body at once, as massive_acc_pairs.
+__device__ __forceinline__ void massive_vjp_pairs(const double (*sp)[4], const double (*sg)[3], int ng, double& ox,
+                                                  double& oy, double& oz, double& om) {
+    const int j = threadIdx.x / ng, k = threadIdx.x - j * ng;
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    if (j < ng && j != k) massive_vjp_pair(sp, sg, j, k, v[0], v[1], v[2], v[3]);
+    ox = pair_sum(v[0], ng); oy = pair_sum(v[1], ng); oz = pair_sum(v[2], ng); om = pair_sum(v[3], ng);
 }
 
 __global__ void massive_reverse_kernel(int ng, double dt, const Body* Ps, const double* mu, int n0, int n1,
@@ -237,8 +272,11 @@ __global__ void massive_reverse_kernel(int ng, double dt, const Body* Ps, const 
             }
             __syncwarp();
             double ox = 0, oy = 0, oz = 0, om = 0;
+            if (ng <= kPairBodies) massive_vjp_pairs(sp, sg, ng, ox, oy, oz, om);
+            else if (on)
+                for (int q = 0; q < ng; ++q)
+                    if (q != j) massive_vjp_pair(sp, sg, j, q, ox, oy, oz, om);
             if (on) {
-                massive_vjp(sp, sg, ng, j, ox, oy, oz, om);
                 const double* m4 = mu + (((size_t)k * 4 + s) * ng + j) * 4;
                 LP[0] = ox + m4[0]; LP[1] = oy + m4[1]; LP[2] = oz + m4[2];
                 lm += om + m4[3];
@@ -823,12 +861,21 @@ dust_reverse_step_kernel(AdjArgs A, const double* __restrict__ seg, int k, int n
         for (int c = 0; c < 3; ++c) { lam[c * nd + i] = Lx[c]; lam[(3 + c) * nd + i] = Lv[c]; }
 }
 
-// mu[k][s][j][c] = sum over blocks of part[b][k][s][j][c], in block order.
-__global__ void reduce_parts_kernel(const double* __restrict__ part, int nblk, int per_block, double* __restrict__ mu) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= per_block) return;
+// mu[k][s][j][c] = sum over blocks of part[b][k][s][j][c]: 32 values per block, warp w adds blocks
+// w, w + kPartWarps, ..., the warps' sums are added in warp order (512 blocks, 25 steps of three
+// bodies: 66 us with a thread per value, 9 us so).
+constexpr int kPartWarps = 16;
+__global__ void __launch_bounds__(32 * kPartWarps)
+reduce_parts_kernel(const double* __restrict__ part, int nblk, int per_block, double* __restrict__ mu) {
+    __shared__ double sums[kPartWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
     double t = 0.0;
-    for (int b = 0; b < nblk; ++b) t += part[(size_t)b * per_block + e];
+    if (e < per_block)
+        for (int b = warp; b < nblk; b += kPartWarps) t += part[(size_t)b * per_block + e];
+    sums[warp][lane] = t;
+    __syncthreads();
+    if (warp != 0 || e >= per_block) return;
+    for (int w = 1; w < kPartWarps; ++w) t += sums[w][lane];
     mu[e] = t;
 }
 
@@ -1048,7 +1095,11 @@ struct AdjointScratch {
     ddx_view view{};
     ImageList il{};
     bool ready = false;
-    // buffers
+    // one block of memory, kept for the next forward of a like size (allocating and freeing it on
+    // every call cost 0.5 ms of 10.8 with 65,536 tracers over 50 steps), and the parts of it
+    char* arena = nullptr;
+    size_t cap = 0;
+    cudaEvent_t used = nullptr;           // the last forward's or backward's work on it
     double *xv_m = nullptr, *y0 = nullptr, *y = nullptr, *N0 = nullptr, *N = nullptr, *ck = nullptr,
            *seg = nullptr, *lam = nullptr, *part = nullptr, *mu = nullptr, *lam_m = nullptr, *lam_mass = nullptr;
     int* idv = nullptr;
@@ -1057,17 +1108,20 @@ struct AdjointScratch {
     unsigned char* active = nullptr;
     Body* Ps = nullptr;
     ViewConst* vc = nullptr;
-    size_t bytes = 0;
 };
 
 void adjoint_free(AdjointScratch*& a) {
     if (!a) return;
-    cudaFree(a->xv_m); cudaFree(a->y0); cudaFree(a->y); cudaFree(a->N0); cudaFree(a->N); cudaFree(a->ck);
-    cudaFree(a->seg); cudaFree(a->lam); cudaFree(a->part); cudaFree(a->mu); cudaFree(a->lam_m);
-    cudaFree(a->lam_mass); cudaFree(a->idv); cudaFree(a->active); cudaFree(a->Ps); cudaFree(a->vc);
-    cudaFree(a->md); cudaFree(a->macc); cudaFree(a->lamS);
+    cudaFree(a->arena);
+    if (a->used) cudaEventDestroy(a->used);
     delete a;
     a = nullptr;
+}
+
+// Marks the end of a call's work on the scratch (a captured call leaves none behind).
+static void mark_used(AdjointScratch& a, cudaStream_t st) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) cudaEventRecord(a.used, st);
 }
 
 // Recompute record per tracer per step: state + a1..a3, then per stage 1/R^2 and 1/R of
@@ -1093,34 +1147,47 @@ static AdjArgs adj_args(const AdjointScratch& a, const SizeBin* bins) {
 int adjoint_forward(AdjointScratch*& a, const ddx_state& s, int ng, int nd, double dt, int n_steps, int K,
                     const StepArgs& sa, const ddx_view& view, const ImageList& il, const SizeBin* bins,
                     const OpticsDev& o, double* image, cudaStream_t st) {
-    adjoint_free(a);
-    a = new AdjointScratch();
-    a->ng = ng; a->nd = nd; a->dt = dt; a->n_steps = n_steps; a->K = K; a->sa = sa; a->view = view; a->il = il;
-    a->nck = n_steps / K + 1;
-    a->nblk = (nd + kThreads - 1) / kThreads;
-    const size_t nd6 = 6ull * nd;
+    const int nblk = (nd + kThreads - 1) / kThreads;
+    const size_t nck = n_steps / K + 1, nd6 = 6ull * nd;
     // a large massive set keeps one step's block sums, a small one a whole segment's
     const bool large = ng > kMaxGrav;
-    const size_t part_words = large ? (size_t)a->nblk * 4 * ng * 4 : (size_t)a->nblk * K * 4 * ng * 4;
+    const size_t part_words = large ? (size_t)nblk * 4 * ng * 4 : (size_t)nblk * K * 4 * ng * 4;
     const size_t mu_words = large ? (size_t)4 * ng * 4 : (size_t)K * 4 * ng * 4;
-    bool fail = cudaMalloc(&a->xv_m, sizeof(double) * 7 * ng) || cudaMalloc(&a->y0, sizeof(double) * nd6) ||
-                cudaMalloc(&a->y, sizeof(double) * nd6) || cudaMalloc(&a->N0, sizeof(double) * nd) ||
-                cudaMalloc(&a->N, sizeof(double) * nd) || cudaMalloc(&a->ck, sizeof(double) * nd6 * a->nck) ||
-                cudaMalloc(&a->seg, sizeof(double) * (size_t)record_comps(ng) * nd * K) ||
-                cudaMalloc(&a->lam, sizeof(double) * nd6) ||
-                cudaMalloc(&a->part, sizeof(double) * (part_words > 0 ? part_words : 1)) ||
-                cudaMalloc(&a->mu, sizeof(double) * mu_words) ||
-                cudaMalloc(&a->md, sizeof(double) * (nd > 0 ? nd : 1)) ||
-                (large && (cudaMalloc(&a->macc, sizeof(double) * 6 * ng) ||
-                           cudaMalloc(&a->lamS, sizeof(double) * 27 * ng))) ||
-                cudaMalloc(&a->lam_m, sizeof(double) * 6 * ng) || cudaMalloc(&a->lam_mass, sizeof(double) * ng) ||
-                cudaMalloc(&a->idv, sizeof(int) * nd) || cudaMalloc(&a->active, nd) ||
-                cudaMalloc(&a->Ps, sizeof(Body) * (size_t)n_steps * 4 * ng) || cudaMalloc(&a->vc, sizeof(ViewConst));
-    if (fail) {
-        adjoint_free(a);
-        cudaGetLastError();
-        return DDX_ERR_NOMEM;
+    const size_t D = sizeof(double);
+    const size_t sizes[] = {D * 7 * ng, D * nd6, D * nd6, D * nd, D * nd, D * nd6 * nck,
+                            D * record_comps(ng) * nd * K, D * nd6, D * part_words, D * mu_words, D * nd,
+                            large ? D * 6 * ng : 0, large ? D * 27 * ng : 0, D * 6 * ng, D * ng, sizeof(int) * nd,
+                            (size_t)nd, sizeof(Body) * (size_t)n_steps * 4 * ng, sizeof(ViewConst)};
+    auto padded = [](size_t n) { return (n + 255) / 256 * 256; };
+    size_t total = 0;
+    for (const size_t n : sizes) total += padded(n);
+    // much larger memory than needed is given back
+    if (a && (a->cap < total || a->cap / 4 > total + (16u << 20))) adjoint_free(a);
+    if (!a) {
+        a = new AdjointScratch();
+        if (cudaMalloc((void**)&a->arena, total) != cudaSuccess ||
+            cudaEventCreateWithFlags(&a->used, cudaEventDisableTiming) != cudaSuccess) {
+            adjoint_free(a);
+            cudaGetLastError();
+            return DDX_ERR_NOMEM;
+        }
+        a->cap = total;
+    } else if (cudaStreamWaitEvent(st, a->used, 0) != cudaSuccess) {   // work on it on another stream
+        return DDX_ERR_CUDA;
     }
+    a->ready = false;
+    a->ng = ng; a->nd = nd; a->dt = dt; a->n_steps = n_steps; a->K = K; a->sa = sa; a->view = view; a->il = il;
+    a->nck = (int)nck;
+    a->nblk = nblk;
+    char* at = a->arena;
+    int part = 0;
+    auto take = [&](auto*& p) {
+        p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(at);
+        at += padded(sizes[part++]);
+    };
+    take(a->xv_m); take(a->y0); take(a->y); take(a->N0); take(a->N); take(a->ck); take(a->seg); take(a->lam);
+    take(a->part); take(a->mu); take(a->md); take(a->macc); take(a->lamS); take(a->lam_m); take(a->lam_mass);
+    take(a->idv); take(a->active); take(a->Ps); take(a->vc);
     const int thr = 256;
     const int blk = ((nd > ng ? nd : ng) + thr - 1) / thr;
     gather_state_kernel<<<blk, thr, 0, st>>>(s, ng, nd, a->xv_m, a->y0, a->N0, a->idv, a->md);
@@ -1150,6 +1217,7 @@ int adjoint_forward(AdjointScratch*& a, const ddx_state& s, int ng, int nd, doub
     if (nd > 0)
         image_splat_kernel<<<(nd + 255) / 256, 256, 0, st>>>(a->y, a->N, a->idv, nd, a->vc, o, il, image);
     if (cudaGetLastError() != cudaSuccess) return DDX_ERR_CUDA;
+    mark_used(*a, st);
     a->ready = true;
     return DDX_OK;
 }
@@ -1181,7 +1249,7 @@ int adjoint_backward(AdjointScratch* a, const double* G, double* grad_state, dou
             if (ng <= kMaxGrav) {
                 dust_reverse_kernel<<<a->nblk, kThreads, 0, st>>>(A, a->seg, n0, n1, a->lam, a->active, a->part);
                 const int per = Kseg * 4 * ng * 4;
-                reduce_parts_kernel<<<(per + 255) / 256, 256, 0, st>>>(a->part, a->nblk, per, a->mu);
+                reduce_parts_kernel<<<(per + 31) / 32, 32 * kPartWarps, 0, st>>>(a->part, a->nblk, per, a->mu);
             }
         } else {
             cudaMemsetAsync(a->mu, 0, sizeof(double) * (size_t)(ng <= kMaxGrav ? Kseg : 1) * 4 * ng * 4, st);
@@ -1198,7 +1266,7 @@ int adjoint_backward(AdjointScratch* a, const double* G, double* grad_state, dou
             if (nd > 0) {
                 dust_reverse_step_kernel<<<a->nblk, kThreads, 0, st>>>(A, a->seg, n - n0, n, a->lam, a->active,
                                                                        a->part);
-                reduce_parts_kernel<<<(per + 255) / 256, 256, 0, st>>>(a->part, a->nblk, per, a->mu);
+                reduce_parts_kernel<<<(per + 31) / 32, 32 * kPartWarps, 0, st>>>(a->part, a->nblk, per, a->mu);
             }
             massive_rev_init_kernel<<<(ng + tb - 1) / tb, tb, 0, st>>>(ng, a->dt, a->lam_m, a->lamS);
             for (int sg = 3; sg >= 0; --sg)
@@ -1211,6 +1279,7 @@ int adjoint_backward(AdjointScratch* a, const double* G, double* grad_state, dou
     cudaMemcpyAsync(grad_mass, a->lam_mass, sizeof(double) * ng, cudaMemcpyDeviceToDevice, st);
     // restore the final state for a later image/backward (the recompute overwrote y and N)
     if (cudaGetLastError() != cudaSuccess) return DDX_ERR_CUDA;
+    mark_used(*a, st);
     a->ready = false;
     return DDX_OK;
 }
