@@ -463,9 +463,11 @@ massive_slice_kernel(StepArgs a, MassiveScratch ms, int sa, int per, int np, dou
 constexpr int kGatherTargets = 32;
 constexpr int kGatherThreads = 256;
 
-template <int PASS>
+// n_pull: the bodies 0..n_pull-1 whose FP64 pulls the sums leave out; PREC: the precision whose
+// stage records pass 1 writes.
+template <int PASS, int PREC>
 __global__ void __launch_bounds__(kGatherThreads)
-massive_gather_kernel(ddx_state s, StepArgs a, MassiveScratch ms, int slices, int np,
+massive_gather_kernel(ddx_state s, StepArgs a, MassiveScratch ms, int n_pull, int slices, int np,
                       const double* __restrict__ part) {
     after_previous();
     constexpr int kWarps = kGatherThreads / 32;
@@ -494,7 +496,7 @@ massive_gather_kernel(ddx_state s, StepArgs a, MassiveScratch ms, int slices, in
 #pragma unroll
         for (int q = 0; q < 3; ++q) d[q] = sums[0][3 * warp + q][lane];
         const Body p = ms.P[st * c + i];
-        for (int j = 0; j < a.n_exact && j < a.n_grav; ++j)
+        for (int j = 0; j < n_pull && j < a.n_grav; ++j)
             if (j != i) pair64(p, ms.P[st * c + j], d[0], d[1], d[2]);
 #pragma unroll
         for (int q = 0; q < 3; ++q) sums[0][3 * warp + q][lane] = d[q];
@@ -503,8 +505,77 @@ massive_gather_kernel(ddx_state s, StepArgs a, MassiveScratch ms, int slices, in
     if (warp != 0 || i >= a.n_grav) return;
 #pragma unroll
     for (int q = 0; q < 6; ++q) acc[q] = sums[0][q][lane];
-    if (PASS == 1) pass1_update(s, a, ms, i, acc, DDX_PREC_MIXED);
+    if (PASS == 1) pass1_update(s, a, ms, i, acc, PREC);
     else pass2_update(s, a, ms, i, acc);
+}
+
+// ---------------------------------------------------------------------------------------
+// FP64 all-pairs over pairs of bodies
+// ---------------------------------------------------------------------------------------
+// FP64 issue bounds the all-pairs sums, and a pair's separation and r^-3 serve both of its bodies:
+// 20 FP64 operations a pair instead of 32.  A block takes two groups I < J of kPairBlock bodies at one
+// of the pass's two stages.  A thread holds a body of I; a warp goes through 32 bodies of J
+// in 32 steps, lane l taking body (l + step) mod 32, and the sums of J's bodies move one lane
+// with each step, so each ends where it began.  The four warps' sums are added in order.  A
+// block I = J takes every body's pulls on its own.  Every block writes sums of its own, row J for the
+// bodies of I and row I for those of J, which massive_gather_kernel adds in row order: the same
+// on every run.  4,099 bodies: 1460 us for both passes of a step, 2330 us with a warp per body.
+constexpr int kPairBlock = 128;
+// Bodies from which on it pays (FP64 steps of 2,000 tracers, us with / without: 1,503 bodies 1286 / 1248,
+// 2,003 1576 / 1787; below, the blocks are too few), and up to which the sums fit into the scratch
+// that every step keeps (MassiveScratch::part).
+constexpr int kPairsFrom = 1664, kPairsTo = 34 * kPairBlock;
+
+__global__ void __launch_bounds__(kPairBlock)
+massive_pairs_kernel(StepArgs a, MassiveScratch ms, int sa, int np, double* __restrict__ part) {
+    after_previous();
+    __shared__ Body src[kPairBlock];
+    __shared__ double red[kPairBlock / 32][3][32];
+    // blockIdx.x = J (J + 1) / 2 + I, I <= J
+    int J = (int)((sqrtf(8.f * (float)blockIdx.x + 1.f) - 1.f) * 0.5f);
+    while ((J + 1) * (J + 2) / 2 <= (int)blockIdx.x) ++J;
+    while (J * (J + 1) / 2 > (int)blockIdx.x) --J;
+    const int I = (int)blockIdx.x - J * (J + 1) / 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const Body* const P = ms.P + (size_t)(sa + blockIdx.y) * ms.cap;
+    const Body none = make_body(1e18, 1e18, 1e18, 0.0);
+    const int i = I * kPairBlock + threadIdx.x, j0 = J * kPairBlock;
+    const Body p = i < a.n_grav ? P[i] : none;
+    src[threadIdx.x] = j0 + (int)threadIdx.x < a.n_grav ? P[j0 + threadIdx.x] : none;
+    __syncthreads();
+    double* const rowI = part + ((size_t)I * 6 + 3 * blockIdx.y) * np;
+    double* const rowJ = part + ((size_t)J * 6 + 3 * blockIdx.y) * np;
+    double acc[3] = {0.0, 0.0, 0.0};
+    if (I == J) {
+#pragma unroll 4
+        for (int k = 0; k < kPairBlock; ++k)
+            if (k != (int)threadIdx.x) pair64(p, src[k], acc[0], acc[1], acc[2]);
+    } else {
+        for (int j = 0; j < kPairBlock; j += 32) {
+            double b[3] = {0.0, 0.0, 0.0};
+#pragma unroll 4
+            for (int step = 0; step < 32; ++step) {
+                const Body q = src[j + ((lane + step) & 31)];
+                const double dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
+                const double RR = dx * dx + dy * dy + dz * dz;
+                const double f = positive64(RR) ? pull64(1.0, RR) : 0.0, fi = f * q.m, fj = f * p.m;
+                acc[0] = fma(fi, dx, acc[0]); acc[1] = fma(fi, dy, acc[1]); acc[2] = fma(fi, dz, acc[2]);
+                b[0] = fma(-fj, dx, b[0]); b[1] = fma(-fj, dy, b[1]); b[2] = fma(-fj, dz, b[2]);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) b[c] = __shfl_sync(0xffffffffu, b[c], (lane + 1) & 31);
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) red[warp][c][lane] = b[c];
+            __syncthreads();
+            if (warp < 3) {
+                double t = red[0][warp][lane];
+                for (int w = 1; w < kPairBlock / 32; ++w) t += red[w][warp][lane];
+                rowI[(size_t)warp * np + j0 + j + lane] = t;
+            }
+            __syncthreads();
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) rowJ[(size_t)c * np + i] = acc[c];
 }
 
 // ---------------------------------------------------------------------------------------
@@ -741,8 +812,25 @@ cudaError_t launch_sliced(const ddx_state& s, const StepArgs& a, MassiveScratch&
         launch_with(a.n_grav <= kOverlapPasses, massive_slice_kernel, grid, kSliceWorkers, 0, st, a, slotted(ms, a),
                     PASS == 1 ? 0 : 2, per, np, ms.part);
     }
-    launch_after(massive_gather_kernel<PASS>, (a.n_grav + kGatherTargets - 1) / kGatherTargets, kGatherThreads, 0, st,
-                 s, a, slotted(ms, a), S, np, ms.part);
+    launch_after(massive_gather_kernel<PASS, DDX_PREC_MIXED>, (a.n_grav + kGatherTargets - 1) / kGatherTargets,
+                 kGatherThreads, 0, st, s, a, slotted(ms, a), a.n_exact, S, np, ms.part);
+    return cudaGetLastError();
+}
+
+// The FP64 all-pairs pass over pairs of bodies (FP64 and compensated steps).
+bool pairs_fit(const StepArgs& a, const MassiveScratch& ms) {
+    const long long nb = (a.n_grav + kPairBlock - 1) / kPairBlock;
+    return a.n_grav >= kPairsFrom && a.n_grav <= kPairsTo && ms.part && ms.part_words >= 6 * nb * nb * kPairBlock;
+}
+
+template <int PASS>
+cudaError_t launch_pairs(const ddx_state& s, const StepArgs& a, MassiveScratch& ms, int precision, cudaStream_t st) {
+    const int nb = (a.n_grav + kPairBlock - 1) / kPairBlock, np = nb * kPairBlock;
+    launch_first(massive_pairs_kernel, dim3(nb * (nb + 1) / 2, 2), kPairBlock, 0, st, a, ms, PASS == 1 ? 0 : 2, np, ms.part);
+    launch_after(precision == DDX_PREC_FP64 ? massive_gather_kernel<PASS, DDX_PREC_FP64>
+                                            : massive_gather_kernel<PASS, DDX_PREC_MIXED>,
+                 (a.n_grav + kGatherTargets - 1) / kGatherTargets, kGatherThreads, 0, st, s, a,
+                 precision == DDX_PREC_FP64 ? ms : slotted(ms, a), 0, nb, np, ms.part);
     return cudaGetLastError();
 }
 }  // namespace
@@ -762,6 +850,7 @@ long long massive_part_words(int cap) { return massive_part_words_for(cap, sm_co
 cudaError_t launch_massive_pass1(const ddx_state& s, const StepArgs& a, MassiveScratch& ms,
                                  int precision, cudaStream_t st) {
     if (precision == DDX_PREC_MIXED && sliced_fits(a, ms)) return launch_sliced<1>(s, a, ms, st);
+    if (precision != DDX_PREC_MIXED && pairs_fit(a, ms)) return launch_pairs<1>(s, a, ms, precision, st);
     const int threads = 128;  // 4 targets per block
     const int blocks = (a.n_grav * 32 + threads - 1) / threads;
     if (precision == DDX_PREC_COMPENSATED)   // the massive set in FP64
@@ -777,6 +866,7 @@ cudaError_t launch_massive_pass1(const ddx_state& s, const StepArgs& a, MassiveS
 cudaError_t launch_massive_pass2(const ddx_state& s, const StepArgs& a, MassiveScratch& ms,
                                  int precision, cudaStream_t st) {
     if (precision == DDX_PREC_MIXED && sliced_fits(a, ms)) return launch_sliced<2>(s, a, ms, st);
+    if (precision != DDX_PREC_MIXED && pairs_fit(a, ms)) return launch_pairs<2>(s, a, ms, precision, st);
     const int threads = 128;
     const int blocks = (a.n_grav * 32 + threads - 1) / threads;
     if (precision == DDX_PREC_COMPENSATED)

@@ -196,3 +196,36 @@ def test_few_tracers_pulls(engine, n_plsml):
         m = one_step(engine, s, s.state, prec)
         np.testing.assert_array_equal(m["N"] == 0, f["N"] == 0)
         check_velocities(s, f, m, rows[f["N"][rows] != 0], rel)
+
+
+# FP64 all-pairs over pairs of bodies from 1,664 to 4,352 massive bodies (3 of them star and planets), in
+# blocks of 128
+@pytest.mark.parametrize("n_grav", [1663, 1664, 1665, 1791, 1792, 1793, 4223, 4351, 4352, 4353])
+@pytest.mark.parametrize("prec", [abi.DDX_PREC_FP64, abi.DDX_PREC_COMPENSATED])
+def test_massive_set_in_fp64(engine, n_grav, prec):
+    """Against the sums in FP64 on the CPU, without the later stages: a step so short that the
+    velocity's change is dt times the first acceleration.  4,000 roundings are 4e-13 of the pulls'
+    magnitudes, and the bodies' motion within the step, a dt^2 against the nearest at some 0.01 AU, is
+    as much: 1e-9 leaves room for pairs a thousand times nearer, and one pull left out is 2e-4 / 10."""
+    s = heavy_ring(n_grav - 3, 8)
+    st = {k: v.copy() for k, v in s.state.items()}
+    for c in "xyz":
+        st["v" + c][:n_grav] = 0.0               # so that the change of velocity is the velocity
+    dt = 1e-6
+    engine.set_size_table(**s.size_table)
+    d = DeviceState.from_numpy(st)
+    engine.step(d, s.n_grav, dt, make_phys(**s.phys), prec, abi.DDX_MODE_FIXED)
+    torch.cuda.synchronize()
+    got = d.to_numpy()
+    x, m = np.stack([st[c][:n_grav] for c in "xyz"], 1), st["m"][:n_grav]
+    rows = np.r_[0:40, 100:n_grav:37, n_grav - 40:n_grav]
+    for i in rows:
+        dx = x - x[i]
+        r2 = (dx ** 2).sum(1)
+        r2[i] = 1.0
+        w = m / (r2 * np.sqrt(r2))
+        w[i] = 0.0
+        want = dt * (w[:, None] * dx).sum(0)
+        mag = dt * (w * np.sqrt(r2)).sum()
+        v = np.array([got["v" + c][i] for c in "xyz"])
+        assert np.abs(v - want).max() <= 1e-9 * mag, (i, np.abs(v - want).max() / mag)
