@@ -801,7 +801,7 @@ def solar_leg(local, fp64_peak, n_steps=1000, reps=3):
             "roofline": {"kernel": "whole step (dust_rk4_kernel<fp64> + massive passes)", "bound": "fp64_pipe",
                          "achieved": flops / t / 1e12, "peak": fp64_peak, "unit": "TFLOP/s",
                          "frac": flops / t / 1e12 / fp64_peak,
-                         "note": "16,384 tracers fill 64 blocks of 256 on 152 SMs: launch- and occupancy-bound"}}
+                         "note": "16,384 tracers fill 256 blocks of 64 on 152 SMs: launch- and occupancy-bound"}}
 
 
 def imaging_leg(local, reps=5):
