@@ -1178,12 +1178,13 @@ cudaError_t cells_ensure(CellScratch*& c, int n_src) {
     static CellTables tab;
     static const bool tab_ok = make_tables(tab);
     if (!tab_ok) return cudaErrorInvalidValue;
-    // Nodes: every split cell has more than CellGrid::leaf groups near it, and a group is near
-    // some 700 cells of a level in space (95 in a disk), so the planetesimals bound the tree;
-    // a belt of 4,096 with a million tracers takes about 32,000 nodes, a belt with a wide halo
-    // of 20,000 some 560,000 when its cells are split at 24 groups.  A level that does not fit
-    // is left out (its parents stay leaves).
-    const int cap = cap_src <= 8192 ? 262144 : 1048576;
+    // Nodes: a level that does not fit would be left out (its parents stay leaves), and then the
+    // tracers together decide how far cells are split, so there is room for the worst case: a
+    // ball of planetesimals with tracers everywhere in it.  Its radius is the mean distance R or
+    // so, the finest edge R / 24 (n / 4,096)^(-1/4) or more, so the four stages have at most 4 (pi / 6) 48^3
+    // (n / 4,096)^(3/4) finest cells and a seventh as many coarser ones: 262,000 for 4,096, 441,000 for
+    // 8,192.  A belt of 4,096 with a million tracers takes 32,000, one with a wide halo 120,000.
+    const int cap = cap_src < 32768 ? 64 * cap_src : 2097152;
     const int groups = cap_src / kGroupSrc, words = (groups + 31) / 32;
     const int G = grid_dim(cap_src);
     const size_t marks = 3 * 4 * (size_t)cell_word0(G, grid_levels(G));

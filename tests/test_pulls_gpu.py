@@ -229,3 +229,24 @@ def test_massive_set_in_fp64(engine, n_grav, prec):
         mag = dt * (w * np.sqrt(r2)).sum()
         v = np.array([got["v" + c][i] for c in "xyz"])
         assert np.abs(v - want).max() <= 1e-9 * mag, (i, np.abs(v - want).max() / mag)
+
+
+def test_grains_in_a_ball_step_alike_alone_and_among_many(engine):
+    """A ball of planetesimals with tracers everywhere in it needs the most cells; all of them fit, so
+    the first 5,000 grains come out the same alone and among 1,500,000."""
+    n_dust = 1_500_000
+    s = heavy_ring(8100, n_dust)
+    g = np.random.default_rng(6)
+    ng = s.n_grav
+    for rows in (slice(3, ng), slice(ng, None)):
+        n = len(s.state["x"][rows])
+        u = g.normal(size=(3, n))
+        u *= 140.0 * g.uniform(0.01, 1.0, n) ** (1 / 3) / np.linalg.norm(u, axis=0)
+        for k, c in enumerate("xyz"):
+            s.state[c][rows] = u[k]
+            s.state["v" + c][rows] *= 0.3
+    got = []
+    for n in (5000, n_dust):
+        m = one_step(engine, s, {k: np.asarray(v)[:ng + n].copy() for k, v in s.state.items()}, abi.DDX_PREC_MIXED)
+        got.append(np.stack([m[c][:ng + 5000] for c in ("x", "y", "z", "vx", "vy", "vz", "N")]))
+    np.testing.assert_array_equal(got[0], got[1])
