@@ -57,8 +57,8 @@ namespace {
 
 constexpr float kFarEdge = 4.5f;
 // A cell is split while more groups than this are near it, and the finest cell edge is about
-// this share of the planetesimals' mean distance for 4,096 of them (as their number to the
-// -1/4), for a narrow belt and for a set spread over more than half an octave of distance.
+// this share of the planetesimals' mean distance for 4,096 of them (edge_scale for other
+// numbers), for a narrow belt and for a set spread over more than half an octave of distance.
 // A spread set's tracers share fewer cells, so a cell has to cost less (us a step, start = all
 // planetesimals one by one, 24 and 1/30 / 40 and 1/24 / 64 and 1/20):
 //   belt of 4,096 with a million tracers              7930 / 2170 / 2560 / 3220
@@ -190,6 +190,15 @@ bool make_tables(CellTables& t) {
 
 constexpr int kSetupThreads = 256;
 
+// The finest edge's share of the mean distance over that for 4,096 planetesimals: it goes as n^(-1/4),
+// but as n^(-1/8) from 4,096 to 32,768 (us a step with -1/4 / -1/8: belts of 9,000 with 300,000 tracers 2166 /
+// 1869, 30,000 with 20,000 5084 / 4564, halos of 20,000 with 30,000 and 500,000 3871 / 3517 and 8624 / 8130; beyond,
+// a halo of 40,000 with 300,000 16182 / 17004, a belt of 65,536 with two million 48100 / 73000).
+__device__ __forceinline__ float edge_scale(float n) {
+    const float q = sqrtf(rsqrtf(fmaxf(n, 1.f) / 4096.f));
+    return n > 4096.f && n <= 32768.f ? sqrtf(q) : q;
+}
+
 // The grids of this step from the geometric mean distance of the planetesimals to the star
 // (largest coordinate difference), which one or two far-flung bodies do not move.  Integer
 // sums: the same on every run.  sums: [0] sum of the logarithms, [1] their number, [2] blocks
@@ -247,7 +256,7 @@ cells_setup_kernel(const Body* __restrict__ P, int n_exact, int n_src, int G, un
     const double var = num > 0 ? (double)sum2 / (double)num / 65536.0 - lm * lm : 0.0;
     const bool spread = var > (double)kSpreadOctaves * kSpreadOctaves;
     g.leaf = spread ? (num < 8192 ? kLeafSpread : kLeafSpreadMany) : kLeafNarrow;
-    const float want = mean * (spread ? kEdgeSpread : kEdgeNarrow) * sqrtf(rsqrtf(fmaxf((float)num, 1.f) / 4096.f));
+    const float want = mean * (spread ? kEdgeSpread : kEdgeNarrow) * edge_scale((float)num);
     // the nearest of 2^e and 3 2^(e-1): a centre, an odd multiple of half an edge, is exact
     const float l = log2f(want);
     int e = (int)floorf(l);
