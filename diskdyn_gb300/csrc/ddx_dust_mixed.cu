@@ -70,8 +70,11 @@
 namespace ddx {
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kTilePairs = 256;                 // pair records per tile (16 KiB)
+constexpr int kThreads = 256;                    // and pair records per tile (16 KiB)
+// From this many tracers on, blocks and tiles of half the size: they spread more evenly over the SMs (us a
+// step with 256 / 128; mixed, 256 planetesimals: 65,536 tracers 158 / 156, 131,072 227 / 203, a million 1081 / 1015; 900:
+// 299 / 301, 484 / 457, 2386 / 2366; 20,003 tracers 230 / 234; compensated, 1,500: 131,072 2157 / 2098).
+constexpr int kManyTracers = 100000;
 // Four lanes share a tracer up to these numbers of tracers, from kLanesMinSources planetesimals on: one
 // thread's chain of pulls then takes longer than four threads' shares with the star term and the
 // sums repeated in each (us a step with one / four lanes; mixed, 900 planetesimals: 2,003 tracers 220 / 174,
@@ -387,15 +390,15 @@ __device__ __forceinline__ uint32_t span_bits(const uint32_t* w, int j0, int n) 
 // needs more than 64): 22.75 ms on the dusty ring against 23.0 ms with two blocks of 128.
 // T = 4: four lanes share a tracer.  Each takes every fourth span of a tile; the spans' sums are then
 // added by all four in span order, so the bits are those of T = 1.
-template <bool COMP, int T>
-__global__ void __launch_bounds__(kThreads, COMP ? 3 : 4)
+template <bool COMP, int T, int NT>
+__global__ void __launch_bounds__(NT, (COMP ? 3 : 4) * kThreads / NT)
 dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __restrict__ bins,
                       const int* __restrict__ perm, bool boxes, const int* __restrict__ src) {
     after_previous();
     constexpr int NB = COMP ? 8 : 7;              // box values: 3 x (min, max), largest own[, smallest own]
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) unsigned long long mbar[2];
-    __shared__ float bred[kThreads / 32][NB];
+    __shared__ float bred[NT / 32][NB];
     __shared__ float bbox[NB];                    // the block's box at the current stage, largest own
     __shared__ uint32_t allfar[kFlagSpans / 32], allnear[kFlagSpans / 32];
     __shared__ uint32_t allcomp[COMP ? kFlagSpans / 32 : 1], nocomp[COMP ? kFlagSpans / 32 : 1];
@@ -426,7 +429,7 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
     }
 
     const int npairs = pair_count(ng - a.n_exact);
-    const int ntiles = (npairs + kTilePairs - 1) / kTilePairs;
+    const int ntiles = (npairs + NT - 1) / NT;
     const int G = 4 * ntiles;                       // tiles over all four stages
     const uint32_t mb[2] = {smem_u32(&mbar[0]), smem_u32(&mbar[1])};
     if (tid == 0) {
@@ -441,10 +444,10 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
     int in_flight[2] = {-1, -1};
     auto issue = [&](int g) {
         if (g == a.lose_tile) return;
-        const int stg = g / ntiles, first = (g - stg * ntiles) * kTilePairs;
-        const unsigned bytes = (unsigned)(min(kTilePairs, npairs - first) * sizeof(BodyPair));
+        const int stg = g / ntiles, first = (g - stg * ntiles) * NT;
+        const unsigned bytes = (unsigned)(min(NT, npairs - first) * sizeof(BodyPair));
         mbar_expect_tx(mb[g & 1], bytes);
-        bulk_load(smem_u32(tiles + (g & 1) * kTilePairs), ms.PP + (size_t)stg * ms.pcap + first, bytes,
+        bulk_load(smem_u32(tiles + (g & 1) * NT), ms.PP + (size_t)stg * ms.pcap + first, bytes,
                   mb[g & 1]);
         in_flight[g & 1] = g;
     };
@@ -562,9 +565,9 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
             if (!mbar_wait(mb[g & 1], (g >> 1) & 1, a.wait_ns)) { lost = 1; continue; }
             if (tid == 0) in_flight[g & 1] = -1;
             if (!alive) continue;
-            const BodyPair* const T_ = tiles + (g & 1) * kTilePairs;
-            const int cnt = min(kTilePairs, npairs - tt * kTilePairs);   // a multiple of kPairSpan
-            static_assert(kTilePairs / kPairSpan <= 32, "one mask bit per span of a tile");
+            const BodyPair* const T_ = tiles + (g & 1) * NT;
+            const int cnt = min(NT, npairs - tt * NT);   // a multiple of kPairSpan
+            static_assert(NT / kPairSpan <= 32, "one mask bit per span of a tile");
             uint32_t fm = 0u, cm = 0u;   // far spans, compensated spans (compensated wins)
             const uint32_t all = cnt / kPairSpan == 32 ? 0xFFFFFFFFu : (1u << (cnt / kPairSpan)) - 1u;
             if (COMP) {
@@ -573,7 +576,7 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
                 } else {
                     uint32_t open = all;
                     if (flags) {
-                        const int j0 = tt * (kTilePairs / kPairSpan);
+                        const int j0 = tt * (NT / kPairSpan);
                         const uint32_t ac = span_bits(allcomp, j0, cnt / kPairSpan);
                         cm = ac;
                         open = all & ~(ac | span_bits(nocomp, j0, cnt / kPairSpan));
@@ -591,7 +594,7 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
             if (boxes) {
                 uint32_t open = all & ~cm;
                 if (flags) {
-                    const int j0 = tt * (kTilePairs / kPairSpan);   // the tile's first span
+                    const int j0 = tt * (NT / kPairSpan);   // the tile's first span
                     const uint32_t af = span_bits(allfar, j0, cnt / kPairSpan);
                     fm = af & ~cm;
                     open = all & ~cm & ~(af | span_bits(allnear, j0, cnt / kPairSpan));
@@ -607,11 +610,11 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
             }
             for (int k0 = 0; k0 < cnt; k0 += T * kPairSpan) {
                 const int k = k0 + sub * kPairSpan;               // this lane's span
-                const f2* ML = COMP ? reinterpret_cast<const f2*>(ms.PM + (size_t)st * ms.pcap + tt * kTilePairs) : nullptr;
+                const f2* ML = COMP ? reinterpret_cast<const f2*>(ms.PM + (size_t)st * ms.pcap + tt * NT) : nullptr;
                 // span k's pulls again with the near ones, in FP64, added to the acceleration
                 auto with_near = [&](int k, f2& px, f2& py, f2& pz) {
                     px = py = pz = 0;
-                    near_span<kPairSpan>(T_ + k, 2 * (tt * kTilePairs + k), XH, XL, YH, YL, ZH, ZL, join3(XH, XL, xr),
+                    near_span<kPairSpan>(T_ + k, 2 * (tt * NT + k), XH, XL, YH, YL, ZH, ZL, join3(XH, XL, xr),
                                          join3(YH, YL, yr), join3(ZH, ZL, zr), inv_near, Pn, src, px, py, pz, kx, ky, kz);
                 };
                 f2 px = 0, py = 0, pz = 0;
@@ -665,7 +668,7 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
                 if (T == 1) {
                     if (ff) {
                         if (mx > inv_near)   // a source within the near radius: its pull in FP64
-                            near_span_ff(T_ + k, ML + k, 2 * (tt * kTilePairs + k), XH, XL, YH, YL, ZH, ZL, xr, yr, zr,
+                            near_span_ff(T_ + k, ML + k, 2 * (tt * NT + k), XH, XL, YH, YL, ZH, ZL, xr, yr, zr,
                                          inv_near, Pn, src, SH, SL, kx, ky, kz);
                         kx += ff_total(SH[0], SL[0]); ky += ff_total(SH[1], SL[1]); kz += ff_total(SH[2], SL[2]);
                         continue;
@@ -692,7 +695,7 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
                                        __longlong_as_double((long long)vz_)};
                         if ((nears >> q) & 1u) {
                             f2 H[3], L[3];
-                            near_span_ff(T_ + kq, ML + kq, 2 * (tt * kTilePairs + kq), XH, XL, YH, YL, ZH, ZL, xr, yr, zr,
+                            near_span_ff(T_ + kq, ML + kq, 2 * (tt * NT + kq), XH, XL, YH, YL, ZH, ZL, xr, yr, zr,
                                          inv_near, Pn, src, H, L, kx, ky, kz);
                             for (int c = 0; c < 3; ++c) t[c] = ff_total(H[c], L[c]);
                         }
@@ -751,23 +754,32 @@ cudaError_t launch_dust_mixed(const ddx_state& s, const StepArgs& a, const Massi
     // cell expansions from kCellMinSources planetesimals on (the lost-copy test hook needs tiles)
     if (!comp && ms.cells && ms.dust_order.cap >= a.n_dust && a.n_grav - a.n_exact >= kCellMinSources && a.lose_tile < 0)
         return launch_dust_cells(s, a, ms, bins, st);
-    const size_t smem = 2 * (size_t)kTilePairs * sizeof(BodyPair);
+    // four lanes per tracer while the GPU is not full without (kLanesFew)
     const bool lanes = a.n_grav - a.n_exact >= kLanesMinSources && a.n_dust <= (comp ? kLanesFewComp : kLanesFew);
-    auto* const kernel = comp ? (lanes ? dust_rk4_mixed_kernel<true, 4> : dust_rk4_mixed_kernel<true, 1>)
-                              : (lanes ? dust_rk4_mixed_kernel<false, 4> : dust_rk4_mixed_kernel<false, 1>);
+    const bool many = a.n_dust >= kManyTracers;
+    constexpr int kHalf = kThreads / 2;
+    auto* const kernel = comp ? (lanes  ? dust_rk4_mixed_kernel<true, 4, kThreads>
+                                 : many ? dust_rk4_mixed_kernel<true, 1, kHalf>
+                                        : dust_rk4_mixed_kernel<true, 1, kThreads>)
+                              : (lanes  ? dust_rk4_mixed_kernel<false, 4, kThreads>
+                                 : many ? dust_rk4_mixed_kernel<false, 1, kHalf>
+                                        : dust_rk4_mixed_kernel<false, 1, kThreads>);
+    const size_t smem = 2 * (size_t)(many ? kHalf : kThreads) * sizeof(BodyPair);
     static bool attr_set[128] = {};   // the attributes are set once per device
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 128) return cudaErrorInvalidDevice;
     if (!attr_set[dev]) {
-        for (const void* f : {(const void*)dust_rk4_mixed_kernel<true, 4>, (const void*)dust_rk4_mixed_kernel<true, 1>,
-                              (const void*)dust_rk4_mixed_kernel<false, 4>, (const void*)dust_rk4_mixed_kernel<false, 1>}) {
-            const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const size_t most = 2 * (size_t)kThreads * sizeof(BodyPair);
+        for (const void* f :
+             {(const void*)dust_rk4_mixed_kernel<true, 4, kThreads>, (const void*)dust_rk4_mixed_kernel<true, 1, kThreads>,
+              (const void*)dust_rk4_mixed_kernel<false, 4, kThreads>, (const void*)dust_rk4_mixed_kernel<false, 1, kThreads>}) {
+            const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
             if (e != cudaSuccess) return e;
         }
         attr_set[dev] = true;
     }
-    const int threads = dust_block_threads(lanes ? 4 * a.n_dust : a.n_dust);   // 256 unless the grains are few
+    const int threads = many ? kHalf : dust_block_threads(lanes ? 4 * a.n_dust : a.n_dust);   // 256 unless the grains are few
     const int blocks = (int)((a.n_dust * (lanes ? 4LL : 1LL) + threads - 1) / threads);
     // the tracers' visiting order and the spans' boxes, when the context keeps their scratch
     const int* perm = nullptr;

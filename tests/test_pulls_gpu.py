@@ -250,3 +250,16 @@ def test_grains_in_a_ball_step_alike_alone_and_among_many(engine):
         m = one_step(engine, s, {k: np.asarray(v)[:ng + n].copy() for k, v in s.state.items()}, abi.DDX_PREC_MIXED)
         got.append(np.stack([m[c][:ng + 5000] for c in ("x", "y", "z", "vx", "vy", "vz", "N")]))
     np.testing.assert_array_equal(got[0], got[1])
+
+
+# 100,000 tracers: blocks and tiles of half the size
+@pytest.mark.parametrize("n_plsml", [100, 257, 1100])
+@pytest.mark.parametrize("prec", [abi.DDX_PREC_MIXED, abi.DDX_PREC_COMPENSATED])
+def test_blocks_of_half_the_size_give_the_same_bits(engine, prec, n_plsml):
+    s = scattered(n_plsml, 100000)
+    ng = s.n_grav
+    got = []
+    for n in (99999, 100000):
+        m = one_step(engine, s, {k: np.asarray(v)[:ng + n].copy() for k, v in s.state.items()}, prec)
+        got.append(np.stack([m[c][:ng + 99999] for c in ("x", "y", "z", "vx", "vy", "vz", "N")]))
+    np.testing.assert_array_equal(got[0], got[1])
