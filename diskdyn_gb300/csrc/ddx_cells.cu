@@ -1182,8 +1182,7 @@ void cells_free(CellScratch*& c) {
 
 cudaError_t cells_ensure(CellScratch*& c, int n_src) {
     if (c && c->cap_src >= n_src) return cudaSuccess;
-    int cap_src = 1024;
-    while (cap_src < n_src) cap_src *= 2;
+    const int cap_src = (n_src + 1023) / 1024 * 1024;
     static CellTables tab;
     static const bool tab_ok = make_tables(tab);
     if (!tab_ok) return cudaErrorInvalidValue;

@@ -26,9 +26,9 @@ constexpr float kReach = 0.55f;
 constexpr int kDistantNode = -2;        // the tracer takes the distant expansion
 // Few tracers leave most of the GPU idle, so 8 or 4 lanes share one below these numbers (us a
 // step with 8 / 4 lanes at 7,000 tracers: 452 / 479 for 2,100 planetesimals, 1131 / 1192 for 9,000;
-// with 4 / 1 at 41,000: 634 / 665 and 1680 / 1831, a narrow belt of 4,096 748 / 731; at 80,000: 790 / 716
-// and 2046 / 2029).
-constexpr int kLanes8 = 8000, kLanes4 = 48000;
+// at 9,000: 498 / 490 for 3,001; with 4 / 1 at 32,000: 582 / 617 and 1425 / 1539, a narrow belt of 4,096 635 /
+// 634; at 40,000, more than one wave of 4 lanes: 664 / 638, 1572 / 1577, 695 / 653).
+constexpr int kLanes8 = 8000, kLanes4 = 34000;
 
 __host__ __device__ constexpr float harm_g(int n, int m) {
     return (float)((double)((n - 1) * (n - 1) - m * m) / (double)((2 * n - 1) * (2 * n - 3)));
@@ -338,8 +338,12 @@ __device__ __forceinline__ void pull_groups(const CellView& v, int n, bool on, c
     }
 }
 
+// Six blocks an SM (80 registers): us a step with 6 / 7 / 8 for one lane per tracer, 4,096 planetesimals with a
+// million tracers 2075 / 2065 / 2147, with 60,000 684 / 700 / 734, 3,001 with a halo and 500,003 1645 / 1639 / 1736, 9,000
+// with a halo and 300,003 2743 / 2841 / 2952.  Seven with four and eight lanes (4,096 with 28,000: 618 / 623 /
+// 634, but 30,000 tracers no longer fit into one wave of six: 3,001 with a halo 617 / 594 / 600).
 template <int T>
-__global__ void __launch_bounds__(kThreads, 8)
+__global__ void __launch_bounds__(kThreads, T > 1 ? 7 : 6)
 dust_cells_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __restrict__ bins,
                   const int* __restrict__ perm, CellView v, const int* __restrict__ src) {
     after_previous();

@@ -104,11 +104,11 @@ def test_tracer_pulls(engine, n_plsml, make):
 
 def test_lanes_per_tracer_give_the_same_bits(engine):
     """Few tracers are shared by 8 or 4 lanes each; the first 100 grains come out the same
-    among 100, 7,999, 8,000, 47,999 and 48,000."""
+    among 100, 7,999, 8,000, 33,999, 34,000 and 48,000."""
     s = scattered(3000, 48000)
     ng = s.n_grav
     first = None
-    for n in (100, 7999, 8000, 47999, 48000):
+    for n in (100, 7999, 8000, 33999, 34000, 48000):
         state = {k: np.asarray(v)[:ng + n].copy() for k, v in s.state.items()}
         m = one_step(engine, s, state, abi.DDX_PREC_MIXED)
         got = np.stack([m[c][:ng + 100] for c in ("x", "y", "z", "vx", "vy", "vz", "N")])
