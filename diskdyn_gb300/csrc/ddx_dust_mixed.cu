@@ -75,6 +75,10 @@ constexpr int kThreads = 256;                    // and pair records per tile (1
 // step with 256 / 128; mixed, 256 planetesimals: 65,536 tracers 158 / 156, 131,072 227 / 203, a million 1081 / 1015; 900:
 // 299 / 301, 484 / 457, 2386 / 2366; 20,003 tracers 230 / 234; compensated, 1,500: 131,072 2157 / 2098).
 constexpr int kManyTracers = 100000;
+// Blocks of 256 threads an SM for the compensated step with many planetesimals (kOrderMinSources), whose
+// float-float pairs want the registers: us a step with 2 / 3, 4,096 planetesimals and 131,072 tracers 5064 / 5425,
+// 40,003 tracers 3255 / 3494, 1,500 and 40,003 1134 / 1227; 300 and 262,144 1778 / 1722.
+constexpr int kCompBlocks = 2;
 // Four lanes share a tracer up to these numbers of tracers, from kLanesMinSources planetesimals on: one
 // thread's chain of pulls then takes longer than four threads' shares with the star term and the
 // sums repeated in each (us a step with one / four lanes; mixed, 900 planetesimals: 2,003 tracers 220 / 174,
@@ -386,12 +390,12 @@ __device__ __forceinline__ uint32_t span_bits(const uint32_t* w, int j0, int n) 
 // spills were slower than three.  With the near-source test in (8.64 ms at 24 KiB tiles),
 // smaller tiles leave more of the SM's 256 KiB to L1, where the spilled values live:
 // 8.55 ms at 12 KiB, 8.47 ms at 16 KiB, 8.53 ms at 20 KiB.
-// COMP: the compensated variant, three blocks per SM (80 registers; its float-float pair
-// needs more than 64): 22.75 ms on the dusty ring against 23.0 ms with two blocks of 128.
+// COMP: the compensated variant, whose float-float pair needs more than 64 registers.
+// MB: blocks of 256 threads per SM.
 // T = 4: four lanes share a tracer.  Each takes every fourth span of a tile; the spans' sums are then
 // added by all four in span order, so the bits are those of T = 1.
-template <bool COMP, int T, int NT>
-__global__ void __launch_bounds__(NT, (COMP ? 3 : 4) * kThreads / NT)
+template <bool COMP, int T, int NT, int MB>
+__global__ void __launch_bounds__(NT, MB * kThreads / NT)
 dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __restrict__ bins,
                       const int* __restrict__ perm, bool boxes, const int* __restrict__ src) {
     after_previous();
@@ -758,12 +762,18 @@ cudaError_t launch_dust_mixed(const ddx_state& s, const StepArgs& a, const Massi
     const bool lanes = a.n_grav - a.n_exact >= kLanesMinSources && a.n_dust <= (comp ? kLanesFewComp : kLanesFew);
     const bool many = a.n_dust >= kManyTracers;
     constexpr int kHalf = kThreads / 2;
-    auto* const kernel = comp ? (lanes  ? dust_rk4_mixed_kernel<true, 4, kThreads>
-                                 : many ? dust_rk4_mixed_kernel<true, 1, kHalf>
-                                        : dust_rk4_mixed_kernel<true, 1, kThreads>)
-                              : (lanes  ? dust_rk4_mixed_kernel<false, 4, kThreads>
-                                 : many ? dust_rk4_mixed_kernel<false, 1, kHalf>
-                                        : dust_rk4_mixed_kernel<false, 1, kThreads>);
+    // blocks of 256 threads an SM (kCompBlocks)
+    const bool wide = comp && a.n_grav - a.n_exact >= kOrderMinSources;
+    auto* const kernel =
+        wide   ? (lanes  ? dust_rk4_mixed_kernel<true, 4, kThreads, kCompBlocks>
+                  : many ? dust_rk4_mixed_kernel<true, 1, kHalf, kCompBlocks>
+                         : dust_rk4_mixed_kernel<true, 1, kThreads, kCompBlocks>)
+        : comp ? (lanes  ? dust_rk4_mixed_kernel<true, 4, kThreads, 3>
+                  : many ? dust_rk4_mixed_kernel<true, 1, kHalf, 3>
+                         : dust_rk4_mixed_kernel<true, 1, kThreads, 3>)
+               : (lanes  ? dust_rk4_mixed_kernel<false, 4, kThreads, 4>
+                  : many ? dust_rk4_mixed_kernel<false, 1, kHalf, 4>
+                         : dust_rk4_mixed_kernel<false, 1, kThreads, 4>);
     const size_t smem = 2 * (size_t)(many ? kHalf : kThreads) * sizeof(BodyPair);
     static bool attr_set[128] = {};   // the attributes are set once per device
     int dev = 0;
@@ -772,8 +782,11 @@ cudaError_t launch_dust_mixed(const ddx_state& s, const StepArgs& a, const Massi
     if (!attr_set[dev]) {
         const size_t most = 2 * (size_t)kThreads * sizeof(BodyPair);
         for (const void* f :
-             {(const void*)dust_rk4_mixed_kernel<true, 4, kThreads>, (const void*)dust_rk4_mixed_kernel<true, 1, kThreads>,
-              (const void*)dust_rk4_mixed_kernel<false, 4, kThreads>, (const void*)dust_rk4_mixed_kernel<false, 1, kThreads>}) {
+             {(const void*)dust_rk4_mixed_kernel<true, 4, kThreads, 3>, (const void*)dust_rk4_mixed_kernel<true, 1, kThreads, 3>,
+              (const void*)dust_rk4_mixed_kernel<true, 4, kThreads, kCompBlocks>,
+              (const void*)dust_rk4_mixed_kernel<true, 1, kThreads, kCompBlocks>,
+              (const void*)dust_rk4_mixed_kernel<false, 4, kThreads, 4>,
+              (const void*)dust_rk4_mixed_kernel<false, 1, kThreads, 4>}) {
             const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
             if (e != cudaSuccess) return e;
         }
