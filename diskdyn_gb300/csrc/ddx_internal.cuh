@@ -195,13 +195,17 @@ class DeviceGuard {
 };
 
 // Mixed massive passes over source slices (ddx_step.cu): targets per block, and the blocks
-// per SM the slices aim at.  The slice sums of a system of up to cap bodies on a GPU with
-// sms SMs take massive_part_words_for(cap, sms) doubles: S slices * np targets with
-// S <= kSliceBlocksPerSM * sms / groups + 1, so S * np <= (kSliceBlocksPerSM * sms + groups) * 256.
+// per SM the slices aim at: fewer and longer slices for few bodies, whose gather reads all of
+// their sums, more for many, which a last wave of long ones would hold up (us a step of 4,000
+// tracers with 2 / 3 / 4 / 8 / 12: 4,096 planetesimals 467 / 462 / 474 / 505 / 537, 9,000 914 / 883 / 873 / 864 /
+// 874, 20,000 2368 / 2213 / 2131 / 2053 / 2040, 65,536 16.7 / 16.7 / 16.9 / 15.7 / 15.8 ms).
+// The slice sums of a system of up to cap bodies on a GPU with sms SMs take
+// massive_part_words_for(cap, sms) doubles: S slices * np targets with S <= blocks * sms / groups + 1,
+// so S * np <= (blocks * sms + groups) * 256.
 constexpr int kSliceThreads = 256;
-constexpr int kSliceBlocksPerSM = 4;
+constexpr int slice_blocks_per_sm(int n) { return n <= 6144 ? 3 : n <= 8192 ? 4 : 8; }
 constexpr long long massive_part_words_for(int cap, int sms) {
-    return 6LL * kSliceThreads * ((long long)kSliceBlocksPerSM * sms + (cap + kSliceThreads - 1) / kSliceThreads);
+    return 6LL * kSliceThreads * ((cap <= 8192 ? 4LL : 8LL) * sms + (cap + kSliceThreads - 1) / kSliceThreads);
 }
 
 // Precisions the step entry points take.

@@ -838,7 +838,7 @@ cudaError_t launch_pairs(const ddx_state& s, const StepArgs& a, MassiveScratch& 
 int massive_slices(int n_grav, int n_exact) {
     const int groups = (n_grav + kSliceThreads - 1) / kSliceThreads;
     const int spans = pair_count(n_grav - n_exact) / kPairSpan;
-    int S = (kSliceBlocksPerSM * sm_count() + groups - 1) / groups;
+    int S = (slice_blocks_per_sm(n_grav) * sm_count() + groups - 1) / groups;
     if (S > kMaxSlices) S = kMaxSlices;
     if (S > spans) S = spans;
     return S < 1 ? 1 : S;

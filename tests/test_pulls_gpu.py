@@ -54,8 +54,10 @@ def check_velocities(s, f, m, rows, rel=2e-6):
 
 
 # a slice block's 256 targets and 128 threads, a tile's pairs, the one-launch order's threshold
-# 1,024 and its list of 1,024 keys a block, and 8,192, where the order goes to the radix sort
-@pytest.mark.parametrize("n_plsml", [2, 125, 126, 253, 254, 1023, 1024, 1025, 2047, 2049, 8191, 8192, 8193])
+# 1,024 and its list of 1,024 keys a block, 6,144 and 8,192 bodies, where the slices become more, and 8,192
+# planetesimals, where the order goes to the radix sort
+@pytest.mark.parametrize("n_plsml", [2, 125, 126, 253, 254, 1023, 1024, 1025, 2047, 2049, 6141, 6142, 8189, 8190, 8191, 8192,
+                                     8193])
 def test_massive_set_pulls(engine, n_plsml):
     s = heavy_ring(n_plsml, 64)
     f = one_step(engine, s, s.state, abi.DDX_PREC_FP64)
