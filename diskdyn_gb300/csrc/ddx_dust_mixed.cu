@@ -24,6 +24,9 @@
 // the lanes test only the rest.  This runs from kOrderMinSources planetesimals on; with
 // fewer, every span takes the full separation in index order.
 //
+// From kCellMinSources planetesimals on the mixed step takes the far ones through cell
+// expansions instead (ddx_cells.cu, ddx_dust_cells.cu); this kernel then serves the compensated step.
+//
 // Blackwell mapping:
 //  - perturbers arrive as 64-byte pair records (two bodies per record, one quantity of
 //    both bodies per 8-byte slot), and every FP32 operation of the pair force runs as one
@@ -758,7 +761,6 @@ cudaError_t launch_dust_mixed(const ddx_state& s, const StepArgs& a, const Massi
     // cell expansions from kCellMinSources planetesimals on (the lost-copy test hook needs tiles)
     if (!comp && ms.cells && ms.dust_order.cap >= a.n_dust && a.n_grav - a.n_exact >= kCellMinSources && a.lose_tile < 0)
         return launch_dust_cells(s, a, ms, bins, st);
-    // four lanes per tracer while the GPU is not full without (kLanesFew)
     const bool lanes = a.n_grav - a.n_exact >= kLanesMinSources && a.n_dust <= (comp ? kLanesFewComp : kLanesFew);
     const bool many = a.n_dust >= kManyTracers;
     constexpr int kHalf = kThreads / 2;
