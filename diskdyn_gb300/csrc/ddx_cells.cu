@@ -697,24 +697,22 @@ cells_split_kernel(CellView v, int level, float near_eta) {
     }
 }
 
-// The expansions of every node's newly far groups (near the parent, not near the node), all
-// levels in one launch: the coarse levels' nodes have thousands of sources and take a block
-// each, the others a warp each, handed out as blocks and warps become free.  What bounds it is the FP32 pipe, about 60 % busy: about 200
-// instructions a source, most of them f32x2, and 900 per node (belt of 4,096 with a million
-// tracers: 32,000 nodes, 12 million sources, 190 us).
+// The expansions of every node's newly far groups (near the parent, not near the node), all levels at
+// once: a warp per node, handed out from the top level down as warps become free (with a block of four
+// warps for every node above the finest two levels 4,096 planetesimals with 16,384 tracers took 657 us a
+// step, 608 so, 3,001 with a halo and 500,003 1862 and 1769).  What bounds it
+// is the FP32 pipe, about 60 % busy: about 200 instructions a source, most of them f32x2, and
+// 900 per node (belt of 4,096 with a million tracers: 32,000 nodes, 12 million sources, 190 us).
 constexpr int kFarList = 256;                    // far groups listed at once per node
 constexpr int kRedParts = (kReal + 31) / 32, kRedRows = (kReal + kRedParts - 1) / kRedParts, kRedStride = 36;
 struct FarShared {
     unsigned char list[kNodeWarps][kFarList];
     float red[kNodeWarps][kRedRows][kRedStride];
     float sum[kNodeWarps][kReal];
-    int item;
 };
 
-template <int W>
 __device__ __forceinline__ void far_sums(const CellView& v, int k, FarShared& sh) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int w0 = W > 1 ? warp : 0, lead = W > 1 ? 0 : warp;   // this warp's share of the node, the node's first warp
     auto& list = sh.list[warp];
     auto& red = sh.red;
     auto& sum = sh.sum;
@@ -727,8 +725,7 @@ __device__ __forceinline__ void far_sums(const CellView& v, int k, FarShared& sh
 #pragma unroll
     for (int q = 0; q < kAcc; ++q) acc[q] = 0;
     float S[3] = {0.f, 0.f, 0.f}, C[3] = {0.f, 0.f, 0.f};
-    // every warp lists the node's far groups (the same list), 8 words of groups at a time, and
-    // takes its share of them
+    // the node's far groups are listed, 8 words of groups at a time
     for (int w = 0; w < v.words; w += kFarList / 32) {
         uint32_t far = 0;
         if (lane < kFarList / 32 && w + lane < v.words) {
@@ -745,7 +742,7 @@ __device__ __forceinline__ void far_sums(const CellView& v, int k, FarShared& sh
         __syncwarp();
         // 32 sources at a time, one per lane; the next ones are loaded ahead
         constexpr int kPerIt = 32 / kGroupSrc;    // groups
-        int e = kPerIt * w0 + lane / kGroupSrc;
+        int e = lane / kGroupSrc;
         const int u = lane & (kGroupSrc - 1);
         float4 h, l;
         int q = -1;
@@ -755,10 +752,10 @@ __device__ __forceinline__ void far_sums(const CellView& v, int k, FarShared& sh
                 h = src[2 * q];
                 l = src[2 * q + 1];
             }
-            e += kPerIt * W;
+            e += kPerIt;
         };
         fetch();
-        for (int b = kPerIt * w0; b < n; b += kPerIt * W) {
+        for (int b = 0; b < n; b += kPerIt) {
             const bool use = q < v.n_src;
             const float dx = ((h.x - cx) + l.x) * inv_s, dy = ((h.y - cy) + l.y) * inv_s;
             const float dz = ((h.z - cz) + l.z) * inv_s, m = h.w;
@@ -814,21 +811,11 @@ __device__ __forceinline__ void far_sums(const CellView& v, int k, FarShared& sh
         if (lane < kRedRows && part * kRedRows + lane < kReal) sum[warp][part * kRedRows + lane] = t;
         __syncwarp();
     });
-    if constexpr (W > 1) __syncthreads();
-    if (w0 == 0)
-        for (int i = lane; i < kReal; i += 32) {
-            float t = 0.f, c = 0.f;
-#pragma unroll
-            for (int j = 0; j < W; ++j) kahan_sum(t, c, sum[lead + j][i]);
-            if (W > 1 && i < 32) {                // degree 1: what the warps' sum lost goes to its low part
-                const float c0 = __shfl_sync(0xffffffffu, c, 0), c2 = __shfl_sync(0xffffffffu, c, 2);
-                const float c3 = __shfl_sync(0xffffffffu, c, 3);
-                if (is_low(i)) t -= i == low_of(0) ? c0 : i == low_of(2) ? c2 : c3;
-            }
-            v.lam[(size_t)k * kReal + i] = is_low(i) || low_of(i) >= 0 ? t : t * v.tab->w[i];   // degree 1: w = 1
-        }
-    if constexpr (W > 1) __syncthreads();
-    else __syncwarp();
+    for (int i = lane; i < kReal; i += 32) {
+        const float t = sum[warp][i];
+        v.lam[(size_t)k * kReal + i] = is_low(i) || low_of(i) >= 0 ? t : t * v.tab->w[i];   // degree 1: w = 1
+    }
+    __syncwarp();
 }
 
 // The expansion of all planetesimals about the origin, per stage, for distant
@@ -996,27 +983,18 @@ cells_far_kernel(CellView v, int distant_blocks) {
         distant_sums(v, blockIdx.x / distant_blocks, blockIdx.x % distant_blocks, distant_blocks, sh.distant);
         __syncthreads();
     }
-    // the levels from the top down are one range of nodes; its first part is coarse
-    int coarse = 0, total = 0;
+    // the levels from the top down are one range of nodes
+    int total = 0;
     for (int l = v.levels - 1; l >= 0; --l) {
         int first;
         total += level_nodes(v, l, first);
-        if (l >= 2) coarse = total;
-    }
-    for (;;) {
-        if (threadIdx.x == 0) sh.far.item = (int)atomicAdd(&v.grid->taken[0], 1u);
-        __syncthreads();
-        const int k = sh.far.item;
-        __syncthreads();
-        if (k >= coarse) break;
-        far_sums<kNodeWarps>(v, k, sh.far);
     }
     for (;;) {
         int k = 0;
-        if ((threadIdx.x & 31) == 0) k = coarse + (int)atomicAdd(&v.grid->taken[1], 1u);
+        if ((threadIdx.x & 31) == 0) k = (int)atomicAdd(&v.grid->taken, 1u);
         k = __shfl_sync(0xffffffffu, k, 0);
         if (k >= total) break;
-        far_sums<1>(v, k, sh.far);
+        far_sums(v, k, sh.far);
     }
 }
 
@@ -1030,7 +1008,7 @@ __device__ __forceinline__ float add_exact(float& a, float b) {
 
 // One level: the parents' expansions, translated, added to the nodes', and the terms of the
 // force components.  A block takes kShiftNodes nodes, a thread per coefficient.
-constexpr int kShiftNodes = 8;
+constexpr int kShiftNodes = 4;
 constexpr int kShiftThreads = (kReal + 31) / 32 * 32;
 constexpr int kForceSplit = kShiftThreads / kCellForce;     // nodes whose force terms are formed at once
 
@@ -1280,7 +1258,7 @@ cudaError_t cells_build(CellScratch* c, const ddx_state& s, const StepArgs& a, c
     launch_after(cells_ancestors_kernel, dim3(chunks, 3), 1024, 0, st, v);
     launch_after(cells_roots_kernel, kCellTop * kCellTop * kCellTop / kRootThreads, kRootThreads, 0, st, v);
     for (int l = v.levels - 1; l >= 0; --l)
-        launch_after(cells_split_kernel, 608, kNodeThreads, 0, st, v, l, a.near_eta);
+        launch_after(cells_split_kernel, 1216, kNodeThreads, 0, st, v, l, a.near_eta);
     const int db = (v.n_src + 4 * kNodeThreads - 1) / (4 * kNodeThreads);
     launch_after(cells_far_kernel, 456, kNodeThreads, 0, st, v, db < kMultiBlocks ? db : kMultiBlocks);
     for (int l = v.levels - 1; l >= 0; --l) launch_after(cells_shift_kernel, 1520, kShiftThreads, 0, st, v, l);

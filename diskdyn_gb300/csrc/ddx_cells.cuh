@@ -33,7 +33,7 @@ struct CellGrid {
     int   leaf;                // most groups near a cell that is not split
     int   min_level;           // levels below it were dropped (out of nodes)
     uint32_t cnt[kCellMaxLevels];     // nodes per level
-    uint32_t taken[2];                // coarse nodes and fine nodes taken by cells_far_kernel
+    uint32_t taken;                   // nodes taken by cells_far_kernel
     uint32_t first[kCellMaxLevels];   // first node of each level (the top's is 0)
 };
 
