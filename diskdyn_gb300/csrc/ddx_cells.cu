@@ -41,6 +41,7 @@
 #include <vector>
 #include "ddx_launch.cuh"
 #include "ddx_cells.cuh"
+#include "ddx_shift.cuh"
 #include "ddx_scan.cuh"
 
 namespace ddx {
@@ -1087,19 +1088,8 @@ cells_shift_kernel(CellView v, int level) {
             }
             __syncthreads();
             if (i < kReal) {
-                float acc[kShiftNodes];
-#pragma unroll
-                for (int j = 0; j < kShiftNodes; ++j) acc[j] = 0.f;
-#pragma unroll 4
-                for (int e = e0; e < e1; ++e) {
-                    const float c = sh_val[e];
-                    const float4* p = reinterpret_cast<const float4*>(par[sh_idx[e]]);
-                    const float4 p0 = p[0], p1 = p[1];
-                    acc[0] = fmaf(c, p0.x, acc[0]); acc[1] = fmaf(c, p0.y, acc[1]);
-                    acc[2] = fmaf(c, p0.z, acc[2]); acc[3] = fmaf(c, p0.w, acc[3]);
-                    acc[4] = fmaf(c, p1.x, acc[4]); acc[5] = fmaf(c, p1.y, acc[5]);
-                    acc[6] = fmaf(c, p1.z, acc[6]); acc[7] = fmaf(c, p1.w, acc[7]);
-                }
+                float acc[kShiftNodes] = {};
+                shift_sums(par, sh_val, sh_idx, e0, e1, acc);
 #pragma unroll
                 for (int j = 0; j < kShiftNodes; ++j) {
                     const float rest = __popc(flip & neg[j]) & 1 ? -acc[j] : acc[j];
