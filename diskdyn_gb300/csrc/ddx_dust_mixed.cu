@@ -569,8 +569,12 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
             lost = __syncthreads_or(lost);      // also: every thread is done with tile g-1
             if (lost) break;
             if (tid == 0 && g + 1 < G) issue(g + 1);
-            if (!mbar_wait(mb[g & 1], (g >> 1) & 1, a.wait_ns)) { lost = 1; continue; }
-            if (tid == 0) in_flight[g & 1] = -1;
+            const bool landed = mbar_wait(mb[g & 1], (g >> 1) & 1, a.wait_ns);
+            if (tid == 0 && landed) in_flight[g & 1] = -1;
+            // Every lane times its own wait, and a copy can land after one lane's limit and before its
+            // neighbour's: the lanes of a team go on together, or some would wait for the others
+            // in the team's ballot and these for them at the barrier.
+            if (!(T > 1 ? __all_sync(team, landed) : landed)) { lost = 1; continue; }
             if (!alive) continue;
             const BodyPair* const T_ = tiles + (g & 1) * NT;
             const int cnt = min(NT, npairs - tt * NT);   // a multiple of kPairSpan
@@ -734,8 +738,9 @@ dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin*
         if (tid == 0) {
             atomicOr(ms.status, kStatusTimeout);
             // let this block's copies that are still in flight land before it exits
+            const unsigned long long limit = a.wait_ns > kDefaultWaitNs ? a.wait_ns : kDefaultWaitNs;
             for (int b = 0; b < 2; ++b)
-                if (in_flight[b] >= 0) mbar_wait(mb[b], (in_flight[b] >> 1) & 1, a.wait_ns);
+                if (in_flight[b] >= 0) mbar_wait(mb[b], (in_flight[b] >> 1) & 1, limit);
         }
         return;
     }
