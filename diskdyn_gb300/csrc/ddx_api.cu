@@ -34,6 +34,7 @@ struct ddx_ctx {
     float near_eta = -1.f;                      // FP64 pulls within near_eta * |coordinate| (< 0: defaults)
     float comp_eta = kDefaultCompEta;           // compensated path: float-float spans within comp_eta * |coordinate|
     int inject_lose_tile = -1;                  // one-shot test hook for the next mixed dust launch
+    int inject_cells_most = -1;                 // test hook: no room for cells of more planetesimals (< 0: off)
     unsigned long long inject_wait_ns = 0;
     CollideScratch* collide = nullptr;          // spatial-hash buffers, grown on demand
     AdjointScratch* adjoint = nullptr;          // trajectory checkpoints of the last adjoint forward
@@ -78,9 +79,23 @@ void free_massive(MassiveScratch& ms) {
 
 int alloc_massive(ddx_ctx* c, int n_grav);
 
+// The cells' scratch for n planetesimals.  Without it the mixed step takes every planetesimal one
+// by one.  A refused size is not asked for again with this massive scratch, so that a run's
+// steps stay alike; a stream that is capturing takes what is there.
+void ensure_cells(ddx_ctx* c, int n, cudaStream_t st) {
+    if (cells_hold(c->ms.cells, n) || (c->ms.cells_refused && n >= c->ms.cells_refused)) return;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return;
+    const bool room = c->inject_cells_most < 0 || n <= c->inject_cells_most;
+    if (!room || cells_ensure(c->ms.cells, n, c->ms.cap) != cudaSuccess) {
+        cudaGetLastError();
+        c->ms.cells_refused = n;
+    }
+}
+
 // The massive set's scratch for n_grav bodies and, for the mixed path, the scratch of the
 // spatial order of the sources and of n_dust tracers (grown on demand).
-int ensure_massive(ddx_ctx* c, int n_grav, int n_dust, int precision) {
+int ensure_massive(ddx_ctx* c, int n_grav, int n_dust, int precision, cudaStream_t st) {
     if (!(c->ms.cap >= n_grav && c->ms.P)) {
         const int r = alloc_massive(c, n_grav);
         if (r) return r;
@@ -91,9 +106,7 @@ int ensure_massive(ddx_ctx* c, int n_grav, int n_dust, int precision) {
             return DDX_ERR_NOMEM;
         }
     }
-    // without room for the cells' scratch the mixed step takes every planetesimal one by one
-    if (precision == DDX_PREC_MIXED && n_grav > kCellMinSources && cells_ensure(c->ms.cells, n_grav) != cudaSuccess)
-        cudaGetLastError();
+    if (precision == DDX_PREC_MIXED && n_dust > 0 && n_grav > kCellMinSources) ensure_cells(c, n_grav, st);
     return DDX_OK;
 }
 
@@ -396,8 +409,8 @@ int ddx_step_host(ddx_ctx* c, const ddx_host_state* in, ddx_host_state* out, con
     int r = make_step_args(c, phys, n_grav, n_dust, dt, mode, a, precision);
     if (r) return r;
     DeviceGuard dg(c->device);
-    if ((r = ensure_massive(c, n_grav, n_dust, precision)) || (r = ensure_pipeline(c))) return r;
     cudaStream_t st = (cudaStream_t)stream;
+    if ((r = ensure_massive(c, n_grav, n_dust, precision, st)) || (r = ensure_pipeline(c))) return r;
     take_injection(c, a);
     // the massive bodies: in, step, out (small)
     if (!h2d_range(*s, *in, 0, n_grav, st)) return DDX_ERR_CUDA;
@@ -444,8 +457,8 @@ int ddx_evolve(ddx_ctx* c, const ddx_state* s, int n_grav, int n_dust, double dt
     int r = make_step_args(c, phys, n_grav, n_dust, dt, mode, a, precision);
     if (r) return r;
     DeviceGuard dg(c->device);
-    if ((r = ensure_massive(c, n_grav, n_dust, precision))) return r;
     cudaStream_t st = (cudaStream_t)stream;
+    if ((r = ensure_massive(c, n_grav, n_dust, precision, st))) return r;
     for (int k = 0; k < n_steps; ++k)
         if ((r = enqueue_step(c, *s, a, precision, st))) return r;
     return DDX_OK;
@@ -453,13 +466,13 @@ int ddx_evolve(ddx_ctx* c, const ddx_state* s, int n_grav, int n_dust, double dt
 
 namespace {
 int prepare_call(ddx_ctx* c, const ddx_state* s, int n_grav, int n_dust, double dt,
-                 const ddx_phys* phys, int precision, int mode, StepArgs& a) {
+                 const ddx_phys* phys, int precision, int mode, StepArgs& a, void* stream) {
     if (!c || !state_ok(s)) return DDX_ERR_ARG;
     if (!step_precision_ok(precision)) return DDX_ERR_ARG;
     if (!c->bins) return DDX_ERR_STATE;
     int r = make_step_args(c, phys, n_grav, n_dust, dt, mode, a, precision);
     if (r) return r;
-    return ensure_massive(c, n_grav, n_dust, precision);   // the caller made c's device current
+    return ensure_massive(c, n_grav, n_dust, precision, (cudaStream_t)stream);   // the caller made c's device current
 }
 }  // namespace
 
@@ -468,7 +481,7 @@ int ddx_massive_rk4(ddx_ctx* c, const ddx_state* s, int n_grav, int n_dust, doub
     if (!c) return DDX_ERR_ARG;
     DeviceGuard dg(c->device);
     StepArgs a;
-    int r = prepare_call(c, s, n_grav, n_dust, dt, phys, precision, mode, a);
+    int r = prepare_call(c, s, n_grav, n_dust, dt, phys, precision, mode, a, stream);
     if (r) return r;
     cudaStream_t st = (cudaStream_t)stream;
     if (a.n_grav == 1 && a.mode == DDX_MODE_REFERENCE) {
@@ -484,7 +497,7 @@ int ddx_small_rk4(ddx_ctx* c, const ddx_state* s, int n_grav, int n_dust, double
     if (!c) return DDX_ERR_ARG;
     DeviceGuard dg(c->device);
     StepArgs a;
-    int r = prepare_call(c, s, n_grav, n_dust, dt, phys, precision, mode, a);
+    int r = prepare_call(c, s, n_grav, n_dust, dt, phys, precision, mode, a, stream);
     if (r) return r;
     take_injection(c, a);
     return cuda_status(launch_dust(*s, a, c->ms, c->bins, precision, (cudaStream_t)stream));
@@ -620,12 +633,18 @@ int ddx_debug_lose_tile_copy(ddx_ctx* c, int tile, unsigned long long wait_ns) {
     return DDX_OK;
 }
 
+int ddx_debug_limit_cells(ddx_ctx* c, int most) {
+    if (!c) return DDX_ERR_ARG;
+    c->inject_cells_most = most;
+    return DDX_OK;
+}
+
 int ddx_massive_final(ddx_ctx* c, const ddx_state* s, int n_grav, int n_dust, double dt,
                       const ddx_phys* phys, int precision, int mode, void* stream) {
     if (!c) return DDX_ERR_ARG;
     DeviceGuard dg(c->device);
     StepArgs a;
-    int r = prepare_call(c, s, n_grav, n_dust, dt, phys, precision, mode, a);
+    int r = prepare_call(c, s, n_grav, n_dust, dt, phys, precision, mode, a, stream);
     if (r) return r;
     if (a.n_grav == 1 && a.mode == DDX_MODE_REFERENCE) return DDX_OK;
     return cuda_status(launch_massive_pass2(*s, a, c->ms, precision, (cudaStream_t)stream));

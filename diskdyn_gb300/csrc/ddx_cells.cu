@@ -38,6 +38,7 @@
 #include <cmath>
 #include <complex>
 #include <cstring>
+#include <new>
 #include <vector>
 #include "ddx_launch.cuh"
 #include "ddx_cells.cuh"
@@ -48,6 +49,7 @@ namespace ddx {
 
 struct CellScratch {
     char* arena = nullptr;
+    CellScratch* outgrown = nullptr;
     CellView v{};
     uint32_t *count = nullptr, *start = nullptr, *temp = nullptr;   // the tracers' counting sort
     unsigned long long* sums = nullptr;                             // of cells_setup_kernel
@@ -1142,15 +1144,19 @@ size_t round256(size_t n) { return (n + 255) / 256 * 256; }
 }  // namespace
 
 void cells_free(CellScratch*& c) {
-    if (!c) return;
-    cudaFree(c->arena);
-    delete c;
-    c = nullptr;
+    while (c) {
+        CellScratch* const next = c->outgrown;
+        cudaFree(c->arena);
+        delete c;
+        c = next;
+    }
 }
 
-cudaError_t cells_ensure(CellScratch*& c, int n_src) {
-    if (c && c->cap_src >= n_src) return cudaSuccess;
-    const int cap_src = (n_src + 1023) / 1024 * 1024;
+bool cells_hold(const CellScratch* c, int n_src) { return c && c->cap_src >= n_src; }
+
+cudaError_t cells_ensure(CellScratch*& c, int n_src, int most) {
+    if (cells_hold(c, n_src)) return cudaSuccess;
+    const int want = c && most > n_src ? most : n_src, cap_src = (want + 1023) / 1024 * 1024;
     static CellTables tab;
     static const bool tab_ok = make_tables(tab);
     if (!tab_ok) return cudaErrorInvalidValue;
@@ -1175,7 +1181,11 @@ cudaError_t cells_ensure(CellScratch*& c, int n_src) {
     char* arena = nullptr;
     cudaError_t e = cudaMalloc((void**)&arena, total);
     if (e != cudaSuccess) return e;
-    CellScratch* n = new CellScratch();
+    CellScratch* n = new (std::nothrow) CellScratch();
+    if (!n) {
+        cudaFree(arena);
+        return cudaErrorMemoryAllocation;
+    }
     n->arena = arena;
     n->cap_src = cap_src;
     char* p = arena;
@@ -1210,13 +1220,14 @@ cudaError_t cells_ensure(CellScratch*& c, int n_src) {
         cells_free(n);
         return e;
     }
-    cells_free(c);
+    n->outgrown = c;
     c = n;
     return cudaSuccess;
 }
 
 cudaError_t cells_build(CellScratch* c, const ddx_state& s, const StepArgs& a, const MassiveScratch& ms,
                         const SizeBin* bins, CellView& v, cudaStream_t st) {
+    if (!cells_hold(c, a.n_grav - a.n_exact)) return cudaErrorInvalidValue;
     v = c->v;
     v.n_src = a.n_grav - a.n_exact;
     v.n_groups = (v.n_src + kGroupSrc - 1) / kGroupSrc;

@@ -764,7 +764,8 @@ cudaError_t launch_dust_mixed(const ddx_state& s, const StepArgs& a, const Massi
     if (a.n_dust <= 0) return cudaSuccess;
     const bool comp = precision == DDX_PREC_COMPENSATED;
     // cell expansions from kCellMinSources planetesimals on (the lost-copy test hook needs tiles)
-    if (!comp && ms.cells && ms.dust_order.cap >= a.n_dust && a.n_grav - a.n_exact >= kCellMinSources && a.lose_tile < 0)
+    if (!comp && a.n_grav - a.n_exact >= kCellMinSources && cells_hold(ms.cells, a.n_grav - a.n_exact) &&
+        ms.dust_order.cap >= a.n_dust && a.lose_tile < 0)
         return launch_dust_cells(s, a, ms, bins, st);
     const bool lanes = a.n_grav - a.n_exact >= kLanesMinSources && a.n_dust <= (comp ? kLanesFewComp : kLanesFew);
     const bool many = a.n_dust >= kManyTracers;

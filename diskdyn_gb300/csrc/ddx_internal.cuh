@@ -136,9 +136,13 @@ __host__ __device__ inline bool spatial_order_on(const StepArgs& a) {
     return a.n_grav - a.n_exact >= kOrderMinSources;
 }
 
-// Buffers of the mixed step's cell expansions (ddx_cells.cu), for up to n_src planetesimals.
+// Buffers of the mixed step's cell expansions (ddx_cells.cu).  cells_ensure makes them hold n_src
+// planetesimals, or `most` when they have to grow; on failure they stay as they were, so a step
+// asks cells_hold before it uses them.  Buffers that were outgrown live on until cells_free: a captured step may
+// replay with them.
 struct CellScratch;
-cudaError_t cells_ensure(CellScratch*& c, int n_src);
+cudaError_t cells_ensure(CellScratch*& c, int n_src, int most);
+bool cells_hold(const CellScratch* c, int n_src);
 void cells_free(CellScratch*& c);
 
 // The mixed step takes far planetesimals through cell expansions (ddx_cells.cu) from this many
@@ -171,6 +175,7 @@ struct MassiveScratch {
     OrderScratch src_order;    // ordering of the FP32 sources (cap bodies)
     OrderScratch dust_order;   // ordering of the tracers of one dust launch
     CellScratch *cells;        // trees of the mixed dust kernel with many planetesimals (ddx_cells.cu)
+    int      cells_refused;    // planetesimals from which on there was no room for them (0: none known)
 };
 
 // Makes `device` current for the scope of an entry point and makes the caller's current

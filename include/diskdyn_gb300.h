@@ -135,7 +135,11 @@ int ddx_set_optics(ddx_ctx *ctx, int n_grid, int n_wav, int n_theta, const doubl
  * FP32 high parts alone.  From 2,048 planetesimals on, those far from a tracer's cell of
  * space act through the cell's expansion (harmonics to degree 10; at most 2.6e-6 of one
  * such pull is left out, the size of the FP32 pulls' own rounding over all of them) and only
- * the others one by one.
+ * the others one by one.  The cells take device memory on the context's first such step: 0.5 GB
+ * at 2,049 massive bodies, 0.8 GB at 4,099, 3.4 GB at 20,000, 6.2 GB at 65,539.  Where there is
+ * no room for it, or that first step is being captured, every planetesimal is taken one by
+ * one, in more time and with other last bits; a size once refused is not asked for again until
+ * the number of massive bodies passes the next power of two.
  * Each tracer's result depends on its own data and the massive set only (not on the
  * other tracers or their order), and the result is the same from run to run. */
 int ddx_step(ddx_ctx *ctx, const ddx_state *s, int n_grav, int n_dust, double dt,
@@ -380,6 +384,11 @@ int ddx_set_compensated_radius(ddx_ctx *ctx, double eta);
  * unchanged.  Nothing faults or hangs; the context stays usable.  That launch takes every
  * planetesimal one by one (cell expansions have no tiles). */
 int ddx_debug_lose_tile_copy(ddx_ctx *ctx, int tile, unsigned long long wait_ns);
+
+/* Failure-detection test hook (no counterpart in the reference).  From now on the device memory
+ * of the cell expansions is refused to this context for more than `most` planetesimals, as if
+ * it had run out; negative: no more.  What the context has already is not taken away. */
+int ddx_debug_limit_cells(ddx_ctx *ctx, int most);
 
 /* Error string for a status code. */
 const char *ddx_status_string(int status);
