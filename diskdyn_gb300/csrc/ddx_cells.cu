@@ -315,13 +315,14 @@ __device__ __forceinline__ uint32_t hilbert(uint32_t (&X)[D]) {
 // Place of a position (relative to the origin) in the tracers' visiting order, 21 bits: the
 // Hilbert order of 128^3 cells of edge s0 (G = 128; 2 s0 at 256), or, in a thin disk, of
 // 256 x 256 x 32 cells of half that edge (32^3 blocks in Hilbert order, the 8 x 8 cells of a
-// block in the plane's), clamped at their border.  inside: it is not clamped.
+// block in the plane's), clamped at their border.  inside: its cell is not at the border, so it
+// holds no clamped position.
 __device__ __forceinline__ uint32_t order_code(const CellGrid& g, int G, const CellPos& p, bool& inside) {
     const float sc = g.inv_s0 * (128.f / (float)G);
     if (g.thin) {
         const float ux = floorf(p.x * sc * 2.f) + 128.f, uy = floorf(p.y * sc * 2.f) + 128.f;
         const float uz = floorf(p.z * sc * 2.f) + 16.f;
-        inside = ux >= 0.f && ux < 256.f && uy >= 0.f && uy < 256.f && uz >= 0.f && uz < 32.f;
+        inside = ux >= 1.f && ux < 255.f && uy >= 1.f && uy < 255.f && uz >= 1.f && uz < 31.f;
         const uint32_t x = (uint32_t)(int)fminf(fmaxf(ux, 0.f), 255.f);   // NaN gives 0
         const uint32_t y = (uint32_t)(int)fminf(fmaxf(uy, 0.f), 255.f);
         const uint32_t z = (uint32_t)(int)fminf(fmaxf(uz, 0.f), 31.f);
@@ -329,7 +330,7 @@ __device__ __forceinline__ uint32_t order_code(const CellGrid& g, int G, const C
         return hilbert<3, 5>(hi) << 6 | hilbert<2, 3>(lo);
     }
     const float ux = floorf(p.x * sc) + 64.f, uy = floorf(p.y * sc) + 64.f, uz = floorf(p.z * sc) + 64.f;
-    inside = ux >= 0.f && ux < 128.f && uy >= 0.f && uy < 128.f && uz >= 0.f && uz < 128.f;
+    inside = ux >= 1.f && ux < 127.f && uy >= 1.f && uy < 127.f && uz >= 1.f && uz < 127.f;
     uint32_t c[3] = {(uint32_t)(int)fminf(fmaxf(ux, 0.f), 127.f), (uint32_t)(int)fminf(fmaxf(uy, 0.f), 127.f),
                      (uint32_t)(int)fminf(fmaxf(uz, 0.f), 127.f)};
     return hilbert<3, 7>(c);
@@ -342,11 +343,18 @@ __device__ __forceinline__ void mark_cell(const CellView& v, int set, const Cell
     if (!(*(volatile uint32_t*)w & bit)) atomicOr(w, bit);
 }
 
+// No position in p's finest cell is distant (a hundredth of slack for the roundings).
+__device__ __forceinline__ bool cell_within_distant(const CellGrid& g, const CellPos& p) {
+    const float ax = fabsf(p.x) + g.s0, ay = fabsf(p.y) + g.s0, az = fabsf(p.z) + g.s0;
+    return ax * ax + ay * ay + az * az < 0.99f * kDistant * kDistant * __uint_as_float(g.b2);
+}
+
 // Per tracer: its place in the visiting order (by its expected position in the middle of the
 // step; removed tracers last) with an atomic rank in it, and the marks of the cells where
 // it is expected to be during the step.  The marks are what this kernel waits for
 // (scattered words that every SM reads), so the middle's cell is marked by the first of its
-// tracers alone where the order's cells are no larger than the tree's.
+// tracers alone where all tracers of a cell of the order would mark the same one: the order's cells
+// are no larger than the tree's finest, the cell holds no clamped position and no distant one.
 __global__ void cells_keys_kernel(ddx_state s, StepArgs a, const SizeBin* __restrict__ bins, CellView v,
                                   uint32_t* __restrict__ key, uint32_t* __restrict__ rank,
                                   uint32_t* __restrict__ count) {
@@ -373,8 +381,7 @@ __global__ void cells_keys_kernel(ddx_state s, StepArgs a, const SizeBin* __rest
                 if (cell_distant(g, p.x, p.y, p.z)) continue;
                 const CellAt at = cell_at(g, v.G, v.levels, p);
                 if (at.level < 0) continue;
-                // the first tracer of a cell of the order marks it where that is no larger than a tree cell
-                if (k == 1 && first != 0 && at.level == 0 && inside && (v.G == 128 || g.thin)) continue;
+                if (k == 1 && first != 0 && inside && (v.G == 128 || g.thin) && cell_within_distant(g, p)) continue;
                 mark_cell(v, mark_set(k), at);
             }
         }
