@@ -12,8 +12,9 @@
 // part by part, 16 bytes a record, and a tracer starts at the record given by the group's
 // number: lanes with different groups then read different banks (a belt of 4,096 with
 // a million tracers 1575 -> 1515 us, 3,001 planetesimals with 30,000 tracers 234 -> 171 us).
-// A tracer outside every grid, with a non-finite position, or further from its cell's centre
-// than kReach edges (it moved more in the step than expected) takes every planetesimal.
+// A tracer outside every grid, with a non-finite position, further from its cell's centre
+// than kReach edges (it moved more in the step than expected), or expected to be distant but out
+// of the distant expansion's reach takes every planetesimal.
 #include "ddx_launch.cuh"
 #include "ddx_cells.cuh"
 #include "ddx_pull.cuh"
@@ -80,6 +81,16 @@ __device__ __forceinline__ void l2p(const float4* __restrict__ F, float x, float
     f2_split(SX, s, t); ax = s + t;
     f2_split(SY, s, t); ay = s + t;
     f2_split(SZ, s, t); az = s + t;
+}
+
+// Whether a tracer that is expected to be distant may take the distant expansion at (x, y, z) from the
+// origin: still kDistantReach times the core's largest distance away (the series is then as good
+// as a cell's, 1 / 5.5 against 0.21), and with no planetesimal of the core within its near radius, near_eta times
+// its largest |coordinate| own (each is at least 1 - 1 / 5.5 of its distance away).
+constexpr float kDistantReach = 5.5f;
+__device__ __forceinline__ bool distant_reach(const CellGrid& g, float x, float y, float z, float near_eta, float own) {
+    const float r2 = fmaf(x, x, fmaf(y, y, z * z)), near = 1.25f * near_eta * own;
+    return r2 >= kDistantReach * kDistantReach * __uint_as_float(g.b2) && r2 >= near * near;
 }
 
 // The acceleration of the distant expansion at (x, y, z) from the origin, in its unit.
@@ -412,16 +423,19 @@ dust_cells_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __r
         if (alive) {
             const CellGrid& g = *v.grid;
             float dx = (X[0] - g.ox) + X[1], dy = (X[2] - g.oy) + X[3], dz = (X[4] - g.oz) + X[5];
-            if (cell_distant(g, dx, dy, dz)) {
-                node = kDistantNode;
-                const float u = g.inv_s0 * (1.f / kFarUnit);
-                m2p(v.distant + (size_t)st * kFarForce4, dx * u, dy * u, dz * u, fx, fy, fz);
-                add_point(v.point[st], col, st, a);
+            // the expected place decides, as it did when the cells were marked: another place could
+            // send the tracer to a cell that only others' marks have built
+            const CellPos at = cell_predict(g, col.get(qX), col.get(qY), col.get(qZ), col.get(qVx), col.get(qVy),
+                                            col.get(qVz), red, dtf, st);
+            if (cell_distant(g, at.x, at.y, at.z)) {
+                if (distant_reach(g, dx, dy, dz, a.near_eta, fmaxf(fabsf(X[0]), fmaxf(fabsf(X[2]), fabsf(X[4]))))) {
+                    node = kDistantNode;
+                    const float u = g.inv_s0 * (1.f / kFarUnit);
+                    m2p(v.distant + (size_t)st * kFarForce4, dx * u, dy * u, dz * u, fx, fy, fz);
+                    add_point(v.point[st], col, st, a);
+                }
             } else {
-                const CellAt at = cell_at(g, v.G, v.levels, cell_predict(g, col.get(qX), col.get(qY), col.get(qZ),
-                                                                         col.get(qVx), col.get(qVy), col.get(qVz), red,
-                                                                         dtf, st));
-                node = find_node(v, at, st, X[0], X[1], X[2], X[3], X[4], X[5], dx, dy, dz);
+                node = find_node(v, cell_at(g, v.G, v.levels, at), st, X[0], X[1], X[2], X[3], X[4], X[5], dx, dy, dz);
                 if (node >= 0) l2p(v.force + (size_t)node * kCellForce4, dx, dy, dz, uni, fx, fy, fz);
             }
         }
