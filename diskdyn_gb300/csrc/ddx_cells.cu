@@ -1161,6 +1161,18 @@ void cells_free(CellScratch*& c) {
 
 bool cells_hold(const CellScratch* c, int n_src) { return c && c->cap_src >= n_src; }
 
+cudaError_t cells_count(const CellScratch* c, long long* nodes, long long* room, int* dropped, cudaStream_t st) {
+    CellGrid g;
+    cudaError_t e = cudaMemcpyAsync(&g, c->v.grid, sizeof(g), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return e;
+    *nodes = 0;
+    for (int l = g.min_level; l < kCellMaxLevels; ++l) *nodes += g.cnt[l];
+    *room = c->v.cap;
+    *dropped = g.min_level;
+    return cudaSuccess;
+}
+
 cudaError_t cells_ensure(CellScratch*& c, int n_src, int most) {
     if (cells_hold(c, n_src)) return cudaSuccess;
     const int want = c && most > n_src ? most : n_src, cap_src = (want + 1023) / 1024 * 1024;

@@ -110,7 +110,7 @@ struct OrderScratch {
     uint32_t *key, *rank;      // [cap] cell of each body, its rank in the cell
     uint32_t *count, *start;   // [kOrderBins + 1] bodies per cell, first position of each cell
     uint32_t *temp;            // scan scratch
-    int      *box;             // [6] bounding box, min then max per axis (ordered-int floats)
+    int      *box;             // [6] bounding box, min then max per axis (ordered-int floats); then bodies per octave
     int      *perm;            // [cap] the order: perm[position] = body
     int       cap;
     bool      stable;          // stable radix sort (timing-independent order) instead of atomics
@@ -123,7 +123,8 @@ void order_free(OrderScratch& o);
 // bounding box (64^3 cells; 32^3 and equal codes in index order when o is stable): the
 // Hilbert index on cubic cells when hilbert, else the Morton code on cells stretched to the
 // box per axis.  perm[position] = body - first and, when inv is given, inv[body - first] =
-// position.  With dead_last, bodies with N == 0 come last.  Stream-ordered.
+// position.  With dead_last, bodies with N == 0 come last.  A stable order leaves the few bodies far
+// beyond the others out of the box and puts them last.  Stream-ordered.
 cudaError_t order_bodies(const ddx_state& s, int first, int n, bool dead_last, const OrderScratch& o, int* perm,
                          int* inv, bool hilbert, cudaStream_t st);
 
@@ -143,6 +144,8 @@ __host__ __device__ inline bool spatial_order_on(const StepArgs& a) {
 struct CellScratch;
 cudaError_t cells_ensure(CellScratch*& c, int n_src, int most);
 bool cells_hold(const CellScratch* c, int n_src);
+// Cells of the last step (in use, room for, finest levels left out for want of room); waits for st.
+cudaError_t cells_count(const CellScratch* c, long long* nodes, long long* room, int* dropped, cudaStream_t st);
 void cells_free(CellScratch*& c);
 
 // The mixed step takes far planetesimals through cell expansions (ddx_cells.cu) from this many

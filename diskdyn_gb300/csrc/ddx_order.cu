@@ -16,6 +16,10 @@
 //    2.0e-9, 5.0e-10 and 4.7e-10 from FP64 at 24.8 ms a step, where the Hilbert order gave
 //    1.5e-9, 1.9e-9, 6.3e-10 and 8.9e-10 at 21.8 ms, and needed the float-float radius doubled
 //    (30.6 ms) to come to 8.6e-10, 1.8e-9, 8.6e-10 and 8.6e-10.
+// A few planetesimals scattered far out would stretch the box until the others share a few of
+// its cells (a belt of 4,096 with a million tracers, one of them at 30,000 AU: 16.0 ms a mixed step, 2.1 ms
+// without it).  So the sources' box leaves out those beyond the octave of distance to the star
+// that all but 1 in kFarFew reach (Octaves), and they come last.
 // The codes are sorted in one of two ways:
 //  - counting sort (the tracers: 6 bits per axis): an atomic increment gives each body its
 //    rank in its cell, an exclusive scan of the cell counts the cells' first positions, and
@@ -51,10 +55,72 @@ __device__ __forceinline__ bool removed(const ddx_state& s, int i) {
     return (((unsigned long long)__double_as_longlong(s.N[i])) << 1) == 0ull;   // N == +-0
 }
 
-__global__ void order_init_kernel(uint32_t* __restrict__ count, int* __restrict__ box) {
+// Bodies per octave of their distance from body 0 (largest coordinate difference in FP32; the
+// octave is the exponent's bits, 255: not finite), and the last octave that the box takes: beyond
+// it lies 1 body in kFarFew at most.
+constexpr int kOctaves = 256, kFarFew = 32;
+__device__ __forceinline__ int octave(const ddx_state& s, const float* v) {
+    const float m = fmaxf(fabsf(v[0] - d2f_toward0(s.x[0])), fmaxf(fabsf(v[1] - d2f_toward0(s.y[0])),
+                                                                   fabsf(v[2] - d2f_toward0(s.z[0]))));
+    const bool nan = !(v[0] == v[0] && v[1] == v[1] && v[2] == v[2]);   // fmaxf leaves NaN out
+    return nan ? kOctaves - 1 : (int)(__float_as_uint(m) >> 23);
+}
+// All lanes of a warp call it and get the result.
+__device__ __forceinline__ int last_octave(const uint32_t* hist, int n) {
+    const int lane = threadIdx.x & 31;
+    constexpr int kPer = kOctaves / 32;
+    uint32_t c[kPer], sum = 0;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) sum += c[q] = hist[lane * kPer + q];
+    uint32_t above = sum;                         // of this lane's octaves and the later lanes'
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_down_sync(0xffffffffu, above, o);
+        if (lane + o < 32) above += u;
+    }
+    above -= sum;
+    const uint32_t few = (uint32_t)n / kFarFew;
+    int last = -1;
+#pragma unroll
+    for (int q = kPer - 1; q >= 0; --q) {
+        if (above <= few && above + c[q] > few) last = lane * kPer + q;
+        above += c[q];
+    }
+    return (int)__reduce_max_sync(0xffffffffu, last);
+}
+
+__global__ void order_octaves_kernel(ddx_state s, int first, int n, uint32_t* __restrict__ hist) {
+    after_previous();
+    __shared__ uint32_t h[kOctaves];
+    static_assert(kThreads == kOctaves, "a thread per octave");
+    h[threadIdx.x] = 0;
+    __syncthreads();
+    const int k = blockIdx.x * kThreads + threadIdx.x;
+    if (k < n) {
+        const float v[3] = {d2f_toward0(s.x[first + k]), d2f_toward0(s.y[first + k]), d2f_toward0(s.z[first + k])};
+        atomicAdd(&h[octave(s, v)], 1u);
+    }
+    __syncthreads();
+    if (h[threadIdx.x]) atomicAdd(&hist[threadIdx.x], h[threadIdx.x]);
+}
+
+// hist: the octaves' counts (null: the box takes every body).
+__device__ __forceinline__ int block_last_octave(const uint32_t* hist, int n) {
+    if (!hist) return kOctaves;                   // the same for every thread
+    __shared__ int last;
+    if (threadIdx.x < 32) {
+        const int l = last_octave(hist, n);
+        if (threadIdx.x == 0) last = l;
+    }
+    __syncthreads();
+    return last;
+}
+
+__global__ void order_init_kernel(uint32_t* __restrict__ count, int* __restrict__ box, uint32_t* __restrict__ hist) {
     after_previous();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k <= kOrderBins) count[k] = 0;
+    if (k < kOctaves) hist[k] = 0;
     if (k < 3) {
         box[k] = ord_of(INFINITY);
         box[3 + k] = ord_of(-INFINITY);
@@ -63,17 +129,20 @@ __global__ void order_init_kernel(uint32_t* __restrict__ count, int* __restrict_
 
 // Bounding box of the bodies' FP32 positions (NaN left out): a block reduction, then one
 // atomic per block and bound.
-__global__ void order_box_kernel(ddx_state s, int first, int n, bool dead_last, int* __restrict__ box) {
+__global__ void order_box_kernel(ddx_state s, int first, int n, bool dead_last, const uint32_t* __restrict__ hist,
+                                 int* __restrict__ box) {
     after_previous();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int last = block_last_octave(hist, n);
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     if (k < n && !(dead_last && removed(s, first + k))) {
         const float v[3] = {d2f_toward0(s.x[first + k]), d2f_toward0(s.y[first + k]), d2f_toward0(s.z[first + k])};
+        if (!hist || octave(s, v) <= last)
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            lo[a] = fminf(lo[a], v[a]);
-            hi[a] = fmaxf(hi[a], v[a]);
-        }
+            for (int a = 0; a < 3; ++a) {
+                lo[a] = fminf(lo[a], v[a]);
+                hi[a] = fmaxf(hi[a], v[a]);
+            }
     }
 #pragma unroll
     for (int a = 0; a < 3; ++a)
@@ -168,7 +237,10 @@ order_small_keys_kernel(ddx_state s, int first, int n, bool dead_last, bool hilb
     after_previous();
     __shared__ float red[kSmallThreads / 32][6];
     __shared__ float box[6];
+    __shared__ uint32_t hist[kOctaves];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if (t < kOctaves) hist[t] = 0;
+    __syncthreads();
     constexpr int kBits = kOrderBits - 1, kPer = kSmallOrder / kSmallThreads;
     float x[kPer][3];
     bool in[kPer];
@@ -180,6 +252,13 @@ order_small_keys_kernel(ddx_state s, int first, int n, bool dead_last, bool hilb
         if (!in[j]) continue;
         x[j][0] = d2f_toward0(s.x[first + k]); x[j][1] = d2f_toward0(s.y[first + k]); x[j][2] = d2f_toward0(s.z[first + k]);
     }
+#pragma unroll
+    for (int j = 0; j < kPer; ++j)
+        if (in[j]) atomicAdd(&hist[octave(s, x[j])], 1u);
+    __syncthreads();
+    const int last = block_last_octave(hist, n);
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) in[j] = in[j] && octave(s, x[j]) <= last;
 #pragma unroll
     for (int j = 0; j < kPer; ++j)
         if (in[j])
@@ -236,14 +315,15 @@ __global__ void order_from_pos_kernel(int n, const int* __restrict__ pos, int* _
     if (k < n) perm[pos[k]] = k;
 }
 
-// Code of each body's cell (bits per axis; removed bodies get 1 << 3 bits when
-// dead_last).  count given: rank[k] = the body's rank in its cell by an atomic increment;
+// Code of each body's cell (bits per axis; removed bodies when dead_last, and those that the box leaves
+// out, get 1 << 3 bits).  count given: rank[k] = the body's rank in its cell by an atomic increment;
 // else rank[k] = k (the values of the stable sort).
 __global__ void order_keys_kernel(ddx_state s, int first, int n, bool dead_last, int bits, bool hilbert,
-                                  const int* __restrict__ box,
+                                  const int* __restrict__ box, const uint32_t* __restrict__ hist,
                                   uint32_t* __restrict__ key, uint32_t* __restrict__ rank,
                                   uint32_t* __restrict__ count) {
     after_previous();
+    const int last = block_last_octave(hist, n);
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     uint32_t bin = 1u << (3 * bits);
@@ -251,7 +331,7 @@ __global__ void order_keys_kernel(ddx_state s, int first, int n, bool dead_last,
         const float v[3] = {d2f_toward0(s.x[first + k]), d2f_toward0(s.y[first + k]), d2f_toward0(s.z[first + k])};
         const float lo[3] = {float_of(box[0]), float_of(box[1]), float_of(box[2])};
         const float hi[3] = {float_of(box[3]), float_of(box[4]), float_of(box[5])};
-        bin = cell_code(v, lo, hi, bits, hilbert);
+        if (!hist || octave(s, v) <= last) bin = cell_code(v, lo, hi, bits, hilbert);
     }
     key[k] = bin;
     rank[k] = count ? atomicAdd(&count[bin], 1u) : (uint32_t)k;
@@ -378,7 +458,7 @@ cudaError_t order_alloc(OrderScratch& o, int cap, bool stable) {
     const size_t tw = stable ? radix_temp_words(cap) : scan_temp_words((int)bins);
     if (cudaMalloc(&n.key, 4ull * cap) || cudaMalloc(&n.rank, 4ull * cap) || cudaMalloc(&n.perm, 4ull * cap) ||
         cudaMalloc(&n.count, 4 * bins) || cudaMalloc(&n.start, 4 * bins) || cudaMalloc(&n.temp, 4 * tw) ||
-        cudaMalloc(&n.box, 6 * sizeof(int))) {
+        cudaMalloc(&n.box, (6 + kOctaves) * sizeof(int))) {
         order_free(n);
         return cudaErrorMemoryAllocation;
     }
@@ -406,22 +486,22 @@ cudaError_t order_bodies(const ddx_state& s, int first, int n, bool dead_last, c
         return cudaGetLastError();
     }
     const int blk = (n + kThreads - 1) / kThreads;
-    launch_first(order_init_kernel, (kOrderBins + 1 + kThreads - 1) / kThreads, kThreads, 0, st, o.count, o.box);
-    launch_after(order_box_kernel, blk, kThreads, 0, st, s, first, n, dead_last, o.box);
+    uint32_t* const hist = reinterpret_cast<uint32_t*>(o.box + 6);
+    launch_first(order_init_kernel, (kOrderBins + 1 + kThreads - 1) / kThreads, kThreads, 0, st, o.count, o.box, hist);
+    if (o.stable) launch_after(order_octaves_kernel, blk, kThreads, 0, st, s, first, n, hist);
+    launch_after(order_box_kernel, blk, kThreads, 0, st, s, first, n, dead_last, o.stable ? hist : nullptr, o.box);
     if (o.stable) {
         constexpr int kBits = kOrderBits - 1;   // 32^3 cells: two 8-bit digit passes
-        launch_after(order_keys_kernel, blk, kThreads, 0, st, s, first, n, dead_last, kBits, hilbert, o.box, o.key,
-                     o.rank,
-                                                    nullptr);
+        launch_after(order_keys_kernel, blk, kThreads, 0, st, s, first, n, dead_last, kBits, hilbert, o.box, hist,
+                     o.key, o.rank, nullptr);
         uint32_t *ko = nullptr, *vo = nullptr;
         cudaError_t e = radix_sort_stable(o.key, o.rank, n, 3 * kBits + 1, o.temp, &ko, &vo, st);
         if (e != cudaSuccess) return e;
         launch_after(order_from_sorted_kernel, blk, kThreads, 0, st, n, vo, perm, inv);
         return cudaGetLastError();
     }
-    launch_after(order_keys_kernel, blk, kThreads, 0, st, s, first, n, dead_last, kOrderBits, hilbert, o.box, o.key,
-                 o.rank,
-                                                o.count);
+    launch_after(order_keys_kernel, blk, kThreads, 0, st, s, first, n, dead_last, kOrderBits, hilbert, o.box, nullptr,
+                 o.key, o.rank, o.count);
     cudaError_t e = exclusive_scan(o.count, o.start, (int)kOrderBins + 1, o.temp, nullptr, st);
     if (e != cudaSuccess) return e;
     launch_after(order_scatter_kernel, blk, kThreads, 0, st, n, o.key, o.rank, o.start, perm, inv);
