@@ -285,9 +285,10 @@ __device__ __forceinline__ double pull64(double m, double x) {
     return zero_at_infinity(x, fma(f * e, fma(e, 1.875, 1.5), f));
 }
 __device__ __forceinline__ bool finite64(double x) { return (__double2hiint(x) & 0x7FFFFFFF) < 0x7FF00000; }
-// x > 0, normal and finite, without the FP64 pipe.
+// x > 0 and not subnormal, +infinity included (a pull of 0 times an infinite separation, so NaN), without the
+// FP64 pipe.
 __device__ __forceinline__ bool positive64(double x) {
-    return (unsigned)__double2hiint(x) - 0x00100000u < 0x7FE00000u;
+    return (unsigned)__double2hiint(x) - 0x00100000u <= 0x7FE00000u;
 }
 
 // Star term of the dust kernels but DDX_MODE_REFERENCE's FP64 one: the same force as star_term

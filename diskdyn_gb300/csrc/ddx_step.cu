@@ -537,10 +537,16 @@ massive_pairs_kernel(StepArgs a, MassiveScratch ms, int sa, int np, double* __re
     while (J * (J + 1) / 2 > (int)blockIdx.x) --J;
     const int I = (int)blockIdx.x - J * (J + 1) / 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const Body* const P = ms.P + (size_t)(sa + blockIdx.y) * ms.cap;
-    const Body none = make_body(1e18, 1e18, 1e18, 0.0);
+    // past the last body, and for one without a position (NaN, a pair of which pair64 leaves out): no mass, and so
+    // far away that its pulls are 0 both ways
+    auto body = [&](int k) {
+        const Body none = make_body(1e150, 1e150, 1e150, 0.0);
+        const Body b = k < a.n_grav ? P[k] : none;
+        return b.x == b.x && b.y == b.y && b.z == b.z ? b : none;
+    };
     const int i = I * kPairBlock + threadIdx.x, j0 = J * kPairBlock;
-    const Body p = i < a.n_grav ? P[i] : none;
-    src[threadIdx.x] = j0 + (int)threadIdx.x < a.n_grav ? P[j0 + threadIdx.x] : none;
+    const Body p = body(i);
+    src[threadIdx.x] = body(j0 + threadIdx.x);
     __syncthreads();
     double* const rowI = part + ((size_t)I * 6 + 3 * blockIdx.y) * np;
     double* const rowJ = part + ((size_t)J * 6 + 3 * blockIdx.y) * np;
