@@ -639,11 +639,11 @@ int ddx_debug_limit_cells(ddx_ctx* c, int most) {
     return DDX_OK;
 }
 
-int ddx_debug_cell_nodes(ddx_ctx* c, long long* nodes, long long* room, int* dropped, void* stream) {
-    if (!c || !nodes || !room || !dropped) return DDX_ERR_ARG;
+int ddx_debug_cell_nodes(ddx_ctx* c, long long* nodes, long long* room, int* dropped, double* near, void* stream) {
+    if (!c || !nodes || !room || !dropped || !near) return DDX_ERR_ARG;
     if (!c->ms.cells) return DDX_ERR_STATE;
     DeviceGuard dg(c->device);
-    return cuda_status(cells_count(c->ms.cells, nodes, room, dropped, (cudaStream_t)stream));
+    return cuda_status(cells_count(c->ms.cells, nodes, room, dropped, near, (cudaStream_t)stream));
 }
 
 int ddx_massive_final(ddx_ctx* c, const ddx_state* s, int n_grav, int n_dust, double dt,

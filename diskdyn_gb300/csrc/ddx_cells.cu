@@ -203,13 +203,13 @@ __device__ __forceinline__ float edge_scale(float n) {
 }
 
 // The grids of this step from the geometric mean distance of the planetesimals to the star
-// (largest coordinate difference), which one or two far-flung bodies do not move.  Integer
-// sums: the same on every run.  sums: [0] sum of the logarithms, [1] their number, [2] blocks
+// (largest coordinate difference) and its spread, without the few beyond the last octave of their order.
+// Integer sums: the same on every run.  sums: [0] sum of the logarithms, [1] their number, [2] blocks
 // done, [3] sum of the logarithms of |z|, [4] of the logarithms' squares (all zero before); the
 // last block to finish writes the grid.
 __global__ void __launch_bounds__(kSetupThreads)
-cells_setup_kernel(const Body* __restrict__ P, int n_exact, int n_src, int G, unsigned long long* __restrict__ sums,
-                   CellGrid* __restrict__ grid) {
+cells_setup_kernel(const Body* __restrict__ P, int n_exact, int n_src, int G, const int* __restrict__ last_octave,
+                   unsigned long long* __restrict__ sums, CellGrid* __restrict__ grid) {
     after_previous();
     __shared__ bool last;
     const Body s = P[0];
@@ -219,7 +219,7 @@ cells_setup_kernel(const Body* __restrict__ P, int n_exact, int n_src, int G, un
     if (k < n_src) {
         const Body b = P[n_exact + k];
         const float m = fmaxf(fabsf((float)(b.x - s.x)), fmaxf(fabsf((float)(b.y - s.y)), fabsf((float)(b.z - s.z))));
-        if (m > 1e-30f && m < 1e30f) {
+        if (m > 1e-30f && m < 1e30f && (int)(__float_as_uint(m) >> 23) <= *last_octave) {
             const float l = log2f(m);
             sum = (long long)(l * 65536.f);
             sum2 = (long long)(l * l * 65536.f);
@@ -1146,6 +1146,13 @@ cells_shift_kernel(CellView v, int level) {
     }
 }
 
+// Sum of the nodes' numbers of near groups (diagnostics).
+__global__ void cells_near_kernel(const CellNode* __restrict__ node, int n, unsigned long long* __restrict__ sum) {
+    unsigned long long t = 0;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) t += (unsigned)node[k].n_near;
+    if (t) atomicAdd(sum, t);
+}
+
 size_t round256(size_t n) { return (n + 255) / 256 * 256; }
 
 }  // namespace
@@ -1161,7 +1168,8 @@ void cells_free(CellScratch*& c) {
 
 bool cells_hold(const CellScratch* c, int n_src) { return c && c->cap_src >= n_src; }
 
-cudaError_t cells_count(const CellScratch* c, long long* nodes, long long* room, int* dropped, cudaStream_t st) {
+cudaError_t cells_count(const CellScratch* c, long long* nodes, long long* room, int* dropped, double* near,
+                        cudaStream_t st) {
     CellGrid g;
     cudaError_t e = cudaMemcpyAsync(&g, c->v.grid, sizeof(g), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -1170,7 +1178,16 @@ cudaError_t cells_count(const CellScratch* c, long long* nodes, long long* room,
     for (int l = g.min_level; l < kCellMaxLevels; ++l) *nodes += g.cnt[l];
     *room = c->v.cap;
     *dropped = g.min_level;
-    return cudaSuccess;
+    unsigned long long sum = 0;               // in the setup's sums, which the next step clears
+    e = cudaMemsetAsync(c->sums, 0, sizeof(sum), st);
+    if (e == cudaSuccess) {
+        launch_first(cells_near_kernel, 152, 256, 0, st, c->v.node, (int)*nodes, c->sums);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&sum, c->sums, sizeof(sum), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    *near = *nodes ? (double)sum / (double)*nodes : 0.0;
+    return e;
 }
 
 cudaError_t cells_ensure(CellScratch*& c, int n_src, int most) {
@@ -1262,8 +1279,7 @@ cudaError_t cells_build(CellScratch* c, const ddx_state& s, const StepArgs& a, c
     if (e == cudaSuccess) e = cudaMemsetAsync(c->sums, 0, 5 * sizeof(unsigned long long) + 4 * (1 + (size_t)v.words) * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
     launch_first(cells_setup_kernel, (v.n_src + kSetupThreads - 1) / kSetupThreads, kSetupThreads, 0, st, ms.P,
-                 a.n_exact,
-                 v.n_src, v.G, c->sums, v.grid);
+                 a.n_exact, v.n_src, v.G, last_octave_of(ms.src_order), c->sums, v.grid);
     launch_after(cells_boxes_kernel, (4 * v.n_groups * kGroupSrc + 127) / 128, 128, 0, st, ms.PP, ms.pcap, v);
     const int blk = (a.n_dust + 255) / 256;
     launch_after(cells_keys_kernel, blk, 256, 0, st, s, a, bins, v, o.key, o.rank, c->count);

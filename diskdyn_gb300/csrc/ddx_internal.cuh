@@ -110,11 +110,14 @@ struct OrderScratch {
     uint32_t *key, *rank;      // [cap] cell of each body, its rank in the cell
     uint32_t *count, *start;   // [kOrderBins + 1] bodies per cell, first position of each cell
     uint32_t *temp;            // scan scratch
-    int      *box;             // [6] bounding box, min then max per axis (ordered-int floats); then bodies per octave
+    int      *box;             // [6] bounding box, min then max per axis (ordered-int floats); then bodies per octave,
+                               // and (a stable order's) the last octave in the box
     int      *perm;            // [cap] the order: perm[position] = body
     int       cap;
     bool      stable;          // stable radix sort (timing-independent order) instead of atomics
 };
+constexpr int kOctaves = 256;                                   // of the distance to the star (ddx_order.cu)
+inline const int* last_octave_of(const OrderScratch& o) { return o.box + 6 + kOctaves; }
 constexpr int kOrderBits = 6;                                   // cell index bits per axis
 constexpr uint32_t kOrderBins = 1u << (3 * kOrderBits);         // cells; one more for removed bodies
 cudaError_t order_alloc(OrderScratch& o, int cap, bool stable);
@@ -144,8 +147,10 @@ __host__ __device__ inline bool spatial_order_on(const StepArgs& a) {
 struct CellScratch;
 cudaError_t cells_ensure(CellScratch*& c, int n_src, int most);
 bool cells_hold(const CellScratch* c, int n_src);
-// Cells of the last step (in use, room for, finest levels left out for want of room); waits for st.
-cudaError_t cells_count(const CellScratch* c, long long* nodes, long long* room, int* dropped, cudaStream_t st);
+// Cells of the last step (in use, room for, finest levels left out for want of room, groups near a cell
+// in the mean); waits for st.
+cudaError_t cells_count(const CellScratch* c, long long* nodes, long long* room, int* dropped, double* near,
+                        cudaStream_t st);
 void cells_free(CellScratch*& c);
 
 // The mixed step takes far planetesimals through cell expansions (ddx_cells.cu) from this many

@@ -58,7 +58,7 @@ __device__ __forceinline__ bool removed(const ddx_state& s, int i) {
 // Bodies per octave of their distance from body 0 (largest coordinate difference in FP32; the
 // octave is the exponent's bits, 255: not finite), and the last octave that the box takes: beyond
 // it lies 1 body in kFarFew at most.
-constexpr int kOctaves = 256, kFarFew = 32;
+constexpr int kFarFew = 32;
 __device__ __forceinline__ int octave(const ddx_state& s, const float* v) {
     const float m = fmaxf(fabsf(v[0] - d2f_toward0(s.x[0])), fmaxf(fabsf(v[1] - d2f_toward0(s.y[0])),
                                                                    fabsf(v[2] - d2f_toward0(s.z[0]))));
@@ -134,6 +134,7 @@ __global__ void order_box_kernel(ddx_state s, int first, int n, bool dead_last, 
     after_previous();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int last = block_last_octave(hist, n);
+    if (hist && k == 0) box[6 + kOctaves] = last;
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     if (k < n && !(dead_last && removed(s, first + k))) {
         const float v[3] = {d2f_toward0(s.x[first + k]), d2f_toward0(s.y[first + k]), d2f_toward0(s.z[first + k])};
@@ -233,7 +234,7 @@ constexpr int kSmallOrder = 8192;        // index < 2^13 below the 15-bit code +
 constexpr int kSmallThreads = 1024;
 __global__ void __launch_bounds__(kSmallThreads)
 order_small_keys_kernel(ddx_state s, int first, int n, bool dead_last, bool hilbert, uint32_t* __restrict__ key,
-                        int* __restrict__ pos) {
+                        int* __restrict__ pos, int* __restrict__ last_out) {
     after_previous();
     __shared__ float red[kSmallThreads / 32][6];
     __shared__ float box[6];
@@ -257,6 +258,7 @@ order_small_keys_kernel(ddx_state s, int first, int n, bool dead_last, bool hilb
         if (in[j]) atomicAdd(&hist[octave(s, x[j])], 1u);
     __syncthreads();
     const int last = block_last_octave(hist, n);
+    if (t == 0) *last_out = last;
 #pragma unroll
     for (int j = 0; j < kPer; ++j) in[j] = in[j] && octave(s, x[j]) <= last;
 #pragma unroll
@@ -458,7 +460,7 @@ cudaError_t order_alloc(OrderScratch& o, int cap, bool stable) {
     const size_t tw = stable ? radix_temp_words(cap) : scan_temp_words((int)bins);
     if (cudaMalloc(&n.key, 4ull * cap) || cudaMalloc(&n.rank, 4ull * cap) || cudaMalloc(&n.perm, 4ull * cap) ||
         cudaMalloc(&n.count, 4 * bins) || cudaMalloc(&n.start, 4 * bins) || cudaMalloc(&n.temp, 4 * tw) ||
-        cudaMalloc(&n.box, (6 + kOctaves) * sizeof(int))) {
+        cudaMalloc(&n.box, (6 + kOctaves + 1) * sizeof(int))) {
         order_free(n);
         return cudaErrorMemoryAllocation;
     }
@@ -479,7 +481,8 @@ cudaError_t order_bodies(const ddx_state& s, int first, int n, bool dead_last, c
     if (n > o.cap) return cudaErrorInvalidValue;
     if (o.stable && n <= kSmallOrder) {
         int* const pos = inv ? inv : reinterpret_cast<int*>(o.rank);
-        launch_first(order_small_keys_kernel, 1, kSmallThreads, 0, st, s, first, n, dead_last, hilbert, o.key, pos);
+        launch_first(order_small_keys_kernel, 1, kSmallThreads, 0, st, s, first, n, dead_last, hilbert, o.key, pos,
+                     o.box + 6 + kOctaves);
         launch_after(order_small_rank_kernel, dim3((n + kThreads - 1) / kThreads, (n + kRankKeys - 1) / kRankKeys),
                      kThreads, 0, st, n, o.key, pos);
         if (perm) launch_after(order_from_pos_kernel, (n + kThreads - 1) / kThreads, kThreads, 0, st, n, pos, perm);

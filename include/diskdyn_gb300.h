@@ -391,10 +391,11 @@ int ddx_debug_lose_tile_copy(ddx_ctx *ctx, int tile, unsigned long long wait_ns)
 int ddx_debug_limit_cells(ddx_ctx *ctx, int most);
 
 /* Diagnostics (no counterpart in the reference).  The cells of the last DDX_PREC_MIXED step that took
- * far planetesimals through cell expansions: how many it built, for how many there is room, and
- * how many of the finest levels were left out because they did not fit (0: none).
- * Synchronises `stream`.  DDX_ERR_STATE before the first such step. */
-int ddx_debug_cell_nodes(ddx_ctx *ctx, long long *nodes, long long *room, int *dropped, void *stream);
+ * far planetesimals through cell expansions: how many it built, for how many there is room,
+ * how many of the finest levels were left out because they did not fit (0: none), and how many
+ * groups of 16 planetesimals are taken one by one in a cell, in the mean.  Synchronises `stream`.
+ * DDX_ERR_STATE before the first such step. */
+int ddx_debug_cell_nodes(ddx_ctx *ctx, long long *nodes, long long *room, int *dropped, double *near, void *stream);
 
 /* Error string for a status code. */
 const char *ddx_status_string(int status);

@@ -1,6 +1,6 @@
-"""A few planetesimals scattered far out leave the others' order alone: the belt's groups stay compact, so the
-mixed step needs about as many cells as without them (in one cell of a 30,000 AU order every group spans the ring
-and every cell is split to the finest)."""
+"""A few planetesimals scattered far out leave the others' order alone: the belt's groups stay compact, and a cell
+has about as many of them near as without those bodies (in one cell of a 30,000 AU order every group spans the
+ring and is near every cell)."""
 import ctypes as C
 
 import numpy as np
@@ -17,11 +17,12 @@ def cells_of_a_step(engine, s, state):
     engine.set_size_table(**s.size_table)
     st = DeviceState.from_numpy(state)
     engine.step(st, s.n_grav, s.dt, make_phys(**s.phys), abi.DDX_PREC_MIXED)
-    nodes, room, dropped = C.c_longlong(), C.c_longlong(), C.c_int()
-    abi.check(engine.lib.ddx_debug_cell_nodes(engine.ctx, C.byref(nodes), C.byref(room), C.byref(dropped), None), "cells")
+    nodes, room, dropped, near = C.c_longlong(), C.c_longlong(), C.c_int(), C.c_double()
     torch.cuda.synchronize()
+    abi.check(engine.lib.ddx_debug_cell_nodes(engine.ctx, C.byref(nodes), C.byref(room), C.byref(dropped), C.byref(near),
+                                              None), "cells")
     assert dropped.value == 0 and nodes.value <= room.value
-    return nodes.value, st.to_numpy()
+    return near.value, st.to_numpy()
 
 
 # the order in one block / by radix sort; one body in 32 at most may lie far out
@@ -39,7 +40,7 @@ def test_scattered_planetesimals_do_not_stretch_the_order(engine, n_plsml, share
     for k, c in enumerate("xyz"):
         state[c][rows] = u[k]
     got, out = cells_of_a_step(engine, s, state)
-    # 1 in 40 fewer on the ring; their groups, a dozen at most, are near a part of its cells
-    assert got < 1.5 * want, (got, want)
+    # the groups of the bodies far out, and the one that they share with the ring's last, may be near every cell
+    assert got <= 1.1 * want + n / 16 + 2, (got, want)
     live = out["N"][s.n_grav:] != 0
     assert np.isfinite(out["x"][s.n_grav:][live]).all()
