@@ -19,7 +19,7 @@
 // A few planetesimals scattered far out would stretch the box until the others share a few of
 // its cells (a belt of 4,096 with a million tracers, one of them at 30,000 AU: 16.0 ms a mixed step, 2.1 ms
 // without it).  So the sources' box leaves out those beyond the octave of distance to the star
-// that all but 1 in kFarFew reach (Octaves), and they come last.
+// that all but 1 in kFarFew reach (Octaves), and they come last, in the order of the box's cells nearest to them.
 // The codes are sorted in one of two ways:
 //  - counting sort (the tracers: 6 bits per axis): an atomic increment gives each body its
 //    rank in its cell, an exclusive scan of the cell counts the cells' first positions, and
@@ -244,7 +244,7 @@ order_small_keys_kernel(ddx_state s, int first, int n, bool dead_last, bool hilb
     __syncthreads();
     constexpr int kBits = kOrderBits - 1, kPer = kSmallOrder / kSmallThreads;
     float x[kPer][3];
-    bool in[kPer];
+    bool in[kPer], far[kPer];
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
@@ -260,10 +260,10 @@ order_small_keys_kernel(ddx_state s, int first, int n, bool dead_last, bool hilb
     const int last = block_last_octave(hist, n);
     if (t == 0) *last_out = last;
 #pragma unroll
-    for (int j = 0; j < kPer; ++j) in[j] = in[j] && octave(s, x[j]) <= last;
+    for (int j = 0; j < kPer; ++j) far[j] = in[j] && octave(s, x[j]) > last;
 #pragma unroll
     for (int j = 0; j < kPer; ++j)
-        if (in[j])
+        if (in[j] && !far[j])
 #pragma unroll
             for (int a = 0; a < 3; ++a) { lo[a] = fminf(lo[a], x[j][a]); hi[a] = fmaxf(hi[a], x[j][a]); }
 #pragma unroll
@@ -286,7 +286,7 @@ order_small_keys_kernel(ddx_state s, int first, int n, bool dead_last, bool hilb
     for (int j = 0; j < kPer; ++j) {
         const int k = t + j * kSmallThreads;
         if (k >= n) break;
-        const uint32_t code = in[j] ? cell_code(x[j], box, box + 3, kBits, hilbert) : 1u << (3 * kBits);
+        const uint32_t code = (in[j] ? cell_code(x[j], box, box + 3, kBits, hilbert) : 0u) | (uint32_t)(!in[j] || far[j]) << (3 * kBits);
         key[k] = code << 13 | (uint32_t)k;
         pos[k] = 0;
     }
@@ -317,8 +317,8 @@ __global__ void order_from_pos_kernel(int n, const int* __restrict__ pos, int* _
     if (k < n) perm[pos[k]] = k;
 }
 
-// Code of each body's cell (bits per axis; removed bodies when dead_last, and those that the box leaves
-// out, get 1 << 3 bits).  count given: rank[k] = the body's rank in its cell by an atomic increment;
+// Code of each body's cell (bits per axis; removed bodies get 1 << 3 bits when dead_last, and those that the
+// box leaves out have that bit set).  count given: rank[k] = the body's rank in its cell by an atomic increment;
 // else rank[k] = k (the values of the stable sort).
 __global__ void order_keys_kernel(ddx_state s, int first, int n, bool dead_last, int bits, bool hilbert,
                                   const int* __restrict__ box, const uint32_t* __restrict__ hist,
@@ -333,7 +333,7 @@ __global__ void order_keys_kernel(ddx_state s, int first, int n, bool dead_last,
         const float v[3] = {d2f_toward0(s.x[first + k]), d2f_toward0(s.y[first + k]), d2f_toward0(s.z[first + k])};
         const float lo[3] = {float_of(box[0]), float_of(box[1]), float_of(box[2])};
         const float hi[3] = {float_of(box[3]), float_of(box[4]), float_of(box[5])};
-        if (!hist || octave(s, v) <= last) bin = cell_code(v, lo, hi, bits, hilbert);
+        bin = cell_code(v, lo, hi, bits, hilbert) | (uint32_t)(hist && octave(s, v) > last) << (3 * bits);
     }
     key[k] = bin;
     rank[k] = count ? atomicAdd(&count[bin], 1u) : (uint32_t)k;

@@ -22,7 +22,7 @@ def cells_of_a_step(engine, s, state):
     abi.check(engine.lib.ddx_debug_cell_nodes(engine.ctx, C.byref(nodes), C.byref(room), C.byref(dropped), C.byref(near),
                                               None), "cells")
     assert dropped.value == 0 and nodes.value <= room.value
-    return near.value, st.to_numpy()
+    return near.value, st.to_numpy(), nodes.value
 
 
 # the order in one block / by radix sort; one body in 32 at most may lie far out
@@ -30,7 +30,7 @@ def cells_of_a_step(engine, s, state):
 @pytest.mark.parametrize("share", ["one", "some"])
 def test_scattered_planetesimals_do_not_stretch_the_order(engine, n_plsml, share):
     s = synth.dusty_ring(n_dust=20000, n_plsml=n_plsml, seed=51, n_steps=1)
-    want, _ = cells_of_a_step(engine, s, s.state)
+    want, _, _ = cells_of_a_step(engine, s, s.state)
     g = np.random.default_rng(3)
     state = {k: v.copy() for k, v in s.state.items()}
     n = 1 if share == "one" else n_plsml // 40
@@ -39,8 +39,27 @@ def test_scattered_planetesimals_do_not_stretch_the_order(engine, n_plsml, share
     u *= (30000.0 if n == 1 else 10 ** g.uniform(2.8, 4.5, n)) / np.linalg.norm(u, axis=0)
     for k, c in enumerate("xyz"):
         state[c][rows] = u[k]
-    got, out = cells_of_a_step(engine, s, state)
+    got, out, _ = cells_of_a_step(engine, s, state)
     # the groups of the bodies far out, and the one that they share with the ring's last, may be near every cell
     assert got <= 1.1 * want + n / 16 + 2, (got, want)
     live = out["N"][s.n_grav:] != 0
     assert np.isfinite(out["x"][s.n_grav:][live]).all()
+
+
+def test_order_of_a_disk_that_just_reaches_into_an_octave(engine):
+    """The octave at the disk's edge holds fewer than 1 in 32 of its planetesimals, or the disk ends before it: as
+    many cells for the same disk."""
+    n_plsml, n_dust, nodes = 20000, 20000, []
+    for scale in (126.0, 138.0):
+        s = synth.dusty_ring(n_dust=n_dust, n_plsml=n_plsml, seed=52, n_steps=1)
+        g = np.random.default_rng(5)
+        n = n_plsml + n_dust
+        a, t = scale * g.uniform(0.1, 1.0, n), g.uniform(0.0, 2 * np.pi, n)
+        pos = np.stack([a * np.cos(t), a * np.sin(t), 0.01 * a * g.normal(size=n)])
+        m = np.abs(pos[:, :n_plsml]).max(0)
+        assert 0.005 < (m > 128.0).mean() < 1 / 32 if scale > 128 else (m < 128.0).all()
+        for k, c in enumerate("xyz"):
+            s.state[c][3:] = pos[k]
+        nodes.append(cells_of_a_step(engine, s, s.state)[2])
+    # the finest edges are 2 AU in both, 9 % less of the larger disk: 1.19 times the cells of a flat set
+    assert nodes[1] <= 1.2 * nodes[0], nodes
