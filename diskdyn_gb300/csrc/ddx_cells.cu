@@ -43,6 +43,7 @@
 #include "ddx_launch.cuh"
 #include "ddx_cells.cuh"
 #include "ddx_shift.cuh"
+#include "ddx_pull.cuh"
 #include "ddx_scan.cuh"
 
 namespace ddx {
@@ -70,6 +71,23 @@ constexpr float kFarEdge = 4.5f;
 constexpr int kLeafNarrow = 24, kLeafSpread = 40, kLeafSpreadMany = 64;      // Many: from 8,192 planetesimals
 constexpr float kEdgeNarrow = 1.f / 30.f, kEdgeSpread = 1.f / 24.f;
 constexpr float kSpreadOctaves = 0.35f;                   // standard deviation of log2 of the distance
+
+// Cells are for flat sets (disks at any tilt) spread over a few octaves of distance.  Tracers lie where the
+// planetesimals do, more or less, and in a thick set few share a cell, whose expansion costs as much as
+// some thousand pulls: every planetesimal one by one is then faster below several 100,000 tracers.  The
+// choice is the planetesimals' alone, as a tracer's result is not to hang on how many others there are.
+// kFlat: smallest eigenvalue of the mean of r r^T over the planetesimals' directions r from the star, 5.1e-3
+// for inclinations up to 10 degrees, 7.3e-3 up to 12, 1/3 for a ball.  us a step with every pair / with cells, 4,093
+// planetesimals and 16,000 - 33,000 - 500,000 tracers spread like them (a shell: 2,000 - 30,000 - 500,000):
+//   ring, up to 3 degrees              721 / 520     756 / 571     3977 / 1185
+//   disk of 20 to 200 AU, up to 10     751 / 714     778 / 814     3967 / 1811
+//   the same, up to 12                 752 / 762     774 / 869     3986 / 1919
+//   the same, up to 15                 730 / 844     786 / 969     3999 / 2044
+//   shell                              549 / 627     778 / 2123    4000 / 4984
+//   disk over one decade, up to 3      702 / 643     718 / 698     3970 / 1622
+//   disk over two decades, up to 3     845 / 997     891 / 1109    4547 / 2651
+constexpr double kFlat = 6e-3;
+constexpr double kMostOctaves = 1.25;                     // as kSpreadOctaves: 0.96 for one decade, 1.92 for two
 
 __host__ __device__ constexpr int coef_at(int n, int m) { return n * (n + 1) / 2 - 1 + m; }
 // A lane's sums of the irregular harmonics, in f2: order 0 in pairs of degrees (2, 3), (4, 5), ..;
@@ -205,8 +223,9 @@ __device__ __forceinline__ float edge_scale(float n) {
 // The grids of this step from the geometric mean distance of the planetesimals to the star
 // (largest coordinate difference) and its spread, without the few beyond the last octave of their order.
 // Integer sums: the same on every run.  sums: [0] sum of the logarithms, [1] their number, [2] blocks
-// done, [3] sum of the logarithms of |z|, [4] of the logarithms' squares (all zero before); the
-// last block to finish writes the grid.
+// done, [3] sum of the logarithms of |z|, [4] of the logarithms' squares, [5..9] of 2^20 times xx, xy, xz, yy, yz of
+// the directions (all zero before); the last block to finish writes the grid.
+constexpr int kSetupSums = 10;
 __global__ void __launch_bounds__(kSetupThreads)
 cells_setup_kernel(const Body* __restrict__ P, int n_exact, int n_src, int G, const int* __restrict__ last_octave,
                    unsigned long long* __restrict__ sums, CellGrid* __restrict__ grid) {
@@ -215,16 +234,21 @@ cells_setup_kernel(const Body* __restrict__ P, int n_exact, int n_src, int G, co
     const Body s = P[0];
     const int k = blockIdx.x * kSetupThreads + threadIdx.x;
     long long sum = 0, sumz = 0, sum2 = 0;
-    int n = 0;
+    int n = 0, dir[5] = {0, 0, 0, 0, 0};
     if (k < n_src) {
         const Body b = P[n_exact + k];
-        const float m = fmaxf(fabsf((float)(b.x - s.x)), fmaxf(fabsf((float)(b.y - s.y)), fabsf((float)(b.z - s.z))));
+        const float x = (float)(b.x - s.x), y = (float)(b.y - s.y), z = (float)(b.z - s.z);
+        const float m = fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z)));
         if (m > 1e-30f && m < 1e30f && (int)(__float_as_uint(m) >> 23) <= *last_octave) {
             const float l = log2f(m);
             sum = (long long)(l * 65536.f);
             sum2 = (long long)(l * l * 65536.f);
-            sumz = (long long)(log2f(fmaxf(fabsf((float)(b.z - s.z)), 1e-30f)) * 65536.f);
+            sumz = (long long)(log2f(fmaxf(fabsf(z), 1e-30f)) * 65536.f);
             n = 1;
+            const float i = 1.f / m, ux = x * i, uy = y * i, uz = z * i;
+            const float f = 1048576.f / (ux * ux + uy * uy + uz * uz);
+            dir[0] = __float2int_rn(f * ux * ux); dir[1] = __float2int_rn(f * ux * uy); dir[2] = __float2int_rn(f * ux * uz);
+            dir[3] = __float2int_rn(f * uy * uy); dir[4] = __float2int_rn(f * uy * uz);
         }
     }
 #pragma unroll
@@ -234,11 +258,21 @@ cells_setup_kernel(const Body* __restrict__ P, int n_exact, int n_src, int G, co
         sum2 += __shfl_xor_sync(0xffffffffu, sum2, o);
         n += __shfl_xor_sync(0xffffffffu, n, o);
     }
-    if ((threadIdx.x & 31) == 0 && n > 0) {
-        atomicAdd(&sums[0], (unsigned long long)sum);
-        atomicAdd(&sums[1], (unsigned long long)n);
-        atomicAdd(&sums[3], (unsigned long long)sumz);
-        atomicAdd(&sums[4], (unsigned long long)sum2);
+#pragma unroll
+    for (int q = 0; q < 5; ++q) dir[q] = __reduce_add_sync(0xffffffffu, dir[q]);
+    // a block's sums, then one atomic each
+    __shared__ long long part[kSetupThreads / 32][kSetupSums];
+    if ((threadIdx.x & 31) == 0) {
+        long long* const p = part[threadIdx.x >> 5];
+        p[0] = sum; p[1] = n; p[2] = 0; p[3] = sumz; p[4] = sum2;
+#pragma unroll
+        for (int q = 0; q < 5; ++q) p[5 + q] = dir[q];
+    }
+    __syncthreads();
+    if (threadIdx.x < kSetupSums && threadIdx.x != 2) {
+        long long t = 0;
+        for (int w = 0; w < kSetupThreads / 32; ++w) t += part[w][threadIdx.x];
+        atomicAdd(&sums[threadIdx.x], (unsigned long long)t);
         __threadfence();
     }
     __syncthreads();
@@ -271,8 +305,14 @@ cells_setup_kernel(const Body* __restrict__ P, int n_exact, int n_src, int G, co
     g.sx = (float)s.x; g.sy = (float)s.y; g.sz = (float)s.z; g.m0 = (float)s.m;
     const float qx = rintf(g.sx / g.s0), qy = rintf(g.sy / g.s0), qz = rintf(g.sz / g.s0);
     g.ox = qx * g.s0; g.oy = qy * g.s0; g.oz = qz * g.s0;
+    // flat: the mean of r r^T less kFlat times the identity is not positive definite (Sylvester's minors)
+    double d[5];
+    for (int q = 0; q < 5; ++q) d[q] = (double)(long long)*(volatile unsigned long long*)&sums[5 + q] / (1048576.0 * (double)num);
+    const double axx = d[0] - kFlat, ayy = d[3] - kFlat, azz = 1.0 - d[0] - d[3] - kFlat, m2 = axx * ayy - d[1] * d[1];
+    const double m3 = azz * m2 - axx * d[4] * d[4] - ayy * d[2] * d[2] + 2.0 * d[1] * d[2] * d[4];
+    const bool flat = !(axx > 0.0 && m2 > 0.0 && m3 > 0.0);
     // centres are exact while the origin is at most 2^20 cells away
-    g.ok = num > 0 && fabsf(qx) < 1048576.f && fabsf(qy) < 1048576.f && fabsf(qz) < 1048576.f;
+    g.ok = num > 0 && flat && var <= kMostOctaves * kMostOctaves && fabsf(qx) < 1048576.f && fabsf(qy) < 1048576.f && fabsf(qz) < 1048576.f;
     g.thin = num > 0 && exp2f((float)(sumz / num) * (1.f / 65536.f)) < 0.07f * mean;
     *grid = g;
 }
@@ -457,17 +497,21 @@ cells_ancestors_kernel(CellView v) {
 }
 
 // Per stage: the sources in slot order as (high parts, mass) and (low parts), and the boxes of
-// the source groups (a lane per source, high parts).
-__global__ void cells_boxes_kernel(const BodyPair* __restrict__ PP, int pcap, CellView v) {
+// the source groups (a lane per source, high parts) and of the spans, two groups each, for the span
+// kernel (store_span_box).  A warp takes a span.
+static_assert(2 * kGroupSrc == 2 * kPairSpan && 2 * kGroupSrc == 32, "a span is two groups and a warp");
+__global__ void cells_boxes_kernel(BodyPair* __restrict__ PP, int pcap, CellView v) {
     after_previous();
-    const int k = (blockIdx.x * blockDim.x + threadIdx.x) / kGroupSrc;             // stage * n_groups + group
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, spans = (v.n_groups + 1) / 2;   // stage * spans + span
     const int u = threadIdx.x % kGroupSrc;
     const unsigned part = ((1u << kGroupSrc) - 1u) << (threadIdx.x & 31 & ~(kGroupSrc - 1));
-    if (k >= 4 * v.n_groups) return;                                        // a group's lanes leave together
-    const int stage = k / v.n_groups, grp = k - stage * v.n_groups;
+    if (w >= 4 * spans) return;                                             // a span's lanes leave together
+    const int stage = w / spans, span = w - stage * spans, grp = 2 * span + ((threadIdx.x & 31) >= kGroupSrc);
+    const bool real = grp < v.n_groups;
+    const int k = stage * v.n_groups + grp;
     const int q = grp * kGroupSrc + u;
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    bool bad = false;
+    bool bad = false, nan = false;
     if (q < v.n_src) {
         const BodyPair& r = PP[(size_t)stage * pcap + (q >> 1)];
         const float p[3] = {r.hx[q & 1], r.hy[q & 1], r.hz[q & 1]};
@@ -476,6 +520,7 @@ __global__ void cells_boxes_kernel(const BodyPair* __restrict__ PP, int pcap, Ce
         S[1] = make_float4(r.lx[q & 1], r.ly[q & 1], r.lz[q & 1], 0.f);
         for (int a = 0; a < 3; ++a) {
             bad = bad || !(fabsf(p[a]) < 1e18f);
+            nan = nan || !(p[a] == p[a]);
             lo[a] = hi[a] = p[a];
         }
         bad = bad || !(fabsf(r.m[q & 1]) < 1e30f);
@@ -486,7 +531,7 @@ __global__ void cells_boxes_kernel(const BodyPair* __restrict__ PP, int pcap, Ce
             N[2 * kGroupPairs] = *reinterpret_cast<const ulonglong2*>(r.lx);
             N[3 * kGroupPairs].x = *reinterpret_cast<const unsigned long long*>(r.lz);
         }
-    } else if ((u & 1) == 0) {                    // an empty record: no mass
+    } else if (real && (u & 1) == 0) {            // an empty record: no mass
         for (int part = 0; part < 4; ++part)
             v.near_rec[(size_t)k * 4 * kGroupPairs + part * kGroupPairs + (u >> 1)] = make_ulonglong2(0, 0);
     }
@@ -498,7 +543,15 @@ __global__ void cells_boxes_kernel(const BodyPair* __restrict__ PP, int pcap, Ce
             hi[a] = fmaxf(hi[a], __shfl_xor_sync(part, hi[a], o));
         }
     bad = (__ballot_sync(part, bad) & part) != 0u;
-    if (u == 0) {   // the box's farthest corner bounds its sources' distances
+    nan = __any_sync(0xffffffffu, nan);
+    float slo[3], shi[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        slo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], kGroupSrc));
+        shi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], kGroupSrc));
+    }
+    store_span_box(PP + (size_t)stage * pcap + (size_t)span * kPairSpan, slo, shi, nan);
+    if (real && u == 0) {   // the box's farthest corner bounds its sources' distances
         const CellGrid& g = *v.grid;
         const float dx = fmaxf(hi[0] - g.ox, g.ox - lo[0]), dy = fmaxf(hi[1] - g.oy, g.oy - lo[1]);
         const float dz = fmaxf(hi[2] - g.oz, g.oz - lo[2]);
@@ -538,9 +591,10 @@ cells_roots_kernel(CellView v) {
     after_previous();
     const int top = v.levels - 1, c = blockIdx.x * kRootThreads + threadIdx.x;   // cell of the top grid
     const CellGrid& g = *v.grid;
+    if (!g.ok) return;
     int first = -1;
     const uint32_t* const w = v.mark + cell_word0(v.G, top) + (c >> 5);
-    if (g.ok && ((w[0] | w[v.mark_words] | w[2 * v.mark_words]) >> (c & 31) & 1u)) {
+    if (((w[0] | w[v.mark_words] | w[2 * v.mark_words]) >> (c & 31) & 1u)) {
         first = (int)atomicAdd(&v.grid->cnt[top], 4u);
         if (first + 4 > v.cap) first = -1;
         else
@@ -983,6 +1037,7 @@ __device__ __forceinline__ void distant_sums(const CellView& v, int stage, int b
 __global__ void __launch_bounds__(kNodeThreads, 3)
 cells_far_kernel(CellView v, int distant_blocks) {
     after_previous();
+    if (!v.grid->ok) return;
     union Shared {
         FarShared far;
         DistantShared distant;
@@ -1208,7 +1263,7 @@ cudaError_t cells_ensure(CellScratch*& c, int n_src, int most) {
     const size_t marks = 3 * 4 * (size_t)cell_word0(G, grid_levels(G));
     const size_t sizes[] = {sizeof(CellGrid), sizeof(CellNode) * cap, 4ull * kReal * cap, 16ull * kCellForce4 * cap,
                             4ull * words * cap, 2ull * kNearList * cap, 4ull * kCellTop * kCellTop * kCellTop, 2 * marks,
-                            32ull * 4 * groups, 32ull * 4 * (cap_src + 16), 4ull * 64 * kGroupPairs * (groups + 1), 5 * sizeof(unsigned long long) + 4 * (1 + words) * sizeof(uint32_t),
+                            32ull * 4 * groups, 32ull * 4 * (cap_src + 16), 4ull * 64 * kGroupPairs * (groups + 1), kSetupSums * sizeof(unsigned long long) + 4 * (1 + words) * sizeof(uint32_t),
                             4ull * 4 * kMultiBlocks * 2 * kMultiCoef, 8ull * 4 * kMultiBlocks * 4,
                             16ull * 4 * kFarForce4, 4 * sizeof(Body), sizeof(CellTables), 4ull * (kCellBins + 1),
                             4ull * (kCellBins + 1), 4ull * scan_temp_words(kCellBins + 1)};
@@ -1240,7 +1295,7 @@ cudaError_t cells_ensure(CellScratch*& c, int n_src, int most) {
     v.src = (float4*)take();
     v.near_rec = (ulonglong2*)take();
     n->sums = (unsigned long long*)take();
-    v.done = (uint32_t*)(n->sums + 5);
+    v.done = (uint32_t*)(n->sums + kSetupSums);
     v.outlier = v.done + 4;
     v.multi = (float*)take();
     v.moments = (double*)take();
@@ -1276,11 +1331,11 @@ cudaError_t cells_build(CellScratch* c, const ddx_state& s, const StepArgs& a, c
     const OrderScratch& o = ms.dust_order;
     cudaError_t e = cudaMemsetAsync(v.own, 0, 2 * marks, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->count, 0, 4 * ((size_t)kCellBins + 1), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->sums, 0, 5 * sizeof(unsigned long long) + 4 * (1 + (size_t)v.words) * sizeof(uint32_t), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->sums, 0, kSetupSums * sizeof(unsigned long long) + 4 * (1 + (size_t)v.words) * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
     launch_first(cells_setup_kernel, (v.n_src + kSetupThreads - 1) / kSetupThreads, kSetupThreads, 0, st, ms.P,
                  a.n_exact, v.n_src, v.G, last_octave_of(ms.src_order), c->sums, v.grid);
-    launch_after(cells_boxes_kernel, (4 * v.n_groups * kGroupSrc + 127) / 128, 128, 0, st, ms.PP, ms.pcap, v);
+    launch_after(cells_boxes_kernel, (4 * ((v.n_groups + 1) / 2) * 32 + 127) / 128, 128, 0, st, ms.PP, ms.pcap, v);
     const int blk = (a.n_dust + 255) / 256;
     launch_after(cells_keys_kernel, blk, 256, 0, st, s, a, bins, v, o.key, o.rank, c->count);
     e = exclusive_scan(c->count, c->start, (int)kCellBins + 1, c->temp, nullptr, st);

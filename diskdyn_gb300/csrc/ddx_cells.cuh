@@ -28,7 +28,7 @@ struct CellGrid {
     float sx, sy, sz, m0;      // star at the start of the step (predicted stage positions)
     uint32_t b2;               // bits of the core's largest squared distance to the origin (all stages)
     uint32_t outliers;         // groups outside the core (all stages)
-    int   ok;                  // 0: no cells this step (every tracer takes every source)
+    int   ok;                  // 0: no cells this step (the span kernel takes every source)
     int   thin;                // a disk: the tracer order cuts it finer in its plane
     int   leaf;                // most groups near a cell that is not split
     int   min_level;           // levels below it were dropped (out of nodes)
@@ -109,12 +109,14 @@ __host__ __device__ inline int cell_word0(int G, int l) {
 }
 
 // Builds the trees of one step for the tracers of s from the massive set's stage records (ms:
-// P, PP and the tracer order's buffers), orders the tracers into ms.dust_order.perm and
-// fills v for the dust kernel.  Stream-ordered.
+// P, PP and the tracer order's buffers), unless the planetesimals are none for cells (CellGrid::ok),
+// orders the tracers into ms.dust_order.perm and fills v for the dust kernel.  Stream-ordered.
 cudaError_t cells_build(CellScratch* c, const ddx_state& s, const StepArgs& a, const MassiveScratch& ms,
                         const SizeBin* bins, CellView& v, cudaStream_t st);
+// The tracers' step with cells.  done: on the device, 0 when the planetesimals were none for cells and
+// the tracers are as they were.
 cudaError_t launch_dust_cells(const ddx_state& s, const StepArgs& a, const MassiveScratch& ms, const SizeBin* bins,
-                              cudaStream_t st);
+                              const int*& done, cudaStream_t st);
 
 // x^(-1/2) within an FP32 rounding: rsqrt.approx and one Newton step whose residual 1 - x y^2 is
 // formed with the square's rounding error.  (With a factor near one instead, y (1.5 - x y^2 / 2),

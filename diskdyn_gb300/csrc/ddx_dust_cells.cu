@@ -1,5 +1,6 @@
 // Mixed-precision RK4 of the dust tracers with cell expansions (ddx_cells.cu), for
-// kCellMinSources planetesimals or more.  The physics and the precisions are those of
+// kCellMinSources planetesimals or more in a flat set (CellGrid::ok; else it leaves at once and
+// ddx_dust_mixed.cu's kernel takes the step).  The physics and the precisions are those of
 // ddx_dust_mixed.cu: FP64 state, star term, planets and RK4 combination; FP32 hi/lo
 // separations, sums over 16 planetesimals with one FP32 Kahan sum per axis across them, and
 // FP64 pulls within the near radius.  The difference is which planetesimals are taken one by
@@ -358,6 +359,7 @@ __global__ void __launch_bounds__(kThreads, T > 1 ? 7 : 6)
 dust_cells_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __restrict__ bins,
                   const int* __restrict__ perm, CellView v, const int* __restrict__ src) {
     after_previous();
+    if (!v.grid->ok) return;
     __shared__ double held[qKept][kThreads];
     const Column col{(uint32_t)__cvta_generic_to_shared(&held[0][threadIdx.x])};
     const int slot = (blockIdx.x * blockDim.x + threadIdx.x) / T;
@@ -471,10 +473,11 @@ dust_cells_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __r
 }  // namespace
 
 cudaError_t launch_dust_cells(const ddx_state& s, const StepArgs& a, const MassiveScratch& ms, const SizeBin* bins,
-                              cudaStream_t st) {
+                              const int*& done, cudaStream_t st) {
     CellView v;
     const cudaError_t e = cells_build(ms.cells, s, a, ms, bins, v, st);
     if (e != cudaSuccess) return e;
+    done = &v.grid->ok;
     const int* const perm = ms.dust_order.perm;
     const int* const src = ms.slot ? ms.src : nullptr;
     const int lanes = a.n_dust < kLanes8 ? 8 : a.n_dust < kLanes4 ? 4 : 1;

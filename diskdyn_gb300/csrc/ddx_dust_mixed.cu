@@ -24,8 +24,8 @@
 // the lanes test only the rest.  This runs from kOrderMinSources planetesimals on; with
 // fewer, every span takes the full separation in index order.
 //
-// From kCellMinSources planetesimals on the mixed step takes the far ones through cell
-// expansions instead (ddx_cells.cu, ddx_dust_cells.cu); this kernel then serves the compensated step.
+// From kCellMinSources planetesimals on the mixed step takes the far ones of a flat set through cell
+// expansions instead (ddx_cells.cu, ddx_dust_cells.cu).
 //
 // Blackwell mapping:
 //  - perturbers arrive as 64-byte pair records (two bodies per record, one quantity of
@@ -219,11 +219,7 @@ __device__ __forceinline__ void pair_ff(const BodyPair* r, f2 ml, f2 XH, f2 XL, 
     acc_ff(fh, fl, dzh, dzl, SH[2], SL[2]);
 }
 
-// Box of every span's sources (high parts, padding slots left out) at every stage, written
-// into the pad slots of the span's first four pair records, so it reaches shared memory with
-// the tile: record 0 {min x, max x}, record 1 {min y, max y}, record 2 {min z, max z},
-// record 3 {max |coordinate|, 0}; the maximum is NaN when a coordinate is NaN (such a span
-// never counts as far).
+// The boxes of all spans (store_span_box).
 // One warp per (stage, span): lane u reads source slot u of the span's 32.
 __global__ void span_box_kernel(BodyPair* __restrict__ PP, int pcap, int n_src, int nspans) {
     after_previous();
@@ -254,16 +250,7 @@ __global__ void span_box_kernel(BodyPair* __restrict__ PP, int pcap, int n_src, 
             hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
         }
     nan = __any_sync(0xffffffffu, nan);
-    if (u < 3) {
-        R[u].pad[0] = lo[u];
-        R[u].pad[1] = hi[u];
-    } else if (u == 3) {
-        float xm = 0.f;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) xm = fmaxf(xm, fmaxf(fabsf(lo[a]), fabsf(hi[a])));
-        R[3].pad[0] = nan ? __int_as_float(0x7FC00000) : xm;
-        R[3].pad[1] = 0.f;
-    }
+    store_span_box(R, lo, hi, nan);
 }
 
 // The test of one tracer (high parts xh, yh, zh; own = its largest |coordinate|) against one
@@ -400,8 +387,10 @@ __device__ __forceinline__ uint32_t span_bits(const uint32_t* w, int j0, int n) 
 template <bool COMP, int T, int NT, int MB>
 __global__ void __launch_bounds__(NT, MB * kThreads / NT)
 dust_rk4_mixed_kernel(ddx_state s, StepArgs a, MassiveScratch ms, const SizeBin* __restrict__ bins,
-                      const int* __restrict__ perm, bool boxes, const int* __restrict__ src) {
+                      const int* __restrict__ perm, bool boxes, const int* __restrict__ src,
+                      const int* __restrict__ done) {
     after_previous();
+    if (done && *done) return;                    // the cells' kernel has taken the step
     constexpr int NB = COMP ? 8 : 7;              // box values: 3 x (min, max), largest own[, smallest own]
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) unsigned long long mbar[2];
@@ -763,10 +752,15 @@ cudaError_t launch_dust_mixed(const ddx_state& s, const StepArgs& a, const Massi
                               const SizeBin* bins, int precision, cudaStream_t st) {
     if (a.n_dust <= 0) return cudaSuccess;
     const bool comp = precision == DDX_PREC_COMPENSATED;
-    // cell expansions from kCellMinSources planetesimals on (the lost-copy test hook needs tiles)
-    if (!comp && a.n_grav - a.n_exact >= kCellMinSources && cells_hold(ms.cells, a.n_grav - a.n_exact) &&
-        ms.dust_order.cap >= a.n_dust && a.lose_tile < 0)
-        return launch_dust_cells(s, a, ms, bins, st);
+    // cell expansions from kCellMinSources planetesimals on (the lost-copy test hook needs tiles); where the
+    // planetesimals turn out to be none for cells, this kernel takes the step after all
+    const int* done = nullptr;
+    const bool cells = !comp && a.n_grav - a.n_exact >= kCellMinSources && cells_hold(ms.cells, a.n_grav - a.n_exact) &&
+                       ms.dust_order.cap >= a.n_dust && a.lose_tile < 0;
+    if (cells) {
+        const cudaError_t e = launch_dust_cells(s, a, ms, bins, done, st);
+        if (e != cudaSuccess) return e;
+    }
     const bool lanes = a.n_grav - a.n_exact >= kLanesMinSources && a.n_dust <= (comp ? kLanesFewComp : kLanesFew);
     const bool many = a.n_dust >= kManyTracers;
     constexpr int kHalf = kThreads / 2;
@@ -807,19 +801,22 @@ cudaError_t launch_dust_mixed(const ddx_state& s, const StepArgs& a, const Massi
     bool boxes = false;
     const int n_src = a.n_grav - a.n_exact;
     if (ms.slot && ms.dust_order.cap >= a.n_dust && spatial_order_on(a)) {
-        cudaError_t e =
-            order_bodies(s, a.n_grav, a.n_dust, true, ms.dust_order, ms.dust_order.perm, nullptr, !comp, st);
-        if (e != cudaSuccess) return e;
-        const int nspans = pair_count(n_src) / kPairSpan;
-        launch_after(span_box_kernel, (4 * nspans * 32 + 127) / 128, 128, 0, st, ms.PP, ms.pcap, n_src, nspans);
+        if (!cells) {                             // the cells' kernels have ordered the tracers and formed the boxes
+            const cudaError_t e =
+                order_bodies(s, a.n_grav, a.n_dust, true, ms.dust_order, ms.dust_order.perm, nullptr, !comp, st);
+            if (e != cudaSuccess) return e;
+            const int nspans = pair_count(n_src) / kPairSpan;
+            launch_after(span_box_kernel, (4 * nspans * 32 + 127) / 128, 128, 0, st, ms.PP, ms.pcap, n_src, nspans);
+        }
         perm = ms.dust_order.perm;
         boxes = true;
     }
     // the source of each pair slot, for the FP64 pulls of near sources: the sources sit in
     // cell order when the step ordered them (massive_prepare), else slot q holds source q
     const int* src = ms.slot && spatial_order_on(a) ? ms.src : nullptr;
-    launch_with(a.n_grav <= kOverlapDust && !a.after_event, kernel, blocks, threads, smem, st, s, a, ms, bins, perm,
-                boxes, src);
+    // behind the cells' kernel one of the two leaves at once, so their overlap crowds nothing
+    launch_with(cells || (a.n_grav <= kOverlapDust && !a.after_event), kernel, blocks, threads, smem, st, s, a, ms, bins, perm,
+                boxes, src, done);
     return cudaGetLastError();
 }
 

@@ -153,7 +153,7 @@ cudaError_t cells_count(const CellScratch* c, long long* nodes, long long* room,
                         cudaStream_t st);
 void cells_free(CellScratch*& c);
 
-// The mixed step takes far planetesimals through cell expansions (ddx_cells.cu) from this many
+// The mixed step takes far planetesimals of a flat set through cell expansions (ddx_cells.cu) from this many
 // on; with fewer, building them costs small numbers of tracers more than it saves (us a step
 // with every pair / with cells: 1,100 planetesimals and 50,000 tracers 395 / 517, 2,100 and 10,000
 // 519 / 491, 2,100 and 500,000 2312 / 1513).

@@ -7,6 +7,25 @@
 namespace ddx {
 namespace {
 
+// Box of a span's sources (high parts, padding slots left out) at one stage, written
+// into the pad slots of the span's first four pair records R, so it reaches shared memory with
+// the tile: record 0 {min x, max x}, record 1 {min y, max y}, record 2 {min z, max z},
+// record 3 {max |coordinate|, 0}; the maximum is NaN when a coordinate is NaN (such a span
+// never counts as far).  Every lane of the span's warp has the whole box and calls it.
+__device__ __forceinline__ void store_span_box(BodyPair* R, const float (&lo)[3], const float (&hi)[3], bool nan) {
+    const int u = threadIdx.x & 31;
+    if (u < 3) {
+        R[u].pad[0] = u == 0 ? lo[0] : u == 1 ? lo[1] : lo[2];
+        R[u].pad[1] = u == 0 ? hi[0] : u == 1 ? hi[1] : hi[2];
+    } else if (u == 3) {
+        float xm = 0.f;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) xm = fmaxf(xm, fmaxf(fabsf(lo[a]), fabsf(hi[a])));
+        R[3].pad[0] = nan ? __int_as_float(0x7FC00000) : xm;
+        R[3].pad[1] = 0.f;
+    }
+}
+
 // N pair records (slots q0 .. q0 + 2 N - 1) summed again for a tracer with a near source
 // among them: the FP32 partial sum, added to (px, py, pz), of the sources at or beyond the
 // near radius (the same operations as the main loop, so each of their pulls is the same), and

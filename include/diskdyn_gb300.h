@@ -132,7 +132,8 @@ int ddx_set_optics(ddx_ctx *ctx, int n_grid, int n_wav, int n_theta, const doubl
  * DDX_PREC_MIXED with 1,024 planetesimals or more visits the tracers and reads the FP32
  * planetesimals in a spatial order (Hilbert cells) and takes spans of 32 planetesimals that
  * lie at least a quarter of the largest |coordinate| of the two away from a tracer with the
- * FP32 high parts alone.  From 2,048 planetesimals on, those far from a tracer's cell of
+ * FP32 high parts alone.  From 2,048 planetesimals on, where they lie flat (a disk inclined up to
+ * some 10 degrees, at any tilt) and within a few octaves of distance, those far from a tracer's cell of
  * space act through the cell's expansion (harmonics to degree 10; at most 2.6e-6 of one
  * such pull is left out, the size of the FP32 pulls' own rounding over all of them) and only
  * the others one by one.  The cells take device memory on the context's first such step: 0.5 GB
