@@ -555,7 +555,7 @@ __global__ void cells_boxes_kernel(BodyPair* __restrict__ PP, int pcap, CellView
         const CellGrid& g = *v.grid;
         const float dx = fmaxf(hi[0] - g.ox, g.ox - lo[0]), dy = fmaxf(hi[1] - g.oy, g.oy - lo[1]);
         const float dz = fmaxf(hi[2] - g.oz, g.oz - lo[2]);
-        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz)), core = kCoreEdges * g.s0;
+        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz)), core = core_edges(v.G) * g.s0;
         if (!bad && r2 <= core * core) {
             atomicMax(&v.grid->b2, __float_as_uint(r2));
         } else {
@@ -1221,6 +1221,8 @@ void cells_free(CellScratch*& c) {
     }
 }
 
+constexpr long long kCellBytes = 32ll << 30;    // of nodes, at most (reached at 135,000 planetesimals)
+
 bool cells_hold(const CellScratch* c, int n_src) { return c && c->cap_src >= n_src; }
 
 cudaError_t cells_count(const CellScratch* c, long long* nodes, long long* room, int* dropped, double* near,
@@ -1251,14 +1253,18 @@ cudaError_t cells_ensure(CellScratch*& c, int n_src, int most) {
     static CellTables tab;
     static const bool tab_ok = make_tables(tab);
     if (!tab_ok) return cudaErrorInvalidValue;
-    // Nodes: a level that does not fit would be left out (its parents stay leaves), and then the
-    // tracers together decide how far cells are split, so there is room for the worst case: a
-    // ball of planetesimals with tracers everywhere in it.  Its radius is the mean distance R or
-    // so, the finest edge R / 24 (n / 4,096)^(-1/4) or more, so the four stages have at most 4 (pi / 6) 48^3
-    // (n / 4,096)^(3/4) finest cells and a seventh as many coarser ones: 262,000 for 4,096, 441,000 for
-    // 8,192.  A belt of 4,096 with a million tracers takes 32,000, one with a wide halo 120,000.
-    const int cap = cap_src < 32768 ? 64 * cap_src : 2097152;
+    // Nodes: a level that does not fit is left out (its parents stay leaves), and then the
+    // tracers together decide how far cells are split, so there is room for planetesimals whose surroundings
+    // are full of tracers out to the distant expansion.  Measured with six million tracers, the edge just
+    // above its rounding's thresholds (the finest it gets), flat rings, disks, two rings and clumps, inclined up to
+    // 10 degrees and tilted: at most 81, 88, 83, 85, 82, 70, 61, 54 and 42 nodes per planetesimal at 2,048, 3,069,
+    // 4,093, 8,189, 9,000, 16,000, 40,000, 65,536 and 131,072; there is room for 100 and 56.  A belt of 4,096
+    // with a million tracers in it takes 32,000, one with a wide halo 120,000.
     const int groups = cap_src / kGroupSrc, words = (groups + 31) / 32;
+    const long long bytes = sizeof(CellNode) + 4 * kReal + 16 * kCellForce4 + 4ll * words + 2 * kNearList;
+    const long long want_nodes = 56ll * cap_src + 44ll * (cap_src < 16384 ? cap_src : 16384);
+    const long long most_nodes = kCellBytes / bytes > 2097152 ? kCellBytes / bytes : 2097152;
+    const size_t cap = (size_t)(want_nodes < most_nodes ? want_nodes : most_nodes);
     const int G = grid_dim(cap_src);
     const size_t marks = 3 * 4 * (size_t)cell_word0(G, grid_levels(G));
     const size_t sizes[] = {sizeof(CellGrid), sizeof(CellNode) * cap, 4ull * kReal * cap, 16ull * kCellForce4 * cap,
@@ -1305,7 +1311,7 @@ cudaError_t cells_ensure(CellScratch*& c, int n_src, int most) {
     n->count = (uint32_t*)take();
     n->start = (uint32_t*)take();
     n->temp = (uint32_t*)take();
-    v.cap = cap;
+    v.cap = (int)cap;
     e = cudaMemcpy((void*)v.tab, &tab, sizeof(tab), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         cells_free(n);

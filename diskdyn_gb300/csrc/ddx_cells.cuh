@@ -137,10 +137,11 @@ __device__ __forceinline__ float star_reduction(const SizeBin* __restrict__ bins
 
 // Tracers at kDistant times the core's largest distance or more from the origin take it
 // through one expansion about the origin (the error bound is that of a cell's).  The core:
-// the groups within kCoreEdges finest cell edges of the origin (the grids reach kDistant times
-// as far); they take the others, planetesimals scattered outwards, one by one.
+// the groups within core_edges finest cell edges of the origin (the grids reach kDistant times
+// as far: 512 edges with 128 cells per axis, 1,024 with 256); they take the others, planetesimals
+// scattered outwards, one by one.
 constexpr float kDistant = 6.f;
-constexpr float kCoreEdges = 80.f;
+__host__ __device__ constexpr float core_edges(int G) { return G == 128 ? 80.f : 160.f; }
 __device__ __forceinline__ bool cell_distant(const CellGrid& g, float rx, float ry, float rz) {
     const float r2 = __fmaf_rn(rx, rx, __fmaf_rn(ry, ry, __fmul_rn(rz, rz)));
     return g.ok && r2 >= __fmul_rn(kDistant * kDistant, __uint_as_float(g.b2)) && r2 < 1e30f;
