@@ -531,9 +531,13 @@ __global__ void cells_boxes_kernel(BodyPair* __restrict__ PP, int pcap, CellView
             N[2 * kGroupPairs] = *reinterpret_cast<const ulonglong2*>(r.lx);
             N[3 * kGroupPairs].x = *reinterpret_cast<const unsigned long long*>(r.lz);
         }
-    } else if (real && (u & 1) == 0) {            // an empty record: no mass
-        for (int part = 0; part < 4; ++part)
-            v.near_rec[(size_t)k * 4 * kGroupPairs + part * kGroupPairs + (u >> 1)] = make_ulonglong2(0, 0);
+    } else if (real && (u & 1) == 0) {            // an empty record: no mass, far from every tracer
+        const f2 away = f2_dup(kFarAway);
+        ulonglong2* const N = v.near_rec + (size_t)k * 4 * kGroupPairs + (u >> 1);
+        N[0] = make_ulonglong2(away, away);
+        N[kGroupPairs] = make_ulonglong2(away, 0);
+        N[2 * kGroupPairs] = make_ulonglong2(0, 0);
+        N[3 * kGroupPairs].x = 0;
     }
 #pragma unroll
     for (int a = 0; a < 3; ++a)

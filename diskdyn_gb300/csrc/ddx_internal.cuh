@@ -96,6 +96,7 @@ struct __align__(16) BodyPair {
     float lx[2], ly[2], lz[2], pad[2];
 };
 
+constexpr float kFarAway = 1.0e18f;   // padding source position, AU (mass 0)
 constexpr int kPairSpan = 16;    // pair records per plain-FP32 partial sum (32 sources)
 
 // Pair records per stage for n_src FP32 sources (bodies n_exact..n_grav-1) in pairs,

@@ -24,8 +24,6 @@ namespace ddx {
 // Massive set
 // ---------------------------------------------------------------------------------------
 
-constexpr float kFarAway = 1.0e18f;  // padding source position, AU (mass 0)
-
 // FP32 source k = i - n_exact (body i >= n_exact) into its slot q of the pair records of a
 // stage: half q & 1 of record q / 2.  The slots follow the sources' cell order when one
 // was made for this step (ms.slot), else q = k.
