@@ -155,6 +155,7 @@ SIGNATURES = [
     ("ddx_sync_status", C.c_int, [C.c_void_p, C.c_void_p]),
     ("ddx_debug_lose_tile_copy", C.c_int, [C.c_void_p, C.c_int, C.c_ulonglong]),
     ("ddx_debug_limit_cells", C.c_int, [C.c_void_p, C.c_int]),
+    ("ddx_debug_limit_image_rows", C.c_int, [C.c_void_p, C.c_longlong]),
     ("ddx_debug_cell_nodes", C.c_int, [C.c_void_p, C.POINTER(C.c_longlong), C.POINTER(C.c_longlong), C.POINTER(C.c_int),
                                        C.POINTER(C.c_double), C.c_void_p]),
     ("ddx_noalloc_sync_status", C.c_int, [C.c_int, C.c_void_p]),

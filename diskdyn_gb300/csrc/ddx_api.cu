@@ -9,6 +9,11 @@
 
 using namespace ddx;
 
+struct ImageRows {
+    float2 *at = nullptr, *outgrown = nullptr;
+    size_t words = 0, refused = 0;
+};
+
 struct ddx_ctx {
     int device = 0;
     // size-bin table
@@ -34,6 +39,7 @@ struct ddx_ctx {
     float near_eta = -1.f;                      // FP64 pulls within near_eta * |coordinate| (< 0: defaults)
     float comp_eta = kDefaultCompEta;           // compensated path: float-float spans within comp_eta * |coordinate|
     int inject_lose_tile = -1;                  // one-shot test hook for the next mixed dust launch
+    long long inject_rows_most = -1;            // test hook: no room for more words of table rows (< 0: off)
     int inject_cells_most = -1;                 // test hook: no room for cells of more planetesimals (< 0: off)
     unsigned long long inject_wait_ns = 0;
     CollideScratch* collide = nullptr;          // spatial-hash buffers, grown on demand
@@ -41,6 +47,7 @@ struct ddx_ctx {
     DetStepScratch* detstep = nullptr;          // body scan of ddx_det_step
     float* img32 = nullptr;                     // FP32 interleaved sums of the mixed images
     size_t img32_words = 0;
+    ImageRows rows;                             // table rows of the mixed images
     // ddx_step_host: copy streams (host to device, device to host) and their events
     cudaStream_t s_in = nullptr, s_out = nullptr;
     cudaEvent_t ev_in = nullptr, ev_comp = nullptr, ev_out = nullptr;
@@ -262,8 +269,36 @@ void free_optics(ddx_ctx* c) {
     c->w = c->in = c->Qabs = c->Qsca = c->Qp = c->Td = c->lQp = c->lTd = c->w5 = nullptr;
     c->lQp32p = nullptr;
     c->lTd32 = nullptr;
+    cudaFree(c->rows.at); cudaFree(c->rows.outgrown);
+    c->rows = ImageRows{};
     c->photo = PhotoConst{};
     c->optics_set = false;
+}
+
+// The mixed images' table rows for n_img wavelengths, null when few tracers do without or there is no
+// room (kept until the optics change: outgrown ones too, which a captured call may replay with; a size once
+// refused is not asked for again, and a stream that is capturing takes what is there).
+float2* image_rows(ddx_ctx* c, int n_img, int n_dust, cudaStream_t st) {
+    const size_t need = image_row_words(c->od, n_img, n_dust);
+    if (need == 0) return nullptr;
+    ImageRows& r = c->rows;
+    if (need <= r.words) return r.at;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if ((r.refused && need >= r.refused) || cudaStreamIsCapturing(st, &capture) != cudaSuccess ||
+        capture != cudaStreamCaptureStatusNone)
+        return nullptr;
+    // growing goes to the most wavelengths at once
+    const size_t most = image_row_words(c->od, kMaxImages, n_dust), words = r.at && most > need ? most : need;
+    float* p = nullptr;
+    if ((c->inject_rows_most >= 0 && words > (size_t)c->inject_rows_most) || dalloc(&p, words) != cudaSuccess) {
+        cudaGetLastError();
+        r.refused = need;
+        return nullptr;
+    }
+    r.outgrown = r.at;
+    r.at = reinterpret_cast<float2*>(p);
+    r.words = words;
+    return r.at;
 }
 
 }  // namespace
@@ -639,6 +674,12 @@ int ddx_debug_limit_cells(ddx_ctx* c, int most) {
     return DDX_OK;
 }
 
+int ddx_debug_limit_image_rows(ddx_ctx* c, long long most) {
+    if (!c) return DDX_ERR_ARG;
+    c->inject_rows_most = most;
+    return DDX_OK;
+}
+
 int ddx_debug_cell_nodes(ddx_ctx* c, long long* nodes, long long* room, int* dropped, double* near, void* stream) {
     if (!c || !nodes || !room || !dropped || !near) return DDX_ERR_ARG;
     if (!c->ms.cells) return DDX_ERR_STATE;
@@ -673,25 +714,19 @@ int ddx_image(ddx_ctx* c, const ddx_state* s, int n_grav, int n_dust, const ddx_
     }
     DeviceGuard dg(c->device);
     if (precision == DDX_PREC_MIXED) {
-        // the sums, then the wavelengths' table rows where there is room for them
-        const size_t sums = (size_t)view->xsize * view->ysize * image_k4(n_img), rows = image_row_words(c->od, n_img);
-        if (sums + rows > c->img32_words) {
+        const size_t need = (size_t)view->xsize * view->ysize * image_k4(n_img);
+        if (need > c->img32_words) {
             cudaFree(c->img32);
             c->img32 = nullptr;
             c->img32_words = 0;
-            size_t need = sums + rows;
             if (dalloc(&c->img32, need) != cudaSuccess) {
                 cudaGetLastError();
-                need = sums;
-                if (dalloc(&c->img32, need) != cudaSuccess) {
-                    cudaGetLastError();
-                    return DDX_ERR_NOMEM;
-                }
+                return DDX_ERR_NOMEM;
             }
             c->img32_words = need;
         }
-        float2* const at = rows && c->img32_words >= sums + rows ? reinterpret_cast<float2*>(c->img32 + sums) : nullptr;
-        return cuda_status(launch_image_mixed(*s, n_grav, n_dust, *view, c->od, il, c->vc, c->photo, Fd, c->img32, at,
+        float2* const rows = image_rows(c, n_img, n_dust, (cudaStream_t)stream);
+        return cuda_status(launch_image_mixed(*s, n_grav, n_dust, *view, c->od, il, c->vc, c->photo, Fd, c->img32, rows,
                                               c->counters, (cudaStream_t)stream));
     }
     return cuda_status(launch_image(*s, n_grav, n_dust, *view, c->od, il, c->vc, Fd, c->counters,

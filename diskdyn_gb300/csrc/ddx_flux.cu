@@ -709,7 +709,8 @@ __global__ void image_rows_kernel(OpticsDev o, ImageList il, int K4, float2* __r
 // From this many tracers on: below, the tables' launch costs what the rows save (ten images, us with / without:
 // 60,000 tracers 38 / 42 at best and 38 / 36 at worst, 200,000 43 / 53, 500,000 55 / 71).
 constexpr int kRowTracers = 100000;
-size_t image_row_words(const OpticsDev& o, int n_img) {
+size_t image_row_words(const OpticsDev& o, int n_img, int n_dust) {
+    if (n_dust < kRowTracers) return 0;
     const size_t n = (size_t)o.n_grid * (o.n_theta - 1) * image_k4(n_img);
     return n < (1u << 27) ? 2 * n : 0;
 }
@@ -976,7 +977,6 @@ cudaError_t launch_image_mixed(const ddx_state& s, int n_grav, int n_dust, const
     const size_t npix = (size_t)view.xsize * view.ysize;
     const int K4 = image_k4(il.n);
     if ((e = cudaMemsetAsync(Fi, 0, sizeof(float) * npix * K4, st)) != cudaSuccess) return e;
-    if (n_dust < kRowTracers) rows = nullptr;
     if (rows) launch_after(image_rows_kernel, 608, 256, 0, st, o, il, K4, rows);
     if (n_dust > 0)
         launch_after(rows ? image_mixed_kernel<true> : image_mixed_kernel<false>, (n_dust + 255) / 256, 256, 0, st, s,

@@ -47,8 +47,9 @@ cudaError_t launch_photo_prepare(const OpticsDev& o, const ViewConst* vc, const 
                                  PhotoConst pc, cudaStream_t st);
 // Mixed images: Fi is an FP32 scratch of npix * image_k4(n_img) floats (256-byte aligned).
 inline int image_k4(int n_img) { return (n_img + 3) / 4 * 4; }
-// 32-bit words of the rows scratch of launch_image_mixed, which takes null as well (0: none).
-size_t image_row_words(const OpticsDev& o, int n_img);
+// 32-bit words of the rows scratch of launch_image_mixed for n_dust tracers (0: they do without), which
+// takes null as well.
+size_t image_row_words(const OpticsDev& o, int n_img, int n_dust);
 cudaError_t launch_image_mixed(const ddx_state& s, int n_grav, int n_dust, const ddx_view& view,
                                const OpticsDev& o, const ImageList& il, ViewConst* vc, PhotoConst pc,
                                double* Fd, float* Fi, float2* rows, unsigned long long* counters, cudaStream_t st);

@@ -394,6 +394,9 @@ int ddx_debug_lose_tile_copy(ddx_ctx *ctx, int tile, unsigned long long wait_ns)
  * it had run out; negative: no more.  What the context has already is not taken away. */
 int ddx_debug_limit_cells(ddx_ctx *ctx, int most);
 
+/* The same for the mixed images' scratch of table rows of more than `most` 4-byte words. */
+int ddx_debug_limit_image_rows(ddx_ctx *ctx, long long most);
+
 /* Diagnostics (no counterpart in the reference).  The cells of the last DDX_PREC_MIXED step that took
  * far planetesimals through cell expansions: how many it built, for how many there is room,
  * how many of the finest levels were left out because they did not fit (0: none), and how many
