@@ -1358,11 +1358,14 @@ cudaError_t cells_build(CellScratch* c, const ddx_state& s, const StepArgs& a, c
     }
     launch_after(cells_ancestors_kernel, dim3(chunks, 3), 1024, 0, st, v);
     launch_after(cells_roots_kernel, kCellTop * kCellTop * kCellTop / kRootThreads, kRootThreads, 0, st, v);
+    // blocks per SM: as many splits and translations as fit, for their latency (a warp or a block per node); the far
+    // sums' three by launch bounds
+    const int sms = sm_count();
     for (int l = v.levels - 1; l >= 0; --l)
-        launch_after(cells_split_kernel, 1216, kNodeThreads, 0, st, v, l, a.near_eta);
+        launch_after(cells_split_kernel, 8 * sms, kNodeThreads, 0, st, v, l, a.near_eta);
     const int db = (v.n_src + 4 * kNodeThreads - 1) / (4 * kNodeThreads);
-    launch_after(cells_far_kernel, 456, kNodeThreads, 0, st, v, db < kMultiBlocks ? db : kMultiBlocks);
-    for (int l = v.levels - 1; l >= 0; --l) launch_after(cells_shift_kernel, 1520, kShiftThreads, 0, st, v, l);
+    launch_after(cells_far_kernel, 3 * sms, kNodeThreads, 0, st, v, db < kMultiBlocks ? db : kMultiBlocks);
+    for (int l = v.levels - 1; l >= 0; --l) launch_after(cells_shift_kernel, 10 * sms, kShiftThreads, 0, st, v, l);
     return cudaGetLastError();
 }
 

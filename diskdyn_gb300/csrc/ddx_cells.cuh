@@ -73,7 +73,7 @@ __host__ __device__ constexpr bool is_low(int i) { return i == 1 || i == 5 || i 
 struct CellView {
     CellGrid*   grid;
     CellNode*   node;          // [cap]
-    float*      lam;           // [cap][2 kCellCoef] potential coefficients (re, im); low parts of degree 1 in kLow
+    float*      lam;           // [cap][2 kCellCoef] potential coefficients (re, im); low parts of degree 1 at low_of
     float4*     force;         // [cap][kCellForce4]
     uint32_t*   near;          // [cap][words] source groups taken one by one
     uint16_t*   list;          // [cap][kNearList] the same as a list

@@ -447,7 +447,7 @@ cudaError_t launch_pixels(const ddx_state& s, int n_grav, int n_dust, const ddx_
     return cudaGetLastError();
 }
 
-// Blocks of the FP64 SED (eight per SM at most), never fewer than the mixed one's.
+// Blocks of the FP64 SED (eight for each of 152 SMs at most), never fewer than the mixed one's.
 int sed_blocks(int n_dust) {
     const int b = n_dust / kSedBatch + 1;
     return b > 1216 ? 1216 : b;
@@ -977,7 +977,7 @@ cudaError_t launch_image_mixed(const ddx_state& s, int n_grav, int n_dust, const
     const size_t npix = (size_t)view.xsize * view.ysize;
     const int K4 = image_k4(il.n);
     if ((e = cudaMemsetAsync(Fi, 0, sizeof(float) * npix * K4, st)) != cudaSuccess) return e;
-    if (rows) launch_after(image_rows_kernel, 608, 256, 0, st, o, il, K4, rows);
+    if (rows) launch_after(image_rows_kernel, 4 * sm_count(), 256, 0, st, o, il, K4, rows);
     if (n_dust > 0)
         launch_after(rows ? image_mixed_kernel<true> : image_mixed_kernel<false>, (n_dust + 255) / 256, 256, 0, st, s,
                      n_grav, n_dust, vc, make_view32(view, o), o, il, pc, rows, Fi, K4, counters);

@@ -126,8 +126,8 @@ void order_free(OrderScratch& o);
 // Orders bodies [first, first + n) of s by the code of their cell on a grid over their
 // bounding box (64^3 cells; 32^3 and equal codes in index order when o is stable): the
 // Hilbert index on cubic cells when hilbert, else the Morton code on cells stretched to the
-// box per axis.  perm[position] = body - first and, when inv is given, inv[body - first] =
-// position.  With dead_last, bodies with N == 0 come last.  A stable order leaves the few bodies far
+// box per axis.  perm[position] = body - first and inv[body - first] = position, where they are given;
+// a stable order gives inv alone.  With dead_last, bodies with N == 0 come last.  A stable order leaves the few bodies far
 // beyond the others out of the box and puts them last.  Stream-ordered.
 cudaError_t order_bodies(const ddx_state& s, int first, int n, bool dead_last, const OrderScratch& o, int* perm,
                          int* inv, bool hilbert, cudaStream_t st);
@@ -377,10 +377,11 @@ cudaError_t launch_massive_pass2(const ddx_state& s, const StepArgs& a, MassiveS
                                  int precision, cudaStream_t st);
 cudaError_t launch_dust(const ddx_state& s, const StepArgs& a, const MassiveScratch& ms,
                         const SizeBin* bins, int precision, cudaStream_t st);
-// Source slices of the mixed massive passes for n_grav bodies (about four blocks per SM),
+// Source slices of the mixed massive passes for n_grav bodies (slice_blocks_per_sm),
 // and the doubles of MassiveScratch::part that cover every system of up to cap bodies on
 // this device (massive_part_words_for with its SM count).
 int massive_slices(int n_grav, int n_exact);
+int sm_count();               // of the current device
 long long massive_part_words(int cap);
 cudaError_t launch_dust_mixed(const ddx_state& s, const StepArgs& a, const MassiveScratch& ms,
                               const SizeBin* bins, int precision, cudaStream_t st);

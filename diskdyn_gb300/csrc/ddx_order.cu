@@ -311,12 +311,6 @@ order_small_rank_kernel(int n, const uint32_t* __restrict__ key, int* __restrict
     if (k < n) atomicAdd(&pos[k], less);
 }
 
-__global__ void order_from_pos_kernel(int n, const int* __restrict__ pos, int* __restrict__ perm) {
-    after_previous();
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) perm[pos[k]] = k;
-}
-
 // Code of each body's cell (bits per axis; removed bodies get 1 << 3 bits when dead_last, and those that the
 // box leaves out have that bit set).  count given: rank[k] = the body's rank in its cell by an atomic increment;
 // else rank[k] = k (the values of the stable sort).
@@ -429,14 +423,10 @@ cudaError_t radix_sort_stable(uint32_t* keys, uint32_t* vals, int n, int key_bit
     return cudaGetLastError();
 }
 
-__global__ void order_from_sorted_kernel(int n, const uint32_t* __restrict__ sorted, int* __restrict__ perm,
-                                         int* __restrict__ inv) {
+__global__ void order_from_sorted_kernel(int n, const uint32_t* __restrict__ sorted, int* __restrict__ inv) {
     after_previous();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const uint32_t k = sorted[p];
-    if (perm) perm[p] = (int)k;
-    if (inv) inv[k] = p;
+    if (p < n) inv[sorted[p]] = p;
 }
 
 __global__ void order_scatter_kernel(int n, const uint32_t* __restrict__ key, const uint32_t* __restrict__ rank,
@@ -478,14 +468,12 @@ void order_free(OrderScratch& o) {
 cudaError_t order_bodies(const ddx_state& s, int first, int n, bool dead_last, const OrderScratch& o, int* perm,
                          int* inv, bool hilbert, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    if (n > o.cap) return cudaErrorInvalidValue;
+    if (n > o.cap || (o.stable && (perm || !inv))) return cudaErrorInvalidValue;
     if (o.stable && n <= kSmallOrder) {
-        int* const pos = inv ? inv : reinterpret_cast<int*>(o.rank);
-        launch_first(order_small_keys_kernel, 1, kSmallThreads, 0, st, s, first, n, dead_last, hilbert, o.key, pos,
+        launch_first(order_small_keys_kernel, 1, kSmallThreads, 0, st, s, first, n, dead_last, hilbert, o.key, inv,
                      o.box + 6 + kOctaves);
         launch_after(order_small_rank_kernel, dim3((n + kThreads - 1) / kThreads, (n + kRankKeys - 1) / kRankKeys),
-                     kThreads, 0, st, n, o.key, pos);
-        if (perm) launch_after(order_from_pos_kernel, (n + kThreads - 1) / kThreads, kThreads, 0, st, n, pos, perm);
+                     kThreads, 0, st, n, o.key, inv);
         return cudaGetLastError();
     }
     const int blk = (n + kThreads - 1) / kThreads;
@@ -500,7 +488,7 @@ cudaError_t order_bodies(const ddx_state& s, int first, int n, bool dead_last, c
         uint32_t *ko = nullptr, *vo = nullptr;
         cudaError_t e = radix_sort_stable(o.key, o.rank, n, 3 * kBits + 1, o.temp, &ko, &vo, st);
         if (e != cudaSuccess) return e;
-        launch_after(order_from_sorted_kernel, blk, kThreads, 0, st, n, vo, perm, inv);
+        launch_after(order_from_sorted_kernel, blk, kThreads, 0, st, n, vo, inv);
         return cudaGetLastError();
     }
     launch_after(order_keys_kernel, blk, kThreads, 0, st, s, first, n, dead_last, kOrderBits, hilbert, o.box, nullptr,

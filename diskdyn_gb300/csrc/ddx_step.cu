@@ -520,8 +520,9 @@ massive_gather_kernel(ddx_state s, StepArgs a, MassiveScratch ms, int n_pull, in
 // on every run.  4,099 bodies: 1460 us for both passes of a step, 2330 us with a warp per body.
 constexpr int kPairBlock = 128;
 // Bodies from which on it pays (FP64 steps of 2,000 tracers, us with / without: 1,503 bodies 1286 / 1248,
-// 2,003 1576 / 1787; below, the blocks are too few), and up to which the sums fit into the scratch
-// that every step keeps (MassiveScratch::part).
+// 2,003 1576 / 1787; below, the blocks are too few), and up to which the sums fit into the scratch that
+// every step keeps for the slices (MassiveScratch::part: 7.5 MB; 8,192 bodies would take 25 MB).  Beyond, a
+// warp per body as before; larger scratch has not been measured.
 constexpr int kPairsFrom = 1664, kPairsTo = 34 * kPairBlock;
 
 __global__ void __launch_bounds__(kPairBlock)
@@ -783,7 +784,6 @@ cudaError_t launch_massive_prepare(const ddx_state& s, const StepArgs& a, Massiv
     return cudaGetLastError();
 }
 
-namespace {
 int sm_count() {
     static int cached[128] = {};
     int dev = 0;
@@ -797,6 +797,7 @@ int sm_count() {
     return cached[dev];
 }
 
+namespace {
 // The sliced mixed pass: slice sums, then their gather with the pass's update.
 // Slice sums are stored [slice][component][np] with np = n_grav rounded up to a block.
 int slice_stride(int n_grav) { return (n_grav + kSliceThreads - 1) / kSliceThreads * kSliceThreads; }
