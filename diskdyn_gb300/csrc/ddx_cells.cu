@@ -86,7 +86,7 @@ constexpr float kSpreadOctaves = 0.35f;                   // standard deviation 
 //   shell                              549 / 627     778 / 2123    4000 / 4984
 //   disk over one decade, up to 3      702 / 643     718 / 698     3970 / 1622
 //   disk over two decades, up to 3     845 / 997     891 / 1109    4547 / 2651
-constexpr double kFlat = 6e-3;
+constexpr float kFlat = 6e-3f;
 constexpr double kMostOctaves = 1.25;                     // as kSpreadOctaves: 0.96 for one decade, 1.92 for two
 
 __host__ __device__ constexpr int coef_at(int n, int m) { return n * (n + 1) / 2 - 1 + m; }
@@ -306,11 +306,12 @@ cells_setup_kernel(const Body* __restrict__ P, int n_exact, int n_src, int G, co
     const float qx = rintf(g.sx / g.s0), qy = rintf(g.sy / g.s0), qz = rintf(g.sz / g.s0);
     g.ox = qx * g.s0; g.oy = qy * g.s0; g.oz = qz * g.s0;
     // flat: the mean of r r^T less kFlat times the identity is not positive definite (Sylvester's minors)
-    double d[5];
-    for (int q = 0; q < 5; ++q) d[q] = (double)(long long)*(volatile unsigned long long*)&sums[5 + q] / (1048576.0 * (double)num);
-    const double axx = d[0] - kFlat, ayy = d[3] - kFlat, azz = 1.0 - d[0] - d[3] - kFlat, m2 = axx * ayy - d[1] * d[1];
-    const double m3 = azz * m2 - axx * d[4] * d[4] - ayy * d[2] * d[2] + 2.0 * d[1] * d[2] * d[4];
-    const bool flat = !(axx > 0.0 && m2 > 0.0 && m3 > 0.0);
+    float d[5];
+    const float per = 1.f / (1048576.f * (float)num);
+    for (int q = 0; q < 5; ++q) d[q] = (float)(long long)*(volatile unsigned long long*)&sums[5 + q] * per;
+    const float axx = d[0] - kFlat, ayy = d[3] - kFlat, azz = 1.f - d[0] - d[3] - kFlat, m2 = axx * ayy - d[1] * d[1];
+    const float m3 = azz * m2 - axx * d[4] * d[4] - ayy * d[2] * d[2] + 2.f * d[1] * d[2] * d[4];
+    const bool flat = !(axx > 0.f && m2 > 0.f && m3 > 0.f);
     // centres are exact while the origin is at most 2^20 cells away
     g.ok = num > 0 && flat && var <= kMostOctaves * kMostOctaves && fabsf(qx) < 1048576.f && fabsf(qy) < 1048576.f && fabsf(qz) < 1048576.f;
     g.thin = num > 0 && exp2f((float)(sumz / num) * (1.f / 65536.f)) < 0.07f * mean;

@@ -762,7 +762,8 @@ cudaError_t launch_dust_mixed(const ddx_state& s, const StepArgs& a, const Massi
         if (e != cudaSuccess) return e;
     }
     const bool lanes = a.n_grav - a.n_exact >= kLanesMinSources && a.n_dust <= (comp ? kLanesFewComp : kLanesFew);
-    const bool many = a.n_dust >= kManyTracers;
+    // (whole blocks behind the cells' kernel: half as many to leave at once)
+    const bool many = a.n_dust >= kManyTracers && !cells;
     constexpr int kHalf = kThreads / 2;
     // blocks of 256 threads an SM (kCompBlocks)
     const bool wide = comp && a.n_grav - a.n_exact >= kOrderMinSources;

@@ -59,9 +59,11 @@ __device__ __forceinline__ bool removed(const ddx_state& s, int i) {
 // octave is the exponent's bits, 255: not finite), and the last octave that the box takes: beyond
 // it lies 1 body in kFarFew at most.
 constexpr int kFarFew = 32;
-__device__ __forceinline__ int octave(const ddx_state& s, const float* v) {
-    const float m = fmaxf(fabsf(v[0] - d2f_toward0(s.x[0])), fmaxf(fabsf(v[1] - d2f_toward0(s.y[0])),
-                                                                   fabsf(v[2] - d2f_toward0(s.z[0]))));
+__device__ __forceinline__ float3 star_place(const ddx_state& s) {
+    return make_float3(d2f_toward0(s.x[0]), d2f_toward0(s.y[0]), d2f_toward0(s.z[0]));
+}
+__device__ __forceinline__ int octave(const float3& star, const float* v) {
+    const float m = fmaxf(fabsf(v[0] - star.x), fmaxf(fabsf(v[1] - star.y), fabsf(v[2] - star.z)));
     const bool nan = !(v[0] == v[0] && v[1] == v[1] && v[2] == v[2]);   // fmaxf leaves NaN out
     return nan ? kOctaves - 1 : (int)(__float_as_uint(m) >> 23);
 }
@@ -92,13 +94,14 @@ __device__ __forceinline__ int last_octave(const uint32_t* hist, int n) {
 __global__ void order_octaves_kernel(ddx_state s, int first, int n, uint32_t* __restrict__ hist) {
     after_previous();
     __shared__ uint32_t h[kOctaves];
+    const float3 star = star_place(s);
     static_assert(kThreads == kOctaves, "a thread per octave");
     h[threadIdx.x] = 0;
     __syncthreads();
     const int k = blockIdx.x * kThreads + threadIdx.x;
     if (k < n) {
         const float v[3] = {d2f_toward0(s.x[first + k]), d2f_toward0(s.y[first + k]), d2f_toward0(s.z[first + k])};
-        atomicAdd(&h[octave(s, v)], 1u);
+        atomicAdd(&h[octave(star, v)], 1u);
     }
     __syncthreads();
     if (h[threadIdx.x]) atomicAdd(&hist[threadIdx.x], h[threadIdx.x]);
@@ -133,12 +136,13 @@ __global__ void order_box_kernel(ddx_state s, int first, int n, bool dead_last, 
                                  int* __restrict__ box) {
     after_previous();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const float3 star = hist ? star_place(s) : make_float3(0.f, 0.f, 0.f);
     const int last = block_last_octave(hist, n);
     if (hist && k == 0) box[6 + kOctaves] = last;
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     if (k < n && !(dead_last && removed(s, first + k))) {
         const float v[3] = {d2f_toward0(s.x[first + k]), d2f_toward0(s.y[first + k]), d2f_toward0(s.z[first + k])};
-        if (!hist || octave(s, v) <= last)
+        if (!hist || octave(star, v) <= last)
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 lo[a] = fminf(lo[a], v[a]);
@@ -239,6 +243,7 @@ order_small_keys_kernel(ddx_state s, int first, int n, bool dead_last, bool hilb
     __shared__ float red[kSmallThreads / 32][6];
     __shared__ float box[6];
     __shared__ uint32_t hist[kOctaves];
+    const float3 star = star_place(s);
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     if (t < kOctaves) hist[t] = 0;
     __syncthreads();
@@ -255,12 +260,12 @@ order_small_keys_kernel(ddx_state s, int first, int n, bool dead_last, bool hilb
     }
 #pragma unroll
     for (int j = 0; j < kPer; ++j)
-        if (in[j]) atomicAdd(&hist[octave(s, x[j])], 1u);
+        if (in[j]) atomicAdd(&hist[octave(star, x[j])], 1u);
     __syncthreads();
     const int last = block_last_octave(hist, n);
     if (t == 0) *last_out = last;
 #pragma unroll
-    for (int j = 0; j < kPer; ++j) far[j] = in[j] && octave(s, x[j]) > last;
+    for (int j = 0; j < kPer; ++j) far[j] = in[j] && octave(star, x[j]) > last;
 #pragma unroll
     for (int j = 0; j < kPer; ++j)
         if (in[j] && !far[j])
@@ -319,6 +324,7 @@ __global__ void order_keys_kernel(ddx_state s, int first, int n, bool dead_last,
                                   uint32_t* __restrict__ key, uint32_t* __restrict__ rank,
                                   uint32_t* __restrict__ count) {
     after_previous();
+    const float3 star = hist ? star_place(s) : make_float3(0.f, 0.f, 0.f);
     const int last = block_last_octave(hist, n);
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
@@ -327,7 +333,7 @@ __global__ void order_keys_kernel(ddx_state s, int first, int n, bool dead_last,
         const float v[3] = {d2f_toward0(s.x[first + k]), d2f_toward0(s.y[first + k]), d2f_toward0(s.z[first + k])};
         const float lo[3] = {float_of(box[0]), float_of(box[1]), float_of(box[2])};
         const float hi[3] = {float_of(box[3]), float_of(box[4]), float_of(box[5])};
-        bin = cell_code(v, lo, hi, bits, hilbert) | (uint32_t)(hist && octave(s, v) > last) << (3 * bits);
+        bin = cell_code(v, lo, hi, bits, hilbert) | (uint32_t)(hist && octave(star, v) > last) << (3 * bits);
     }
     key[k] = bin;
     rank[k] = count ? atomicAdd(&count[bin], 1u) : (uint32_t)k;
