@@ -86,15 +86,15 @@ void free_massive(MassiveScratch& ms) {
 
 int alloc_massive(ddx_ctx* c, int n_grav);
 
-// The cells' scratch for n planetesimals.  Without it the mixed step takes every planetesimal one
+// The cells' scratch for n planetesimals and n_dust tracers.  Without it the mixed step takes every planetesimal one
 // by one.  A refused size is not asked for again with this massive scratch, so that a run's
 // steps stay alike; a stream that is capturing takes what is there.
-void ensure_cells(ddx_ctx* c, int n, cudaStream_t st) {
-    if (cells_hold(c->ms.cells, n) || (c->ms.cells_refused && n >= c->ms.cells_refused)) return;
+void ensure_cells(ddx_ctx* c, int n, int n_dust, cudaStream_t st) {
+    if (cells_hold(c->ms.cells, n, n_dust) || (c->ms.cells_refused && n >= c->ms.cells_refused)) return;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return;
     const bool room = c->inject_cells_most < 0 || n <= c->inject_cells_most;
-    if (!room || cells_ensure(c->ms.cells, n, c->ms.cap) != cudaSuccess) {
+    if (!room || cells_ensure(c->ms.cells, n, n_dust, c->ms.cap) != cudaSuccess) {
         cudaGetLastError();
         c->ms.cells_refused = n;
     }
@@ -113,7 +113,7 @@ int ensure_massive(ddx_ctx* c, int n_grav, int n_dust, int precision, cudaStream
             return DDX_ERR_NOMEM;
         }
     }
-    if (precision == DDX_PREC_MIXED && n_dust > 0 && n_grav > kCellMinSources) ensure_cells(c, n_grav, st);
+    if (precision == DDX_PREC_MIXED && n_dust > 0 && n_grav > kCellMinSources) ensure_cells(c, n_grav, n_dust, st);
     return DDX_OK;
 }
 

@@ -35,6 +35,8 @@
 // g = ((n-1)^2 - m^2) / ((2n-1)(2n-3)) for the regular ones, and the same with z/r^2 and
 // 1/r^2 for the irregular ones (the solid harmonics of W. Dehnen, Comput. Astrophys. Cosmol.
 // 1:1 (2014), divided by their leading factors, which go into the coefficients).
+#include <algorithm>
+#include <climits>
 #include <cmath>
 #include <complex>
 #include <cstring>
@@ -54,7 +56,7 @@ struct CellScratch {
     CellView v{};
     uint32_t *count = nullptr, *start = nullptr, *temp = nullptr;   // the tracers' counting sort
     unsigned long long* sums = nullptr;                             // of cells_setup_kernel
-    int cap_src = 0;
+    int cap_src = 0, cap_dust = 0;
 };
 
 namespace {
@@ -1228,7 +1230,7 @@ void cells_free(CellScratch*& c) {
 
 constexpr long long kCellBytes = 32ll << 30;    // of nodes, at most (reached at 135,000 planetesimals)
 
-bool cells_hold(const CellScratch* c, int n_src) { return c && c->cap_src >= n_src; }
+bool cells_hold(const CellScratch* c, int n_src, int n_dust) { return c && c->cap_src >= n_src && c->cap_dust >= n_dust; }
 
 cudaError_t cells_count(const CellScratch* c, long long* nodes, long long* room, int* dropped, double* near,
                         cudaStream_t st) {
@@ -1252,8 +1254,11 @@ cudaError_t cells_count(const CellScratch* c, long long* nodes, long long* room,
     return e;
 }
 
-cudaError_t cells_ensure(CellScratch*& c, int n_src, int most) {
-    if (cells_hold(c, n_src)) return cudaSuccess;
+cudaError_t cells_ensure(CellScratch*& c, int n_src, int n_dust, int most) {
+    if (cells_hold(c, n_src, n_dust)) return cudaSuccess;
+    int cap_dust = INT_MAX;
+    if (!c && n_dust <= 1 << 29)
+        for (cap_dust = 4096; cap_dust < n_dust;) cap_dust *= 2;
     const int want = c && most > n_src ? most : n_src, cap_src = (want + 1023) / 1024 * 1024;
     static CellTables tab;
     static const bool tab_ok = make_tables(tab);
@@ -1264,13 +1269,14 @@ cudaError_t cells_ensure(CellScratch*& c, int n_src, int most) {
     // above its rounding's thresholds (the finest it gets), flat rings, disks, two rings and clumps, inclined up to
     // 10 degrees and tilted: at most 81, 88, 83, 85, 82, 70, 61, 54 and 42 nodes per planetesimal at 2,048, 3,069,
     // 4,093, 8,189, 9,000, 16,000, 40,000, 65,536 and 131,072; there is room for 100 and 56.  A belt of 4,096
-    // with a million tracers in it takes 32,000, one with a wide halo 120,000.
+    // with a million tracers in it takes 32,000, one with a wide halo 120,000.  A tracer needs one cell a level and
+    // stage at most, which is less for few tracers (16,384 with 4,096 planetesimals: 1.0 GB instead of 1.3).
     const int groups = cap_src / kGroupSrc, words = (groups + 31) / 32;
     const long long bytes = sizeof(CellNode) + 4 * kReal + 16 * kCellForce4 + 4ll * words + 2 * kNearList;
     const long long want_nodes = 56ll * cap_src + 44ll * (cap_src < 16384 ? cap_src : 16384);
     const long long most_nodes = kCellBytes / bytes > 2097152 ? kCellBytes / bytes : 2097152;
-    const size_t cap = (size_t)(want_nodes < most_nodes ? want_nodes : most_nodes);
     const int G = grid_dim(cap_src);
+    const size_t cap = (size_t)std::min({want_nodes, most_nodes, 4ll * grid_levels(G) * cap_dust});
     const size_t marks = 3 * 4 * (size_t)cell_word0(G, grid_levels(G));
     const size_t sizes[] = {sizeof(CellGrid), sizeof(CellNode) * cap, 4ull * kReal * cap, 16ull * kCellForce4 * cap,
                             4ull * words * cap, 2ull * kNearList * cap, 4ull * kCellTop * kCellTop * kCellTop, 2 * marks,
@@ -1290,6 +1296,7 @@ cudaError_t cells_ensure(CellScratch*& c, int n_src, int most) {
     }
     n->arena = arena;
     n->cap_src = cap_src;
+    n->cap_dust = cap_dust;
     char* p = arena;
     int k = 0;
     auto take = [&]() { char* r = p; p += round256(sizes[k++]); return r; };
@@ -1329,7 +1336,7 @@ cudaError_t cells_ensure(CellScratch*& c, int n_src, int most) {
 
 cudaError_t cells_build(CellScratch* c, const ddx_state& s, const StepArgs& a, const MassiveScratch& ms,
                         const SizeBin* bins, CellView& v, cudaStream_t st) {
-    if (!cells_hold(c, a.n_grav - a.n_exact)) return cudaErrorInvalidValue;
+    if (!cells_hold(c, a.n_grav - a.n_exact, a.n_dust)) return cudaErrorInvalidValue;
     v = c->v;
     v.n_src = a.n_grav - a.n_exact;
     v.n_groups = (v.n_src + kGroupSrc - 1) / kGroupSrc;

@@ -755,7 +755,7 @@ cudaError_t launch_dust_mixed(const ddx_state& s, const StepArgs& a, const Massi
     // cell expansions from kCellMinSources planetesimals on (the lost-copy test hook needs tiles); where the
     // planetesimals turn out to be none for cells, this kernel takes the step after all
     const int* done = nullptr;
-    const bool cells = !comp && a.n_grav - a.n_exact >= kCellMinSources && cells_hold(ms.cells, a.n_grav - a.n_exact) &&
+    const bool cells = !comp && a.n_grav - a.n_exact >= kCellMinSources && cells_hold(ms.cells, a.n_grav - a.n_exact, a.n_dust) &&
                        ms.dust_order.cap >= a.n_dust && a.lose_tile < 0;
     if (cells) {
         const cudaError_t e = launch_dust_cells(s, a, ms, bins, done, st);

@@ -142,12 +142,12 @@ __host__ __device__ inline bool spatial_order_on(const StepArgs& a) {
 }
 
 // Buffers of the mixed step's cell expansions (ddx_cells.cu).  cells_ensure makes them hold n_src
-// planetesimals, or `most` when they have to grow; on failure they stay as they were, so a step
-// asks cells_hold before it uses them.  Buffers that were outgrown live on until cells_free: a captured step may
-// replay with them.
+// planetesimals and n_dust tracers, or `most` planetesimals and any number of tracers when they have to grow;
+// on failure they stay as they were, so a step asks cells_hold before it uses them.  Buffers that were
+// outgrown live on until cells_free: a captured step may replay with them.
 struct CellScratch;
-cudaError_t cells_ensure(CellScratch*& c, int n_src, int most);
-bool cells_hold(const CellScratch* c, int n_src);
+cudaError_t cells_ensure(CellScratch*& c, int n_src, int n_dust, int most);
+bool cells_hold(const CellScratch* c, int n_src, int n_dust);
 // Cells of the last step (in use, room for, finest levels left out for want of room, groups near a cell
 // in the mean); waits for st.
 cudaError_t cells_count(const CellScratch* c, long long* nodes, long long* room, int* dropped, double* near,

@@ -138,10 +138,10 @@ int ddx_set_optics(ddx_ctx *ctx, int n_grid, int n_wav, int n_theta, const doubl
  * 2.6e-6 of one such pull is left out, the size of the FP32 pulls' own rounding over all of
  * them) and only the others one by one.  The cells take device memory on the context's first
  * step with so many: 0.8 GB at 2,051 massive bodies, 1.3 GB at 4,099, 4.9 GB at 20,003, 13 GB
- * at 65,539, 34 GB from 135,000 on.  Where there is no room for it, or that first step is being
- * captured, every planetesimal is taken one by one, in more time and with other last bits; a
- * size once refused is not asked for again until the number of massive bodies passes the next
- * power of two.
+ * at 65,539, 34 GB from 135,000 on, and less for tens of thousands of tracers or fewer.  Where
+ * there is no room for it, or that first step is being captured, every planetesimal is taken
+ * one by one, in more time and with other last bits; a size once refused is not asked for again
+ * until the number of massive bodies passes the next power of two.
  * Each tracer's result depends on its own data and the massive set only (not on the
  * other tracers or their order), and the result is the same from run to run.  (With more than
  * 200,000 planetesimals and tracers all around them the finest cells may not fit; whether they

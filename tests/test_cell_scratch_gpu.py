@@ -80,6 +80,21 @@ def test_captured_step_replays_after_growth(contexts):
     assert same(st.to_numpy(), want)
 
 
+def test_captured_step_replays_after_more_tracers(contexts):
+    """The room for cells goes by the tracers too while they are few."""
+    few = ring(2100)
+    many = synth.dusty_ring(n_dust=200000, n_plsml=2100, seed=21, n_steps=1)
+    e = contexts(few)
+    want = stepped(e, few)
+    graph, st = captured(e, few)
+    got = stepped(e, many)
+    assert same(got, stepped(contexts(many), many))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert same(st.to_numpy(), want)
+    assert same(stepped(e, few), want)
+
+
 def test_capture_without_cells_takes_every_planetesimal(contexts):
     """After a compensated step everything but the cells is there."""
     s = ring(2100)
