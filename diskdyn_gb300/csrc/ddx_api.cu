@@ -86,13 +86,20 @@ void free_massive(MassiveScratch& ms) {
 
 int alloc_massive(ddx_ctx* c, int n_grav);
 
+// Whether memory may not be allocated for work on st.
+bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
 // The cells' scratch for n planetesimals and n_dust tracers.  Without it the mixed step takes every planetesimal one
 // by one.  A refused size is not asked for again with this massive scratch, so that a run's
 // steps stay alike; a stream that is capturing takes what is there.
 void ensure_cells(ddx_ctx* c, int n, int n_dust, cudaStream_t st) {
     if (cells_hold(c->ms.cells, n, n_dust) || (c->ms.cells_refused && n >= c->ms.cells_refused)) return;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return;
+    if (capturing(st)) return;
     const bool room = c->inject_cells_most < 0 || n <= c->inject_cells_most;
     if (!room || cells_ensure(c->ms.cells, n, n_dust, c->ms.cap) != cudaSuccess) {
         cudaGetLastError();
@@ -283,10 +290,7 @@ float2* image_rows(ddx_ctx* c, int n_img, int n_dust, cudaStream_t st) {
     if (need == 0) return nullptr;
     ImageRows& r = c->rows;
     if (need <= r.words) return r.at;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if ((r.refused && need >= r.refused) || cudaStreamIsCapturing(st, &capture) != cudaSuccess ||
-        capture != cudaStreamCaptureStatusNone)
-        return nullptr;
+    if ((r.refused && need >= r.refused) || capturing(st)) return nullptr;
     // growing goes to the most wavelengths at once
     const size_t most = image_row_words(c->od, kMaxImages, n_dust), words = r.at && most > need ? most : need;
     float* p = nullptr;

@@ -40,8 +40,8 @@
 #include <cmath>
 #include <complex>
 #include <cstring>
+#include <memory>
 #include <new>
-#include <vector>
 #include "ddx_launch.cuh"
 #include "ddx_cells.cuh"
 #include "ddx_shift.cuh"
@@ -151,7 +151,8 @@ cd regular(int n, int m, double x, double y, double z) {
 bool make_tables(CellTables& t) {
     std::memset(&t, 0, sizeof(t));
     constexpr int N = 2 * kCellCoef;
-    std::vector<double> M((size_t)N * N, 0.0);       // [i][j]: parent coefficient i into child coefficient j
+    const std::unique_ptr<double[]> M(new (std::nothrow) double[(size_t)N * N]());   // [i][j]: parent coefficient i into child coefficient j
+    if (!M) return false;
     for (int n = 1; n <= kCellP; ++n)
         for (int m = 0; m <= n; ++m) {
             double df = 1.0;
