@@ -75,20 +75,24 @@ constexpr float kEdgeNarrow = 1.f / 30.f, kEdgeSpread = 1.f / 24.f;
 constexpr float kSpreadOctaves = 0.35f;                   // standard deviation of log2 of the distance
 
 // Cells are for flat sets (disks at any tilt) spread over a few octaves of distance.  Tracers lie where the
-// planetesimals do, more or less, and in a thick set few share a cell, whose expansion costs as much as
+// planetesimals do, more or less, and in a set that fills much space few share a cell, whose expansion costs as much as
 // some thousand pulls: every planetesimal one by one is then faster below several 100,000 tracers.  The
 // choice is the planetesimals' alone, as a tracer's result is not to hang on how many others there are.
-// kFlat: smallest eigenvalue of the mean of r r^T over the planetesimals' directions r from the star, 5.1e-3
-// for inclinations up to 10 degrees, 7.3e-3 up to 12, 1/3 for a ball.  us a step with every pair / with cells, 4,093
-// planetesimals and 16,000 - 33,000 - 500,000 tracers spread like them (a shell: 2,000 - 30,000 - 500,000):
-//   ring, up to 3 degrees              721 / 520     756 / 571     3977 / 1185
-//   disk of 20 to 200 AU, up to 10     751 / 714     778 / 814     3967 / 1811
-//   the same, up to 12                 752 / 762     774 / 869     3986 / 1919
-//   the same, up to 15                 730 / 844     786 / 969     3999 / 2044
-//   shell                              549 / 627     778 / 2123    4000 / 4984
-//   disk over one decade, up to 3      702 / 643     718 / 698     3970 / 1622
-//   disk over two decades, up to 3     845 / 997     891 / 1109    4547 / 2651
-constexpr float kFlat = 6e-3f;
+// Two limits: kFlat* on the smallest eigenvalue of the mean of r r^T over the planetesimals' directions r from
+// the star (4.6e-4 for inclinations up to 3 degrees, 5.1e-3 up to 10, 1/3 for a ball), and kRoom* on its root times the
+// standard deviation of log2 |r|, the set's room.  us a step with every pair / with cells, 16,000 - 33,000 - 500,000
+// tracers spread like 4,093 planetesimals (a shell: 2,000 - 30,000 - 500,000):
+//   narrow: ring of 120 to 140 AU, up to 3 degrees (room 0.0014)   721 / 520     756 / 571     3977 / 1185
+//           the same, up to 15 (0.0068)                            829 / 779     885 / 937     4005 / 1751
+//           the same, up to 20 (0.0092, over the limit)            716 / 791     740 / 947     4007 / 1733
+//           ring of 100 to 160 AU, up to 5 (0.0069)                803 / 705     839 / 836     4031 / 1612
+//   spread: disk of 20 to 200 AU, up to 6 (0.036)                  716 / 624     746 / 711     3941 / 1651
+//           the same, up to 10 (0.060)                             751 / 714     778 / 814     3967 / 1811
+//           the same, up to 15 (0.089, over)                       730 / 844     786 / 969     3999 / 2044
+//           disk over two decades, up to 3 (1.9 octaves, over)     845 / 997     891 / 1109    4547 / 2651
+//   shell (over)                                                   549 / 627     778 / 2123    4000 / 4984
+// Without cells the kernels that build them leave at once: 0.93 to 1.1 times the speed of a step that never had them.
+constexpr float kFlatNarrow = 1.25e-2f, kFlatSpread = 6e-3f, kRoomNarrow = 7e-3f, kRoomSpread = 6.2e-2f;
 constexpr double kMostOctaves = 1.25;                     // as kSpreadOctaves: 0.96 for one decade, 1.92 for two
 
 __host__ __device__ constexpr int coef_at(int n, int m) { return n * (n + 1) / 2 - 1 + m; }
@@ -227,8 +231,9 @@ __device__ __forceinline__ float edge_scale(float n) {
 // (largest coordinate difference) and its spread, without the few beyond the last octave of their order.
 // Integer sums: the same on every run.  sums: [0] sum of the logarithms, [1] their number, [2] blocks
 // done, [3] sum of the logarithms of |z|, [4] of the logarithms' squares, [5..9] of 2^20 times xx, xy, xz, yy, yz of
-// the directions (all zero before); the last block to finish writes the grid.
-constexpr int kSetupSums = 10;
+// the directions, [10] and [11] as [0] and [4] of the distances themselves (all zero before); the last block to
+// finish writes the grid.
+constexpr int kSetupSums = 12;
 __global__ void __launch_bounds__(kSetupThreads)
 cells_setup_kernel(const Body* __restrict__ P, int n_exact, int n_src, int G, const int* __restrict__ last_octave,
                    unsigned long long* __restrict__ sums, CellGrid* __restrict__ grid) {
@@ -236,7 +241,7 @@ cells_setup_kernel(const Body* __restrict__ P, int n_exact, int n_src, int G, co
     __shared__ bool last;
     const Body s = P[0];
     const int k = blockIdx.x * kSetupThreads + threadIdx.x;
-    long long sum = 0, sumz = 0, sum2 = 0;
+    long long sum = 0, sumz = 0, sum2 = 0, sumr = 0, sumr2 = 0;
     int n = 0, dir[5] = {0, 0, 0, 0, 0};
     if (k < n_src) {
         const Body b = P[n_exact + k];
@@ -249,7 +254,9 @@ cells_setup_kernel(const Body* __restrict__ P, int n_exact, int n_src, int G, co
             sumz = (long long)(log2f(fmaxf(fabsf(z), 1e-30f)) * 65536.f);
             n = 1;
             const float i = 1.f / m, ux = x * i, uy = y * i, uz = z * i;
-            const float f = 1048576.f / (ux * ux + uy * uy + uz * uz);
+            const float u2 = ux * ux + uy * uy + uz * uz, f = 1048576.f / u2, lr = l + 0.5f * log2f(u2);
+            sumr = (long long)(lr * 65536.f);
+            sumr2 = (long long)(lr * lr * 65536.f);
             dir[0] = __float2int_rn(f * ux * ux); dir[1] = __float2int_rn(f * ux * uy); dir[2] = __float2int_rn(f * ux * uz);
             dir[3] = __float2int_rn(f * uy * uy); dir[4] = __float2int_rn(f * uy * uz);
         }
@@ -259,6 +266,8 @@ cells_setup_kernel(const Body* __restrict__ P, int n_exact, int n_src, int G, co
         sum += __shfl_xor_sync(0xffffffffu, sum, o);
         sumz += __shfl_xor_sync(0xffffffffu, sumz, o);
         sum2 += __shfl_xor_sync(0xffffffffu, sum2, o);
+        sumr += __shfl_xor_sync(0xffffffffu, sumr, o);
+        sumr2 += __shfl_xor_sync(0xffffffffu, sumr2, o);
         n += __shfl_xor_sync(0xffffffffu, n, o);
     }
 #pragma unroll
@@ -270,6 +279,7 @@ cells_setup_kernel(const Body* __restrict__ P, int n_exact, int n_src, int G, co
         p[0] = sum; p[1] = n; p[2] = 0; p[3] = sumz; p[4] = sum2;
 #pragma unroll
         for (int q = 0; q < 5; ++q) p[5 + q] = dir[q];
+        p[10] = sumr; p[11] = sumr2;
     }
     __syncthreads();
     if (threadIdx.x < kSetupSums && threadIdx.x != 2) {
@@ -308,16 +318,20 @@ cells_setup_kernel(const Body* __restrict__ P, int n_exact, int n_src, int G, co
     g.sx = (float)s.x; g.sy = (float)s.y; g.sz = (float)s.z; g.m0 = (float)s.m;
     const float qx = rintf(g.sx / g.s0), qy = rintf(g.sy / g.s0), qz = rintf(g.sz / g.s0);
     g.ox = qx * g.s0; g.oy = qy * g.s0; g.oz = qz * g.s0;
-    // flat: the mean of r r^T less kFlat times the identity is not positive definite (Sylvester's minors)
+    // flat: the mean of r r^T less the limit times the identity is not positive definite (Sylvester's minors)
     float d[5];
     const float per = 1.f / (1048576.f * (float)num);
     for (int q = 0; q < 5; ++q) d[q] = (float)(long long)*(volatile unsigned long long*)&sums[5 + q] * per;
-    const float axx = d[0] - kFlat, ayy = d[3] - kFlat, azz = 1.f - d[0] - d[3] - kFlat, m2 = axx * ayy - d[1] * d[1];
+    const double lr = num > 0 ? (double)(long long)*(volatile unsigned long long*)&sums[10] / (double)num / 65536.0 : 0.0;
+    const double varr = num > 0 ? (double)(long long)*(volatile unsigned long long*)&sums[11] / (double)num / 65536.0 - lr * lr : 0.0;
+    const float room = spread ? kRoomSpread : kRoomNarrow;
+    const float most = fminf(spread ? kFlatSpread : kFlatNarrow, room * room / fmaxf((float)varr, 1e-12f));
+    const float axx = d[0] - most, ayy = d[3] - most, azz = 1.f - d[0] - d[3] - most, m2 = axx * ayy - d[1] * d[1];
     const float m3 = azz * m2 - axx * d[4] * d[4] - ayy * d[2] * d[2] + 2.f * d[1] * d[2] * d[4];
     const bool flat = !(axx > 0.f && m2 > 0.f && m3 > 0.f);
     // centres are exact while the origin is at most 2^20 cells away
     g.ok = num > 0 && flat && var <= kMostOctaves * kMostOctaves && fabsf(qx) < 1048576.f && fabsf(qy) < 1048576.f && fabsf(qz) < 1048576.f;
-    g.thin = num > 0 && exp2f((float)(sumz / num) * (1.f / 65536.f)) < 0.07f * mean;
+    g.thin = g.ok && exp2f((float)(sumz / num) * (1.f / 65536.f)) < 0.07f * mean;
     *grid = g;
 }
 
@@ -1229,7 +1243,7 @@ void cells_free(CellScratch*& c) {
     }
 }
 
-constexpr long long kCellBytes = 32ll << 30;    // of nodes, at most (reached at 135,000 planetesimals)
+constexpr long long kCellBytes = 32ll << 30;    // of nodes, at most (reached at 147,000 planetesimals)
 
 bool cells_hold(const CellScratch* c, int n_src, int n_dust) { return c && c->cap_src >= n_src && c->cap_dust >= n_dust; }
 
@@ -1267,14 +1281,14 @@ cudaError_t cells_ensure(CellScratch*& c, int n_src, int n_dust, int most) {
     // Nodes: a level that does not fit is left out (its parents stay leaves), and then the
     // tracers together decide how far cells are split, so there is room for planetesimals whose surroundings
     // are full of tracers out to the distant expansion.  Measured with six million tracers, the edge just
-    // above its rounding's thresholds (the finest it gets), flat rings, disks, two rings and clumps, inclined up to
-    // 10 degrees and tilted: at most 81, 88, 83, 85, 82, 70, 61, 54 and 42 nodes per planetesimal at 2,048, 3,069,
-    // 4,093, 8,189, 9,000, 16,000, 40,000, 65,536 and 131,072; there is room for 100 and 56.  A belt of 4,096
+    // above its rounding's thresholds (the finest it gets), rings and disks up to the limits of the sets that take
+    // cells, tilted ones and clumps: at most 112, 103, 90, 91, 86, 64, 58, 50 and 36 nodes per planetesimal at 2,048,
+    // 3,069, 4,093, 6,141, 8,189, 16,381, 40,000, 65,536 and 131,072; there is room for 120 (180 at 2,048) and 58.  A belt of 4,096
     // with a million tracers in it takes 32,000, one with a wide halo 120,000.  A tracer needs one cell a level and
-    // stage at most, which is less for few tracers (16,384 with 4,096 planetesimals: 1.0 GB instead of 1.3).
+    // stage at most, which is less for few tracers (16,384 with 4,096 planetesimals: 1.0 GB instead of 1.5).
     const int groups = cap_src / kGroupSrc, words = (groups + 31) / 32;
     const long long bytes = sizeof(CellNode) + 4 * kReal + 16 * kCellForce4 + 4ll * words + 2 * kNearList;
-    const long long want_nodes = 56ll * cap_src + 44ll * (cap_src < 16384 ? cap_src : 16384);
+    const long long want_nodes = 58ll * cap_src + 62ll * (cap_src < 16384 ? cap_src : 16384);
     const long long most_nodes = kCellBytes / bytes > 2097152 ? kCellBytes / bytes : 2097152;
     const int G = grid_dim(cap_src);
     const size_t cap = (size_t)std::min({want_nodes, most_nodes, 4ll * grid_levels(G) * cap_dust});

@@ -132,13 +132,13 @@ int ddx_set_optics(ddx_ctx *ctx, int n_grid, int n_wav, int n_theta, const doubl
  * DDX_PREC_MIXED with 1,024 planetesimals or more visits the tracers and reads the FP32
  * planetesimals in a spatial order (Hilbert cells) and takes spans of 32 planetesimals that
  * lie at least a quarter of the largest |coordinate| of the two away from a tracer with the
- * FP32 high parts alone.  From 2,048 planetesimals on, where they lie flat (a disk inclined up
- * to some 10 degrees, at any tilt) and within a few octaves of distance, those far from a
+ * FP32 high parts alone.  From 2,048 planetesimals on, where they lie flat and fill little room
+ * (a ring inclined up to 15 degrees, a disk up to 10, at any tilt), those far from a
  * tracer's cell of space act through the cell's expansion (harmonics to degree 10; at most
  * 2.6e-6 of one such pull is left out, the size of the FP32 pulls' own rounding over all of
  * them) and only the others one by one.  The cells take device memory on the context's first
- * step with so many: 0.8 GB at 2,051 massive bodies, 1.3 GB at 4,099, 4.9 GB at 20,003, 13 GB
- * at 65,539, 34 GB from 135,000 on, and less for tens of thousands of tracers or fewer.  Where
+ * step with so many: 0.9 GB at 2,051 massive bodies, 1.5 GB at 4,099, 5.7 GB at 20,003, 14 GB
+ * at 65,539, 34 GB from 147,000 on, and less for tens of thousands of tracers or fewer.  Where
  * there is no room for it, or that first step is being captured, every planetesimal is taken
  * one by one, in more time and with other last bits; a size once refused is not asked for again
  * until the number of massive bodies passes the next power of two.

@@ -1,4 +1,4 @@
-"""Which planetesimals act through cells: flat sets (at any tilt) over a few octaves of distance.  The others are taken
+"""Which planetesimals act through cells: flat sets (at any tilt) that fill little room.  The others are taken
 one by one, with the bits of a context that has no memory for cells.  The choice is the planetesimals' alone: a grain's
 step is the same among few tracers and many."""
 import ctypes as C
@@ -31,15 +31,19 @@ def tilted(p, degrees):
     return np.stack([c * p[0] + s * p[2], p[1], -s * p[0] + c * p[2]])
 
 
-# smallest eigenvalue of the directions' mean of r r^T, against 6e-3: 5e-4, 5.1e-3, 7.3e-3, 1/3 (0 for one clump);
-# octaves of distance, against 1.25: 0.96 for a decade, 1.92 for two
+# root of the smallest eigenvalue of the directions' mean of r r^T times the octaves of distance, against 7e-3 where
+# these are few (1.4e-3, 5.4e-3, 7.9e-3, 3.6e-3; 9.6e-3 for the wide ring; 0 for one clump) and 6.2e-2 where they are many
+# (4.8e-2, 7.7e-2, 2.1e-2); 1.92 octaves, against 1.25, for two decades
 SETS = {"ring": (lambda g, n: disk(g, n, 120, 140, 3), True),
-        "inclined 10": (lambda g, n: disk(g, n, 120, 140, 10), True),
-        "inclined 12": (lambda g, n: disk(g, n, 120, 140, 12), False),
+        "inclined 12": (lambda g, n: disk(g, n, 120, 140, 12), True),
+        "inclined 17": (lambda g, n: disk(g, n, 120, 140, 17), False),
         "tilted 90": (lambda g, n: tilted(disk(g, n, 120, 140, 8), 90), True),
         "tilted 37": (lambda g, n: tilted(disk(g, n, 120, 140, 8), 37), True),
+        "wide": (lambda g, n: disk(g, n, 100, 160, 7), False),
         "clump": (lambda g, n: np.array([[90.0], [90.0], [20.0]]) + g.normal(size=(3, n)), True),
         "ball": (ball, False),
+        "disk 8": (lambda g, n: disk(g, n, 20, 200, 8), True),
+        "disk 13": (lambda g, n: disk(g, n, 20, 200, 13), False),
         "decade": (lambda g, n: disk(g, n, 30, 300, 3, log=True), True),
         "two decades": (lambda g, n: disk(g, n, 3, 300, 3, log=True), False)}
 

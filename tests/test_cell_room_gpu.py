@@ -22,21 +22,28 @@ def directions(g, n):
     return u / np.linalg.norm(u, axis=1)[:, None]
 
 
-def planetesimals(n, g):
-    """A wide ring inclined up to 10 degrees: of the sets that take cells the one that needs the most of them."""
-    a, t = g.uniform(100.0, 160.0, n), g.uniform(0.0, 2 * np.pi, n)
-    z = a * np.sin(np.deg2rad(10.0) * g.uniform(0.0, 1.0, n)) * np.sin(g.uniform(0.0, 2 * np.pi, n))
-    return np.stack([a * np.cos(t), a * np.sin(t), z], 1)
+def planetesimals(kind, n, g):
+    """Of the sets that take cells those that need the most of them: a tilted ring inclined up to 11 degrees, and
+    clumps of some 24 groups."""
+    if kind == "ring":
+        a, t = g.uniform(120.0, 140.0, n), g.uniform(0.0, 2 * np.pi, n)
+        z = a * np.sin(np.deg2rad(11.0) * g.uniform(0.0, 1.0, n)) * np.sin(g.uniform(0.0, 2 * np.pi, n))
+        x, y = a * np.cos(t), a * np.sin(t)
+        return np.stack([0.8 * x - 0.6 * z, y, 0.6 * x + 0.8 * z], 1)
+    t = 2 * np.pi * g.integers(0, 8, n) / 8
+    return np.stack([130.0 * np.cos(t), 130.0 * np.sin(t), 0.0 * t], 1) + g.normal(size=(n, 3))
 
 
-# n planetesimals with star and planets a multiple of 1,024 or 8,192; phase: of the finest edge before rounding
-@pytest.mark.parametrize("n,phase,power", [(3069, 0.785, 0.25), (4093, 0.285, 0.25), (8189, 0.285, 0.125), (8189, 0.785, 0.125)])
-def test_no_level_is_left_out(engine, n, phase, power):
+# n planetesimals with star and planets a multiple of 1,024; phase: of the finest edge before rounding
+@pytest.mark.parametrize("kind,n,phase,power", [("clumps", 3069, 0.285, 0.25), ("clumps", 3069, 0.785, 0.25),
+                                                ("ring", 6141, 0.285, 0.125), ("ring", 8189, 0.285, 0.125),
+                                                ("ring", 8189, 0.785, 0.125)])
+def test_no_level_is_left_out(engine, kind, n, phase, power):
     g = np.random.default_rng(n)
     s = synth.dusty_ring(n_dust=N_DUST, n_plsml=n, seed=71, n_steps=1)
     ng = s.n_grav
     s.state["m"][3:ng] = 0.01 * s.state["m"][0] / n
-    p = planetesimals(n, g)
+    p = planetesimals(kind, n, g)
     want = np.log2(np.exp2(np.log2(np.abs(p).max(1)).mean()) / 30.0 * (4096.0 / n) ** power)
     p *= 2.0 ** (phase - (want - np.floor(want)))
     edge = 2.0 ** np.floor(want) * (1.0 if phase < 0.5 else 1.5)
